@@ -360,61 +360,139 @@ struct ExpandRows {
     int n;
 };
 
-// One group of 4 output rows.  Rows are counted locally from P - lead, the
-// 16 B-aligned row at or before the block's first output row P (lead =
-// P mod 4); local row u is block row j = u - lead, valid for lead <= u < span
-// (span = lead + the block's count, below 2^31 + 4).  Block row j copies the
-// input row of the entry k whose list covers j and appends entry j - pos[k]
-// of that list.  A whole group is W 16 B stores (4 rows of W words); the
-// first and last group of a block may be partial.
+// The entry of each of 32 consecutive output rows, one per lane: k0 covers the
+// window's first row j.  A list that begins inside the window sets its row's
+// bit, so a lane's entry is k0 plus the bits at or below it: one shared read
+// and one REDUX a window, where a search per row took ten dependent reads.
+// k0 moves on to the entry of row j + 32.  j may be "negative" (modulo 2^32)
+// by up to 3 rows, before the block's first row.
+__device__ __forceinline__ int window_entries(const ExpandRows &xr, int n, uint32_t j, int lane, int &k0) {
+    const int i = k0 + 1 + lane;
+    const uint32_t p = xr.pos[i < n ? i : n] - j;   // > 0; entry n holds the block's total
+    const unsigned heads = __reduce_or_sync(FULL, p < 32u && i < n ? 1u << p : 0u);
+    const int k = k0 + __popc(heads & (0xffffffffu >> (31 - lane)));
+    k0 += __popc(__ballot_sync(FULL, p <= 32u && i < n));
+    return k;
+}
+
+// A window's output row as the lane holds it, stored to shared memory in the
+// widest words that the row's width keeps aligned.
 template <int W>
-__device__ __forceinline__ void k2u_write_group(uint32_t u, uint32_t lead, uint32_t span, const ExpandRows &er_,
-                                                const int32_t *__restrict__ rows, const int32_t *__restrict__ edges,
-                                                int32_t *__restrict__ obase) {
-    constexpr int C = W - 1;
-    int k = row_of(er_.pos, er_.n, u >= lead ? u - lead : 0u);
-    uint32_t nxt = er_.pos[k + 1];
-    int32_t v[4 * W];
-    int kp = -1;       // entry of the previous output row of the group, if valid
-    uint32_t er = 0;   // erel[kp]
+__device__ __forceinline__ void stage_row(int32_t *dst, const int32_t (&v)[W]) {
+    if constexpr (W % 4 == 0) {
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-        const uint32_t uq = u + (uint32_t)q;
-        if (uq >= lead && uq < span) {
-            const uint32_t j = uq - lead;
-            while (j >= nxt) nxt = er_.pos[++k + 1];   // one step per list boundary
-            if (q > 0 && k == kp) {
-                // the same input row as the previous output row: copied from registers
+        for (int c = 0; c < W; c += 4)
+            *reinterpret_cast<int4 *>(dst + c) = make_int4(v[c], v[c + 1], v[c + 2], v[c + 3]);
+    } else if constexpr (W % 2 == 0) {
 #pragma unroll
-                for (int c = 0; c < C; ++c) v[q * W + c] = v[(q - 1) * W + c];
-            } else {
-                const int32_t *src = rows + (int)er_.row[k] * C;
-#pragma unroll
-                for (int c = 0; c < C; ++c) v[q * W + c] = __ldg(src + c);
-                er = er_.erel[k];
-            }
-            v[q * W + C] = __ldg(edges + (er + j));
-            kp = k;
-        } else {
-#pragma unroll
-            for (int c = 0; c < W; ++c) v[q * W + c] = 0;
-            kp = -1;
-        }
-    }
-    int32_t *g = obase + (size_t)u * W;
-    if (u >= lead && u + 4u <= span) {
-#pragma unroll
-        for (int k2 = 0; k2 < W; ++k2)
-            reinterpret_cast<int4 *>(g)[k2] = make_int4(v[4 * k2], v[4 * k2 + 1], v[4 * k2 + 2], v[4 * k2 + 3]);
+        for (int c = 0; c < W; c += 2) *reinterpret_cast<int2 *>(dst + c) = make_int2(v[c], v[c + 1]);
     } else {
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const uint32_t uq = u + (uint32_t)q;
-            if (uq >= lead && uq < span) {
+        for (int c = 0; c < W; ++c) dst[c] = v[c];
+    }
+}
+
+constexpr int kChunk = 64;   // output rows a warp stages at a time: two windows
+
+// Output rows [u, u + kChunk) of a warp, W = 2..8 columns.  Rows are counted
+// locally from P - lead, the 16 B-aligned row at or before the block's first
+// output row P (lead = P mod 4); local row u is block row u - lead, valid for
+// lo <= u < hi.  A lane gathers the row it owns in each window (its input row
+// through L1, lanes of one list reading one row; its list entry, consecutive
+// lanes reading consecutive entries), the warp stages the rows packed in
+// shared memory and writes them as consecutive 16 B vectors.
+//
+// The stores bound this kernel before DRAM does: with each thread storing its
+// own four rows, 4 W words apart in a warp's instruction, every 16 B store was
+// a half-filled sector of its own.  Consecutive vectors took the k2u op (count
+// and expansion) on 120k -> 12M rows of 4 columns from 65.6 to 47.0 us (3.7 to
+// 5.1 TB/s of its input, list entries and output) and on 9M -> 18.6M rows of
+// 6 columns from 185.9 to 159.0 us (4.0 to 4.6 TB/s).
+template <int W>
+__device__ __forceinline__ void write_chunk(uint32_t u, uint32_t lead, uint32_t lo, uint32_t hi, const ExpandRows &xr,
+                                            int n, int &k0, const int32_t *__restrict__ rows,
+                                            const int32_t *__restrict__ edges, int32_t *__restrict__ obase,
+                                            int32_t *stg, int lane) {
+    constexpr int C = W - 1, kWin = kChunk / 32;
+    int32_t v[kWin][W];
 #pragma unroll
-                for (int c = 0; c < W; ++c) g[q * W + c] = v[q * W + c];
-            }
+    for (int q = 0; q < kWin; ++q) {
+        const uint32_t j = u + 32u * q - lead, uq = u + 32u * q + (uint32_t)lane;
+        int k = window_entries(xr, n, j, lane, k0);
+        if (uq >= lo && uq < hi) {
+            const int32_t *src = rows + (int)xr.row[k] * C;
+#pragma unroll
+            for (int c = 0; c < C; ++c) v[q][c] = __ldg(src + c);
+            v[q][C] = __ldg(edges + (xr.erel[k] + (uq - lead)));
+        } else {
+#pragma unroll
+            for (int c = 0; c < W; ++c) v[q][c] = 0;
         }
+    }
+#pragma unroll
+    for (int q = 0; q < kWin; ++q) stage_row<W>(stg + (q * 32 + lane) * W, v[q]);
+    __syncwarp();
+    int32_t *g = obase + (size_t)u * W;
+    if (u >= lo && u + kChunk <= hi) {
+#pragma unroll
+        for (int i = 0; i < kChunk * W / 4; i += 32)
+            if (i + lane < kChunk * W / 4)
+                reinterpret_cast<int4 *>(g)[i + lane] = reinterpret_cast<const int4 *>(stg)[i + lane];
+    } else {
+        const int w0 = lo > u ? (int)(lo - u) * W : 0;
+        const int w1 = (hi > u ? (hi - u < (uint32_t)kChunk ? (int)(hi - u) : kChunk) : 0) * W;
+        for (int i = w0 + lane; i < w1; i += 32) g[i] = stg[i];
+    }
+    __syncwarp();   // the staging area is written again by the next chunk
+}
+
+// As write_chunk for one window of 32 output rows of any width, without
+// staging: lane l takes the window's vectors l, l + 32, ... of four words and
+// fetches each word from the input row, or the list entry, that the lane
+// holding the word's output row knows.  A table of 10 columns (800k -> 1.66M
+// rows of 11) took 72.3 us with one output row per thread and scalar stores,
+// 45.7 so.
+__device__ __forceinline__ void write_window_any(uint32_t u, uint32_t lead, uint32_t lo, uint32_t hi, int C,
+                                                 const ExpandRows &xr, int n, int &k0,
+                                                 const int32_t *__restrict__ rows, const int32_t *__restrict__ edges,
+                                                 int32_t *__restrict__ obase, int lane) {
+    const int W = C + 1;
+    const uint32_t uq = u + (uint32_t)lane;
+    const int k = window_entries(xr, n, u - lead, lane, k0);
+    int src = 0;
+    int32_t nb = 0;
+    if (uq >= lo && uq < hi) {
+        src = (int)xr.row[k] * C;
+        nb = __ldg(edges + (xr.erel[k] + (uq - lead)));
+    }
+    int32_t *g = obase + (size_t)u * W;
+    const int words = 32 * W;
+    const int w0 = lo > u ? (int)(lo - u) * W : 0;
+    const int w1 = (hi > u ? (hi - u < 32u ? (int)(hi - u) : 32) : 0) * W;
+    int r = 4 * lane / W, c = 4 * lane % W;                 // row and column of the lane's first word
+    const int dr = 124 / W, dc = 124 % W;                   // from a vector's last word + 1 to the next's first
+    for (int i = 0; i < words; i += 128) {                  // the same trips in every lane
+        const int at = i + 4 * lane;
+        int32_t v[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int rr = r & 31;
+            const int s = __shfl_sync(FULL, src, rr);
+            const int32_t e = __shfl_sync(FULL, nb, rr);
+            v[q] = e;
+            if (c < C && at + q >= w0 && at + q < w1) v[q] = __ldg(rows + s + c);
+            if (++c == W) { c = 0; ++r; }
+        }
+        if (at >= w0 && at + 4 <= w1) {
+            *reinterpret_cast<int4 *>(g + at) = make_int4(v[0], v[1], v[2], v[3]);
+        } else {
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+                if (at + q >= w0 && at + q < w1) g[at + q] = v[q];
+        }
+        r += dr;
+        c += dc;
+        if (c >= W) { c -= W; ++r; }
     }
 }
 
@@ -422,13 +500,14 @@ __device__ __forceinline__ void k2u_write_group(uint32_t u, uint32_t lead, uint3
 // kSliceRows) of block b, where block b's slices are numbered from s_b (the
 // slices of the blocks before it) and k' = k - s_b; locate_slice finds b, s_b
 // and the block's output prefix.  W = C + 1 output columns for
-// 2 <= W <= 8; W = 0 for any width (one output row per thread and step,
-// scalar stores).  History rows are read through L1 (consecutive output rows
-// of one input row reuse it).
+// 2 <= W <= 8; W = 0 for any width.  Each warp takes a contiguous run of the
+// slice's chunks, so it searches for its first entry once and walks on from
+// there.  History rows are read through L1 (consecutive output rows of one
+// input row reuse it).
 // CTAs per SM the register budget is set for: the widest instantiations need
 // more registers to avoid spills
 template <int W>
-constexpr int expand_min_ctas() { return (W >= 2 && W <= 4) || W == 0 ? 8 : (W <= 7 ? 6 : 4); }
+constexpr int expand_min_ctas() { return W <= 6 ? 8 : 6; }
 
 template <int W>
 __global__ void __launch_bounds__(kThreads, expand_min_ctas<W>())
@@ -440,6 +519,7 @@ k2u_expand_kernel(const int32_t *__restrict__ hist, int64_t R, int C_rt, const i
     static_assert(kRPT == 4, "4 input rows per thread");
     __shared__ ExpandRows xr;
     __shared__ uint32_t s_w[2][kThreads / 32];
+    __shared__ __align__(16) int32_t stage[W >= 2 ? (kThreads / 32) * kChunk * W : 1];
     const int C = W >= 2 ? W - 1 : C_rt;
     const int t = threadIdx.x, lane = t & 31, wid = t >> 5;
     allow_dependent_grid();
@@ -501,26 +581,23 @@ k2u_expand_kernel(const int32_t *__restrict__ hist, int64_t R, int C_rt, const i
     const uint32_t T = loc.T;
     const int32_t *hblk = hist + r0 * C;
 
-    // 3. the slice's share of output rows [P, P + T)
-    if constexpr (W >= 2) {
-        const uint32_t lead = (uint32_t)(P & 3ull), span = T + lead;
-        const uint32_t u0 = slice * (uint32_t)kSliceRows;
-        const uint32_t u1 = u0 >= span ? u0 : (span - u0 < (uint32_t)kSliceRows ? span : u0 + (uint32_t)kSliceRows);
-        int32_t *obase = out + (P - lead) * W;
-        for (uint32_t u = u0 + 4u * (uint32_t)t; u < u1; u += 4u * kThreads)
-            k2u_write_group<W>(u, lead, span, xr, hblk, edges, obase);
-    } else {
-        const int Wd = C + 1;
-        int32_t *oblk = out + P * Wd;
-        const uint32_t j0 = slice * (uint32_t)kSliceRows;
-        const uint32_t j1 = j0 >= T ? j0 : (T - j0 < (uint32_t)kSliceRows ? T : j0 + (uint32_t)kSliceRows);
-        for (uint32_t j = j0 + (uint32_t)t; j < j1; j += kThreads) {
-            const int k = row_of(xr.pos, xr.n, j);
-            int32_t *dst = oblk + (size_t)j * Wd;
-            const int32_t *src = hblk + (int64_t)xr.row[k] * C;
-            for (int c = 0; c < C; ++c) dst[c] = __ldg(src + c);
-            dst[C] = __ldg(edges + (xr.erel[k] + j));
-        }
+    // 3. the slice's share of output rows [P, P + T): a run of chunks per warp
+    constexpr int kStep = W >= 2 ? kChunk : 32;
+    const uint32_t lead = (uint32_t)(P & 3ull), span = T + lead;
+    const uint32_t u0 = slice * (uint32_t)kSliceRows;
+    const uint32_t u1 = u0 >= span ? u0 : (span - u0 < (uint32_t)kSliceRows ? span : u0 + (uint32_t)kSliceRows);
+    const uint32_t lo = u0 > lead ? u0 : lead;
+    const uint32_t per = ((u1 - u0 + kStep - 1) / kStep + kThreads / 32 - 1) / (kThreads / 32) * kStep;
+    uint32_t u = u0 + (uint32_t)wid * per;
+    const uint32_t ue = u < u1 ? (u1 - u < per ? u1 : u + per) : u;
+    if (u >= ue) return;   // the same in every lane
+    int32_t *obase = out + ((int64_t)P - lead) * (C + 1);
+    int k0 = row_of(xr.pos, xr.n, u >= lead ? u - lead : 0u);
+    for (; u < ue; u += kStep) {
+        if constexpr (W >= 2)
+            write_chunk<W>(u, lead, lo, u1, xr, xr.n, k0, hblk, edges, obase, stage + wid * (kChunk * W), lane);
+        else
+            write_window_any(u, lead, lo, u1, C, xr, xr.n, k0, hblk, edges, obase, lane);
     }
 }
 
