@@ -1,0 +1,550 @@
+// k2u, k2k and k2c over a dense functional direction in one launch (sm_103a).
+//
+// A direction that keeps one neighbour per id (PredView::nb) answers a row
+// with one 4 B read and gives at most one output row per input row, so the
+// output is sized by the input, and nothing has to reach the host between
+// counting and writing:
+//
+//   k2u     : the rows that have a neighbour, with it appended
+//   k2k/k2c : the rows whose neighbour is the end value
+//
+// What bounds it.  Counting is bound by the look-ups: a random 4 B read is one
+// L1 tag look-up per lane and a 32 B sector from L2, at most 245 G/s on this
+// chip however the load is written (12M of them take 49 us), while DRAM is
+// half idle.  Writing streams: the table in, the output out.  As two kernels
+// in a row each leaves the other's resource idle, and the second reads the
+// table from DRAM again.  Here both kinds of CTA run at once: CTAs are ordered
+// so that the count of block b + lag and the writing of block b are neighbours,
+// with a lag of some 1200 blocks of 1024 rows.  What a write CTA needs has then
+// been counted before (1216 CTAs are in flight at most), and most of the rows
+// it reads are still in L2.  The op is left bound by L2 bandwidth (1.1 GB
+// through it in 130 us on 12M rows of 4 columns, a third of it look-ups).
+//
+// Two kernels and a host round trip before, this launch after, us a call:
+// k2u on 12M rows of 4 columns 163 -> 138, k2k on 10M rows of 3 105.7 -> 89,
+// k2c on 3M rows of 6 49 -> 42; k2u on 50k rows of 6 about 49 -> 22.  A
+// single pass with a decoupled look-back was slower (177 / 139 / 65): every tile
+// waited for the slowest load among the 300 tiles in flight before it.
+//
+// A write CTA checks that the groups of 256 blocks up to its own have been
+// counted, and waits if not.  It depends only on CTAs before it in the grid,
+// which the device starts in order, so the wait ends; it is bounded all the
+// same, and an op whose wait ran out runs again as two kernels.
+//
+// Per-block counts and per-group sums are those of the two-kernel ops: a
+// group's word holds its counted blocks (low 16 bits) and kept rows.  One CTA
+// placed behind the last count waits for every group and writes the op's
+// totals into pinned host memory, so that the host goes on while the last
+// blocks are still written.
+#include "wk_kernels.h"
+#include "wk_probe.cuh"
+
+namespace wk {
+namespace dev {
+
+#define FULL 0xffffffffu
+
+constexpr int kOct = 8;              // blocks per step of the CTA order
+constexpr int kPublishPolls = 1 << 20;
+constexpr int kWritePolls = 1 << 22;   // above the publisher's: it reports first
+
+__device__ __forceinline__ unsigned long long ld_acquire64(const unsigned long long *p) {
+    unsigned long long v;
+    asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+    return v;
+}
+
+__device__ __forceinline__ unsigned long long warp_add(unsigned long long v) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(FULL, v, o);
+    return v;
+}
+
+struct Fused {
+    const int32_t *hist;
+    int64_t R, nblk;
+    int C, scol, ecol;            // k2k: the end column; k2c: ecol < 0 and end_const
+    int32_t end_const;
+    uint32_t dir;
+    const int32_t *nb;            // the direction's neighbour array, ids [vmin, vmin + dn)
+    uint32_t vmin, dn;
+    int32_t *nbr;                 // k2u: per row, the neighbour or -1
+    uint32_t *mask;               // filter: a bit per row
+    unsigned int *blk_nz;         // kept rows per block
+    unsigned long long *gs;       // two words per group, zero at launch
+    int *err;
+    unsigned long long *clear;    // the other sums buffer, cleared for the next op
+    int64_t nclear;
+    int32_t *out;
+    unsigned long long *pub;      // pinned host words: [0] seq, [2] error bits, [3] rows, [4] second count
+    unsigned long long seq;
+    int steps, lag;               // octets of blocks, and how many the writing trails by
+};
+
+// What CTA `i` does: role 0 counts unit `unit` of octet `oct`, 1 writes it, 2
+// publishes.  nc count and nw write CTAs per octet; the first `lag` octets'
+// counts, then per octet its counts and an earlier one's writes, the
+// publisher, and the last `lag` octets' writes.
+struct Role {
+    int kind, oct, unit;
+};
+__device__ __forceinline__ Role role_of(int i, int steps, int lag, int nc, int nw) {
+    const int head = lag * nc, mid = (steps - lag) * (nc + nw);
+    Role r;
+    if (i < head) {
+        r.kind = 0;
+        r.oct = i / nc;
+        r.unit = i % nc;
+    } else if (i < head + mid) {
+        const int j = i - head, s = j / (nc + nw), u = j % (nc + nw);
+        r.kind = u < nc ? 0 : 1;
+        r.oct = u < nc ? s + lag : s;
+        r.unit = u < nc ? u : u - nc;
+    } else if (i == head + mid) {
+        r.kind = 2;
+        r.oct = r.unit = 0;
+    } else {
+        const int j = i - head - mid - 1;
+        r.kind = 1;
+        r.oct = steps - lag + j / nw;
+        r.unit = j % nw;
+    }
+    return r;
+}
+
+// Wait until groups 0 .. g are counted; the sum of the kept rows of groups
+// before g, the same in every thread (and of all of them when g is past the
+// last group).  False when the wait ran out.
+struct WaitShared {
+    unsigned long long sum[2][kThreads / 32];
+    int there[2][kThreads / 32];
+};
+__device__ __forceinline__ bool groups_before(const Fused &a, int64_t g, int polls, WaitShared &sh,
+                                              unsigned long long &sum) {
+    const int64_t ng = (a.nblk + (1 << kGroupShift) - 1) >> kGroupShift;
+    const int64_t last = g < ng ? g : ng - 1;
+    const int t = threadIdx.x;
+    for (int poll = 0;; ++poll) {
+        bool there = true;
+        unsigned long long x = 0ull;
+        for (int64_t i = t; i <= last; i += kThreads) {
+            const int64_t left = a.nblk - (i << kGroupShift);
+            const unsigned long long w = ld_acquire64(a.gs + 2 * i);
+            there = there && (w & 0xffffull) == (unsigned long long)(left < (1 << kGroupShift) ? left : (1 << kGroupShift));
+            if (i < g) x += w >> 16;
+        }
+        // a group's sum is at most 2^18: a warp's fits 32 bits for up to 2^16 groups
+        x = ng <= (1 << 16) ? (unsigned long long)__reduce_add_sync(FULL, (unsigned int)x) : warp_add(x);
+        there = __all_sync(FULL, there);
+        if ((t & 31) == 0) {
+            sh.sum[poll & 1][t >> 5] = x;
+            sh.there[poll & 1][t >> 5] = there;
+        }
+        __syncthreads();   // one a poll: the polls alternate between two sets of words
+        int all = 1;
+        sum = 0ull;
+#pragma unroll
+        for (int w = 0; w < kThreads / 32; ++w) {
+            all &= sh.there[poll & 1][w];
+            sum += sh.sum[poll & 1][w];
+        }
+        if (all) return true;
+        if (poll >= polls) return false;
+        __nanosleep(100);
+    }
+}
+
+// A row whose start is an index key (a value of 0), looked up in the hash
+// table: whether its list holds v, and the entries a linear scan touches.
+__device__ __forceinline__ bool index_key_holds(const PredView &pv, uint32_t dir, int32_t v, unsigned int *scanned,
+                                             int *err) {
+    uint32_t off;
+    const uint32_t deg = probe_seg(pv.buckets, pv.nmain, pv.nover, seg_key(0u, dir), &off, err);
+    const int32_t *e = pv.edges + off;
+    uint32_t lo = 0, hi = deg;
+    while (lo < hi) {
+        const uint32_t mid = (lo + hi) >> 1;
+        if (__ldg(e + mid) < v) lo = mid + 1;
+        else hi = mid;
+    }
+    const bool f = lo < deg && __ldg(e + lo) == v;
+    *scanned = f ? lo + 1 : deg;
+    return f;
+}
+
+// Count BPC blocks from block b0: every start vertex, then every neighbour, in
+// flight together (4 BPC rounds of 32 rows a warp).
+template <int CT, bool FILTER, int BPC>
+__device__ __forceinline__ void count_blocks(const Fused &a, const PredView &pv, int64_t b0, unsigned int (*s_n)[kThreads / 32],
+                                             unsigned long long *s_x) {
+    constexpr int kRounds = kRowsPerBlock / kThreads, NR = kRounds * BPC;
+    const int C = CT > 0 ? CT : a.C;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    auto row_at = [&](int rd) -> int64_t {
+        return (b0 + rd / kRounds) * kRowsPerBlock + warp * (kRounds * 32) + (rd % kRounds) * 32 + lane;
+    };
+    int32_t v[NR], tg[FILTER ? NR : 1];
+#pragma unroll
+    for (int rd = 0; rd < NR; ++rd) {
+        const int64_t r = row_at(rd);
+        v[rd] = r < a.R ? __ldg(a.hist + r * C + a.scol) : -1;
+        if constexpr (FILTER) tg[rd] = r < a.R && a.ecol >= 0 ? __ldg(a.hist + r * C + a.ecol) : a.end_const;
+    }
+    unsigned zeros = 0u;   // rounds in which this lane's row starts at an index key
+    int32_t g[NR];
+#pragma unroll
+    for (int rd = 0; rd < NR; ++rd) {
+        const uint32_t x = (uint32_t)v[rd] - a.vmin;   // wraps above dn below vmin
+        g[rd] = (v[rd] > 0 && x < a.dn) ? __ldg(a.nb + x) : -1;
+        if (v[rd] == 0) zeros |= 1u << rd;
+    }
+    unsigned int n[BPC];
+    unsigned long long extra = 0ull;   // in lane 0 unless a row started at an index key
+    bool keyed = false;
+#pragma unroll
+    for (int j = 0; j < BPC; ++j) n[j] = 0u;
+#pragma unroll
+    for (int rd = 0; rd < NR; ++rd) {
+        const int64_t r = row_at(rd);
+        bool keep = g[rd] >= 0;
+        if constexpr (FILTER) {
+            const unsigned had = __ballot_sync(FULL, keep);
+            extra += lane == 0 ? (unsigned long long)__popc(had) : 0ull;   // entries a linear scan touches
+            keep = keep && g[rd] == tg[rd];
+            if (__any_sync(FULL, (zeros >> rd) & 1u)) {
+                unsigned int sc = 0u;
+                if ((zeros >> rd) & 1u) keep = index_key_holds(pv, a.dir, tg[rd], &sc, a.err);
+                extra += sc;   // of every lane: summed over the warp below
+                keyed = true;
+            }
+            const unsigned m = __ballot_sync(FULL, keep);
+            if (lane == 0 && r < a.R) a.mask[r >> 5] = m;
+            n[rd / kRounds] += (unsigned)__popc(m);
+        } else {
+            if (r < a.R) a.nbr[r] = g[rd];
+            n[rd / kRounds] += (unsigned)__popc(__ballot_sync(FULL, keep));
+        }
+    }
+    if constexpr (!FILTER) extra = __any_sync(FULL, zeros != 0u) ? 1ull : 0ull;   // the op reruns unspecialised
+    if (keyed) extra = warp_add(extra);   // the same in every lane
+    if (lane == 0) {
+#pragma unroll
+        for (int j = 0; j < BPC; ++j) s_n[j][warp] = n[j];
+        s_x[warp] = extra;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        unsigned long long sum = 0ull, x = 0ull;
+        unsigned int done = 0u;
+#pragma unroll
+        for (int j = 0; j < BPC; ++j) {
+            unsigned int c = 0u;
+#pragma unroll
+            for (int w = 0; w < kThreads / 32; ++w) c += s_n[j][w];
+            if (b0 + j < a.nblk) {
+                a.blk_nz[b0 + j] = c;
+                sum += c;
+                ++done;
+            }
+        }
+#pragma unroll
+        for (int w = 0; w < kThreads / 32; ++w) x += s_x[w];
+        unsigned long long *gw = a.gs + 2 * (b0 >> kGroupShift);
+        if (x) atomicAdd(gw + 1, x);
+        __threadfence();   // the CTA's rows and counts, before the group's word says so
+        if (done) atomicAdd(gw, (sum << 16) | done);
+    }
+}
+
+// One row of C words, in the widest loads that C (and the table's alignment) allows.
+template <int C>
+__device__ __forceinline__ void copy_row_regs(const int32_t *__restrict__ src, int32_t *v, bool aligned) {
+    if (C % 4 == 0 && aligned) {
+#pragma unroll
+        for (int c = 0; c + 3 < C; c += 4) {
+            const int4 x = __ldg(reinterpret_cast<const int4 *>(src + c));
+            v[c] = x.x; v[c + 1] = x.y; v[c + 2] = x.z; v[c + 3] = x.w;
+        }
+    } else if (C % 2 == 0 && aligned) {
+#pragma unroll
+        for (int c = 0; c + 1 < C; c += 2) {
+            const int2 x = __ldg(reinterpret_cast<const int2 *>(src + c));
+            v[c] = x.x; v[c + 1] = x.y;
+        }
+    } else {
+#pragma unroll
+        for (int c = 0; c < C; ++c) v[c] = __ldg(src + c);
+    }
+}
+
+// The kept rows of this thread's block of group g before block b, by warps
+// (at most 2^18).
+__device__ __forceinline__ unsigned int blocks_before(const Fused &a, int64_t b) {
+    static_assert(kThreads == (1 << kGroupShift), "one thread per block of a group");
+    const int64_t i = ((b >> kGroupShift) << kGroupShift) + threadIdx.x;
+    return __reduce_add_sync(FULL, i < b ? __ldcg(a.blk_nz + i) : 0u);
+}
+
+// Write block b of a k2u op: its matched rows with the neighbour appended,
+// packed in shared memory at the output's 16 B phase and stored as vectors.
+// The rows are loaded before the wait for the groups: nearly every row of a
+// functional step is kept, and they are in L2.  False when the wait ran out.
+template <int C>
+__device__ __forceinline__ bool write_k2u(const Fused &a, int64_t b, WaitShared &s_wait, int32_t *buf,
+                                          unsigned int *s_w, unsigned int *s_b) {
+    constexpr int W = C + 1, kPasses = kRowsPerBlock / kThreads;
+    const int t = threadIdx.x, lane = t & 31, wid = t >> 5;
+    const int64_t r0 = b * kRowsPerBlock;
+    const int n = (int)((a.R - r0) < kRowsPerBlock ? (a.R - r0) : kRowsPerBlock);
+    const bool aligned = ((uintptr_t)a.hist & 15u) == 0;
+    int32_t x[kPasses], v[kPasses][W];
+    unsigned m[kPasses], kept = 0u;
+#pragma unroll
+    for (int q = 0; q < kPasses; ++q) {
+        const int r = wid * (32 * kPasses) + q * 32 + lane;
+        if (r < n) copy_row_regs<C>(a.hist + (r0 + r) * C, v[q], aligned);
+    }
+    unsigned long long P;
+    if (!groups_before(a, b >> kGroupShift, kWritePolls, s_wait, P)) return false;
+#pragma unroll
+    for (int q = 0; q < kPasses; ++q) {
+        const int r = wid * (32 * kPasses) + q * 32 + lane;
+        x[q] = r < n ? __ldcg(a.nbr + r0 + r) : -1;
+    }
+    const unsigned int before = blocks_before(a, b);
+#pragma unroll
+    for (int q = 0; q < kPasses; ++q) {
+        m[q] = __ballot_sync(FULL, x[q] >= 0);
+        kept += (unsigned)__popc(m[q]);
+    }
+    if (lane == 0) { s_w[wid] = kept; s_b[wid] = before; }
+    __syncthreads();
+    unsigned at = 0u, T = 0u;
+#pragma unroll
+    for (int w = 0; w < kThreads / 32; ++w) {
+        if (w == wid) at = T;
+        T += s_w[w];
+        P += s_b[w];
+    }
+    const int lead = (int)((P * W) & 3ull), end = lead + (int)T * W;
+    const unsigned below = (1u << lane) - 1u;
+#pragma unroll
+    for (int q = 0; q < kPasses; ++q) {
+        if (x[q] >= 0) {
+            v[q][C] = x[q];
+            int32_t *d = buf + lead + (at + (unsigned)__popc(m[q] & below)) * W;
+            if constexpr (W % 4 == 0) {          // lead is 0
+#pragma unroll
+                for (int c = 0; c < W; c += 4)
+                    *reinterpret_cast<int4 *>(d + c) = make_int4(v[q][c], v[q][c + 1], v[q][c + 2], v[q][c + 3]);
+            } else if constexpr (W % 2 == 0) {   // lead is 0 or 2
+#pragma unroll
+                for (int c = 0; c < W; c += 2) *reinterpret_cast<int2 *>(d + c) = make_int2(v[q][c], v[q][c + 1]);
+            } else {
+#pragma unroll
+                for (int c = 0; c < W; ++c) d[c] = v[q][c];
+            }
+        }
+        at += (unsigned)__popc(m[q]);
+    }
+    __syncthreads();
+    int32_t *o = a.out + (P * W - (unsigned)lead);
+    for (int i = 4 * t; i < end; i += 4 * kThreads) {
+        if (i >= lead && i + 4 <= end) {
+            __stcs(reinterpret_cast<int4 *>(o + i), *reinterpret_cast<const int4 *>(buf + i));
+        } else {
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                if (i + j >= lead && i + j < end) o[i + j] = buf[i + j];
+        }
+    }
+    return true;
+}
+
+// Write a filter's octet of blocks, one per warp: the block's kept rows from
+// its mask words, its output words as vectors, each gathered from its row.
+template <int CT>
+__device__ __forceinline__ void write_filter(const Fused &a, int64_t b0, unsigned long long P, uint16_t *sel,
+                                             unsigned int *s_nz, unsigned int *s_b) {
+    const int C = CT > 0 ? CT : a.C;
+    const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+    const unsigned int before = blocks_before(a, b0);
+    if (lane == 0) s_b[w] = before;
+    if (t < kOct) s_nz[t] = b0 + t < a.nblk ? __ldcg(a.blk_nz + b0 + t) : 0u;
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < kThreads / 32; ++i) P += s_b[i];
+    for (int i = 0; i < w; ++i) P += s_nz[i];
+    const unsigned int nb = s_nz[w];
+    if (nb == 0u) return;   // the warp's block keeps nothing (or lies past the table)
+    const int64_t r0 = (b0 + w) * kRowsPerBlock;
+    const int64_t wi = (r0 >> 5) + lane, nwords = (a.R + 31) >> 5;
+    uint32_t m = wi < nwords ? __ldcg(a.mask + wi) : 0u;   // bits past R are 0
+    const unsigned int c = __popc(m);
+    unsigned int pos = c;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned int v = __shfl_up_sync(FULL, pos, o);
+        if (lane >= o) pos += v;
+    }
+    pos -= c;
+    uint16_t *ws = sel + w * kRowsPerBlock;
+    while (m) {
+        ws[pos++] = (uint16_t)(lane * 32 + __ffs(m) - 1);
+        m &= m - 1u;
+    }
+    __syncwarp();
+    const int32_t *hb = a.hist + r0 * C;
+    const uint32_t words = nb * (uint32_t)C;
+    const uint32_t lead = (uint32_t)((P * (unsigned long long)C) & 3ull);
+    int32_t *gout = a.out + (P * (unsigned long long)C - lead);
+    for (uint32_t u = (uint32_t)lane; 4u * u < lead + words; u += 32u) {
+        int32_t v[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const uint32_t kk = 4u * u + (uint32_t)j - lead;   // wraps above `words` before the lead
+            v[j] = kk < words ? __ldg(hb + (int)ws[kk / (uint32_t)C] * C + (int)(kk % (uint32_t)C)) : 0;
+        }
+        if (4u * u >= lead && 4u * u + 4u <= lead + words) {
+            reinterpret_cast<int4 *>(gout)[u] = make_int4(v[0], v[1], v[2], v[3]);
+        } else {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const uint32_t kk = 4u * u + (uint32_t)j - lead;
+                if (kk < words) gout[4u * u + j] = v[j];
+            }
+        }
+    }
+}
+
+// CT columns (0: any, filters only).  BPC: blocks per count CTA.
+template <int CT, bool FILTER, int BPC>
+__global__ void __launch_bounds__(kThreads, FILTER ? 6 : (CT <= 4 ? 6 : (CT <= 6 ? 5 : 4)))
+fused_kernel(const __grid_constant__ Fused a, const __grid_constant__ PredView pv) {
+    constexpr int NC = kOct / BPC, NW = FILTER ? 1 : kOct;
+    __shared__ __align__(16) int32_t buf[FILTER ? kOct * kRowsPerBlock / 2 : kRowsPerBlock * (CT + 1) + 4];
+    __shared__ unsigned long long s_part[kThreads / 32];
+    __shared__ unsigned int s_n[BPC][kThreads / 32], s_b[kThreads / 32];
+    __shared__ WaitShared s_wait;
+    asm volatile("griddepcontrol.wait;" ::: "memory");   // the previous op's table and sums are complete
+    asm volatile("griddepcontrol.launch_dependents;");
+    const Role role = role_of((int)blockIdx.x, a.steps, a.lag, NC, NW);
+    if (role.kind == 0) {
+        // the other sums buffer, read by the previous op, is cleared for the next
+        for (int64_t w = ((int64_t)role.oct * NC + role.unit) * kThreads + threadIdx.x; w < a.nclear;
+             w += (int64_t)a.steps * NC * kThreads)
+            a.clear[w] = 0ull;
+        const int64_t b0 = (int64_t)role.oct * kOct + role.unit * BPC;
+        if (b0 < a.nblk) count_blocks<CT, FILTER, BPC>(a, pv, b0, s_n, s_part);
+        return;
+    }
+    unsigned long long P = 0ull;
+    if (role.kind == 2) {
+        // every group counted: the op's totals for the host
+        const int64_t ng = (a.nblk + (1 << kGroupShift) - 1) >> kGroupShift;
+        const bool ok = groups_before(a, ng, kPublishPolls, s_wait, P);
+        unsigned long long x = 0ull;
+        for (int64_t i = threadIdx.x; ok && i < ng; i += kThreads) x += __ldcg(a.gs + 2 * i + 1);
+        x = warp_add(x);
+        if ((threadIdx.x & 31) == 0) s_part[threadIdx.x >> 5] = x;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            x = 0ull;
+#pragma unroll
+            for (int w = 0; w < kThreads / 32; ++w) x += s_part[w];
+            a.pub[2] = (unsigned long long)(unsigned int)atomicOr(a.err, 0) | (ok ? 0ull : (unsigned long long)kErrWait);
+            a.pub[3] = P;
+            a.pub[4] = x;
+            __threadfence_system();
+            *(volatile unsigned long long *)a.pub = a.seq;
+        }
+        return;
+    }
+    const int64_t b = (int64_t)role.oct * kOct + role.unit;
+    if (b >= a.nblk) return;   // the same in every thread
+    bool ok;
+    if constexpr (FILTER) {
+        ok = groups_before(a, b >> kGroupShift, kWritePolls, s_wait, P);
+        if (ok) write_filter<CT>(a, b, P, reinterpret_cast<uint16_t *>(buf), s_n[0], s_b);
+    } else {
+        ok = write_k2u<CT>(a, b, s_wait, buf, s_n[0], s_b);
+    }
+    if (!ok && threadIdx.x == 0) atomicOr(a.err, kErrWait);
+}
+
+bool fused_takes(int C, bool filter) { return filter || C + 1 <= kFusedCols; }
+
+template <int CT, bool FILTER, int BPC>
+static int run_fused(const Fused &a, const PredView &pv, cudaStream_t st) {
+    constexpr int NC = kOct / BPC, NW = FILTER ? 1 : kOct;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned int)(a.steps * (NC + NW) + 1));
+    cfg.blockDim = dim3(kThreads);
+    cfg.stream = st;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return (int)cudaLaunchKernelEx(&cfg, fused_kernel<CT, FILTER, BPC>, a, pv);
+}
+
+int launch_fused(const FusedOp &op, cudaStream_t st) {
+    Fused a;
+    a.hist = op.hist;
+    a.R = op.R;
+    a.nblk = (op.R + kRowsPerBlock - 1) / kRowsPerBlock;
+    a.C = op.C;
+    a.scol = op.scol;
+    a.ecol = op.ecol;
+    a.end_const = op.end_const;
+    a.dir = op.dir;
+    a.nb = op.dir ? op.pv.nb[1] : op.pv.nb[0];
+    a.vmin = op.dir ? op.pv.vmin[1] : op.pv.vmin[0];
+    a.dn = op.dir ? op.pv.dn[1] : op.pv.dn[0];
+    a.nbr = op.nbr;
+    a.mask = op.mask;
+    a.blk_nz = op.blk_nz;
+    a.gs = op.group_sums;
+    a.err = op.err;
+    a.clear = op.clear;
+    a.nclear = op.nclear;
+    a.out = op.out;
+    a.pub = op.pub;
+    a.seq = op.seq;
+    a.steps = (int)((a.nblk + kOct - 1) / kOct);
+    // The writing trails by what the CTAs in flight reach over (6 to 8 a SM, 9 to
+    // 16 an octet) and a group's 256 blocks, no more: the rows should still be in
+    // L2 when they are read again.  222 octets instead of 146 made a k2u op on
+    // 12M rows of 4 columns read 392 instead of 278 MB from DRAM (192 MB is the
+    // table) and took it from 144 to 153 us.
+    const int lag = op.sms * 3 / 4 + (1 << kGroupShift) / kOct;
+    a.lag = a.steps < lag ? a.steps : lag;
+    // two blocks per count CTA (eight look-ups in flight a lane) once there are
+    // enough of them to fill the GPU
+    const bool pair = !op.filter && a.nblk >= 16 * (int64_t)op.sms;
+#define WK_FUSED(CC)                                                      \
+    case CC: return pair ? run_fused<CC, false, 2>(a, op.pv, st) : run_fused<CC, false, 1>(a, op.pv, st)
+    if (!op.filter) {
+        switch (op.C) {
+            WK_FUSED(1); WK_FUSED(2); WK_FUSED(3); WK_FUSED(4); WK_FUSED(5);
+            WK_FUSED(6); WK_FUSED(7); WK_FUSED(8); WK_FUSED(9); WK_FUSED(10);
+        }
+        return (int)cudaErrorInvalidValue;   // not reached: fused_takes
+    }
+#undef WK_FUSED
+    switch (op.C) {
+        case 1: return run_fused<1, true, 1>(a, op.pv, st);
+        case 2: return run_fused<2, true, 1>(a, op.pv, st);
+        case 3: return run_fused<3, true, 1>(a, op.pv, st);
+        case 4: return run_fused<4, true, 1>(a, op.pv, st);
+        case 5: return run_fused<5, true, 1>(a, op.pv, st);
+        case 6: return run_fused<6, true, 1>(a, op.pv, st);
+        case 7: return run_fused<7, true, 1>(a, op.pv, st);
+        case 8: return run_fused<8, true, 1>(a, op.pv, st);
+        default: return run_fused<0, true, 1>(a, op.pv, st);
+    }
+}
+
+}  // namespace dev
+}  // namespace wk

@@ -82,16 +82,16 @@ constexpr int kRounds = kRowsPerBlock / (kThreads / 32) / 32;
 // blk_sum[b] = the block's output rows, added into its group's sums.  Err bit
 // 1 when a block's output count reaches 2^31 (the expansion keeps block-local
 // positions in 32 bits).  FUNC (a direction whose lists hold at most one
-// vertex): deg receives the neighbour itself as an int32, or -1 for no match,
-// and off is unused.  DENSE (the direction is an offsets array): a warp
+// vertex, hashed): deg receives the neighbour itself as an int32, or -1 for no
+// match, and off is unused.  DENSE (the direction is an offsets array): a warp
 // issues the lookups of all its rounds phase by phase -- every round's start
-// vertex, then every round's offsets or neighbour -- and a lane looks up its
-// own key (no shuffles).  BPC blocks per CTA: 2 for a large dense op, so each
+// vertex, then every round's offsets -- and a lane looks up its own key (no
+// shuffles).  BPC blocks per CTA: 2 for a large dense op, so each
 // warp keeps eight rounds of loads in flight and a CTA's fixed costs
 // (reduction, exit) are shared by 2048 rows; 1 otherwise, so a small op still
 // spreads over many CTAs.
 template <bool FUNC, bool DENSE, int BPC>
-__global__ void __launch_bounds__(kThreads, (DENSE && FUNC) ? 8 : 6)
+__global__ void __launch_bounds__(kThreads, 6)
 k2u_count_kernel(const int32_t *__restrict__ hist, int64_t R, int C, int scol, uint32_t dir, PredView pv, uint32_t *__restrict__ deg, uint32_t *__restrict__ off,
                  unsigned long long *__restrict__ blk_sum, unsigned long long *__restrict__ group_sums, int *err,
                  unsigned long long *__restrict__ clear, int64_t nclear) {
@@ -120,50 +120,29 @@ k2u_count_kernel(const int32_t *__restrict__ hist, int64_t R, int C, int scol, u
     for (int j = 0; j < BPC; ++j) my_sum[j] = 0ull;
     if constexpr (DENSE) {
         const uint32_t vmin = dir ? pv.vmin[1] : pv.vmin[0], dn = dir ? pv.dn[1] : pv.dn[0];
-        if constexpr (FUNC) {
-            // a dense functional direction keeps the neighbour per id: one 4 B read
-            const int32_t *nba = dir ? pv.nb[1] : pv.nb[0];
-            int32_t g[NR];
+        const uint32_t *rp = dir ? pv.rp[1] : pv.rp[0];
+        uint32_t a[NR], e[NR];
 #pragma unroll
-            for (int rd = 0; rd < NR; ++rd) {
-                const int32_t vid = v[rd];
-                const uint32_t x = (uint32_t)vid - vmin;   // wraps above dn below vmin
-                g[rd] = (vid > 0 && x < dn) ? __ldg(nba + x) : -1;
-                if (vid == 0) atomicOr(err, 8);   // an index key: the op reruns unspecialised
+        for (int rd = 0; rd < NR; ++rd) {
+            const int32_t vid = v[rd];
+            a[rd] = e[rd] = 0u;
+            const uint32_t x = (uint32_t)vid - vmin;   // wraps above dn below vmin
+            if (vid > 0 && x < dn) {
+                a[rd] = __ldg(rp + x);
+                e[rd] = __ldg(rp + x + 1);
+            } else if (vid == 0) {   // index key: the hash table
+                e[rd] = probe_seg(pv.buckets, pv.nmain, pv.nover, seg_key(0u, dir), &a[rd], err);
+                e[rd] += a[rd];
             }
+        }
 #pragma unroll
-            for (int rd = 0; rd < NR; ++rd) {
-                const int64_t r = row_at(rd);
-                if (r < R) {
-                    reinterpret_cast<int32_t *>(deg)[r] = g[rd];
-                    my_sum[rd / kRounds] += g[rd] >= 0 ? 1ull : 0ull;
-                }
-            }
-        } else {
-            const uint32_t *rp = dir ? pv.rp[1] : pv.rp[0];
-            uint32_t a[NR], e[NR];
-#pragma unroll
-            for (int rd = 0; rd < NR; ++rd) {
-                const int32_t vid = v[rd];
-                a[rd] = e[rd] = 0u;
-                const uint32_t x = (uint32_t)vid - vmin;   // wraps above dn below vmin
-                if (vid > 0 && x < dn) {
-                    a[rd] = __ldg(rp + x);
-                    e[rd] = __ldg(rp + x + 1);
-                } else if (vid == 0) {   // index key: the hash table
-                    e[rd] = probe_seg(pv.buckets, pv.nmain, pv.nover, seg_key(0u, dir), &a[rd], err);
-                    e[rd] += a[rd];
-                }
-            }
-#pragma unroll
-            for (int rd = 0; rd < NR; ++rd) {
-                const int64_t r = row_at(rd);
-                const uint32_t d = e[rd] - a[rd];
-                if (r < R) {
-                    deg[r] = d;
-                    off[r] = a[rd];
-                    my_sum[rd / kRounds] += d;
-                }
+        for (int rd = 0; rd < NR; ++rd) {
+            const int64_t r = row_at(rd);
+            const uint32_t d = e[rd] - a[rd];
+            if (r < R) {
+                deg[r] = d;
+                off[r] = a[rd];
+                my_sum[rd / kRounds] += d;
             }
         }
     } else {
@@ -602,8 +581,8 @@ k2u_expand_kernel(const int32_t *__restrict__ hist, int64_t R, int C_rt, const i
 }
 
 // ------------------------------------------------- k2u expand, functional
-// A direction whose lists hold at most one vertex: the expansion is a
-// compaction of the matched rows with their neighbour appended.  One CTA per
+// A hashed direction whose lists hold at most one vertex (a dense one takes
+// wk_fused.cu): the expansion is a compaction of the matched rows with their neighbour appended.  One CTA per
 // non-empty input block (its only slice).  Warp w takes rows 128 w .. 128 w +
 // 127 in four passes of 32 consecutive rows, finds each matched row's output
 // position by ballots, copies the row and its neighbour into shared memory
@@ -705,29 +684,9 @@ __device__ __forceinline__ bool list_contains(const int32_t *__restrict__ e, uin
     return f;
 }
 
-// The general lookup of the filter probe: probe_warp (runs of equal keys
-// probed once) where every lane takes it; in the NB kernel only a lane with an
-// index key (a start value of 0) gets here, alone, and looks itself up.
-template <bool NB>
-__device__ __forceinline__ void probe_view_or_warp(const PredView &pv, int32_t vid, uint32_t dir, uint32_t &o,
-                                                   uint32_t &d, int *err) {
-    if constexpr (NB) {
-        o = 0u;
-        d = vid >= 0 ? probe_view(pv, (uint32_t)vid, dir, &o, err) : 0u;
-    } else {
-        probe_warp(pv, vid, dir, o, d, err);
-    }
-}
-
 // totals[0] += adjacency entries a linear scan would touch, totals[1] += rows kept.
-// NB: the direction is dense and functional, so its neighbour array answers a
-// membership test with one 4 B read (the list holds that neighbour or
-// nothing; a linear scan touches 1 entry or none); a start value of 0 (an
-// index key, hashed) takes the general path.  All rounds' reads are issued
-// before any is used.
 // One CTA per block of input rows (two blocks per CTA, with eight rounds of
 // loads in flight per lane, took 48 registers and ran slower).
-template <bool NB>
 __global__ void __launch_bounds__(kThreads, 6)
 filter_probe_kernel(const int32_t *__restrict__ hist, int64_t R, int C, int scol, int ecol,
                     int32_t end_const, uint32_t dir, PredView pv,
@@ -750,32 +709,17 @@ filter_probe_kernel(const int32_t *__restrict__ hist, int64_t R, int C, int scol
     }
     unsigned int my_nz = 0u;   // kept rows (lane 0)
     unsigned long long my_scan = 0;
-    int32_t g[kRounds];   // NB: the neighbour, or -1 (none, or not looked up here)
-    if constexpr (NB) {
-        const int32_t *nba = dir ? pv.nb[1] : pv.nb[0];
-        const uint32_t vmin = dir ? pv.vmin[1] : pv.vmin[0], dn = dir ? pv.dn[1] : pv.dn[0];
-#pragma unroll
-        for (int rd = 0; rd < kRounds; ++rd) {
-            const uint32_t x = (uint32_t)v[rd] - vmin;   // wraps above dn below vmin
-            g[rd] = (v[rd] > 0 && x < dn) ? __ldg(nba + x) : -1;
-        }
-    }
 #pragma unroll
     for (int rd = 0; rd < kRounds; ++rd) {
         const int64_t row0 = wrow0 + rd * 32, r = row0 + lane;
         if (row0 >= R) break;   // warp-uniform
         bool found = false;
-        if (NB && v[rd] != 0) {
-            found = r < R && g[rd] >= 0 && g[rd] == tg[rd];
-            my_scan += (r < R && g[rd] >= 0) ? 1u : 0u;
-        } else {
-            uint32_t o, d;
-            probe_view_or_warp<NB>(pv, v[rd], dir, o, d, err);
-            if (r < R && d > 0u) {
-                uint32_t sc = 0;
-                found = list_contains(pv.edges + o, d, tg[rd], &sc);
-                my_scan += sc;
-            }
+        uint32_t o, d;
+        probe_warp(pv, v[rd], dir, o, d, err);
+        if (r < R && d > 0u) {
+            uint32_t sc = 0;
+            found = list_contains(pv.edges + o, d, tg[rd], &sc);
+            my_scan += sc;
         }
         const uint32_t m = __ballot_sync(FULL, found);
         if (lane == 0) {
@@ -913,11 +857,8 @@ void launch_k2u_count(const int32_t *hist, int64_t R, int C, int scol, uint32_t 
         cudaLaunchKernelEx(&cfg, k2u_count_kernel<F, D, B>, hist, R, C, scol, dir, pv, deg, off, blk_sum,         \
                            group_sums, err, clear, nclear);                                                      \
     } while (0)
-    if (func && dense) {
-        if (pair) WK_COUNT(true, true, 2);
-        else WK_COUNT(true, true, 1);
-    } else if (func) {
-        WK_COUNT(true, false, 1);
+    if (func) {
+        WK_COUNT(true, false, 1);   // hashed: a dense one takes wk_fused.cu
     } else if (dense) {
         if (pair) WK_COUNT(false, true, 2);
         else WK_COUNT(false, true, 1);
@@ -998,8 +939,6 @@ int preload_k2u_kernels() {
     get((const void *)k2u_count_kernel<false, true, 1>);
     get((const void *)k2u_count_kernel<false, true, 2>);
     get((const void *)k2u_count_kernel<true, false, 1>);
-    get((const void *)k2u_count_kernel<true, true, 1>);
-    get((const void *)k2u_count_kernel<true, true, 2>);
     get((const void *)publish_kernel);
     get((const void *)k2u_expand_kernel<0>);
     get((const void *)k2u_expand_kernel<2>);
@@ -1017,12 +956,8 @@ void launch_filter_probe(const int32_t *hist, int64_t R, int C, int scol, int ec
                          unsigned long long *group_sums, unsigned long long *clear, int64_t nclear,
                          unsigned long long *totals, int *err, cudaStream_t st) {
     const unsigned int nb = nblocks_rows(R);
-#define WK_PROBE(NBV) \
-    filter_probe_kernel<NBV><<<nb, kThreads, 0, st>>>(hist, R, C, scol, ecol, end_const, dir, pv, mask, blk_nz, \
-                                                      group_sums, clear, nclear, totals, err)
-    if ((dir ? pv.nb[1] : pv.nb[0]) != nullptr) WK_PROBE(true);
-    else WK_PROBE(false);
-#undef WK_PROBE
+    filter_probe_kernel<<<nb, kThreads, 0, st>>>(hist, R, C, scol, ecol, end_const, dir, pv, mask, blk_nz, group_sums,
+                                                 clear, nclear, totals, err);
 }
 
 void launch_filter_write(const int32_t *hist, int64_t R, int C, const uint32_t *mask, const unsigned int *blk_nz,

@@ -87,6 +87,41 @@ void launch_filter_probe(const int32_t *hist, int64_t R, int C, int scol, int ec
 void launch_filter_write(const int32_t *hist, int64_t R, int C, const uint32_t *mask, const unsigned int *blk_nz,
                          const unsigned long long *group_sums, int32_t *out, cudaStream_t st);
 
+// k2u, k2k and k2c over a dense functional direction (pv.nb[dir] set) in one
+// launch; k2u for up to kFusedCols output columns (fused_takes).  out holds R
+// rows of C + 1 (k2u) or C columns and is 16 B aligned; nbr (k2u) holds R
+// words, mask (filters) a bit per row, blk_nz a word per block, group_sums two
+// zero words per group.  clear[0 .. nclear) is set to zero.  The op's totals go
+// to pinned host memory: pub[2] = the error word (bit 0: corrupt overflow
+// chain, kErrWait: a wait ran out and the op has to run as two kernels),
+// pub[3] = output rows, pub[4] = k2u: not 0 when a row's start is an index key
+// (the op has to run unspecialised), filter: entries a linear scan touches;
+// then seq into pub[0].  Returns a cudaError_t.
+constexpr int kFusedCols = 11;
+constexpr int kErrWait = 16;
+struct FusedOp {
+    const int32_t *hist;
+    int64_t R;
+    int C, scol, ecol;
+    int32_t end_const;
+    uint32_t dir;
+    bool filter;
+    PredView pv;
+    int32_t *nbr;
+    uint32_t *mask;
+    unsigned int *blk_nz;
+    unsigned long long *group_sums;
+    int *err;
+    unsigned long long *clear;
+    int64_t nclear;
+    int32_t *out;
+    unsigned long long *pub;
+    unsigned long long seq;
+    int sms;
+};
+bool fused_takes(int C, bool filter);
+int launch_fused(const FusedOp &op, cudaStream_t st);
+
 // Copy an adjacency list (index or constant start) into a one-column table.
 void launch_copy_list(const int32_t *src, int64_t n, int32_t *dst, cudaStream_t st);
 

@@ -210,6 +210,88 @@ int clear_totals(wk_ctx *ctx) {
     return e == cudaSuccess ? WK_OK : cuda_fail(e, "clear totals");
 }
 
+bool alloc_failure_pending(wk_ctx *ctx) { return ctx->inject_alloc_fail.load(std::memory_order_relaxed) > 0; }
+
+// A k2u or filter op over a dense functional direction in one launch
+// (wk_fused.cu): at most one row out per row in, so the output is sized by the
+// input and nothing has to reach the host before it is written.
+// *done is false when the op has to run as two kernels instead: more columns
+// than the launch takes, a start that is an index key (k2u), an output bound
+// that does not fit in device memory, or a device wait that ran out.
+int op_fused(wk_ctx *ctx, wk_history *h, int scol, int ecol, int32_t end_const, uint32_t dir, bool filter,
+             const PredView &pv, OpClock &clk, bool *done) {
+    *done = false;
+    const int C = h->col_num;
+    const int64_t R = h->size / C;
+    const int width = filter ? C : C + 1;
+    if (pv.nb[dir] == nullptr || !dev::fused_takes(C, filter)) return WK_OK;
+    DevBuf &ob = out_buf(ctx, h);
+    const int64_t nblk = (R + dev::kRowsPerBlock - 1) / dev::kRowsPerBlock;
+    const int64_t groups = (nblk + (1 << dev::kGroupShift) - 1) >> dev::kGroupShift;
+    int st;
+    if ((st = filter ? take(ctx, ctx->mask, (size_t)((R + 31) / 32) * 4) : take(ctx, ctx->deg, (size_t)R * 4)) ||
+        (st = take(ctx, ctx->blk_nz, (size_t)nblk * 4)) || (st = reserve_gsum(ctx, groups)))
+        return st;
+    const bool injected = alloc_failure_pending(ctx);
+    if ((st = take(ctx, ob, (size_t)R * width * 4))) {
+        // a k2u op of two kernels asks for its rows only; a filter's asks for as much
+        return injected || st != WK_ENOMEM || filter ? st : WK_OK;
+    }
+    if ((st = clk.begin())) return st;
+    const int par = ctx->gs_par;
+    unsigned long long *gs = gsum_buffer(ctx, par);
+    dev::FusedOp op;
+    op.hist = h->data;
+    op.R = R;
+    op.C = C;
+    op.scol = scol;
+    op.ecol = ecol;
+    op.end_const = end_const;
+    op.dir = dir;
+    op.filter = filter;
+    op.pv = pv;
+    op.nbr = ctx->deg.as<int32_t>();
+    op.mask = ctx->mask.as<uint32_t>();
+    op.blk_nz = ctx->blk_nz.as<unsigned int>();
+    op.group_sums = gs + 2;
+    op.err = reinterpret_cast<int *>(gs);
+    op.clear = gsum_buffer(ctx, par ^ 1);
+    op.nclear = 2 + 2 * ctx->gs_used[par ^ 1];
+    op.out = ob.as<int32_t>();
+    op.pub = ctx->h_gs_dev;
+    op.seq = ++ctx->pub_seq;
+    op.sms = ctx->sms;
+    const cudaError_t le = (cudaError_t)dev::launch_fused(op, ctx->stream);
+    if (le != cudaSuccess) return cuda_fail(le, "one-launch op");
+    if ((st = launch_check("one-launch op")) || (st = clk.end(true))) return st;
+    ctx->gs_par = par ^ 1;
+    ctx->gs_used[par ^ 1] = 0;
+    ctx->gs_used[par] = groups;
+    if ((st = wait_published(ctx, op.seq))) return st;
+    const unsigned long long err = ctx->h_gs[2];
+    const int64_t R_out = (int64_t)ctx->h_gs[3], extra = (int64_t)ctx->h_gs[4];
+    if (err & 1ull)
+        return set_error(WK_EDEVICE, "probe found an overflow chain longer than the segment's overflow area (corrupt store)");
+    if ((err & (unsigned long long)dev::kErrWait) || (!filter && extra)) return WK_OK;
+    if (!filter && R_out > ctx->row_limit)
+        return set_error(WK_EOVERFLOW, "k2u: %lld output rows exceed the context's row limit %lld", (long long)R_out,
+                         (long long)ctx->row_limit);
+    ctx->last.rows_out = R_out;
+    ctx->last.alg_bytes = filter ? 4 * R * C + 16 * R + 4 * extra + 4 * R_out * C
+                                 : 4 * R * C + 16 * R + 4 * R_out + 4 * R_out * (C + 1);
+    if (ctx->timing) {
+        cudaError_t e = cudaStreamSynchronize(ctx->stream);
+        if (e != cudaSuccess) return cuda_fail(e, "one-launch op sync");
+    }
+    clk.finish();
+    h->data = ob.as<int32_t>();
+    h->size = R_out * width;
+    h->col_num = width;
+    h->step++;
+    *done = true;
+    return WK_OK;
+}
+
 // two-pass k2u (count -> host adds up the group sums -> expand)
 int op_k2u(wk_ctx *ctx, wk_history *h, int scol, uint32_t pid, uint32_t dir) {
     const int C = h->col_num;
@@ -230,14 +312,16 @@ int op_k2u(wk_ctx *ctx, wk_history *h, int scol, uint32_t pid, uint32_t dir) {
         h->step++;
         return WK_OK;
     }
+    bool done = false;
+    if ((st = op_fused(ctx, h, scol, -1, 0, dir, false, pv, clk, &done)) || done) return st;
     const int64_t nblk = (R + dev::kRowsPerBlock - 1) / dev::kRowsPerBlock;
     const int64_t groups = (nblk + (1 << dev::kGroupShift) - 1) >> dev::kGroupShift;
     if ((st = take(ctx, ctx->deg, (size_t)R * 4)) || (st = take(ctx, ctx->off, (size_t)R * 4)) ||
         (st = take(ctx, ctx->blk_sum, (size_t)nblk * 8)) || (st = reserve_gsum(ctx, groups)))
         return st;
-    // a functional direction (at most one neighbour per vertex) expands as a
+    // a hashed functional direction (at most one neighbour per vertex) expands as a
     // compaction; if a row hits an index list (vertex 0) the op reruns unspecialised
-    bool func = pv.func[dir] != 0u && C + 1 <= 8;
+    bool func = pv.func[dir] != 0u && pv.nb[dir] == nullptr && C + 1 <= 8;
     int errf = 0;
     unsigned long long *gs = nullptr;
     for (;;) {
@@ -337,6 +421,8 @@ int op_filter(wk_ctx *ctx, wk_history *h, int scol, int ecol, int32_t end_const,
         h->step++;
         return WK_OK;
     }
+    bool done = false;
+    if ((st = op_fused(ctx, h, scol, ecol, end_const, dir, true, pv, clk, &done)) || done) return st;
     const int64_t nblk = (R + dev::kRowsPerBlock - 1) / dev::kRowsPerBlock;
     const int64_t groups = (nblk + (1 << dev::kGroupShift) - 1) >> dev::kGroupShift;
     if ((st = take(ctx, ctx->mask, (size_t)((R + 31) / 32) * 4)) || (st = take(ctx, ctx->blk_nz, (size_t)nblk * 4)) ||
