@@ -16,16 +16,23 @@
 //                 (lanes of one warp may probe different segments), output
 //                 row count (degree, or 0/1 for a filter, 1 for a pass),
 //                 per-tile sums and per-query sums (warp-aggregated atomics)
-//   batch_scan  : one block: exclusive scan of tile sums and of per-query
+//   batch_scan  : two blocks: exclusive scans of tile sums and of per-query
 //                 output rows / ints -> next step's layout; capacity check
-//   batch_write : per tile: block scan of the counts, then every output row
+//   batch_write : per tile: warp scan of the counts, then every output row
 //                 written at out_int_off[q] + pos_in_q * width; rows whose
 //                 output exceeds `split` ints are written warp-cooperatively,
 //                 the rest thread-per-row
+//
+// A tile is the rows one warp takes: total / warps of the grid, from one row
+// up (rows_per_tile).  Light steps are bound by latency, not by bytes: 4096
+// start rows with lists of 100 are 128 warps of 32 rows, or 4 blocks of 1024,
+// that walk their lists one after another, but 4096 warps that walk one list
+// each.  A batch of 4096 light requests (packed, run, results on the host)
+// took 559 us with tiles of 1024 rows a block, 208 so.
 // The three phases run either as three kernels per step or as one
 // cooperative persistent kernel per step (batch_step_kernel) whose blocks
 // meet at two grid barriers -- after the count and after the scan, which
-// block 0 runs -- each wait bounded; the autotuner picks the faster.  Every
+// the first and last block run -- each wait bounded; the autotuner picks the faster.  Every
 // size lives in device memory and every grid is persistent, so the launch
 // sequence of a batch never depends on its data: it is captured once into a
 // CUDA graph and replayed for each new batch.  Each query's rows come out in
@@ -60,17 +67,64 @@ struct BatchTune {
 constexpr int kErrBarrier = 1 << 4;         // flags[0]: a grid-barrier wait ran out
 constexpr long kBarrierIters = 1l << 24;    // polls of a grid-barrier wait (about 1 s with the back-off)
 
-constexpr int kBTMin = 128;                 // the smaller of the two block sizes (128, 256 threads)
-constexpr int kMaxQ = 4096;                 // queries per batch (shared-memory row offsets)
+constexpr int kBTMax = 256;                 // the larger of the two block sizes (128, 256 threads)
+constexpr int kMaxBlocksPerSm = 16;
+constexpr int kMaxQ = 4096;                 // queries per batch
 
-__device__ __forceinline__ int find_query(const int64_t *s_off, int Q, int64_t g) {
-    int lo = 0, hi = Q - 1;   // largest q with s_off[q] <= g
+// largest q with off[q] <= g (off: the step's input row offsets, Q + 1 of
+// them, read through L1)
+__device__ __forceinline__ int find_query(const int64_t *__restrict__ off, int Q, int64_t g) {
+    int lo = 0, hi = Q - 1;
     while (lo < hi) {
         const int mid = (lo + hi + 1) >> 1;
-        if (s_off[mid] <= g) lo = mid;
+        if (__ldg(off + mid) <= g) lo = mid;
         else hi = mid - 1;
     }
     return lo;
+}
+
+// As find_query for one row by a whole warp: each round asks 32 pivots with
+// one load, so 4096 queries take three dependent loads instead of twelve (the
+// step kernels are chains of such loads, each starting with a cold L1).
+__device__ __forceinline__ int find_query_warp(const int64_t *__restrict__ off, int Q, int64_t g, int lane) {
+    int lo = 0, n = Q;
+    while (n > 1) {
+        const int step = (n + 31) >> 5, i = lane * step;
+        const unsigned m = __ballot_sync(FULL, i < n && __ldg(off + lo + i) <= g);
+        const int k = 31 - __clz((int)m);   // off is ascending: the pivots at or below g come first
+        lo += k * step;
+        n = n - k * step < step ? n - k * step : step;
+    }
+    return lo;
+}
+
+// The queries of 32 consecutive rows g0 + lane, whose first belongs to q0: the
+// boundaries of the next 32 queries, one per lane, searched by shuffles; rows
+// past them (behind that many empty queries) search on their own.
+__device__ __forceinline__ int find_queries(const int64_t *__restrict__ off, int Q, int64_t g0, int q0, int lane) {
+    const int64_t rel = q0 + 1 + lane < Q ? __ldg(off + q0 + 1 + lane) - g0 : 64;
+    const int p = rel < 64 ? (int)rel : 64;   // > 0: q0 is the last query that begins at or before g0
+    int k = 0;                                // boundaries at or before row g0 + lane
+#pragma unroll
+    for (int s = 16; s > 0; s >>= 1)
+        if (__shfl_sync(FULL, p, k + s - 1) <= lane) k += s;
+    if (__shfl_sync(FULL, p, k) <= lane) ++k;
+    if (k == 32) return find_query(off, Q, g0 + lane);
+    return q0 + k;
+}
+
+// Rows per tile of a step of `total` rows on a grid of `warps` warps: as many
+// as give every warp a tile (a power of two below 32, then a multiple of 32),
+// at most 32 x rounds.
+__host__ __device__ __forceinline__ int rows_per_tile(int64_t total, int64_t warps, int rounds) {
+    const int64_t need = (total + warps - 1) / warps;
+    if (need >= 32) {
+        const int64_t r = (need + 31) / 32;
+        return 32 * (int)(r < rounds ? r : rounds);
+    }
+    int rho = 1;
+    while (rho < need) rho *= 2;
+    return rho;
 }
 
 __device__ __forceinline__ bool b_contains(const int32_t *e, uint32_t n, int32_t v) {
@@ -98,25 +152,41 @@ struct StepIO {
     int *flags;               // [0] error bits, [1] overflow
     int64_t cap_ints, cap_rows;
     int Q;
+    int64_t warps;            // of the count and write grids
 };
 
-// count: per (query, row) output counts, per-tile and per-query sums (BT
-// threads a block, a tile of BT x rounds rows)
+// tiles of a step and this warp's: warp w of block b takes tiles b + w G,
+// + G BT / 32, ... (G blocks), so few tiles spread over the blocks
+__device__ __forceinline__ int64_t first_tile() {
+    return (int64_t)(threadIdx.x >> 5) * gridDim.x + blockIdx.x;
+}
+
+__device__ __forceinline__ unsigned long long warp_scan(unsigned long long v, int lane) {
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned long long x = __shfl_up_sync(FULL, v, o);
+        if (lane >= o) v += x;
+    }
+    return v;
+}
+
+// count: per (query, row) output counts, per-tile and per-query sums
 template <int BT>
-__device__ __forceinline__ void count_phase(const StepIO &io, int rounds, const int64_t *s_off) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int tile_rows = (BT / 32) * 32 * rounds;
-    const int64_t total = s_off[io.Q];
-    const int64_t ntiles = (total + tile_rows - 1) / tile_rows;
-    __shared__ unsigned long long s_sum[BT / 32];
-    for (int64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+__device__ __forceinline__ void count_phase(const StepIO &io, int rounds) {
+    const int lane = threadIdx.x & 31;
+    const int64_t total = io.in_row_off[io.Q];
+    const int rho = rows_per_tile(total, io.warps, rounds);
+    const int64_t ntiles = (total + rho - 1) / rho;
+    for (int64_t tile = first_tile(); tile < ntiles; tile += (int64_t)gridDim.x * (BT / 32)) {
         unsigned long long my = 0ull;
-        for (int rd = 0; rd < rounds; ++rd) {
-            const int64_t g = tile * tile_rows + (int64_t)warp * 32 * rounds + rd * 32 + lane;
-            const bool valid = g < total;
-            int q = 0;
+        int q0 = find_query_warp(io.in_row_off, io.Q, tile * rho, lane);
+        for (int r0 = 0; r0 < rho && tile * rho + r0 < total; r0 += 32) {
+            const int64_t g = tile * rho + r0 + lane;
+            const bool valid = r0 + lane < rho && g < total;
+            const int q = find_queries(io.in_row_off, io.Q, g - lane, q0, lane);
+            q0 = __shfl_sync(FULL, q, 31);   // the next window's row may begin a later query: found from here
             StepDesc d{BK_NOP, 0, 0, 0, 0, 0};
-            if (valid) { q = find_query(s_off, io.Q, g); d = io.desc[q]; }
+            if (valid) d = io.desc[q];
             PredView pv{};
             int32_t vid = -1;
             bool probe = valid && d.kind != BK_NOP;
@@ -126,7 +196,7 @@ __device__ __forceinline__ void count_phase(const StepIO &io, int rounds, const 
                 if (d.kind == BK_C2U) {
                     vid = d.cst;
                 } else {
-                    const int64_t r = g - s_off[q];
+                    const int64_t r = g - __ldg(io.in_row_off + q);
                     const int32_t *row = io.hist + io.in_int_off[q] + r * io.in_cols[q];
                     vid = __ldg(row + d.scol);
                     target = d.kind == BK_K2K ? __ldg(row + d.ecol) : d.cst;
@@ -156,153 +226,191 @@ __device__ __forceinline__ void count_phase(const StepIO &io, int rounds, const 
             my += c;
         }
         for (int o2 = 16; o2 > 0; o2 >>= 1) my += __shfl_xor_sync(FULL, my, o2);
-        if (lane == 0) s_sum[warp] = my;
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            unsigned long long t = 0ull;
-            for (int w = 0; w < BT / 32; ++w) t += s_sum[w];
-            io.tile_sum[tile] = t;
-        }
-        __syncthreads();
+        if (lane == 0) io.tile_sum[tile] = my;
     }
+}
+
+// Programmatic dependent launch: the step kernels are placed while the kernel
+// before them ends, and each waits for it before reading anything.
+__device__ __forceinline__ void after_prior_kernel() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;");
 }
 
 template <int BT>
 __global__ void __launch_bounds__(BT)
 batch_count_kernel(StepIO io, int rounds) {
-    extern __shared__ int64_t s_off[];   // Q + 1
+    after_prior_kernel();
     if (io.flags[1]) return;
-    for (int i = threadIdx.x; i <= io.Q; i += blockDim.x) s_off[i] = io.in_row_off[i];
+    count_phase<BT>(io, rounds);
+}
+
+// Exclusive scan of the threads' values over the block (any multiple of 32
+// threads up to 1024), and their sum.
+__device__ __forceinline__ unsigned long long block_scan(unsigned long long v, unsigned long long *ws,
+                                                         unsigned long long &all) {
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    const unsigned long long in = warp_scan(v, lane);
+    if (lane == 31) ws[wid] = in;
     __syncthreads();
-    count_phase<BT>(io, rounds, s_off);
+    const unsigned long long x = warp_scan(lane < nw ? ws[lane] : 0ull, lane);   // in every warp
+    all = __shfl_sync(FULL, x, 31);
+    const unsigned long long before = __shfl_sync(FULL, x, wid > 0 ? wid - 1 : 0);
+    __syncthreads();   // ws is free again
+    return in - v + (wid > 0 ? before : 0ull);
 }
 
-// One block (any multiple of 32 threads up to 1024): tile prefix sums,
-// per-query output layout, capacity check.  BT: the count's block size.
-template <int BT>
-__device__ __forceinline__ void scan_phase(const StepIO &io, int rounds) {
-    __shared__ unsigned long long ws[32], wi[32];
-    const int nt = blockDim.x, nw = nt >> 5;
-    const int t = threadIdx.x, lane = t & 31, wid = t >> 5;
-    const int tile_rows = (BT / 32) * 32 * rounds;
+// The scan's two parts, each one block's work: the tiles' prefix sums, and the
+// queries' output layout with the capacity check.  One SM's memory
+// transactions and the chain of its loads bound them, so they run on two SMs, a
+// thread takes neighbouring entries of its neighbours (pairs of tiles, single
+// queries: whole sectors), and a pass's loads are issued together.  (Both on
+// one SM, four consecutive queries a thread and 8 B stores 32 B apart: 14.5 us
+// for 4096 queries; on one SM 11.5; this 9.)  The one-kernel step reads here
+// and in the write phase what other blocks wrote in the same launch: past L1.
+constexpr int kScanPer = 4;   // loads in flight
+__device__ __forceinline__ void scan_tiles(const StepIO &io, int rounds, unsigned long long *ws) {
+    const int nt = blockDim.x, t = threadIdx.x;
     const int64_t total = io.in_row_off[io.Q];
-    const int64_t n = (total + tile_rows - 1) / tile_rows;
-    // (1) exclusive scan of the tile sums, in place
-    {
-        const int64_t per = (n + nt - 1) / nt, a = (int64_t)t * per, b = a + per < n ? a + per : n;
-        unsigned long long ls = 0ull;
-        for (int64_t i = a; i < b; ++i) ls += io.tile_sum[i];
-        unsigned long long is = ls;
-        for (int o = 1; o < 32; o <<= 1) { const unsigned long long v = __shfl_up_sync(FULL, is, o); if (lane >= o) is += v; }
-        if (lane == 31) ws[wid] = is;
-        __syncthreads();
-        if (wid == 0) {
-            unsigned long long x = lane < nw ? ws[lane] : 0ull;
-            for (int o = 1; o < 32; o <<= 1) { const unsigned long long v = __shfl_up_sync(FULL, x, o); if (lane >= o) x += v; }
-            ws[lane] = x;
+    const int rho = rows_per_tile(total, io.warps, rounds);
+    const int64_t n = (total + rho - 1) / rho;
+    unsigned long long carry = 0ull;
+    for (int64_t i0 = 0; i0 < n; i0 += 2 * kScanPer * (int64_t)nt) {
+        ulonglong2 p[kScanPer];
+#pragma unroll
+        for (int k = 0; k < kScanPer; ++k) {
+            const int64_t i = i0 + 2 * ((int64_t)k * nt + t);   // the buffer holds an even number of tiles
+            p[k] = i < n ? __ldcg(reinterpret_cast<const ulonglong2 *>(io.tile_sum + i)) : make_ulonglong2(0ull, 0ull);
+            if (i + 1 >= n) p[k].y = 0ull;
         }
-        __syncthreads();
-        unsigned long long es = is - ls + (wid ? ws[wid - 1] : 0ull);
-        for (int64_t i = a; i < b; ++i) { const unsigned long long v = io.tile_sum[i]; io.tile_sum[i] = es; es += v; }
-        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < kScanPer; ++k) {
+            const int64_t i = i0 + 2 * ((int64_t)k * nt + t);
+            if (i0 + 2 * (int64_t)k * nt >= n) break;   // the same in every thread
+            unsigned long long all;
+            const unsigned long long e = carry + block_scan(p[k].x + p[k].y, ws, all);
+            if (i < n) *reinterpret_cast<ulonglong2 *>(io.tile_sum + i) = make_ulonglong2(e, e + p[k].x);
+            carry += all;
+        }
     }
-    // (2) per-query output rows and ints (Q <= 4096: four per thread of 1024)
-    {
-        const int Q = io.Q, per = (Q + nt - 1) / nt, a = t * per, b = a + per < Q ? a + per : Q;
-        unsigned long long lr = 0ull, li = 0ull;
-        for (int q = a; q < b; ++q) {
-            const StepDesc d = io.desc[q];
-            const int w = (d.kind == BK_K2U) ? io.in_cols[q] + 1 : (d.kind == BK_C2U ? 1 : io.in_cols[q]);
-            lr += io.q_rows[q];
-            li += io.q_rows[q] * (unsigned long long)w;
-        }
-        unsigned long long ir = lr, ii = li;
-        for (int o = 1; o < 32; o <<= 1) {
-            const unsigned long long v = __shfl_up_sync(FULL, ir, o), x = __shfl_up_sync(FULL, ii, o);
-            if (lane >= o) { ir += v; ii += x; }
-        }
-        if (lane == 31) { ws[wid] = ir; wi[wid] = ii; }
-        __syncthreads();
-        if (wid == 0) {
-            unsigned long long x = lane < nw ? ws[lane] : 0ull, y = lane < nw ? wi[lane] : 0ull;
-            for (int o = 1; o < 32; o <<= 1) {
-                const unsigned long long v = __shfl_up_sync(FULL, x, o), u = __shfl_up_sync(FULL, y, o);
-                if (lane >= o) { x += v; y += u; }
+}
+
+__device__ __forceinline__ void scan_queries(const StepIO &io, unsigned long long *ws) {
+    const int nt = blockDim.x, t = threadIdx.x;
+    const int Q = io.Q;
+    unsigned long long row_at = 0ull, int_at = 0ull;
+    for (int q0 = 0; q0 < Q; q0 += kScanPer * nt) {
+        unsigned long long r[kScanPer];
+        int w[kScanPer];
+#pragma unroll
+        for (int k = 0; k < kScanPer; ++k) {
+            const int q = q0 + k * nt + t;
+            r[k] = 0ull;
+            w[k] = 0;
+            if (q < Q) {
+                const int kind = io.desc[q].kind, cols = io.in_cols[q];
+                r[k] = __ldcg(io.q_rows + q);
+                w[k] = kind == BK_K2U ? cols + 1 : (kind == BK_C2U ? 1 : cols);
             }
-            ws[lane] = x;
-            wi[lane] = y;
         }
-        __syncthreads();
-        unsigned long long er = ir - lr + (wid ? ws[wid - 1] : 0ull);
-        unsigned long long ei = ii - li + (wid ? wi[wid - 1] : 0ull);
-        for (int q = a; q < b; ++q) {
-            const StepDesc d = io.desc[q];
-            const int w = (d.kind == BK_K2U) ? io.in_cols[q] + 1 : (d.kind == BK_C2U ? 1 : io.in_cols[q]);
-            const unsigned long long r = io.q_rows[q];
-            io.out_row_off[q] = (int64_t)er;
-            io.out_int_off[q] = (int64_t)ei;
-            io.out_cols[q] = w;
-            io.q_rows[q] = 0ull;   // the next step's count kernel accumulates afresh
-            er += r;
-            ei += r * (unsigned long long)w;
+#pragma unroll
+        for (int k = 0; k < kScanPer; ++k) {
+            const int q = q0 + k * nt + t;
+            if (q0 + k * nt >= Q) break;   // the same in every thread
+            unsigned long long ar, ai;
+            const unsigned long long er = block_scan(r[k], ws, ar), ei = block_scan(r[k] * (unsigned long long)w[k], ws, ai);
+            if (q < Q) {
+                io.out_row_off[q] = (int64_t)(row_at + er);
+                io.out_int_off[q] = (int64_t)(int_at + ei);
+                io.out_cols[q] = w[k];
+                io.q_rows[q] = 0ull;   // the next step's count kernel accumulates afresh
+            }
+            row_at += ar;
+            int_at += ai;
         }
-        if (t == nt - 1) {
-            io.out_row_off[Q] = (int64_t)er;
-            if ((int64_t)er > io.cap_rows || (int64_t)ei > io.cap_ints) io.flags[1] = 1;
-        }
+    }
+    if (t == 0) {
+        io.out_row_off[Q] = (int64_t)row_at;
+        if ((int64_t)row_at > io.cap_rows || (int64_t)int_at > io.cap_ints) io.flags[1] = 1;
     }
 }
 
-template <int BT>
-__global__ void __launch_bounds__(1024)
+constexpr int kScanThreads = 1024;
+__global__ void __launch_bounds__(kScanThreads)
 batch_scan_kernel(StepIO io, int rounds) {
-    if (io.flags[1]) return;
-    scan_phase<BT>(io, rounds);
+    __shared__ unsigned long long ws[32];
+    after_prior_kernel();
+    if (io.flags[1]) return;   // over capacity: so does the write (also when the other block just found it)
+    if (blockIdx.x == 0) scan_tiles(io, rounds, ws);
+    else scan_queries(io, ws);
 }
 
-// Per tile: block scan of the counts, then write.  Rows with more than
-// `split` output ints are queued and written by whole warps.
+// One row's output of nw = c x w ints, by the whole warp: four ints a lane in
+// flight, the row and column of each kept by steps of 32 (no division).
+__device__ __forceinline__ void write_row_warp(int kind, const int32_t *row, const int32_t *e, int32_t *dst, int cin,
+                                               int w, uint32_t c, int lane) {
+    const int64_t nw = (int64_t)c * w;
+    const uint32_t dr = 32u / (uint32_t)w;
+    const int dc = 32 % w;
+    uint32_t r = (uint32_t)lane / (uint32_t)w;
+    int cc = lane % w;
+    for (int64_t x = lane; x < nw; x += 128) {
+        int32_t v[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            if (x + 32 * k < nw) {
+                if (kind == BK_K2U) v[k] = cc < cin ? __ldg(row + cc) : __ldg(e + r);
+                else if (kind == BK_C2U) v[k] = __ldg(e + r);
+                else v[k] = __ldg(row + cc);
+            }
+            r += dr;
+            cc += dc;
+            if (cc >= w) { cc -= w; ++r; }
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            if (x + 32 * k < nw) dst[x + 32 * k] = v[k];
+    }
+}
+
+// Per tile: warp scan of the counts, then write.  A row with more than
+// `split` output ints -- fewer in tiles below 32 rows, whose other lanes are
+// idle -- is written by the whole warp.
 template <int BT>
-__device__ __forceinline__ void write_phase(const StepIO &io, int rounds, int split, const int64_t *s_off) {
-    __shared__ unsigned long long s_w[BT / 32];
-    __shared__ int s_nq;
-    __shared__ int s_big[BT * 8];        // queued rows (local index), rounds <= 8
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int tile_rows = BT * rounds;
-    const int64_t total = s_off[io.Q];
-    const int64_t ntiles = (total + tile_rows - 1) / tile_rows;
-    for (int64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-        if (threadIdx.x == 0) s_nq = 0;
-        // thread t owns rows tile*tile_rows + t*rounds .. + rounds-1
-        const int64_t g0 = tile * tile_rows + (int64_t)threadIdx.x * rounds;
-        unsigned long long my = 0ull;
-        for (int k = 0; k < rounds; ++k) my += (g0 + k < total) ? io.cnt[g0 + k] : 0u;
-        unsigned long long inc = my;
-        for (int o = 1; o < 32; o <<= 1) { const unsigned long long v = __shfl_up_sync(FULL, inc, o); if (lane >= o) inc += v; }
-        if (lane == 31) s_w[warp] = inc;
-        __syncthreads();
-        unsigned long long pos = io.tile_sum[tile] + inc - my;
-        for (int w = 0; w < warp; ++w) pos += s_w[w];
-        for (int k = 0; k < rounds; ++k) {
-            const int64_t g = g0 + k;
-            if (g >= total) break;
-            const uint32_t c = io.cnt[g];
-            if (c == 0u) continue;
-            const int q = find_query(s_off, io.Q, g);
-            const StepDesc d = io.desc[q];
-            const int cin = io.in_cols[q];
-            const int w = (d.kind == BK_K2U) ? cin + 1 : (d.kind == BK_C2U ? 1 : cin);
-            if ((int64_t)c * w > split) {
-                const int slot = atomicAdd(&s_nq, 1);
-                s_big[slot] = (int)(g - tile * tile_rows);
-                // its output position is recomputed by the warp below
-            } else {
-                const int32_t *row = io.hist + io.in_int_off[q] + (g - s_off[q]) * cin;
-                int32_t *dst = io.out + io.out_int_off[q] + ((int64_t)pos - io.out_row_off[q]) * w;
-                if (d.kind == BK_K2U || d.kind == BK_C2U) {
-                    const int32_t *e = io.pvs[d.pid].edges + io.off[g];
+__device__ __forceinline__ void write_phase(const StepIO &io, int rounds, int split) {
+    const int lane = threadIdx.x & 31;
+    const int64_t total = io.in_row_off[io.Q];
+    const int rho = rows_per_tile(total, io.warps, rounds);
+    const int64_t ntiles = (total + rho - 1) / rho;
+    const int64_t most = rho < 32 ? ((int64_t)split * rho + 31) / 32 : split;
+    for (int64_t tile = first_tile(); tile < ntiles; tile += (int64_t)gridDim.x * (BT / 32)) {
+        unsigned long long base = __ldcg(io.tile_sum + tile);
+        int q0 = find_query_warp(io.in_row_off, io.Q, tile * rho, lane);
+        for (int r0 = 0; r0 < rho && tile * rho + r0 < total; r0 += 32) {
+            const int64_t g = tile * rho + r0 + lane;
+            const int q = find_queries(io.in_row_off, io.Q, g - lane, q0, lane);
+            q0 = __shfl_sync(FULL, q, 31);
+            const uint32_t c = r0 + lane < rho && g < total ? __ldcg(io.cnt + g) : 0u;
+            const unsigned long long inc = warp_scan(c, lane);
+            const unsigned long long pos = base + inc - c;
+            base += __shfl_sync(FULL, inc, 31);
+            int kind = BK_NOP, cin = 0, w = 0;
+            const int32_t *row = nullptr, *e = nullptr;
+            int32_t *dst = nullptr;
+            if (c) {
+                const StepDesc d = io.desc[q];
+                kind = d.kind;
+                cin = io.in_cols[q];
+                w = (kind == BK_K2U) ? cin + 1 : (kind == BK_C2U ? 1 : cin);
+                row = io.hist + io.in_int_off[q] + (g - __ldg(io.in_row_off + q)) * cin;
+                dst = io.out + __ldcg(io.out_int_off + q) + ((int64_t)pos - __ldcg(io.out_row_off + q)) * w;
+                if (kind == BK_K2U || kind == BK_C2U) e = io.pvs[d.pid].edges + __ldcg(io.off + g);
+            }
+            const bool big = c != 0u && (int64_t)c * w > most;
+            if (c != 0u && !big) {
+                if (kind == BK_K2U || kind == BK_C2U) {
                     for (uint32_t x = 0; x < c; ++x) {
-                        if (d.kind == BK_K2U) for (int cc = 0; cc < cin; ++cc) dst[cc] = __ldg(row + cc);
+                        if (kind == BK_K2U) for (int cc = 0; cc < cin; ++cc) dst[cc] = __ldg(row + cc);
                         dst[w - 1] = __ldg(e + x);
                         dst += w;
                     }
@@ -310,50 +418,24 @@ __device__ __forceinline__ void write_phase(const StepIO &io, int rounds, int sp
                     for (int cc = 0; cc < cin; ++cc) dst[cc] = __ldg(row + cc);
                 }
             }
-            pos += c;
-        }
-        __syncthreads();
-        // queued rows: one warp per row, lanes stride over the row's output ints
-        const int nq = s_nq;
-        for (int i = warp; i < nq; i += BT / 32) {
-            const int lr = s_big[i];
-            const int64_t g = tile * tile_rows + lr;
-            // output position of row g: tile base + counts of the rows before it in the tile
-            unsigned long long before = 0ull;
-            for (int j = lane; j < lr; j += 32) before += io.cnt[tile * tile_rows + j];
-            for (int o = 16; o > 0; o >>= 1) before += __shfl_xor_sync(FULL, before, o);
-            const unsigned long long p = io.tile_sum[tile] + before;
-            const int q = find_query(s_off, io.Q, g);
-            const StepDesc d = io.desc[q];
-            const int cin = io.in_cols[q];
-            const int w = (d.kind == BK_K2U) ? cin + 1 : (d.kind == BK_C2U ? 1 : cin);
-            const uint32_t c = io.cnt[g];
-            const int32_t *row = io.hist + io.in_int_off[q] + (g - s_off[q]) * cin;
-            int32_t *dst = io.out + io.out_int_off[q] + ((int64_t)p - io.out_row_off[q]) * w;
-            const int32_t *e = (d.kind == BK_K2U || d.kind == BK_C2U) ? io.pvs[d.pid].edges + io.off[g] : nullptr;
-            const int64_t nw = (int64_t)c * w;
-            for (int64_t x = lane; x < nw; x += 32) {
-                const int64_t r = x / w;
-                const int cc = (int)(x - r * w);
-                int32_t v;
-                if (d.kind == BK_K2U) v = (cc < cin) ? __ldg(row + cc) : __ldg(e + r);
-                else if (d.kind == BK_C2U) v = __ldg(e + r);
-                else v = __ldg(row + cc);
-                dst[x] = v;
+            for (unsigned left = __ballot_sync(FULL, big); left; left &= left - 1u) {
+                const int src = __ffs(left) - 1;
+                write_row_warp(__shfl_sync(FULL, kind, src),
+                               reinterpret_cast<const int32_t *>(__shfl_sync(FULL, (unsigned long long)row, src)),
+                               reinterpret_cast<const int32_t *>(__shfl_sync(FULL, (unsigned long long)e, src)),
+                               reinterpret_cast<int32_t *>(__shfl_sync(FULL, (unsigned long long)dst, src)),
+                               __shfl_sync(FULL, cin, src), __shfl_sync(FULL, w, src), __shfl_sync(FULL, c, src), lane);
             }
         }
-        __syncthreads();
     }
 }
 
 template <int BT>
 __global__ void __launch_bounds__(BT)
 batch_write_kernel(StepIO io, int rounds, int split) {
-    extern __shared__ int64_t s_off[];   // Q+1 input row offsets
+    after_prior_kernel();
     if (io.flags[1]) return;
-    for (int i = threadIdx.x; i <= io.Q; i += blockDim.x) s_off[i] = io.in_row_off[i];
-    __syncthreads();
-    write_phase<BT>(io, rounds, split, s_off);
+    write_phase<BT>(io, rounds, split);
 }
 
 __device__ __forceinline__ unsigned int ld_acquire(const unsigned int *p) {
@@ -407,16 +489,15 @@ __device__ __forceinline__ bool grid_barrier(unsigned int *bar, int *flags) {
 template <int BT>
 __global__ void __launch_bounds__(BT)
 batch_step_kernel(StepIO io, int rounds, int split, unsigned int *bar) {
-    extern __shared__ int64_t s_off[];   // Q + 1 input row offsets
     if (io.flags[1]) return;             // set before the launch: the same in every block
-    for (int i = threadIdx.x; i <= io.Q; i += blockDim.x) s_off[i] = io.in_row_off[i];
-    __syncthreads();
-    count_phase<BT>(io, rounds, s_off);
+    count_phase<BT>(io, rounds);
     if (!grid_barrier(bar, io.flags)) return;
-    if (blockIdx.x == 0) scan_phase<BT>(io, rounds);
+    __shared__ unsigned long long ws[32];
+    if (blockIdx.x == 0) scan_tiles(io, rounds, ws);
+    if (blockIdx.x == gridDim.x - 1) scan_queries(io, ws);   // another block where there are two
     if (!grid_barrier(bar, io.flags)) return;
     if (*(volatile int *)(io.flags + 1)) return;   // this step's scan found the batch over capacity
-    write_phase<BT>(io, rounds, split, s_off);
+    write_phase<BT>(io, rounds, split);
 }
 
 // step-0 layout: every query has one virtual row and no columns
@@ -451,12 +532,15 @@ struct wk_batch {
     int32_t *d_hist[2] = {};
     uint32_t *d_cnt = nullptr, *d_off = nullptr;
     unsigned long long *d_tile = nullptr, *d_qrows = nullptr;
-    int *d_flags = nullptr;
+    int *d_flags = nullptr;                 // d_block
     unsigned int *d_bar = nullptr;          // grid barrier of the one-kernel steps (count, generation)
     // host (pinned)
     StepDesc *h_desc = nullptr;
-    int64_t *h_layout = nullptr;            // row_off (Q+1), int_off (Q), cols as int64 (Q)
-    int *h_flags = nullptr;
+    // the flags (one word) and the final tables' layout -- row_off (Q+1), int_off
+    // (Q), cols as int32 (Q) -- on the device, and their pinned copy
+    int64_t *d_block = nullptr, *h_block = nullptr;
+    int64_t *h_layout = nullptr;            // h_block + 1
+    int *h_flags = nullptr;                 // h_block
     // graph
     // executable graphs by batch size (a serving loop's batch sizes vary from
     // batch to batch; each size is captured once), all for graph_tune
@@ -482,11 +566,9 @@ cudaError_t create_priority_stream(cudaStream_t *st) {
     return cudaStreamCreateWithPriority(st, cudaStreamNonBlocking, greatest);
 }
 
-// tiles of the smallest shape (kBTMin threads x rounds rows): the tile-sum
-// buffer holds any tuning's
-int64_t max_tiles(const wk_batch *b, int rounds) {
-    const int64_t tr = (int64_t)kBTMin * rounds;
-    return (b->cap_rows + tr - 1) / tr + 1;
+// most tiles of any tuning: one per warp of the widest grid, or of 32 rows
+int64_t max_tiles(const wk_batch *b) {
+    return std::max((int64_t)b->sms * kMaxBlocksPerSm * (kBTMax / 32), (b->cap_rows + 31) / 32) + 2;   // read in pairs
 }
 
 void free_batch(wk_batch *b) {
@@ -498,15 +580,14 @@ void free_batch(wk_batch *b) {
     if (b->stream) cudaStreamDestroy(b->stream);
     cudaFree(b->d_pvs); cudaFree(b->d_desc);
     for (int i = 0; i < 2; ++i) { cudaFree(b->d_row_off[i]); cudaFree(b->d_int_off[i]); cudaFree(b->d_cols[i]); cudaFree(b->d_hist[i]); }
-    cudaFree(b->d_cnt); cudaFree(b->d_off); cudaFree(b->d_tile); cudaFree(b->d_qrows); cudaFree(b->d_flags);
+    cudaFree(b->d_cnt); cudaFree(b->d_off); cudaFree(b->d_tile); cudaFree(b->d_qrows); cudaFree(b->d_block);
     cudaFree(b->d_bar);
     if (b->h_desc) cudaFreeHost(b->h_desc);
-    if (b->h_layout) cudaFreeHost(b->h_layout);
-    if (b->h_flags) cudaFreeHost(b->h_flags);
+    if (b->h_block) cudaFreeHost(b->h_block);
     delete b;
 }
 
-StepIO make_io(wk_batch *b, int s, int Q) {
+StepIO make_io(wk_batch *b, int s, int Q, int64_t warps) {
     StepIO io;
     const int in = s & 1, out = in ^ 1;
     io.hist = b->d_hist[in];
@@ -527,17 +608,23 @@ StepIO make_io(wk_batch *b, int s, int Q) {
     io.cap_ints = b->cap_ints;
     io.cap_rows = b->cap_rows;
     io.Q = Q;
+    io.warps = warps;
+    if (s == b->max_steps - 1) {   // the final tables' layout, in one range for one copy to the host
+        io.out_row_off = b->d_block + 1;
+        io.out_int_off = b->d_block + Q + 2;
+        io.out_cols = reinterpret_cast<int32_t *>(b->d_block + 2 * Q + 2);
+    }
     return io;
 }
 
 // the max_steps steps of a batch with BT-thread blocks: three kernels per
 // step, or one cooperative kernel
 template <int BT>
-int enqueue_steps(wk_batch *b, int Q, const BatchTune &t, unsigned grid, size_t sm_off, cudaStream_t st) {
+int enqueue_steps(wk_batch *b, int Q, const BatchTune &t, unsigned grid, cudaStream_t st) {
     if (t.fused) {
         // every block of a cooperative launch must be resident at once
         int occ = 0;
-        cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, batch_step_kernel<BT>, BT, sm_off);
+        cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, batch_step_kernel<BT>, BT, 0);
         if (e != cudaSuccess) return cuda_fail(e, "batch step occupancy");
         if (occ < 1) return set_error(WK_EDEVICE, "batch step kernel: no block fits on an SM");
         const unsigned gf = (unsigned)std::min<int64_t>(grid, (int64_t)occ * b->sms);
@@ -550,21 +637,34 @@ int enqueue_steps(wk_batch *b, int Q, const BatchTune &t, unsigned grid, size_t 
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(gf);
         cfg.blockDim = dim3(BT);
-        cfg.dynamicSmemBytes = sm_off;
         cfg.stream = st;
         cfg.attrs = attr;
         cfg.numAttrs = 1;
         for (int s = 0; s < b->max_steps; ++s) {
-            StepIO io = make_io(b, s, Q);
+            StepIO io = make_io(b, s, Q, (int64_t)gf * (BT / 32));
             if ((e = cudaLaunchKernelEx(&cfg, batch_step_kernel<BT>, io, t.rounds, t.split, b->d_bar)) != cudaSuccess)
                 return cuda_fail(e, "batch step launch");
         }
     } else {
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[0].val.programmaticStreamSerializationAllowed = 1;
+        cudaLaunchConfig_t cfg = {};
+        cfg.stream = st;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
         for (int s = 0; s < b->max_steps; ++s) {
-            StepIO io = make_io(b, s, Q);
-            batch_count_kernel<BT><<<grid, BT, sm_off, st>>>(io, t.rounds);
-            batch_scan_kernel<BT><<<1, 1024, 0, st>>>(io, t.rounds);
-            batch_write_kernel<BT><<<grid, BT, sm_off, st>>>(io, t.rounds, t.split);
+            StepIO io = make_io(b, s, Q, (int64_t)grid * (BT / 32));
+            cfg.gridDim = dim3(grid);
+            cfg.blockDim = dim3(BT);
+            cudaError_t e = cudaLaunchKernelEx(&cfg, batch_count_kernel<BT>, io, t.rounds);
+            cfg.gridDim = dim3(2);
+            cfg.blockDim = dim3(kScanThreads);
+            if (e == cudaSuccess) e = cudaLaunchKernelEx(&cfg, batch_scan_kernel, io, t.rounds);
+            cfg.gridDim = dim3(grid);
+            cfg.blockDim = dim3(BT);
+            if (e == cudaSuccess) e = cudaLaunchKernelEx(&cfg, batch_write_kernel<BT>, io, t.rounds, t.split);
+            if (e != cudaSuccess) return cuda_fail(e, "batch step launch");
         }
     }
     return WK_OK;
@@ -579,12 +679,10 @@ int64_t batch_kernels(const wk_batch *b, const BatchTune &t) {
 // write) as three kernels or as one cooperative kernel
 int enqueue(wk_batch *b, int Q, const BatchTune &t, cudaStream_t st) {
     // the Q descriptors of each step (step s's start at s * max_q)
-    for (int s = 0; s < b->max_steps; ++s) {
-        const size_t at = (size_t)s * b->max_q;
-        cudaError_t e = cudaMemcpyAsync(b->d_desc + at, b->h_desc + at, sizeof(StepDesc) * (size_t)Q,
-                                        cudaMemcpyHostToDevice, st);
-        if (e != cudaSuccess) return cuda_fail(e, "batch descriptors");
-    }
+    const size_t pitch = sizeof(StepDesc) * (size_t)b->max_q;
+    cudaError_t ce = cudaMemcpy2DAsync(b->d_desc, pitch, b->h_desc, pitch, sizeof(StepDesc) * (size_t)Q,
+                                       (size_t)b->max_steps, cudaMemcpyHostToDevice, st);
+    if (ce != cudaSuccess) return cuda_fail(ce, "batch descriptors");
     batch_init_kernel<<<(Q + 256) / 256, 256, 0, st>>>(Q, b->d_row_off[0], b->d_int_off[0], b->d_cols[0], b->d_qrows,
                                                        b->d_flags);
     // The step kernels loop over tiles, so any grid gives the same rows.  A
@@ -593,8 +691,7 @@ int enqueue(wk_batch *b, int Q, const BatchTune &t, cudaStream_t st) {
     // light queries then hold a few SMs, not all of them.
     const int64_t full = (int64_t)b->sms * t.blocks_per_sm;
     const unsigned grid = (unsigned)std::min<int64_t>(full, std::max<int64_t>(b->sms / 4, 2 * (int64_t)Q));
-    const size_t sm_off = sizeof(int64_t) * (size_t)(Q + 1);
-    const int st2 = t.bt == 128 ? enqueue_steps<128>(b, Q, t, grid, sm_off, st) : enqueue_steps<256>(b, Q, t, grid, sm_off, st);
+    const int st2 = t.bt == 128 ? enqueue_steps<128>(b, Q, t, grid, st) : enqueue_steps<256>(b, Q, t, grid, st);
     if (st2) return st2;
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_fail(e, "batch launch");
@@ -622,18 +719,17 @@ extern "C" int wk_batch_create(wk_ctx *ctx, int32_t max_queries, int32_t max_ste
     b->cap_rows = capacity_ints;   // every row holds at least one int
     cudaDeviceGetAttribute(&b->sms, cudaDevAttrMultiProcessorCount, ctx->device);
     const size_t npv = ctx->store->views.size();
-    const int64_t tiles = max_tiles(b, 1);
+    const int64_t tiles = max_tiles(b);
     bool ok = cudaMalloc(&b->d_pvs, sizeof(PredView) * npv) == cudaSuccess &&
               cudaMalloc(&b->d_desc, sizeof(StepDesc) * (size_t)max_queries * max_steps) == cudaSuccess &&
               cudaMalloc(&b->d_cnt, 4 * (size_t)b->cap_rows) == cudaSuccess &&
               cudaMalloc(&b->d_off, 4 * (size_t)b->cap_rows) == cudaSuccess &&
               cudaMalloc(&b->d_tile, 8 * (size_t)tiles) == cudaSuccess &&
               cudaMalloc(&b->d_qrows, 8 * (size_t)max_queries) == cudaSuccess &&
-              cudaMalloc(&b->d_flags, 64) == cudaSuccess &&
+              cudaMalloc(&b->d_block, 8 * (size_t)(3 * max_queries + 2)) == cudaSuccess &&
               cudaMalloc(&b->d_bar, 2 * sizeof(unsigned int)) == cudaSuccess &&
               cudaHostAlloc((void **)&b->h_desc, sizeof(StepDesc) * (size_t)max_queries * max_steps, 0) == cudaSuccess &&
-              cudaHostAlloc((void **)&b->h_layout, 8 * (size_t)(3 * max_queries + 1), 0) == cudaSuccess &&
-              cudaHostAlloc((void **)&b->h_flags, 64, 0) == cudaSuccess &&
+              cudaHostAlloc((void **)&b->h_block, 8 * (size_t)(3 * max_queries + 2), 0) == cudaSuccess &&
               create_priority_stream(&b->stream) == cudaSuccess &&
               cudaEventCreateWithFlags(&b->done, cudaEventDisableTiming) == cudaSuccess;
     for (int i = 0; ok && i < 2; ++i)
@@ -646,8 +742,11 @@ extern "C" int wk_batch_create(wk_ctx *ctx, int32_t max_queries, int32_t max_ste
         free_batch(b);
         return set_error(WK_ENOMEM, "wk_batch_create: allocation failed (capacity %lld ints)", (long long)capacity_ints);
     }
+    b->d_flags = reinterpret_cast<int *>(b->d_block);
+    b->h_flags = reinterpret_cast<int *>(b->h_block);
+    b->h_layout = b->h_block + 1;
     e = cudaMemcpy(b->d_pvs, ctx->store->views.data(), sizeof(PredView) * npv, cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMemset(b->d_flags, 0, 64);
+    if (e == cudaSuccess) e = cudaMemset(b->d_flags, 0, 8);
     if (e == cudaSuccess) e = cudaMemset(b->d_bar, 0, 2 * sizeof(unsigned int));
     if (e != cudaSuccess) { int r = cuda_fail(e, "wk_batch_create"); free_batch(b); return r; }
     *out = b;
@@ -660,7 +759,7 @@ extern "C" int wk_batch_destroy(wk_batch *b) {
 }
 
 extern "C" int wk_batch_set_tuning(wk_batch *b, int32_t blocks_per_sm, int32_t rows_per_warp, int32_t split_ints) {
-    if (!b || blocks_per_sm < 1 || blocks_per_sm > 16 || rows_per_warp < 32 || rows_per_warp > 256 ||
+    if (!b || blocks_per_sm < 1 || blocks_per_sm > kMaxBlocksPerSm || rows_per_warp < 32 || rows_per_warp > 256 ||
         rows_per_warp % 32 || split_ints < 1)
         return set_error(WK_EINVAL, "wk_batch_set_tuning: blocks/SM 1..16, rows/warp 32..256 (x32), split >= 1");
     b->tune = BatchTune{blocks_per_sm, rows_per_warp / 32, split_ints, b->tune.fused, b->tune.bt};
@@ -783,13 +882,9 @@ extern "C" int wk_batch_launch(wk_batch *b, const int64_t *cmd_chains, const int
     ctx->launches += batch_kernels(b, b->tune);
     b->last_q = nq;
     b->final_buf = b->max_steps & 1;
-    // layout of the final tables + flags, then the completion event
-    const int fb = b->final_buf;
-    if ((e = cudaMemcpyAsync(b->h_flags, b->d_flags, 8, cudaMemcpyDeviceToHost, s)) != cudaSuccess ||
-        (e = cudaMemcpyAsync(b->h_layout, b->d_row_off[fb], 8 * (size_t)(nq + 1), cudaMemcpyDeviceToHost, s)) != cudaSuccess ||
-        (e = cudaMemcpyAsync(b->h_layout + nq + 1, b->d_int_off[fb], 8 * (size_t)nq, cudaMemcpyDeviceToHost, s)) != cudaSuccess ||
-        (e = cudaMemcpyAsync(reinterpret_cast<int32_t *>(b->h_layout + 2 * nq + 1), b->d_cols[fb], 4 * (size_t)nq,
-                             cudaMemcpyDeviceToHost, s)) != cudaSuccess ||
+    // the flags and the layout of the final tables, then the completion event
+    if ((e = cudaMemcpyAsync(b->h_block, b->d_block, 8 * (2 * (size_t)nq + 2) + 4 * (size_t)nq, cudaMemcpyDeviceToHost,
+                             s)) != cudaSuccess ||
         (e = cudaEventRecord(b->done, s)) != cudaSuccess)
         return cuda_fail(e, "batch layout readback");
     return WK_OK;
