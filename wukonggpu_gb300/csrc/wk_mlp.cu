@@ -18,7 +18,8 @@
 // layers' activation runs in the GEMM's epilogue: the forward product writes
 // GELU(Z) in bf16 (row-major and transposed) beside Z, and the input-gradient
 // product of the layer above writes dZ = dH * GELU'(Z) with the bias
-// gradient (its column sums), so dH itself is never stored.
+// gradient (its column sums), so dH itself is never stored.  Prediction, which
+// keeps nothing for a backward pass, is one kernel (wk_mlp_forward.cuh).
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -29,6 +30,7 @@
 
 #include "wk_runtime.h"
 #include "wk_tc_gemm.cuh"
+#include "wk_mlp_forward.cuh"
 
 namespace wk {
 namespace mlp {
@@ -212,6 +214,11 @@ struct wk_mlp {
     int status = 0;              // a host-side GEMM failure since the last check
     int sms = 152;               // multiprocessors of the device (GEMM tile width choice)
     bool broken = false;         // a GEMM left work in flight: no further GEMM is launched
+    // prediction: two buffers of features in flight, the outputs and ids, a stream for the copies in, and a pinned block for small calls
+    DevBuf stage[2], pred;
+    cudaStream_t copy = nullptr;
+    cudaEvent_t copied[2] = {}, used[2] = {};
+    unsigned char *h_small = nullptr, *h_small_dev = nullptr;
 };
 
 namespace {
@@ -341,7 +348,7 @@ int check_status(wk_mlp *m, cudaStream_t s, const char *what) {
     return WK_OK;
 }
 
-// forward over M rows already uploaded (feats, pids); Y in z[3] col 0
+// forward of a training step over M rows already uploaded (feats, pids); Y in z[3] col 0
 void forward(wk_mlp *m, int M, cudaStream_t s) {
     const int Mp = pad64(M);
     build_input_kernel<<<nblk((int64_t)Mp * kX), 256, 0, s>>>(m->feats, m->pids, M, Mp, m->params + m->off_emb,
@@ -356,8 +363,47 @@ void forward(wk_mlp *m, int M, cudaStream_t s) {
         kin = kH;
     }
     gemm(m, in, kH, m->wb[3], kH, m->z[3], kOutPad, Mp, kOutPad, kH, nullptr, s);
-    // output bias (layer 4 has one real output): added in the loss / predict read
+    // output bias (layer 4 has one real output): added before the loss
     m->kernels += 1;
+}
+
+// Calls of up to kSmallRows samples go through the pinned block, which the
+// kernel reads and writes in place: one host copy of at most 100 KB instead of
+// two device copies in and one out, each some 10 us whatever it holds.
+constexpr int kSmallRows = 512;
+constexpr size_t kSmallPids = sizeof(float) * kIn * kSmallRows, kSmallOut = kSmallPids + sizeof(int32_t) * kSmallRows;
+constexpr size_t kSmallBytes = kSmallOut + sizeof(float) * kSmallRows;
+
+// predictions for n samples in device-readable memory (wk_mlp_forward.cuh)
+void predict(wk_mlp *m, const float *feats, const int32_t *pids, int64_t n, float *out, cudaStream_t s) {
+    if (m->broken) {
+        if (!m->status)
+            m->status = set_error(WK_EDEVICE, "estimator: an earlier tensor-core GEMM left work in flight; "
+                                              "destroy the estimator");
+        return;
+    }
+    mlpf::Args a;
+    a.feats = feats;
+    a.pids = pids;
+    for (int l = 0; l < 4; ++l) a.bias[l] = m->params + m->off_b[l];
+    a.emb = m->params + m->off_emb;
+    a.out = out;
+    a.err = m->d_err;
+    a.n_ids = m->n_ids;
+    a.n = n;
+    CUtensorMap w[4];
+    bool ok = (((uintptr_t)feats | (uintptr_t)a.emb) & 15u) == 0;
+    for (int l = 0; ok && l < 4; ++l)
+        ok = tc::make_map(&w[l], m->wb[l], (uint64_t)kRowsPad[l], (uint64_t)kCols[l], (uint64_t)kCols[l],
+                          l < 3 ? (uint32_t)kH : 32u);
+    if (!ok) {
+        if (!m->status) m->status = set_error(WK_EDEVICE, "estimator: tensor map or alignment of the prediction");
+        return;
+    }
+    const int64_t tiles = (n + mlpf::kTile - 1) / mlpf::kTile;
+    mlpf::forward_kernel<<<(unsigned)std::min<int64_t>(tiles, m->sms), mlpf::kThreads, mlpf::kSmem, s>>>(w[0], w[1], w[2],
+                                                                                                       w[3], a);
+    m->kernels++;
 }
 
 // loss + backward + Adam on M rows (targets uploaded)
@@ -411,11 +457,7 @@ void backward_step(wk_mlp *m, int M, float lr, bool update, cudaStream_t s) {
     }
 }
 
-__global__ void add_bias_read_kernel(const float *Y, const float *b4, int M, float *out) {
-    for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < M; r += gridDim.x * blockDim.x) out[r] = Y[(size_t)r * kOutPad] + b4[0];
-}
-
-// add the output bias to column 0 of Y in place (so loss and predict see y = H3 . w4 + b4)
+// add the output bias to column 0 of Y in place (so the loss sees y = H3 . w4 + b4)
 __global__ void add_out_bias_kernel(float *Y, const float *b4, int M) {
     for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < M; r += gridDim.x * blockDim.x) Y[(size_t)r * kOutPad] += b4[0];
 }
@@ -442,6 +484,12 @@ void free_mlp(wk_mlp *m) {
     cudaFree(m->bidx);
     cudaFree(m->cbias);
     if (m->h_err) cudaFreeHost(m->h_err);
+    if (m->h_small) cudaFreeHost(m->h_small);
+    for (int i = 0; i < 2; ++i) {
+        if (m->copied[i]) cudaEventDestroy(m->copied[i]);
+        if (m->used[i]) cudaEventDestroy(m->used[i]);
+    }
+    if (m->copy) cudaStreamDestroy(m->copy);
     delete m;
 }
 
@@ -485,6 +533,15 @@ extern "C" int wk_mlp_create(wk_ctx *ctx, int32_t n_ids, int32_t max_batch, uint
          cudaMalloc(&m->loss, 16) == cudaSuccess && cudaMalloc(&m->pids, 4 * Mp) == cudaSuccess &&
          cudaMalloc(&m->d_err, sizeof(int)) == cudaSuccess && cudaMalloc(&m->bidx, sizeof(int)) == cudaSuccess &&
          cudaHostAlloc((void **)&m->h_err, sizeof(int), 0) == cudaSuccess &&
+         cudaHostAlloc((void **)&m->h_small, kSmallBytes, cudaHostAllocMapped) == cudaSuccess &&
+         cudaHostGetDevicePointer((void **)&m->h_small_dev, m->h_small, 0) == cudaSuccess &&
+         cudaStreamCreateWithFlags(&m->copy, cudaStreamNonBlocking) == cudaSuccess &&
+         cudaEventCreateWithFlags(&m->copied[0], cudaEventDisableTiming) == cudaSuccess &&
+         cudaEventCreateWithFlags(&m->copied[1], cudaEventDisableTiming) == cudaSuccess &&
+         cudaEventCreateWithFlags(&m->used[0], cudaEventDisableTiming) == cudaSuccess &&
+         cudaEventCreateWithFlags(&m->used[1], cudaEventDisableTiming) == cudaSuccess &&
+         cudaFuncSetAttribute(mlpf::forward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mlpf::kSmem) ==
+             cudaSuccess &&
          set_gemm_smem_all<tc::kEpiStore>() && set_gemm_smem_all<tc::kEpiGeluFwd>() &&
          set_gemm_smem_all<tc::kEpiGeluBwd>();
     if (!ok) {
@@ -678,19 +735,51 @@ extern "C" int wk_mlp_train(wk_mlp *m, const float *feats, const int32_t *pids, 
     return finish(WK_OK);
 }
 
-// Predictions (log(1 + rows)) for n samples, in chunks of the batch capacity.
+// Predictions (log(1 + rows)) for n samples: a small call through the pinned
+// block, a larger one in chunks of two tiles per SM, whose copies in run on
+// their own stream while the chunk before is computed.
 extern "C" int wk_mlp_predict(wk_mlp *m, const float *feats, const int32_t *pids, int64_t n, float *out) {
     if (!m || (n > 0 && (!feats || !pids || !out)) || n < 0) return set_error(WK_EINVAL, "wk_mlp_predict");
     cudaSetDevice(m->ctx->device);
     cudaStream_t s = m->ctx->stream;
-    for (int64_t b0 = 0; b0 < n; b0 += m->cap_m) {
-        const int M = (int)std::min<int64_t>(m->cap_m, n - b0);
-        int st = upload(m, feats + b0 * kIn, pids + b0, nullptr, M, s);
-        if (st) return st;
-        forward(m, M, s);
-        add_bias_read_kernel<<<nblk(M), 256, 0, s>>>(m->z[3], m->params + m->off_b[3], M, m->tgt);
-        cudaError_t e = cudaMemcpyAsync(out + b0, m->tgt, sizeof(float) * (size_t)M, cudaMemcpyDeviceToHost, s);
-        if (e != cudaSuccess) return cuda_fail(e, "wk_mlp_predict");
+    int st = WK_OK;
+    if (n > 0 && n <= kSmallRows) {
+        std::memcpy(m->h_small, feats, sizeof(float) * (size_t)n * kIn);
+        std::memcpy(m->h_small + kSmallPids, pids, sizeof(int32_t) * (size_t)n);
+        predict(m, reinterpret_cast<const float *>(m->h_small_dev),
+                reinterpret_cast<const int32_t *>(m->h_small_dev + kSmallPids), n,
+                reinterpret_cast<float *>(m->h_small_dev + kSmallOut), s);
+        if ((st = check_status(m, s, "wk_mlp_predict"))) return st;
+        std::memcpy(out, m->h_small + kSmallOut, sizeof(float) * (size_t)n);
+    } else if (n > 0) {
+        const int64_t chunk = std::min<int64_t>(n, 2 * (int64_t)mlpf::kTile * m->sms);
+        for (int i = 0; i < (n > chunk ? 2 : 1); ++i)
+            if ((st = m->stage[i].reserve(sizeof(float) * (size_t)chunk * kIn))) return st;
+        if ((st = m->pred.reserve(2 * sizeof(float) * (size_t)n))) return st;   // the outputs, then the ids
+        cudaStream_t in = n > chunk ? m->copy : s;
+        int32_t *p = m->pred.as<int32_t>() + n;
+        cudaError_t e = cudaMemcpyAsync(p, pids, sizeof(int32_t) * (size_t)n, cudaMemcpyHostToDevice, in);
+        for (int64_t b0 = 0, k = 0; b0 < n && e == cudaSuccess; b0 += chunk, ++k) {
+            const int64_t rows = std::min<int64_t>(chunk, n - b0);
+            const int b = (int)(k & 1);
+            float *f = m->stage[b].as<float>();
+            if (k >= 2) e = cudaStreamWaitEvent(in, m->used[b], 0);   // the chunk two before has read the buffer
+            if (e == cudaSuccess) e = cudaMemcpyAsync(f, feats + b0 * kIn, sizeof(float) * (size_t)rows * kIn, cudaMemcpyHostToDevice, in);
+            if (in != s) {
+                if (e == cudaSuccess) e = cudaEventRecord(m->copied[b], in);
+                if (e == cudaSuccess) e = cudaStreamWaitEvent(s, m->copied[b], 0);
+            }
+            if (e != cudaSuccess) break;
+            predict(m, f, p + b0, rows, m->pred.as<float>() + b0, s);
+            if (in != s) e = cudaEventRecord(m->used[b], s);
+        }
+        if (e == cudaSuccess)
+            e = cudaMemcpyAsync(out, m->pred.ptr, sizeof(float) * (size_t)n, cudaMemcpyDeviceToHost, s);
+        if (e != cudaSuccess) {
+            cudaStreamSynchronize(m->copy);   // nothing still reads the caller's arrays
+            cudaStreamSynchronize(s);
+            return cuda_fail(e, "wk_mlp_predict");
+        }
         if ((st = check_status(m, s, "wk_mlp_predict"))) return st;
     }
     m->ctx->launches += m->kernels;
