@@ -177,6 +177,8 @@ unsigned long long *gsum_buffer(wk_ctx *ctx, int par) {
 }
 }  // namespace
 
+int wk::reserve_published(wk_ctx *ctx, int64_t words) { return reserve_gsum(ctx, (words + 1) / 2); }
+
 int wk::reserve_op_scratch(wk_ctx *ctx, int64_t rows) {
     if (!ctx || rows < 0) return set_error(WK_EINVAL, "reserve_op_scratch: bad arguments");
     if (ctx->device < 0) return WK_OK;

@@ -316,7 +316,6 @@ wk_ctx::~wk_ctx() {
     dscal.release();
     part_cnt.release();
     part_scan.release();
-    part_bound.release();
     if (h_scal) cudaFreeHost(h_scal);
     if (h_gs) cudaFreeHost(h_gs);
     for (auto &e : tev) cudaEventDestroy(e);

@@ -98,8 +98,8 @@ struct wk_ctx {
     unsigned long long pub_seq = 0;  // the last count kernel's sequence number
     wk::DevBuf dscal;                // [0] error flags, [8..32) totals
     // wk_history_partition: rows per (owner, tile) and their scan's block
-    // sums, and the parts' bounds (grown on demand, kept for the next call)
-    wk::DevBuf part_cnt, part_scan, part_bound;
+    // sums (grown on demand, kept for the next call)
+    wk::DevBuf part_cnt, part_scan;
     unsigned long long *h_scal = nullptr;   // pinned mirror of the totals
 
     // timing
@@ -137,4 +137,8 @@ int noalloc_prepare(unsigned char **scratch);
 // Reserve a context's per-op scratch (per-row degree/offset/mask, per-block
 // counts and look-back words) for steps of up to `rows` input rows.
 int reserve_op_scratch(wk_ctx *ctx, int64_t rows);
+
+// Room for `words` words from index 2 of the context's pinned, device-mapped
+// words (h_gs), in which a kernel leaves what the host reads after it.
+int reserve_published(wk_ctx *ctx, int64_t words);
 }  // namespace wk
