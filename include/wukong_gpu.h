@@ -194,7 +194,7 @@ int wk_const_to_unknown(wk_ctx *ctx, wk_history *h, int64_t start, int32_t direc
  * WK_EINVAL); *out_rows receives the output row count
  * (also when the output does not fit: WK_EOVERFLOW).  The call allocates
  * nothing: its scratch is one fixed device array inside the library (about
- * 2.1 MB), which wk_ctx_create loads on the context's device -- with the
+ * 3.2 MB), which wk_ctx_create loads on the context's device -- with the
  * kernels this call launches -- and looks up, so no call loads a module or
  * takes device memory; the array stays on that GPU until the process exits.
  * Limits: at most 262,144 input rows per call; the output is bounded by

@@ -4,21 +4,18 @@
 // probe, then streaming reads of history/adjacency and streaming writes of the
 // new table.  No tensor cores are involved.
 //
-//   k2u     : count (probe; per-row degree and edge offset; per-block output
-//             count; per-group sums of output rows and of slices, a slice
-//             being at most kSliceRows output rows of one block) -> the host
-//             adds up the group sums, sizes the output and passes the groups'
-//             prefixes -> expand (one CTA per slice: finds its block from the
-//             group prefixes and the group's block counts, the block's local
-//             scan, the slice's rows written)
-//   k2k/k2c : probe + membership (per-row ballot masks; per-block count; op
-//             total) -> filtered copy (per input block: output prefix by
-//             look-back, selected rows copied)
+//   k2u     : count (probe; per block of rows, those with a list: their first
+//             output row, list offset and row; per-block output count;
+//             per-group sums of output rows and of slices, a slice being at
+//             most kSliceRows output rows of one block) -> publish (the group
+//             sums to the host, which adds them up and sizes the output; one
+//             record per slice for the expansion) -> expand (one CTA per
+//             slice: its record, its block's entries, its rows written)
+//   k2k/k2c : probe + membership (per-row ballot masks; per-block counts;
+//             per-group sums) -> filtered copy (per input block: output prefix
+//             from the group sums and its group's counts, selected rows copied)
 //
-// The filter's look-back never waits: the first kernel of the op has written
-// every block's count before the second kernel starts, so a block finds its
-// output prefix by adding its predecessors' counts back to the nearest
-// predecessor that has already published its inclusive prefix (or to block 0).
+// A dense functional direction takes one launch for either (wk_fused.cu).
 //
 // Result order equals the reference CPU engine's (core/engine.hpp:126-225):
 // output rows follow input row order, and for k2u each input row's block of
@@ -79,20 +76,66 @@ __device__ __forceinline__ void allow_dependent_grid() { asm volatile("griddepco
 // probed, so the history read does not sit in front of every bucket read.
 constexpr int kRounds = kRowsPerBlock / (kThreads / 32) / 32;
 
-// blk_sum[b] = the block's output rows, added into its group's sums.  Err bit
-// 1 when a block's output count reaches 2^31 (the expansion keeps block-local
-// positions in 32 bits).  FUNC (a direction whose lists hold at most one
-// vertex, hashed): deg receives the neighbour itself as an int32, or -1 for no
-// match, and off is unused.  DENSE (the direction is an offsets array): a warp
-// issues the lookups of all its rounds phase by phase -- every round's start
-// vertex, then every round's offsets -- and a lane looks up its own key (no
-// shuffles).  BPC blocks per CTA: 2 for a large dense op, so each
-// warp keeps eight rounds of loads in flight and a CTA's fixed costs
-// (reduction, exit) are shared by 2048 rows; 1 otherwise, so a small op still
-// spreads over many CTAs.
+// Which of a lane's NR start vertices a direction can hold at all: a bit per
+// round.  A hashed direction with a presence bitmap answers with one 4 B read a
+// row, all rounds' reads in flight together and equal neighbours' reads merged
+// by the load unit; the run search and bucket reads of probe_warp are then only
+// for rounds that hold one (a sparse predicate's rounds rarely do).  Going
+// through probe_warp for every round took 116 instructions a round of 32 rows
+// and one read's latency after another: the count of 9M rows of 5 columns 49
+// us, 39 so.
+template <int NR>
+__device__ __forceinline__ unsigned may_hold(const PredView &pv, uint32_t dir, const int32_t (&v)[NR]) {
+    unsigned present = 0u;
+    const uint32_t *bm = dir ? pv.bm[1] : pv.bm[0];
+    if (bm != nullptr) {
+        const uint32_t bvmin = dir ? pv.bvmin[1] : pv.bvmin[0], bn = dir ? pv.bn[1] : pv.bn[0];
+        uint32_t w[NR];
+#pragma unroll
+        for (int rd = 0; rd < NR; ++rd) {
+            const uint32_t x = (uint32_t)v[rd] - bvmin;   // wraps above bn below bvmin
+            w[rd] = (v[rd] > 0 && x < bn) ? __ldg(bm + (x >> 5)) : 0u;
+        }
+#pragma unroll
+        for (int rd = 0; rd < NR; ++rd) {
+            const uint32_t x = (uint32_t)v[rd] - bvmin;
+            present |= (v[rd] == 0 ? 1u : (w[rd] >> (x & 31u)) & 1u) << rd;   // an index key: always hashed
+        }
+    } else {
+#pragma unroll
+        for (int rd = 0; rd < NR; ++rd) present |= (v[rd] >= 0 ? 1u : 0u) << rd;
+    }
+    return present;
+}
+
+// where a block's number of entries sits in its blk_sum word
+constexpr int kEntryShift = 48;
+constexpr unsigned long long kSumMask = (1ull << kEntryShift) - 1;
+
+// blk_sum[b] = the block's output rows, added into its group's sums, and from
+// bit 48 on its rows with a list.  Err bit 1 when a block's output count
+// reaches 2^31 (block-local positions are 32 bits).
+//
+// A block's rows with a list are its entries, written in order from the
+// block's first row on: pos = the entry's first output row within the block
+// (and the block's total behind the last), rel = its list offset minus pos
+// (modulo 2^32: rel + j is the list entry of output row j), row = its row in
+// the block.  The expansion's CTAs, several of them for a block with a large
+// fan-out, then copy what they need instead of scanning 1024 degrees each
+// (half of their instructions on a step of low fan-out), and rows without a
+// list -- 99% of them for a sparse predicate -- cost no traffic.
+//
+// FUNC (a direction whose lists hold at most one vertex, hashed): pos receives
+// the neighbour of every row as an int32, or -1 for no match; no entries.
+// DENSE (the direction is an offsets array): a warp issues the lookups of all
+// its rounds phase by phase -- every round's start vertex, then every round's
+// offsets -- and a lane looks up its own key (no shuffles).  BPC blocks per
+// CTA: 2 for a large dense op, so each warp keeps eight rounds of loads in
+// flight and a CTA's fixed costs (reduction, exit) are shared by 2048 rows; 1
+// otherwise, so a small op still spreads over many CTAs.
 template <bool FUNC, bool DENSE, int BPC>
 __global__ void __launch_bounds__(kThreads, 6)
-k2u_count_kernel(const int32_t *__restrict__ hist, int64_t R, int C, int scol, uint32_t dir, PredView pv, uint32_t *__restrict__ deg, uint32_t *__restrict__ off,
+k2u_count_kernel(const int32_t *__restrict__ hist, int64_t R, int C, int scol, uint32_t dir, PredView pv, Entries en,
                  unsigned long long *__restrict__ blk_sum, unsigned long long *__restrict__ group_sums, int *err,
                  unsigned long long *__restrict__ clear, int64_t nclear) {
     constexpr int NR = kRounds * BPC;   // rounds of 32 rows per warp
@@ -116,77 +159,114 @@ k2u_count_kernel(const int32_t *__restrict__ hist, int64_t R, int C, int scol, u
         v[rd] = r < R ? __ldg(hist + r * C + scol) : -1;
     }
     unsigned long long my_sum[BPC];
+    unsigned int nent[BPC], run[BPC];   // the warp's entries and output rows so far
 #pragma unroll
-    for (int j = 0; j < BPC; ++j) my_sum[j] = 0ull;
+    for (int j = 0; j < BPC; ++j) { my_sum[j] = 0ull; nent[j] = run[j] = 0u; }
+    uint32_t o[NR], d[NR];   // a row's list offset; its degree, then its first output row within the warp's
+    unsigned has = 0u;       // rounds in which the lane's row has a list
     if constexpr (DENSE) {
         const uint32_t vmin = dir ? pv.vmin[1] : pv.vmin[0], dn = dir ? pv.dn[1] : pv.dn[0];
         const uint32_t *rp = dir ? pv.rp[1] : pv.rp[0];
-        uint32_t a[NR], e[NR];
 #pragma unroll
         for (int rd = 0; rd < NR; ++rd) {
             const int32_t vid = v[rd];
-            a[rd] = e[rd] = 0u;
+            o[rd] = d[rd] = 0u;
             const uint32_t x = (uint32_t)vid - vmin;   // wraps above dn below vmin
             if (vid > 0 && x < dn) {
-                a[rd] = __ldg(rp + x);
-                e[rd] = __ldg(rp + x + 1);
+                o[rd] = __ldg(rp + x);
+                d[rd] = __ldg(rp + x + 1);
             } else if (vid == 0) {   // index key: the hash table
-                e[rd] = probe_seg(pv.buckets, pv.nmain, pv.nover, seg_key(0u, dir), &a[rd], err);
-                e[rd] += a[rd];
+                d[rd] = probe_seg(pv.buckets, pv.nmain, pv.nover, seg_key(0u, dir), &o[rd], err);
+                d[rd] += o[rd];
             }
         }
 #pragma unroll
-        for (int rd = 0; rd < NR; ++rd) {
-            const int64_t r = row_at(rd);
-            const uint32_t d = e[rd] - a[rd];
-            if (r < R) {
-                deg[r] = d;
-                off[r] = a[rd];
-                my_sum[rd / kRounds] += d;
-            }
-        }
+        for (int rd = 0; rd < NR; ++rd) d[rd] -= o[rd];   // v is -1 past the table: no list
     } else {
         // hashed: runs of equal keys probed once (probe_warp), a round at a time
+        const unsigned present = may_hold(pv, dir, v);
 #pragma unroll
         for (int rd = 0; rd < NR; ++rd) {
             const int64_t r = row_at(rd);
-            if (r - lane >= R) break;   // warp-uniform
-            uint32_t o, d;
-            probe_warp(pv, v[rd], dir, o, d, err);
-            if (r < R) {
-                if constexpr (FUNC) {
-                    reinterpret_cast<int32_t *>(deg)[r] = d ? __ldg(pv.edges + o) : -1;
-                    if (d > 1u) atomicOr(err, 8);   // an index list: the op reruns unspecialised
-                    // at most one output row per input row, so a block's output never
-                    // exceeds its rows even before the rerun
-                    my_sum[rd / kRounds] += d ? 1u : 0u;
-                } else {
-                    deg[r] = d;
-                    off[r] = o;
-                    my_sum[rd / kRounds] += d;
+            o[rd] = d[rd] = 0u;
+            const bool here = (present >> rd) & 1u;
+            if (__any_sync(FULL, here)) probe_warp(pv, here ? v[rd] : -1, dir, o[rd], d[rd], err);
+            if constexpr (FUNC) {
+                if (r < R) reinterpret_cast<int32_t *>(en.pos)[r] = d[rd] ? __ldg(pv.edges + o[rd]) : -1;
+                if (d[rd] > 1u) atomicOr(err, 8);   // an index list: the op reruns unspecialised
+                // at most one output row per input row, so a block's output never
+                // exceeds its rows even before the rerun
+                my_sum[rd / kRounds] += d[rd] ? 1u : 0u;
+            }
+        }
+    }
+    if constexpr (!FUNC) {
+#pragma unroll
+        for (int rd = 0; rd < NR; ++rd) {
+            const int j = rd / kRounds;
+            const unsigned m = __ballot_sync(FULL, d[rd] != 0u);
+            if (d[rd] != 0u) has |= 1u << rd;
+            my_sum[j] += d[rd];
+            nent[j] += (unsigned)__popc(m);
+            if (m) {   // the same in every lane
+                uint32_t in = d[rd];
+#pragma unroll
+                for (int sh = 1; sh < 32; sh <<= 1) {
+                    const uint32_t x = __shfl_up_sync(FULL, in, sh);
+                    if (lane >= sh) in += x;
                 }
+                d[rd] = run[j] + in - d[rd];
+                run[j] += __shfl_sync(FULL, in, 31);
             }
         }
     }
     // each block's output rows: a warp reduction (one REDUX instruction while the
     // partial sums are small, as every valid block's are) and one barrier
     __shared__ unsigned long long s_part[BPC][kThreads / 32];
+    __shared__ unsigned int s_ent[BPC][kThreads / 32];
 #pragma unroll
     for (int j = 0; j < BPC; ++j) {
         unsigned long long ws;
         if (!__any_sync(FULL, my_sum[j] >= (1ull << 26))) ws = __reduce_add_sync(FULL, (unsigned int)my_sum[j]);
         else ws = warp_sum(my_sum[j]);
-        if (lane == 0) s_part[j][warp] = ws;
+        if (lane == 0) { s_part[j][warp] = ws; s_ent[j][warp] = nent[j]; }
     }
     __syncthreads();
+    if constexpr (!FUNC) {
+#pragma unroll
+        for (int j = 0; j < BPC; ++j) {
+            if (nent[j] == 0u) continue;   // the same in every lane
+            unsigned int at = 0u, base = 0u;
+            for (int w = 0; w < warp; ++w) {
+                at += s_ent[j][w];
+                base += (unsigned int)s_part[j][w];
+            }
+            const int64_t first = (b0 + j) * kRowsPerBlock;
+#pragma unroll
+            for (int q = 0; q < kRounds; ++q) {
+                const int rd = j * kRounds + q;
+                const bool mine = (has >> rd) & 1u;
+                const unsigned m = __ballot_sync(FULL, mine);
+                if (mine) {
+                    const int64_t k = first + at + (unsigned)__popc(m & ((1u << lane) - 1u));
+                    en.pos[k] = base + d[rd];
+                    en.rel[k] = o[rd] - (base + d[rd]);
+                    en.row[k] = (uint16_t)(warp * (kRounds * 32) + q * 32 + lane);
+                }
+                at += (unsigned)__popc(m);
+            }
+        }
+    }
     if (threadIdx.x < BPC) {
         const int j = threadIdx.x;
         const int64_t b = b0 + j;
         unsigned long long sum = 0ull;
+        unsigned int n = 0u;
 #pragma unroll
-        for (int w = 0; w < kThreads / 32; ++w) sum += s_part[j][w];
+        for (int w = 0; w < kThreads / 32; ++w) { sum += s_part[j][w]; n += s_ent[j][w]; }
         if (b < nblk) {
-            blk_sum[b] = sum;
+            if (!FUNC && n < kRowsPerBlock) en.pos[b * kRowsPerBlock + n] = (uint32_t)sum;
+            blk_sum[b] = sum | (unsigned long long)n << kEntryShift;   // a sum past 2^31 is an error
             // group sums spread the atomics over many addresses (256 blocks each);
             // the host adds them up for the op totals, so no address takes one per block
             if (sum) {
@@ -199,22 +279,10 @@ k2u_count_kernel(const int32_t *__restrict__ hist, int64_t R, int C, int scol, u
     }
 }
 
-// One CTA, stream-ordered behind a count kernel: copies the op's error word
-// and group sums into pinned host memory, fences them system-wide, then writes
-// the sequence number the host waits for.
-__global__ void __launch_bounds__(kThreads) publish_kernel(const Publish pub) {
-    wait_prior_grid();   // the count kernel's sums are complete
-    for (long long w = threadIdx.x; w < pub.n; w += blockDim.x) pub.dst[2 + w] = __ldcg(pub.src + w);
-    __threadfence_system();
-    __syncthreads();
-    if (threadIdx.x == 0) *(volatile unsigned long long *)pub.dst = pub.seq;
-}
+// ------------------------------------------------- publish, slice records
+static_assert(kThreads == (1 << kGroupShift), "one thread per block of a group");
 
-// ------------------------------------------------------- k2u slice location
-static_assert(kThreads == (1 << kGroupShift), "one thread per group and per block of a group");
-
-// inclusive scan of (x, y) pairs over the CTA's threads; sw is free again
-// after the caller's next barrier
+// inclusive scan of (x, y) pairs over the CTA's threads
 __device__ __forceinline__ void cta_scan2(unsigned long long &x, unsigned long long &y,
                                           unsigned long long (&sw)[2][kThreads / 32]) {
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -230,88 +298,76 @@ __device__ __forceinline__ void cta_scan2(unsigned long long &x, unsigned long l
         if (w < wid) { x += sw[0][w]; y += sw[1][w]; }
 }
 
-struct SliceLoc {
-    int64_t b;              // the input block
-    unsigned long long P;   // output rows of the blocks before it
-    uint32_t T;             // its output rows
-    uint32_t slice;         // the slice's index within the block
-};
-
-// Where expansion CTA k works: the group whose slices cover k, then the
-// block within it (a scan of the group's 256 block counts).  The group comes
-// from the host's table when the op has one (a uniform binary search, every
-// read a broadcast from the parameter bank), else from a scan of the count
-// kernel's group sums, 256 groups per pass.  Every non-empty block has
-// slices_of(count) slices, in block order.  b is -1 if k is not below the
-// op's slice total.
-__device__ __forceinline__ SliceLoc locate_slice(unsigned long long k, const unsigned long long *__restrict__ blk_sum,
-                                                 const unsigned long long *__restrict__ group_sums, int64_t ngroups,
-                                                 int64_t nblk, const GroupTable &gt) {
-    __shared__ unsigned long long sw[2][kThreads / 32];
-    __shared__ unsigned long long s_tot[2];
-    __shared__ int64_t s_g;
-    __shared__ SliceLoc s_loc;
-    const int t = threadIdx.x;
-    SliceLoc none;
-    none.b = -1;
-    if (t == 0) s_loc.b = -1;
-    int64_t g;
-    unsigned long long opg, spg;
-    if (gt.n > 0) {
-        if (k >= gt.sl[gt.n]) return none;   // the same in every thread
-        int lo = 0, hi = gt.n - 1;
+// The records of the slices of group g, of those in [first, first + cap): the
+// slices are numbered in block order over the op, a block of count output rows
+// having slices_of(count) of them.
+__device__ __forceinline__ void plan_group(const SlicePlan &a, int64_t g) {
+    __shared__ unsigned long long sw[2][kThreads / 32], s_before[2][kThreads / 32];
+    __shared__ unsigned long long s_x[kThreads], s_word[kThreads];
+    __shared__ uint32_t s_y[kThreads + 1];   // a group has fewer than 2^32 slices
+    const int t = threadIdx.x, lane = t & 31, wid = t >> 5;
+    // output rows and slices of the groups before
+    unsigned long long op = 0ull, sp = 0ull;
+    for (int64_t i = t; i < g; i += kThreads) {
+        op += __ldcg(a.group_sums + 2 * i);
+        sp += __ldcg(a.group_sums + 2 * i + 1);
+    }
+    op = warp_sum(op);
+    sp = warp_sum(sp);
+    if (lane == 0) { s_before[0][wid] = op; s_before[1][wid] = sp; }
+    const int64_t bi = (g << kGroupShift) + t;
+    const unsigned long long word = bi < a.nblk ? a.blk_sum[bi] : 0ull;
+    unsigned long long x = word & kSumMask, y = slices_of(word & kSumMask);
+    const unsigned long long x0 = x, y0 = y;
+    cta_scan2(x, y, sw);
+    s_x[t] = x - x0;
+    s_y[t] = (uint32_t)(y - y0);
+    s_word[t] = word;
+    if (t == kThreads - 1) s_y[kThreads] = (uint32_t)y;
+    __syncthreads();
+    op = sp = 0ull;
+#pragma unroll
+    for (int w = 0; w < kThreads / 32; ++w) { op += s_before[0][w]; sp += s_before[1][w]; }
+    const unsigned long long last = a.first + a.cap;   // the group's slices of the window
+    const uint32_t i0 = a.first > sp ? (uint32_t)min(a.first - sp, (unsigned long long)s_y[kThreads]) : 0u;
+    const uint32_t i1 = last > sp ? (uint32_t)min(last - sp, (unsigned long long)s_y[kThreads]) : 0u;
+    for (uint32_t i = i0 + t; i < i1; i += kThreads) {
+        const unsigned long long k = sp + i;
+        int lo = 0, hi = kThreads - 1;   // the last block whose slices begin at or before i
         while (lo < hi) {
             const int mid = (lo + hi + 1) >> 1;
-            if (gt.sl[mid] <= k) lo = mid;
+            if (s_y[mid] <= i) lo = mid;
             else hi = mid - 1;
         }
-        g = lo;
-        opg = gt.out[lo];
-        spg = gt.sl[lo];
-    } else {
-        unsigned long long op = 0ull, sp = 0ull;   // sums of the groups before the pass
-        for (int64_t g0 = 0;; g0 += kThreads) {
-            const int64_t gi = g0 + t;
-            const unsigned long long x0 = gi < ngroups ? group_sums[2 * gi] : 0ull;
-            const unsigned long long y0 = gi < ngroups ? group_sums[2 * gi + 1] : 0ull;
-            unsigned long long x = x0, y = y0;
-            cta_scan2(x, y, sw);
-            if (t == kThreads - 1) { s_tot[0] = x; s_tot[1] = y; }
-            // the groups that end at or before slice k are a prefix of the pass
-            const int before = __syncthreads_count(gi < ngroups && sp + y <= k);
-            if (before < kThreads) {
-                if (t == before) {
-                    s_tot[0] = op + x - x0;
-                    s_tot[1] = sp + y - y0;
-                    s_g = gi < ngroups ? gi : -1;
-                }
-                __syncthreads();
-                break;
-            }
-            op += s_tot[0];
-            sp += s_tot[1];
-            __syncthreads();   // s_tot and sw are written again by the next pass
-        }
-        g = s_g;
-        if (g < 0) return none;   // the same in every thread
-        opg = s_tot[0];
-        spg = s_tot[1];
+        SliceRec r;
+        r.P = op + s_x[lo];
+        r.block = (uint32_t)((g << kGroupShift) + lo);
+        r.T = (uint32_t)(s_word[lo] & kSumMask);   // below 2^31 (the count kernel flags larger blocks)
+        r.slice = i - s_y[lo];
+        r.n = (uint32_t)(s_word[lo] >> kEntryShift);
+        r.pad[0] = r.pad[1] = 0u;
+        uint4 *dst = reinterpret_cast<uint4 *>(a.slices + (k - a.first));
+        const uint4 *src = reinterpret_cast<const uint4 *>(&r);
+        dst[0] = src[0];
+        dst[1] = src[1];
     }
-    const unsigned long long kk = k - spg;
-    const int64_t bi = (g << kGroupShift) + t;
-    const unsigned long long x0 = bi < nblk ? blk_sum[bi] : 0ull;
-    const unsigned long long y0 = slices_of(x0);
-    unsigned long long x = x0, y = y0;
-    cta_scan2(x, y, sw);
-    const int before = __syncthreads_count(bi < nblk && y <= kk);
-    if (t == before && bi < nblk) {
-        s_loc.b = bi;
-        s_loc.P = opg + x - x0;
-        s_loc.T = (uint32_t)x0;   // below 2^31 (the count kernel flags larger blocks)
-        s_loc.slice = (uint32_t)(kk - (y - y0));
+}
+
+// Stream-ordered behind a count kernel.  CTA 0 copies the op's error word and
+// group sums into pinned host memory, fences them system-wide, then writes the
+// sequence number the host waits for; CTA 1 + g writes the slice records of
+// group g, while the host adds up the sums and launches the expansion.
+__global__ void __launch_bounds__(kThreads) publish_kernel(const Publish pub, const SlicePlan plan) {
+    wait_prior_grid();   // the count kernel's sums are complete
+    if (blockIdx.x > 0) {
+        plan_group(plan, (int64_t)blockIdx.x - 1);
+        return;
     }
+    if (pub.dst == nullptr) return;
+    for (long long w = threadIdx.x; w < pub.n; w += blockDim.x) pub.dst[2 + w] = __ldcg(pub.src + w);
+    __threadfence_system();
     __syncthreads();
-    return s_loc;
+    if (threadIdx.x == 0) *(volatile unsigned long long *)pub.dst = pub.seq;
 }
 
 // -------------------------------------------------------------- k2u expand
@@ -327,16 +383,14 @@ __device__ __forceinline__ int row_of(const uint32_t *pos, int n, uint32_t j) {
     return lo;
 }
 
-// The block's input rows whose list is not empty, compacted in order:
-// entry k is block row row[k], its first output row pos[k] (block-local), its
-// list offset minus pos[k] in erel[k] (modulo 2^32: erel + j is the entry
-// index of output row j), and pos[n] = the block's total.  A sparse direction
-// leaves most rows empty, so searches and walks over the entries skip them.
+// The block's entries as the count kernel left them: entry k is block row
+// row[k], its first output row pos[k] (block-local), its list offset minus
+// pos[k] in erel[k] (modulo 2^32: erel + j is the entry index of output row
+// j), and pos[n] = the block's total.
 struct ExpandRows {
-    uint32_t pos[kRowsPerBlock + 1];
-    uint32_t erel[kRowsPerBlock];
-    uint16_t row[kRowsPerBlock];
-    int n;
+    alignas(16) uint32_t pos[kRowsPerBlock + 4];
+    alignas(16) uint32_t erel[kRowsPerBlock];
+    alignas(16) uint16_t row[kRowsPerBlock];
 };
 
 // The entry of each of 32 consecutive output rows, one per lane: k0 covers the
@@ -371,6 +425,22 @@ __device__ __forceinline__ void stage_row(int32_t *dst, const int32_t (&v)[W]) {
     }
 }
 
+// Shared memory to global by the copy engine (both 16 B aligned, bytes a
+// multiple of 16), in a group of the calling thread's own; and the wait until
+// its copies have read their source.
+__device__ __forceinline__ void bulk_store(int32_t *dst, const int32_t *src, uint32_t bytes) {
+    asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;\n\tcp.async.bulk.commit_group;" ::"l"(dst),
+                 "r"((uint32_t)__cvta_generic_to_shared(src)), "r"(bytes)
+                 : "memory");
+}
+__device__ __forceinline__ void bulk_read_done() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
+
+// 16 B from global to shared memory without registers
+__device__ __forceinline__ void copy16(void *dst, const void *src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
+                 : "memory");
+}
+
 constexpr int kChunk = 64;   // output rows a warp stages at a time: two windows
 
 // Output rows [u, u + kChunk) of a warp, W = 2..8 columns.  Rows are counted
@@ -393,36 +463,43 @@ __device__ __forceinline__ void write_chunk(uint32_t u, uint32_t lead, uint32_t 
                                             const int32_t *__restrict__ edges, int32_t *__restrict__ obase,
                                             int32_t *stg, int lane) {
     constexpr int C = W - 1, kWin = kChunk / 32;
+    const bool whole = u >= lo && u + kChunk <= hi;   // the same in every lane
     int32_t v[kWin][W];
+    auto gather = [&](int q, int k) {
+        const int32_t *src = rows + (int)xr.row[k] * C;
 #pragma unroll
-    for (int q = 0; q < kWin; ++q) {
-        const uint32_t j = u + 32u * q - lead, uq = u + 32u * q + (uint32_t)lane;
-        int k = window_entries(xr, n, j, lane, k0);
-        if (uq >= lo && uq < hi) {
-            const int32_t *src = rows + (int)xr.row[k] * C;
+        for (int c = 0; c < C; ++c) v[q][c] = __ldg(src + c);
+        v[q][C] = __ldg(edges + (xr.erel[k] + (u + 32u * q - lead) + (uint32_t)lane));
+    };
+    if (whole) {
 #pragma unroll
-            for (int c = 0; c < C; ++c) v[q][c] = __ldg(src + c);
-            v[q][C] = __ldg(edges + (xr.erel[k] + (uq - lead)));
-        } else {
+        for (int q = 0; q < kWin; ++q) gather(q, window_entries(xr, n, u + 32u * q - lead, lane, k0));
+    } else {
 #pragma unroll
-            for (int c = 0; c < W; ++c) v[q][c] = 0;
+        for (int q = 0; q < kWin; ++q) {
+            const uint32_t uq = u + 32u * q + (uint32_t)lane;
+            const int k = window_entries(xr, n, u + 32u * q - lead, lane, k0);
+            if (uq >= lo && uq < hi) gather(q, k);
         }
     }
+    // the chunk before has left the staging area (lane 0 issued its copy); the
+    // wait comes after this chunk's loads
+    if (lane == 0) bulk_read_done();
+    __syncwarp();
 #pragma unroll
     for (int q = 0; q < kWin; ++q) stage_row<W>(stg + (q * 32 + lane) * W, v[q]);
-    __syncwarp();
     int32_t *g = obase + (size_t)u * W;
-    if (u >= lo && u + kChunk <= hi) {
-#pragma unroll
-        for (int i = 0; i < kChunk * W / 4; i += 32)
-            if (i + lane < kChunk * W / 4)
-                reinterpret_cast<int4 *>(g)[i + lane] = reinterpret_cast<const int4 *>(stg)[i + lane];
+    if (whole) {
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) bulk_store(g, stg, kChunk * W * 4);
     } else {
+        __syncwarp();
         const int w0 = lo > u ? (int)(lo - u) * W : 0;
         const int w1 = (hi > u ? (hi - u < (uint32_t)kChunk ? (int)(hi - u) : kChunk) : 0) * W;
         for (int i = w0 + lane; i < w1; i += 32) g[i] = stg[i];
+        __syncwarp();   // the staging area is written again by the next chunk
     }
-    __syncwarp();   // the staging area is written again by the next chunk
 }
 
 // As write_chunk for one window of 32 output rows of any width, without
@@ -475,89 +552,117 @@ __device__ __forceinline__ void write_window_any(uint32_t u, uint32_t lead, uint
     }
 }
 
-// One CTA per slice: CTA k writes local rows [k' kSliceRows, (k' + 1)
-// kSliceRows) of block b, where block b's slices are numbered from s_b (the
-// slices of the blocks before it) and k' = k - s_b; locate_slice finds b, s_b
-// and the block's output prefix.  W = C + 1 output columns for
-// 2 <= W <= 8; W = 0 for any width.  Each warp takes a contiguous run of the
-// slice's chunks, so it searches for its first entry once and walks on from
-// there.  History rows are read through L1 (consecutive output rows of one
-// input row reuse it).
+// As write_chunk for one window of 32 output rows of C + 1 columns, 9 to
+// kMaxStaged: the lane's row goes to shared memory word by word, starting at
+// column lane of an even pitch (an odd pitch needs no turn), so that the 32
+// lanes' words fall in different banks.  The expansion of 800k -> 1.66M rows of 11
+// columns took 41.4 us with write_window_any (ten instructions a word), 26.8 us
+// so; both with cold caches.
+__device__ __forceinline__ void write_window_staged(uint32_t u, uint32_t lead, uint32_t lo, uint32_t hi, int C,
+                                                    const ExpandRows &xr, int n, int &k0,
+                                                    const int32_t *__restrict__ rows,
+                                                    const int32_t *__restrict__ edges, int32_t *__restrict__ obase,
+                                                    int32_t *stg, int lane) {
+    const int W = C + 1;
+    const uint32_t uq = u + (uint32_t)lane;
+    const bool whole = u >= lo && u + 32u <= hi;   // the same in every lane
+    const int k = window_entries(xr, n, u - lead, lane, k0);
+    if (lane == 0) bulk_read_done();   // the window before has left the staging area
+    __syncwarp();
+    if (uq >= lo && uq < hi) {
+        const int32_t *src = rows + (int)xr.row[k] * C;
+        int32_t *dst = stg + lane * W;
+        const int32_t nb = __ldg(edges + (xr.erel[k] + (uq - lead)));
+        int c = W % 2 == 0 ? lane % C : 0;
+        int i = 0;
+        for (; i + 4 <= C; i += 4) {
+            int32_t v[4];
+            int at[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                at[q] = c;
+                v[q] = __ldg(src + c);
+                c = c + 1 < C ? c + 1 : 0;
+            }
+#pragma unroll
+            for (int q = 0; q < 4; ++q) dst[at[q]] = v[q];
+        }
+        for (; i < C; ++i) {
+            dst[c] = __ldg(src + c);
+            c = c + 1 < C ? c + 1 : 0;
+        }
+        dst[C] = nb;
+    }
+    int32_t *g = obase + (size_t)u * W;
+    if (whole) {
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) bulk_store(g, stg, 32u * (uint32_t)W * 4u);
+    } else {
+        __syncwarp();
+        const int w0 = lo > u ? (int)(lo - u) * W : 0;
+        const int w1 = (hi > u ? (hi - u < 32u ? (int)(hi - u) : 32) : 0) * W;
+        for (int i = w0 + lane; i < w1; i += 32) g[i] = stg[i];
+        __syncwarp();
+    }
+}
+
+// One CTA per slice: CTA k of the launch takes slice record k and writes local
+// rows [slice kSliceRows, (slice + 1) kSliceRows) of its block.  W = C + 1
+// output columns for 2 <= W <= 8; kStaged for 9 to kMaxStaged (32 W words of
+// dynamic shared memory a warp); 0 for any width.  The CTA's chain before
+// its first row is the record, the block's entries (copied asynchronously) and
+// one barrier; finding the block by a scan of its group's counts and scanning
+// the block's degrees there was two thirds of its instructions on steps of low
+// fan-out.  Each warp takes a contiguous run of the slice's chunks, so it
+// searches for its first entry once and walks on from there.  History rows are
+// read through L1 (consecutive output rows of one input row reuse it).
+//
+// On 9M -> 18.6M rows of 6 columns the expansion took 112 us with the scans,
+// 86 us from records (627 MB in and out: 7.3 TB/s), which bounds it by memory;
+// the whole op 159 us before, 129 us after.
+//
+// NT = 128 when the slices are many and mostly full (wide_slices): more and
+// smaller CTAs even out the last wave.  Those CTAs, 15 an SM, take nearly all
+// of an SM's shared memory, and a grid that starts on an SM before they have
+// left it would keep their small L1 for all of its run (a functional step
+// behind one took 165 us more): they don't let it start early.
+//
 // CTAs per SM the register budget is set for: the widest instantiations need
 // more registers to avoid spills
-template <int W>
-constexpr int expand_min_ctas() { return W <= 6 ? 8 : 6; }
+constexpr int kStaged = 1, kMaxStaged = 32;
+template <int W, int NT>
+constexpr int expand_min_ctas() { return (W <= 6 ? 8 : 6) * (kThreads / NT); }
 
-template <int W>
-__global__ void __launch_bounds__(kThreads, expand_min_ctas<W>())
-k2u_expand_kernel(const int32_t *__restrict__ hist, int64_t R, int C_rt, const int32_t *__restrict__ edges,
-                  const uint32_t *__restrict__ deg, const uint32_t *__restrict__ off,
-                  const unsigned long long *__restrict__ blk_sum, const unsigned long long *__restrict__ group_sums,
-                  int64_t ngroups, int64_t nblk, const __grid_constant__ GroupTable gt, int32_t *__restrict__ out) {
-    constexpr int kRPT = kRowsPerBlock / kThreads;
-    static_assert(kRPT == 4, "4 input rows per thread");
+template <int W, int NT>
+__global__ void __launch_bounds__(NT, expand_min_ctas<W, NT>())
+k2u_expand_kernel(const int32_t *__restrict__ hist, int C_rt, const int32_t *__restrict__ edges, const Entries en,
+                  const SliceRec *__restrict__ slices, int32_t *__restrict__ out) {
+    constexpr int kWarps = NT / 32;
     __shared__ ExpandRows xr;
-    __shared__ uint32_t s_w[2][kThreads / 32];
-    __shared__ __align__(16) int32_t stage[W >= 2 ? (kThreads / 32) * kChunk * W : 1];
+    __shared__ __align__(16) int32_t stage[W >= 2 ? kWarps * kChunk * W : 4];
+    extern __shared__ __align__(16) int32_t stage_any[];   // kStaged
     const int C = W >= 2 ? W - 1 : C_rt;
     const int t = threadIdx.x, lane = t & 31, wid = t >> 5;
-    allow_dependent_grid();
+    if constexpr (NT == kThreads) allow_dependent_grid();   // see above
 
-    // 1. the slice's block, the block's output prefix and count
-    const SliceLoc loc = locate_slice(blockIdx.x, blk_sum, group_sums, ngroups, nblk, gt);
-    if (loc.b < 0) return;   // the same in every thread
-    const int64_t b = loc.b;
-    const uint32_t slice = loc.slice;
-    const int64_t r0 = b * kRowsPerBlock;
-    const int n = (int)((R - r0) < kRowsPerBlock ? (R - r0) : kRowsPerBlock);
+    // 1. the slice
+    const uint4 ra = __ldg(reinterpret_cast<const uint4 *>(slices + blockIdx.x));
+    const uint4 rb = __ldg(reinterpret_cast<const uint4 *>(slices + blockIdx.x) + 1);
+    const unsigned long long P = (unsigned long long)ra.y << 32 | ra.x;   // SliceRec: P, block, T | slice, n
+    const uint32_t T = ra.w, slice = rb.x;
+    const int n = (int)rb.y;
+    const int64_t r0 = (int64_t)ra.z * kRowsPerBlock;
 
-    // 2. the block's degrees and edge offsets, 4 rows per thread; local
-    //    exclusive scans of the degrees and of the non-empty rows
-    const int q0 = t * kRPT;
-    uint32_t d[kRPT], o[kRPT];
-    if (q0 + kRPT <= n) {
-        const uint4 dv = *reinterpret_cast<const uint4 *>(deg + r0 + q0);
-        const uint4 ov = *reinterpret_cast<const uint4 *>(off + r0 + q0);
-        d[0] = dv.x; d[1] = dv.y; d[2] = dv.z; d[3] = dv.w;
-        o[0] = ov.x; o[1] = ov.y; o[2] = ov.z; o[3] = ov.w;
-    } else {
-#pragma unroll
-        for (int q = 0; q < kRPT; ++q) {
-            d[q] = q0 + q < n ? deg[r0 + q0 + q] : 0u;
-            o[q] = q0 + q < n ? off[r0 + q0 + q] : 0u;
-        }
+    // 2. its block's entries, with the total behind the last
+    for (int i = t; i < min(n / 4 + 1, kRowsPerBlock / 4); i += NT) {
+        copy16(xr.pos + 4 * i, en.pos + r0 + 4 * i);
+        if (4 * i < n) copy16(xr.erel + 4 * i, en.rel + r0 + 4 * i);
+        if (i % 2 == 0 && 4 * i < n) copy16(xr.row + 4 * i, en.row + r0 + 4 * i);
     }
-    const uint32_t ls = d[0] + d[1] + d[2] + d[3];
-    const uint32_t lc = (d[0] != 0u) + (d[1] != 0u) + (d[2] != 0u) + (d[3] != 0u);
-    uint32_t is = ls, ic = lc;
-#pragma unroll
-    for (int sh = 1; sh < 32; sh <<= 1) {
-        const uint32_t x = __shfl_up_sync(FULL, is, sh), y = __shfl_up_sync(FULL, ic, sh);
-        if (lane >= sh) { is += x; ic += y; }
-    }
-    if (lane == 31) { s_w[0][wid] = is; s_w[1][wid] = ic; }
+    if (t == 0 && n == kRowsPerBlock) xr.pos[n] = T;
+    asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
-    uint32_t e = is - ls, kk = ic - lc;
-#pragma unroll
-    for (int w = 0; w < kThreads / 32; ++w)
-        if (w < wid) { e += s_w[0][w]; kk += s_w[1][w]; }
-#pragma unroll
-    for (int q = 0; q < kRPT; ++q) {
-        if (d[q]) {
-            xr.pos[kk] = e;
-            xr.erel[kk] = o[q] - e;   // modulo 2^32: erel + j is the entry's index
-            xr.row[kk] = (uint16_t)(q0 + q);
-            ++kk;
-            e += d[q];
-        }
-    }
-    if (t == kThreads - 1) {   // the block's totals; rows >= n have no list
-        xr.pos[kk] = e;
-        xr.n = (int)kk;
-    }
-    __syncthreads();
-    const unsigned long long P = loc.P;
-    const uint32_t T = loc.T;
     const int32_t *hblk = hist + r0 * C;
 
     // 3. the slice's share of output rows [P, P + T): a run of chunks per warp
@@ -566,18 +671,21 @@ k2u_expand_kernel(const int32_t *__restrict__ hist, int64_t R, int C_rt, const i
     const uint32_t u0 = slice * (uint32_t)kSliceRows;
     const uint32_t u1 = u0 >= span ? u0 : (span - u0 < (uint32_t)kSliceRows ? span : u0 + (uint32_t)kSliceRows);
     const uint32_t lo = u0 > lead ? u0 : lead;
-    const uint32_t per = ((u1 - u0 + kStep - 1) / kStep + kThreads / 32 - 1) / (kThreads / 32) * kStep;
+    const uint32_t per = ((u1 - u0 + kStep - 1) / kStep + kWarps - 1) / kWarps * kStep;
     uint32_t u = u0 + (uint32_t)wid * per;
     const uint32_t ue = u < u1 ? (u1 - u < per ? u1 : u + per) : u;
     if (u >= ue) return;   // the same in every lane
     int32_t *obase = out + ((int64_t)P - lead) * (C + 1);
-    int k0 = row_of(xr.pos, xr.n, u >= lead ? u - lead : 0u);
+    int k0 = row_of(xr.pos, n, u >= lead ? u - lead : 0u);
     for (; u < ue; u += kStep) {
         if constexpr (W >= 2)
-            write_chunk<W>(u, lead, lo, u1, xr, xr.n, k0, hblk, edges, obase, stage + wid * (kChunk * W), lane);
+            write_chunk<W>(u, lead, lo, u1, xr, n, k0, hblk, edges, obase, stage + wid * (kChunk * W), lane);
+        else if constexpr (W == kStaged)
+            write_window_staged(u, lead, lo, u1, C, xr, n, k0, hblk, edges, obase, stage_any + wid * 32 * (C + 1), lane);
         else
-            write_window_any(u, lead, lo, u1, C, xr, xr.n, k0, hblk, edges, obase, lane);
+            write_window_any(u, lead, lo, u1, C, xr, n, k0, hblk, edges, obase, lane);
     }
+    if (W != 0 && lane == 0) bulk_read_done();   // the staging area goes with the CTA
 }
 
 // ------------------------------------------------- k2u expand, functional
@@ -592,9 +700,7 @@ k2u_expand_kernel(const int32_t *__restrict__ hist, int64_t R, int C_rt, const i
 template <int W>
 __global__ void __launch_bounds__(kThreads)
 k2u_expand_func_kernel(const int32_t *__restrict__ hist, int64_t R, const int32_t *__restrict__ nbr,
-                       const unsigned long long *__restrict__ blk_sum,
-                       const unsigned long long *__restrict__ group_sums, int64_t ngroups, int64_t nblk,
-                       const __grid_constant__ GroupTable gt, int32_t *__restrict__ out) {
+                       const SliceRec *__restrict__ slices, int32_t *__restrict__ out) {
     constexpr int C = W - 1;
     constexpr int kPitch = W | 1;
     __shared__ int32_t rows[kRowsPerBlock * kPitch];
@@ -603,10 +709,8 @@ k2u_expand_func_kernel(const int32_t *__restrict__ hist, int64_t R, const int32_
     allow_dependent_grid();
 
     // the block (every non-empty block has one slice)
-    const SliceLoc loc = locate_slice(blockIdx.x, blk_sum, group_sums, ngroups, nblk, gt);
-    if (loc.b < 0) return;   // the same in every thread
-    const int64_t b = loc.b;
-    const int64_t r0 = b * kRowsPerBlock;
+    const SliceRec loc = slices[blockIdx.x];
+    const int64_t r0 = (int64_t)loc.block * kRowsPerBlock;
     const int n = (int)((R - r0) < kRowsPerBlock ? (R - r0) : kRowsPerBlock);
 
     // matched rows and their block-local output positions
@@ -709,13 +813,16 @@ filter_probe_kernel(const int32_t *__restrict__ hist, int64_t R, int C, int scol
     }
     unsigned int my_nz = 0u;   // kept rows (lane 0)
     unsigned long long my_scan = 0;
+    const bool dense = (dir ? pv.rp[1] : pv.rp[0]) != nullptr;
+    const unsigned present = dense ? ~0u : may_hold(pv, dir, v);
 #pragma unroll
     for (int rd = 0; rd < kRounds; ++rd) {
         const int64_t row0 = wrow0 + rd * 32, r = row0 + lane;
         if (row0 >= R) break;   // warp-uniform
         bool found = false;
-        uint32_t o, d;
-        probe_warp(pv, v[rd], dir, o, d, err);
+        uint32_t o = 0u, d = 0u;
+        const bool here = (present >> rd) & 1u;
+        if (__any_sync(FULL, here)) probe_warp(pv, here ? v[rd] : -1, dir, o, d, err);
         if (r < R && d > 0u) {
             uint32_t sc = 0;
             found = list_contains(pv.edges + o, d, tg[rd], &sc);
@@ -836,61 +943,52 @@ static inline unsigned int nblocks_rows(int64_t R) {
     return (unsigned int)((R + kRowsPerBlock - 1) / kRowsPerBlock);
 }
 
-void launch_k2u_count(const int32_t *hist, int64_t R, int C, int scol, uint32_t dir, PredView pv, uint32_t *deg, uint32_t *off, unsigned long long *blk_sum, unsigned long long *group_sums,
-                      int *err, bool func, unsigned long long *clear, int64_t nclear, int sms, cudaStream_t st) {
+static cudaLaunchConfig_t dependent_launch(cudaLaunchAttribute *attr, unsigned int grid, cudaStream_t st) {
+    attr->id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr->val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(kThreads);
+    cfg.stream = st;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cfg;
+}
+
+void launch_k2u_count(const int32_t *hist, int64_t R, int C, int scol, uint32_t dir, PredView pv, const Entries &en,
+                      unsigned long long *blk_sum, unsigned long long *group_sums, int *err, bool func,
+                      unsigned long long *clear, int64_t nclear, int sms, cudaStream_t st) {
     const bool dense = (dir ? pv.rp[1] : pv.rp[0]) != nullptr;
     const unsigned int nb = nblocks_rows(R);
     // two blocks per CTA once the op has enough blocks to fill the GPU with half as many CTAs
     if (sms < 1) sms = 1;
     const bool pair = dense && nb >= 16u * (unsigned int)sms;
     cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t cfg = {};
-    cfg.blockDim = dim3(kThreads);
-    cfg.stream = st;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-#define WK_COUNT(F, D, B)                                                                                         \
-    do {                                                                                                         \
-        cfg.gridDim = dim3((nb + B - 1) / B);                                                                    \
-        cudaLaunchKernelEx(&cfg, k2u_count_kernel<F, D, B>, hist, R, C, scol, dir, pv, deg, off, blk_sum,         \
-                           group_sums, err, clear, nclear);                                                      \
+#define WK_COUNT(F, D, B)                                                                                       \
+    do {                                                                                                       \
+        const cudaLaunchConfig_t cfg = dependent_launch(attr, (nb + B - 1) / B, st);                           \
+        cudaLaunchKernelEx(&cfg, k2u_count_kernel<F, D, B>, hist, R, C, scol, dir, pv, en, blk_sum, group_sums, \
+                           err, clear, nclear);                                                                \
     } while (0)
-    if (func) {
-        WK_COUNT(true, false, 1);   // hashed: a dense one takes wk_fused.cu
-    } else if (dense) {
-        if (pair) WK_COUNT(false, true, 2);
-        else WK_COUNT(false, true, 1);
-    } else {
-        WK_COUNT(false, false, 1);
-    }
+    if (func) WK_COUNT(true, false, 1);   // hashed: a dense one takes wk_fused.cu
+    else if (dense && pair) WK_COUNT(false, true, 2);
+    else if (dense) WK_COUNT(false, true, 1);
+    else WK_COUNT(false, false, 1);
 #undef WK_COUNT
 }
 
-// launched so that its one CTA is in place when the count kernel finishes
-void launch_publish(const Publish &pub, cudaStream_t st) {
+// launched so that its CTAs are in place when the kernel before it finishes
+void launch_publish(const Publish &pub, const SlicePlan &plan, cudaStream_t st) {
     cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(1);
-    cfg.blockDim = dim3(kThreads);
-    cfg.stream = st;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, publish_kernel, pub);
+    const int64_t ng = plan.slices ? (plan.nblk + (1 << kGroupShift) - 1) >> kGroupShift : 0;
+    const cudaLaunchConfig_t cfg = dependent_launch(attr, (unsigned int)(1 + ng), st);
+    cudaLaunchKernelEx(&cfg, publish_kernel, pub, plan);
 }
 
-void launch_k2u_expand_func(const int32_t *hist, int64_t R, int C, const int32_t *nbr,
-                            const unsigned long long *blk_sum, const unsigned long long *group_sums,
-                            const GroupTable &gt, unsigned long long slices, int32_t *out, cudaStream_t st) {
-    if (slices == 0ull) return;
-    const int64_t nblk = (R + kRowsPerBlock - 1) / kRowsPerBlock;
-    const int64_t ng = (nblk + (1 << kGroupShift) - 1) >> kGroupShift;
-    const unsigned int g = (unsigned int)slices;
-#define WK_EXPAND_F(WC) \
-    k2u_expand_func_kernel<WC><<<g, kThreads, 0, st>>>(hist, R, nbr, blk_sum, group_sums, ng, nblk, gt, out)
+void launch_k2u_expand_func(const int32_t *hist, int64_t R, int C, const int32_t *nbr, const SliceRec *slices,
+                            unsigned int n, int32_t *out, cudaStream_t st) {
+    if (n == 0u) return;
+#define WK_EXPAND_F(WC) k2u_expand_func_kernel<WC><<<n, kThreads, 0, st>>>(hist, R, nbr, slices, out)
     switch (C + 1) {
         case 2: WK_EXPAND_F(2); break;
         case 3: WK_EXPAND_F(3); break;
@@ -903,17 +1001,28 @@ void launch_k2u_expand_func(const int32_t *hist, int64_t R, int C, const int32_t
 #undef WK_EXPAND_F
 }
 
-void launch_k2u_expand(const int32_t *hist, int64_t R, int C, const int32_t *edges, const uint32_t *deg,
-                       const uint32_t *off, const unsigned long long *blk_sum, const unsigned long long *group_sums,
-                       const GroupTable &gt, unsigned long long slices, int32_t *out, cudaStream_t st) {
-    if (slices == 0ull) return;
-    const int64_t nblk = (R + kRowsPerBlock - 1) / kRowsPerBlock;
-    const int64_t ng = (nblk + (1 << kGroupShift) - 1) >> kGroupShift;
-    const unsigned int g = (unsigned int)slices;
-#define WK_EXPAND(WC) \
-    k2u_expand_kernel<WC><<<g, kThreads, 0, st>>>(hist, R, C, edges, deg, off, blk_sum, group_sums, ng, nblk, gt, \
-                                                 out)
-    switch (C + 1) {
+// More slices than CTAs of 256 threads fit at once, half full on average or
+// more: 120k rows of fan-out 100 (1524 slices, 1.25 waves of such CTAs) take
+// 43.2 us with 128 threads a CTA and 47.7 us with 256.  On steps of low fan-out,
+// a slice per block of rows, each CTA copies more than it writes: 9M -> 18.6M
+// rows take 144 us with 128 threads and 129 us with 256.
+bool wide_slices(unsigned long long slices, unsigned long long rows_out, int sms) {
+    return slices > 8ull * (unsigned long long)(sms < 1 ? 1 : sms) && rows_out / slices >= kSliceRows / 2;
+}
+
+void launch_k2u_expand(const int32_t *hist, int C, const int32_t *edges, const Entries &en, const SliceRec *slices,
+                       unsigned int n, bool wide, int32_t *out, cudaStream_t st) {
+    if (n == 0u) return;
+    const int W = C + 1;
+    const size_t any = W > 8 && W <= kMaxStaged ? (size_t)32 * W * 4 : 0;   // per warp
+#define WK_EXPAND_T(WC, NT) \
+    k2u_expand_kernel<WC, NT><<<n, NT, any * (NT / 32), st>>>(hist, C, edges, en, slices, out)
+#define WK_EXPAND(WC)                                      \
+    do {                                                   \
+        if (wide) WK_EXPAND_T(WC, 128);                    \
+        else WK_EXPAND_T(WC, 256);                         \
+    } while (0)
+    switch (W) {
         case 2: WK_EXPAND(2); break;
         case 3: WK_EXPAND(3); break;
         case 4: WK_EXPAND(4); break;
@@ -921,9 +1030,13 @@ void launch_k2u_expand(const int32_t *hist, int64_t R, int C, const int32_t *edg
         case 6: WK_EXPAND(6); break;
         case 7: WK_EXPAND(7); break;
         case 8: WK_EXPAND(8); break;
-        default: WK_EXPAND(0); break;
+        default:
+            if (any) WK_EXPAND(kStaged);
+            else WK_EXPAND_T(0, 256);
+            break;
     }
 #undef WK_EXPAND
+#undef WK_EXPAND_T
 }
 
 // Load every k2u count and expansion kernel now (with lazy module loading a
@@ -940,14 +1053,23 @@ int preload_k2u_kernels() {
     get((const void *)k2u_count_kernel<false, true, 2>);
     get((const void *)k2u_count_kernel<true, false, 1>);
     get((const void *)publish_kernel);
-    get((const void *)k2u_expand_kernel<0>);
-    get((const void *)k2u_expand_kernel<2>);
-    get((const void *)k2u_expand_kernel<3>);
-    get((const void *)k2u_expand_kernel<4>);
-    get((const void *)k2u_expand_kernel<5>);
-    get((const void *)k2u_expand_kernel<6>);
-    get((const void *)k2u_expand_kernel<7>);
-    get((const void *)k2u_expand_kernel<8>);
+    get((const void *)k2u_expand_kernel<0, 256>);
+    get((const void *)k2u_expand_kernel<kStaged, 128>);
+    get((const void *)k2u_expand_kernel<kStaged, 256>);
+    get((const void *)k2u_expand_kernel<2, 128>);
+    get((const void *)k2u_expand_kernel<2, 256>);
+    get((const void *)k2u_expand_kernel<3, 128>);
+    get((const void *)k2u_expand_kernel<3, 256>);
+    get((const void *)k2u_expand_kernel<4, 128>);
+    get((const void *)k2u_expand_kernel<4, 256>);
+    get((const void *)k2u_expand_kernel<5, 128>);
+    get((const void *)k2u_expand_kernel<5, 256>);
+    get((const void *)k2u_expand_kernel<6, 128>);
+    get((const void *)k2u_expand_kernel<6, 256>);
+    get((const void *)k2u_expand_kernel<7, 128>);
+    get((const void *)k2u_expand_kernel<7, 256>);
+    get((const void *)k2u_expand_kernel<8, 128>);
+    get((const void *)k2u_expand_kernel<8, 256>);
     return (int)e;
 }
 

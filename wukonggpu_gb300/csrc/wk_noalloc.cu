@@ -13,7 +13,7 @@
 //   - at most kMaxRows input rows per call (262,144); a larger call is
 //     rejected with WK_EINVAL before any device work; the output is bounded
 //     only by the caller's capacity (WK_EOVERFLOW, with the row count);
-//   - the array (about 2.1 MB) is loaded on a device, and its address looked
+//   - the array (about 3.2 MB) is loaded on a device, and its address looked
 //     up, when a context is made for that device (wk_ctx_create calls
 //     noalloc_prepare), together with the kernels this entry point launches:
 //     with lazy module loading both would otherwise be loaded -- and device
@@ -26,6 +26,7 @@
 //     contexts' streams at once) race on the array and must not be issued;
 //   - a context keeps the address it looked up; it must not be used after a
 //     reset of its device.
+#include <algorithm>
 #include <cstdint>
 
 #include "wk_runtime.h"
@@ -42,7 +43,10 @@ constexpr size_t kOffFlags = 0;       // err (int, 16 B), the group's sums (outp
 constexpr size_t kOffDeg = al(kOffFlags + 32);
 constexpr size_t kOffOff = al(kOffDeg + 4 * kMaxRows);
 constexpr size_t kOffBlkSum = al(kOffOff + 4 * kMaxRows);
-constexpr size_t kScratchBytes = al(kOffBlkSum + 8 * kMaxBlocks);
+constexpr size_t kOffRow = al(kOffBlkSum + 8 * kMaxBlocks);
+constexpr size_t kOffSlices = al(kOffRow + 2 * kMaxRows);
+constexpr unsigned long long kSlices = 16384;         // slice records per round of the expansion (134M output rows)
+constexpr size_t kScratchBytes = al(kOffSlices + sizeof(wk::dev::SliceRec) * kSlices);
 
 __device__ __align__(256) unsigned char g_noalloc_scratch[kScratchBytes];
 
@@ -88,8 +92,8 @@ extern "C" int wk_known_to_unknown_noalloc(wk_ctx *ctx, const int32_t *hist, int
     if (!sc) return set_error(WK_EDEVICE, "known_to_unknown_noalloc: the context has no scratch address");
     int *err = reinterpret_cast<int *>(sc + kOffFlags);
     unsigned long long *gsum = reinterpret_cast<unsigned long long *>(sc + kOffFlags) + 2;
-    uint32_t *deg = reinterpret_cast<uint32_t *>(sc + kOffDeg);
-    uint32_t *off = reinterpret_cast<uint32_t *>(sc + kOffOff);
+    const dev::Entries en{reinterpret_cast<uint32_t *>(sc + kOffDeg), reinterpret_cast<uint32_t *>(sc + kOffOff),
+                          reinterpret_cast<uint16_t *>(sc + kOffRow)};
     unsigned long long *blk_sum = reinterpret_cast<unsigned long long *>(sc + kOffBlkSum);
 
     const PredView pv = ctx->store->views[(size_t)predict];
@@ -97,7 +101,7 @@ extern "C" int wk_known_to_unknown_noalloc(wk_ctx *ctx, const int32_t *hist, int
     cudaStream_t s = ctx->stream;
     if ((e = cudaMemsetAsync(sc + kOffFlags, 0, 32, s)) != cudaSuccess) return cuda_fail(e, "noalloc: clear flags");
     // kMaxRows input rows are one group: its two sums are the op's totals
-    dev::launch_k2u_count(hist, rows, cols, scol, (uint32_t)direction, pv, deg, off, blk_sum, gsum, err, false,
+    dev::launch_k2u_count(hist, rows, cols, scol, (uint32_t)direction, pv, en, blk_sum, gsum, err, false,
                           nullptr, 0, ctx->sms, s);
     if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(e, "noalloc: count launch");
     ctx->launches += 1;
@@ -118,17 +122,18 @@ extern "C" int wk_known_to_unknown_noalloc(wk_ctx *ctx, const int32_t *hist, int
                          "known_to_unknown_noalloc: output needs %lld rows of %lld int32 elements, capacity is %lld "
                          "(*out_rows holds the row count)",
                          (long long)R_out, (long long)width, (long long)out_capacity);
-    dev::GroupTable gt;
-    gt.n = 1;
-    gt.out[0] = 0ull;
-    gt.sl[0] = 0u;
-    gt.out[1] = ctx->h_scal[2];
-    // the slices of at most 256 blocks: each block has ceil((count + 3) / 8192)
-    // of them with count below 2^31, so fewer than 2^26 in all
-    gt.sl[1] = (unsigned int)ctx->h_scal[3];
-    dev::launch_k2u_expand(hist, rows, cols, pv.edges, deg, off, blk_sum, gsum, gt, ctx->h_scal[3], out, s);
-    if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(e, "noalloc: expand launch");
-    ctx->launches += 1;
+    const unsigned long long slices = ctx->h_scal[3];
+    const int64_t nblk = (rows + dev::kRowsPerBlock - 1) / dev::kRowsPerBlock;
+    dev::SliceRec *recs = reinterpret_cast<dev::SliceRec *>(sc + kOffSlices);
+    const bool wide = dev::wide_slices(slices, (unsigned long long)R_out, ctx->sms);
+    for (unsigned long long s0 = 0ull; s0 < slices; s0 += kSlices) {
+        const unsigned int n = (unsigned int)std::min(slices - s0, kSlices);
+        dev::launch_publish(dev::Publish{nullptr, nullptr, 0, 0ull},
+                            dev::SlicePlan{blk_sum, gsum, nblk, recs, s0, kSlices}, s);
+        dev::launch_k2u_expand(hist, cols, pv.edges, en, recs, n, wide, out, s);
+        if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(e, "noalloc: expand launch");
+        ctx->launches += 2;
+    }
     if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return cuda_fail(e, "noalloc: sync");
     return WK_OK;
 }

@@ -177,6 +177,18 @@ unsigned long long *gsum_buffer(wk_ctx *ctx, int par) {
 }
 }  // namespace
 
+// Slice records kept for an op of nblk blocks: enough for a mean fan-out of 128;
+// an op with more slices expands in rounds of that many (33M output rows at
+// least).  They lie behind the entries' offsets and rows in the context's `off`
+// buffer, and are few for a small op: as 64k records in a buffer of their own
+// they cost a new context's first light query 110 us of allocation.
+namespace {
+inline int64_t slice_records(int64_t nblk) { return 16 * nblk + 4096; }
+inline size_t off_bytes(int64_t nblk) {
+    return (size_t)nblk * dev::kRowsPerBlock * 6 + (size_t)slice_records(nblk) * sizeof(dev::SliceRec);
+}
+}
+
 int wk::reserve_published(wk_ctx *ctx, int64_t words) { return reserve_gsum(ctx, (words + 1) / 2); }
 
 int wk::reserve_op_scratch(wk_ctx *ctx, int64_t rows) {
@@ -186,7 +198,7 @@ int wk::reserve_op_scratch(wk_ctx *ctx, int64_t rows) {
     if (e != cudaSuccess) return cuda_fail(e, "cudaSetDevice");
     const int64_t nblk = (rows + dev::kRowsPerBlock - 1) / dev::kRowsPerBlock + 1;
     int st;
-    if ((st = ctx->deg.reserve((size_t)rows * 4)) || (st = ctx->off.reserve((size_t)rows * 4)) ||
+    if ((st = ctx->deg.reserve((size_t)nblk * dev::kRowsPerBlock * 4)) || (st = ctx->off.reserve(off_bytes(nblk))) ||
         (st = ctx->mask.reserve((size_t)((rows + 31) / 32) * 4)) || (st = ctx->blk_sum.reserve((size_t)nblk * 8)) ||
         (st = ctx->blk_nz.reserve((size_t)nblk * 4)) ||
         (st = reserve_gsum(ctx, (nblk + (1 << dev::kGroupShift) - 1) >> dev::kGroupShift)))
@@ -318,9 +330,16 @@ int op_k2u(wk_ctx *ctx, wk_history *h, int scol, uint32_t pid, uint32_t dir) {
     if ((st = op_fused(ctx, h, scol, -1, 0, dir, false, pv, clk, &done)) || done) return st;
     const int64_t nblk = (R + dev::kRowsPerBlock - 1) / dev::kRowsPerBlock;
     const int64_t groups = (nblk + (1 << dev::kGroupShift) - 1) >> dev::kGroupShift;
-    if ((st = take(ctx, ctx->deg, (size_t)R * 4)) || (st = take(ctx, ctx->off, (size_t)R * 4)) ||
+    const size_t whole = (size_t)nblk * dev::kRowsPerBlock;   // entries come by whole blocks
+    if ((st = take(ctx, ctx->deg, whole * 4)) || (st = take(ctx, ctx->off, off_bytes(nblk))) ||
         (st = take(ctx, ctx->blk_sum, (size_t)nblk * 8)) || (st = reserve_gsum(ctx, groups)))
         return st;
+    unsigned char *off = ctx->off.as<unsigned char>();
+    const dev::Entries en{ctx->deg.as<uint32_t>(), reinterpret_cast<uint32_t *>(off),
+                          reinterpret_cast<uint16_t *>(off + whole * 4)};
+    dev::SliceRec *recs = reinterpret_cast<dev::SliceRec *>(off + whole * 6);
+    dev::SlicePlan plan{ctx->blk_sum.as<unsigned long long>(), nullptr, nblk, recs, 0ull,
+                        (unsigned long long)slice_records(nblk)};
     // a hashed functional direction (at most one neighbour per vertex) expands as a
     // compaction; if a row hits an index list (vertex 0) the op reruns unspecialised
     bool func = pv.func[dir] != 0u && pv.nb[dir] == nullptr && C + 1 <= 8;
@@ -331,15 +350,17 @@ int op_k2u(wk_ctx *ctx, wk_history *h, int scol, uint32_t pid, uint32_t dir) {
         gs = gsum_buffer(ctx, par);
         if ((st = clk.begin())) return st;
         // the op's error flags and group sums come to the host through pinned
-        // memory (a one-CTA kernel behind the count); the host adds up the totals
+        // memory (the publish kernel behind the count, which also writes the
+        // expansion's slice records); the host adds up the totals
         const dev::Publish pub{gs, ctx->h_gs_dev, 2 + 2 * groups, ++ctx->pub_seq};
-        dev::launch_k2u_count(h->data, R, C, scol, dir, pv, ctx->deg.as<uint32_t>(), ctx->off.as<uint32_t>(),
-                              ctx->blk_sum.as<unsigned long long>(), gs + 2, reinterpret_cast<int *>(gs), func,
-                              gsum_buffer(ctx, par ^ 1), 2 + 2 * ctx->gs_used[par ^ 1], ctx->sms, ctx->stream);
+        dev::launch_k2u_count(h->data, R, C, scol, dir, pv, en, ctx->blk_sum.as<unsigned long long>(), gs + 2,
+                              reinterpret_cast<int *>(gs), func, gsum_buffer(ctx, par ^ 1),
+                              2 + 2 * ctx->gs_used[par ^ 1], ctx->sms, ctx->stream);
         if ((st = launch_check("k2u count")) || (st = clk.end(false))) return st;
         // outside the count's timing events: the op's device span counts it,
         // the count kernel's time does not
-        dev::launch_publish(pub, ctx->stream);
+        plan.group_sums = gs + 2;
+        dev::launch_publish(pub, plan, ctx->stream);
         if ((st = launch_check("k2u publish"))) return st;
         ++ctx->launches;
         ++ctx->last.kernels;
@@ -354,22 +375,10 @@ int op_k2u(wk_ctx *ctx, wk_history *h, int scol, uint32_t pid, uint32_t dir) {
     if (errf & 1)
         return set_error(WK_EDEVICE, "probe found an overflow chain longer than the segment's overflow area (corrupt store)");
     if (errf & 2) return set_error(WK_EOVERFLOW, "k2u: 1024 consecutive input rows expand to 2^31 rows or more");
-    // the op totals, and the groups' prefixes for the expansion
-    dev::GroupTable gt;
-    gt.n = groups <= dev::kTableGroups ? (int)groups : 0;
     unsigned long long rows_out = 0ull, slices = 0ull;
     for (int64_t g = 0; g < groups; ++g) {
-        if (gt.n) {
-            gt.out[g] = rows_out;
-            gt.sl[g] = (unsigned int)slices;
-        }
         rows_out += ctx->h_gs[4 + 2 * g];
         slices += ctx->h_gs[5 + 2 * g];
-    }
-    if (slices >> 32) gt.n = 0;   // not reached: a slice holds up to 8192 of the output rows
-    if (gt.n) {
-        gt.out[gt.n] = rows_out;
-        gt.sl[gt.n] = (unsigned int)slices;
     }
     const int64_t R_out = (int64_t)rows_out;
     if (R_out > ctx->row_limit)
@@ -382,13 +391,19 @@ int op_k2u(wk_ctx *ctx, wk_history *h, int scol, uint32_t pid, uint32_t dir) {
     } else {
         if ((st = take(ctx, ob, (size_t)R_out * (C + 1) * 4))) return st;
         if ((st = clk.begin())) return st;
-        if (func)
-            dev::launch_k2u_expand_func(h->data, R, C, ctx->deg.as<int32_t>(), ctx->blk_sum.as<unsigned long long>(),
-                                        gs + 2, gt, slices, ob.as<int32_t>(), ctx->stream);
-        else
-            dev::launch_k2u_expand(h->data, R, C, pv.edges, ctx->deg.as<uint32_t>(), ctx->off.as<uint32_t>(),
-                                   ctx->blk_sum.as<unsigned long long>(), gs + 2, gt, slices, ob.as<int32_t>(),
-                                   ctx->stream);
+        const bool wide = dev::wide_slices(slices, rows_out, ctx->sms);
+        for (unsigned long long s0 = 0ull;;) {
+            const unsigned int n = (unsigned int)std::min<unsigned long long>(slices - s0, plan.cap);
+            if (func)
+                dev::launch_k2u_expand_func(h->data, R, C, ctx->deg.as<int32_t>(), recs, n, ob.as<int32_t>(), ctx->stream);
+            else
+                dev::launch_k2u_expand(h->data, C, pv.edges, en, recs, n, wide, ob.as<int32_t>(), ctx->stream);
+            if ((s0 += n) >= slices) break;
+            plan.first = s0;   // the next records, behind the expansion that reads these
+            dev::launch_publish(dev::Publish{nullptr, nullptr, 0, 0ull}, plan, ctx->stream);
+            ctx->launches += 2;
+            ctx->last.kernels += 2;
+        }
         if ((st = launch_check("k2u expand")) || (st = clk.end(true))) return st;
         if (ctx->timing) {
             cudaError_t e = cudaStreamSynchronize(ctx->stream);
@@ -451,7 +466,7 @@ int op_filter(wk_ctx *ctx, wk_history *h, int scol, int ecol, int32_t end_const,
     // the error word and totals come to the host through pinned memory, as a
     // k2u op's group sums do
     const dev::Publish pub{ctx->dscal.as<unsigned long long>(), ctx->h_gs_dev, 4, ++ctx->pub_seq};
-    dev::launch_publish(pub, ctx->stream);
+    dev::launch_publish(pub, dev::SlicePlan{}, ctx->stream);
     if ((st = launch_check("filter publish"))) return st;
     ++ctx->launches;
     ++ctx->last.kernels;
