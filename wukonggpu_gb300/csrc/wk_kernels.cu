@@ -328,6 +328,11 @@ __device__ __forceinline__ void plan_group(const SlicePlan &a, int64_t g) {
     op = sp = 0ull;
 #pragma unroll
     for (int w = 0; w < kThreads / 32; ++w) { op += s_before[0][w]; sp += s_before[1][w]; }
+    if (t == 0 && a.head != nullptr && (g + 1) << kGroupShift >= a.nblk) {   // the last group
+        const unsigned long long rows = op + s_x[kThreads - 1] + (s_word[kThreads - 1] & kSumMask);
+        const unsigned long long n = sp + s_y[kThreads];
+        *a.head = *a.err == 0 && n <= a.max_slices && rows <= a.max_rows ? (uint32_t)n : 0u;
+    }
     const unsigned long long last = a.first + a.cap;   // the group's slices of the window
     const uint32_t i0 = a.first > sp ? (uint32_t)min(a.first - sp, (unsigned long long)s_y[kThreads]) : 0u;
     const uint32_t i1 = last > sp ? (uint32_t)min(last - sp, (unsigned long long)s_y[kThreads]) : 0u;
@@ -359,6 +364,8 @@ __device__ __forceinline__ void plan_group(const SlicePlan &a, int64_t g) {
 // group g, while the host adds up the sums and launches the expansion.
 __global__ void __launch_bounds__(kThreads) publish_kernel(const Publish pub, const SlicePlan plan) {
     wait_prior_grid();   // the count kernel's sums are complete
+    // no early start for an expansion behind: its CTAs would keep to the small
+    // shared memory that these leave an SM, and few at a time, for all of its run
     if (blockIdx.x > 0) {
         plan_group(plan, (int64_t)blockIdx.x - 1);
         return;
@@ -434,6 +441,13 @@ __device__ __forceinline__ void bulk_store(int32_t *dst, const int32_t *src, uin
                  : "memory");
 }
 __device__ __forceinline__ void bulk_read_done() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
+
+// 16 B that the grid before has written: after wait_prior_grid, in program order
+__device__ __forceinline__ uint4 load16(const void *p) {
+    uint4 v;
+    asm volatile("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    return v;
+}
 
 // 16 B from global to shared memory without registers
 __device__ __forceinline__ void copy16(void *dst, const void *src) {
@@ -620,7 +634,7 @@ __device__ __forceinline__ void write_window_staged(uint32_t u, uint32_t lead, u
 //
 // On 9M -> 18.6M rows of 6 columns the expansion took 112 us with the scans,
 // 86 us from records (627 MB in and out: 7.3 TB/s), which bounds it by memory;
-// the whole op 159 us before, 129 us after.
+// the whole op 159 us before, 129 us after (124.5 launched ahead of the totals).
 //
 // NT = 128 when the slices are many and mostly full (wide_slices): more and
 // smaller CTAs even out the last wave.  Those CTAs, 15 an SM, take nearly all
@@ -637,18 +651,20 @@ constexpr int expand_min_ctas() { return (W <= 6 ? 8 : 6) * (kThreads / NT); }
 template <int W, int NT>
 __global__ void __launch_bounds__(NT, expand_min_ctas<W, NT>())
 k2u_expand_kernel(const int32_t *__restrict__ hist, int C_rt, const int32_t *__restrict__ edges, const Entries en,
-                  const SliceRec *__restrict__ slices, int32_t *__restrict__ out) {
+                  const SliceRec *__restrict__ slices, const uint32_t *__restrict__ head, int32_t *__restrict__ out) {
     constexpr int kWarps = NT / 32;
     __shared__ ExpandRows xr;
     __shared__ __align__(16) int32_t stage[W >= 2 ? kWarps * kChunk * W : 4];
     extern __shared__ __align__(16) int32_t stage_any[];   // kStaged
     const int C = W >= 2 ? W - 1 : C_rt;
     const int t = threadIdx.x, lane = t & 31, wid = t >> 5;
+    wait_prior_grid();   // the records are complete
     if constexpr (NT == kThreads) allow_dependent_grid();   // see above
 
+    if (head != nullptr && blockIdx.x >= *head) return;
+
     // 1. the slice
-    const uint4 ra = __ldg(reinterpret_cast<const uint4 *>(slices + blockIdx.x));
-    const uint4 rb = __ldg(reinterpret_cast<const uint4 *>(slices + blockIdx.x) + 1);
+    const uint4 ra = load16(slices + blockIdx.x), rb = load16(reinterpret_cast<const uint4 *>(slices + blockIdx.x) + 1);
     const unsigned long long P = (unsigned long long)ra.y << 32 | ra.x;   // SliceRec: P, block, T | slice, n
     const uint32_t T = ra.w, slice = rb.x;
     const int n = (int)rb.y;
@@ -1011,12 +1027,19 @@ bool wide_slices(unsigned long long slices, unsigned long long rows_out, int sms
 }
 
 void launch_k2u_expand(const int32_t *hist, int C, const int32_t *edges, const Entries &en, const SliceRec *slices,
-                       unsigned int n, bool wide, int32_t *out, cudaStream_t st) {
+                       unsigned int n, const uint32_t *head, bool wide, int32_t *out, cudaStream_t st) {
     if (n == 0u) return;
     const int W = C + 1;
     const size_t any = W > 8 && W <= kMaxStaged ? (size_t)32 * W * 4 : 0;   // per warp
-#define WK_EXPAND_T(WC, NT) \
-    k2u_expand_kernel<WC, NT><<<n, NT, any * (NT / 32), st>>>(hist, C, edges, en, slices, out)
+    cudaLaunchAttribute attr[1];
+    cudaLaunchConfig_t cfg = dependent_launch(attr, n, st);
+    if (head == nullptr) cfg.numAttrs = 0;
+#define WK_EXPAND_T(WC, NT)                                                                                \
+    do {                                                                                                   \
+        cfg.blockDim = dim3(NT);                                                                           \
+        cfg.dynamicSmemBytes = any * (NT / 32);                                                            \
+        cudaLaunchKernelEx(&cfg, k2u_expand_kernel<WC, NT>, hist, C, edges, en, slices, head, out);        \
+    } while (0)
 #define WK_EXPAND(WC)                                      \
     do {                                                   \
         if (wide) WK_EXPAND_T(WC, 128);                    \

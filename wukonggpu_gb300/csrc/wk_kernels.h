@@ -60,12 +60,18 @@ struct Publish {
     unsigned long long seq;
 };
 // In the same launch, the records of the op's slices [first, first + cap) (a
-// CTA per group); slices null: none.
+// CTA per group); slices null: none.  head (a device word, or null) receives
+// the number of slices when an expansion launched behind may write them: the
+// count set no error, they are at most max_slices, and the output has at most
+// max_rows rows; else 0.
 struct SlicePlan {
     const unsigned long long *blk_sum, *group_sums;
     int64_t nblk;
     SliceRec *slices;
     unsigned long long first, cap;
+    uint32_t *head;
+    const int *err;
+    unsigned long long max_rows, max_slices;
 };
 void launch_publish(const Publish &pub, const SlicePlan &plan, cudaStream_t st);
 
@@ -78,12 +84,13 @@ int preload_k2u_kernels();
 // non-empty block (n slice records).
 void launch_k2u_expand_func(const int32_t *hist, int64_t R, int C, const int32_t *nbr, const SliceRec *slices,
                             unsigned int n, int32_t *out, cudaStream_t st);
-// k2u pass 2: one CTA for each of n slice records writes its rows (row ||
-// neighbour) of the block's output; out holds the op's output rows of C + 1
-// columns and is 16 B aligned; wide: what wide_slices says of the op.
+// k2u pass 2: the rows (row || neighbour) of n slice records, a CTA each; out
+// holds the op's output rows of C + 1 columns and is 16 B aligned; wide: what
+// wide_slices says of the op.  head (a device word) not null: the number of
+// slices, at most n, is read from there.
 bool wide_slices(unsigned long long slices, unsigned long long rows_out, int sms);
 void launch_k2u_expand(const int32_t *hist, int C, const int32_t *edges, const Entries &en, const SliceRec *slices,
-                       unsigned int n, bool wide, int32_t *out, cudaStream_t st);
+                       unsigned int n, const uint32_t *head, bool wide, int32_t *out, cudaStream_t st);
 
 // k2k/k2c pass 1: probe + membership of the end value; per-row ballot masks,
 // per-block kept-row counts, each added into its group's sum (group_sums[2 g],

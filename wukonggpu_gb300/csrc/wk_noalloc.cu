@@ -129,8 +129,8 @@ extern "C" int wk_known_to_unknown_noalloc(wk_ctx *ctx, const int32_t *hist, int
     for (unsigned long long s0 = 0ull; s0 < slices; s0 += kSlices) {
         const unsigned int n = (unsigned int)std::min(slices - s0, kSlices);
         dev::launch_publish(dev::Publish{nullptr, nullptr, 0, 0ull},
-                            dev::SlicePlan{blk_sum, gsum, nblk, recs, s0, kSlices}, s);
-        dev::launch_k2u_expand(hist, cols, pv.edges, en, recs, n, wide, out, s);
+                            dev::SlicePlan{blk_sum, gsum, nblk, recs, s0, kSlices, nullptr, nullptr, 0ull, 0ull}, s);
+        dev::launch_k2u_expand(hist, cols, pv.edges, en, recs, n, nullptr, wide, out, s);
         if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(e, "noalloc: expand launch");
         ctx->launches += 2;
     }
