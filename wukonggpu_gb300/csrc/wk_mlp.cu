@@ -20,6 +20,14 @@
 // product of the layer above writes dZ = dH * GELU'(Z) with the bias
 // gradient (its column sums), so dH itself is never stored.  Prediction, which
 // keeps nothing for a backward pass, is one kernel (wk_mlp_forward.cuh).
+//
+// A forward and backward pass is eight kernels, each launched ahead of its
+// turn: the input, three layers, the output layer with the loss and the first
+// backward layer, two layers back, and every weight gradient with the
+// embedding's in one.  What bounds a step of 1024 rows is the chain of those
+// launches and a product's latency (5 to 8 us, 64 CTAs).  As 16 kernels and 4
+// copies, each weight gradient in the chain, the step kept the GPU for 155 us,
+// so for 66 us.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -44,86 +52,35 @@ constexpr int kXPadN = 128;   // W1^T rows padded (dX GEMM has N = 80 -> 128)
 constexpr float kB1 = 0.9f, kB2 = 0.999f;   // Adam moment decay rates
 
 // ------------------------------------------------------------ elementwise
-// X0 [Mp x 80] bf16 = [feats | emb[pid]] for real rows, 0 for padding
-__global__ void build_input_kernel(const float *__restrict__ feats, const int32_t *__restrict__ pids, int M, int Mp,
-                                   const float *__restrict__ emb, int n_ids, __nv_bfloat16 *__restrict__ X0,
-                                   __nv_bfloat16 *__restrict__ X0t) {
-    const int64_t n = (int64_t)Mp * kX;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        const int r = (int)(i / kX), c = (int)(i % kX);
+// X0 [Mp x 80] bf16 = [feats | emb[pid]] for real rows, 0 for padding, and its
+// transpose, 32 rows a CTA; and the words that the step adds into, cleared.
+__global__ void __launch_bounds__(256)
+build_input_kernel(const float *__restrict__ feats, const int32_t *__restrict__ pids, int M, int Mp,
+                   const float *__restrict__ emb, int n_ids, __nv_bfloat16 *__restrict__ X0,
+                   __nv_bfloat16 *__restrict__ X0t, float *__restrict__ zero, int64_t nzero, int *done) {
+    __shared__ __nv_bfloat16 tile[kX][34];   // 17 words a column: the transposing reads and writes spread over the banks
+    asm volatile("griddepcontrol.launch_dependents;");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    const int r0 = blockIdx.x * 32, t = threadIdx.x;
+    for (int i = t; i < 32 * kX; i += 256) {
+        const int r = i / kX, c = i % kX, row = r0 + r;
         float v = 0.f;
-        if (r < M) {
-            if (c < kIn) v = feats[(size_t)r * kIn + c];
+        if (row < M) {
+            if (c < kIn) v = feats[(size_t)row * kIn + c];
             else {
-                int p = pids[r];
+                int p = pids[row];
                 p = p < 0 ? 0 : (p > n_ids ? n_ids : p);
                 v = emb[(size_t)p * kEmb + (c - kIn)];
             }
         }
         const __nv_bfloat16 bv = __float2bfloat16(v);
-        X0[i] = bv;
-        X0t[(size_t)c * Mp + r] = bv;
+        X0[(size_t)r0 * kX + i] = bv;
+        tile[c][r] = bv;
     }
-}
-
-// column sums of a bf16 [Mp x N] matrix into fp32 db[N] (one block per column)
-__global__ void colsum_kernel(const __nv_bfloat16 *__restrict__ Dt, int Mp, float *__restrict__ db) {
-    const int c = blockIdx.x;
-    float s = 0.f;
-    for (int r = threadIdx.x; r < Mp; r += blockDim.x) s += __bfloat162float(Dt[(size_t)c * Mp + r]);
-    __shared__ float sh[32];
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = s;
     __syncthreads();
-    if (threadIdx.x < 32) {
-        s = threadIdx.x < (blockDim.x >> 5) ? sh[threadIdx.x] : 0.f;
-        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-        if (threadIdx.x == 0) db[c] = s;
-    }
-}
-
-// loss[0] = mean((y - t)^2) over real rows, also added into loss[1] (the
-// epoch's running sum); dY (bf16, col 0, row-major and transposed) =
-// 2 (y - t) / M.  One block.
-__global__ void loss_kernel(const float *__restrict__ Y, const float *__restrict__ tgt, int M, int Mp,
-                            __nv_bfloat16 *__restrict__ dY, __nv_bfloat16 *__restrict__ dYt, float *__restrict__ loss) {
-    float s = 0.f;
-    for (int r = threadIdx.x; r < Mp; r += blockDim.x) {
-        float g = 0.f;
-        if (r < M) {
-            const float d = Y[(size_t)r * kOutPad] - tgt[r];
-            s += d * d;
-            g = 2.f * d / (float)M;
-        }
-        const __nv_bfloat16 b = __float2bfloat16(g);
-        dY[(size_t)r * kOutPad] = b;
-        dYt[r] = b;   // row 0 of dY^T
-    }
-    __shared__ float sh[32];
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = s;
-    __syncthreads();
-    if (threadIdx.x < 32) {
-        s = threadIdx.x < (blockDim.x >> 5) ? sh[threadIdx.x] : 0.f;
-        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-        if (threadIdx.x == 0) {
-            const float l = s / (float)(M > 0 ? M : 1);
-            loss[0] = l;
-            loss[1] += l;
-        }
-    }
-}
-
-// embedding gradient: demb[pid] += dX[r, 48..79]
-__global__ void emb_grad_kernel(const float *__restrict__ dX, int ldx, const int32_t *__restrict__ pids, int M,
-                                int n_ids, float *__restrict__ demb) {
-    const int64_t n = (int64_t)M * kEmb;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        const int r = (int)(i / kEmb), c = (int)(i % kEmb);
-        int p = pids[r];
-        p = p < 0 ? 0 : (p > n_ids ? n_ids : p);
-        atomicAdd(&demb[(size_t)p * kEmb + c], dX[(size_t)r * ldx + kIn + c]);
-    }
+    for (int i = t; i < 32 * kX; i += 256) X0t[(size_t)(i / 32) * Mp + r0 + i % 32] = tile[i / 32][i % 32];
+    for (int64_t i = (int64_t)blockIdx.x * 256 + t; i < nzero; i += (int64_t)gridDim.x * 256) zero[i] = 0.f;
+    if (blockIdx.x == 0 && t == 0) *done = 0;
 }
 
 // Adam over fp32 master weights; g, m, v, w all of length n.  The bias
@@ -198,10 +155,10 @@ struct wk_mlp {
     // bf16 weights (row-major, padded) and transposes
     __nv_bfloat16 *wb[4] = {}, *wt[4] = {};
     // activations (capacity cap_m)
-    // dz / dzt: two buffers, the layer whose weight gradient is taken and the one below it
-    __nv_bfloat16 *x0 = nullptr, *x0t = nullptr, *h[3] = {}, *ht[3] = {}, *dz[2] = {}, *dzt[2] = {}, *dy = nullptr,
-                  *dyt = nullptr;
-    float *z[4] = {}, *dx = nullptr, *feats = nullptr, *tgt = nullptr, *loss = nullptr;
+    __nv_bfloat16 *x0 = nullptr, *x0t = nullptr, *h[3] = {}, *ht[3] = {}, *dz[3] = {}, *dzt[3] = {};
+    float *z[3] = {}, *feats = nullptr, *tgt = nullptr;
+    float *loss = nullptr;       // the step's, the epoch's sum; then d_err and done, two ints
+    float2 *part = nullptr;      // the output layer's sums per CTA
     int32_t *pids = nullptr;
     int *bidx = nullptr;         // the batch of the epoch a training step takes
     float2 *cbias = nullptr;     // Adam bias corrections of an epoch's steps
@@ -210,7 +167,8 @@ struct wk_mlp {
     int64_t kernels = 0;
     int *d_err = nullptr;        // device flag of the tensor-core GEMM (bit 2: a wait ran out,
                                  // bit 3: work left in flight, TMEM kept)
-    int *h_err = nullptr;        // pinned mirror
+    int *done = nullptr;         // the output layer's CTAs done
+    float *h_loss = nullptr;     // pinned mirror of loss and what follows it
     int status = 0;              // a host-side GEMM failure since the last check
     int sms = 152;               // multiprocessors of the device (GEMM tile width choice)
     bool broken = false;         // a GEMM left work in flight: no further GEMM is launched
@@ -234,28 +192,48 @@ void refresh_bf16(wk_mlp *m, cudaStream_t s) {
     for (int l = 0; l < 4; ++l) {
         // W^T of layer l is [cols x rows_pad]: the dX product takes it as B
         // with N = cols (layer 0 pads 80 -> 128; the extra rows stay zero)
-        const int tcols = (l == 0) ? kXPadN : kH;
+        // (the output layer's is not needed: its dX is row-wise)
+        const int tcols = (l == 0) ? kXPadN : (l == 3 ? 0 : kH);
         weight_copy_kernel<<<nblk((int64_t)kRowsPad[l] * kCols[l]), 256, 0, s>>>(
             m->params + m->off_w[l], kRows[l], kCols[l], m->wb[l], kCols[l], kRowsPad[l], m->wt[l], kRowsPad[l], tcols);
     }
     m->kernels += 4;
 }
 
+// A launch that may take its place before the kernels ahead of it are done
+// (its kernel waits for them before it touches memory).
+template <class... P, class... A>
+void launch_ahead(void (*k)(P...), dim3 grid, unsigned threads, size_t smem, cudaStream_t s, const A &...args) {
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, k, args...);
+}
+
+bool refused(wk_mlp *m) {
+    if (m->broken && !m->status)
+        m->status = set_error(WK_EDEVICE, "estimator: an earlier tensor-core GEMM left work in flight; "
+                                          "destroy the estimator");
+    return m->broken;
+}
+
 // C = A . B^T (+ bias) on the tensor cores (wk_tc_gemm.cuh), with the
 // epilogue EPI; N is a multiple of 64.  The tile width is the widest that still
 // gives a full wave of CTAs, else 32: these products are small, and more CTAs
 // means more copies and products in flight and more warps for the epilogue.
-template <int EPI = tc::kEpiStore>
+template <int EPI>
 void gemm(wk_mlp *m, const __nv_bfloat16 *A, int lda, const __nv_bfloat16 *B, int ldb, float *C, int ldc, int M, int N,
-          int K, const float *bias, cudaStream_t s, const tc::EpiArgs &ea = tc::EpiArgs()) {
-    if (m->broken) {
-        if (!m->status)
-            m->status = set_error(WK_EDEVICE, "estimator: an earlier tensor-core GEMM left work in flight; "
-                                              "destroy the estimator");
-        return;
-    }
+          int K, const float *bias, cudaStream_t s, const tc::EpiArgs &ea) {
+    if (refused(m)) return;
     if (M <= 0 || K <= 0 || N <= 0 || N % 64 || ldc % 4 || ((uintptr_t)C & 15u) || ((uintptr_t)bias & 15u) ||
-        (EPI != tc::kEpiStore && (((uintptr_t)ea.h & 15u) || ea.ldh % 8 || !ea.ht || ea.m_store > M)) ||
+        ((uintptr_t)ea.h & 15u) || ea.ldh % 8 || !ea.ht || ea.m_store > M ||
         (EPI == tc::kEpiGeluBwd && (((uintptr_t)ea.z & 15u) || ea.ldz % 4 || !ea.colsum))) {
         if (!m->status) m->status = set_error(WK_EINVAL, "estimator GEMM: shape or alignment (M %d, N %d, K %d)", M, N, K);
         return;
@@ -271,25 +249,12 @@ void gemm(wk_mlp *m, const __nv_bfloat16 *A, int lda, const __nv_bfloat16 *B, in
         if (!m->status) m->status = set_error(WK_EDEVICE, "estimator GEMM: tensor map (M %d, N %d, K %d)", M, N, K);
         return;
     }
-    const dim3 grid((unsigned)mt, (unsigned)(N / bn));
-    switch (bn) {
-        case 32:
-            tc::gemm_tc_kernel<32, EPI><<<grid, tc::kThreads, tc::smem_bytes(32), s>>>(ta, tb, C, ldc, M, K, bias,
-                                                                                       m->d_err, ea);
-            break;
-        case 64:
-            tc::gemm_tc_kernel<64, EPI><<<grid, tc::kThreads, tc::smem_bytes(64), s>>>(ta, tb, C, ldc, M, K, bias,
-                                                                                       m->d_err, ea);
-            break;
-        case 128:
-            tc::gemm_tc_kernel<128, EPI><<<grid, tc::kThreads, tc::smem_bytes(128), s>>>(ta, tb, C, ldc, M, K, bias,
-                                                                                         m->d_err, ea);
-            break;
-        default:
-            tc::gemm_tc_kernel<256, EPI><<<grid, tc::kThreads, tc::smem_bytes(256), s>>>(ta, tb, C, ldc, M, K, bias,
-                                                                                         m->d_err, ea);
-            break;
-    }
+    auto *k = bn == 32    ? tc::gemm_tc_kernel<32, EPI>
+              : bn == 64  ? tc::gemm_tc_kernel<64, EPI>
+              : bn == 128 ? tc::gemm_tc_kernel<128, EPI>
+                          : tc::gemm_tc_kernel<256, EPI>;
+    launch_ahead(k, dim3((unsigned)mt, (unsigned)(N / bn)), tc::kThreads, tc::smem_bytes(bn), s, ta, tb, C, ldc, M, K,
+                 bias, m->d_err, ea);
     m->kernels++;
 }
 
@@ -322,19 +287,24 @@ bool set_gemm_smem_all() {
            set_gemm_smem<256, EPI>();
 }
 
+// the loss, the epoch's sum and the device flag to their pinned mirror
+cudaError_t copy_status(wk_mlp *m, cudaStream_t s) {
+    return cudaMemcpyAsync(m->h_loss, m->loss, 16, cudaMemcpyDeviceToHost, s);
+}
+
 // the status of the work queued since the last check: a host-side failure, a
 // launch error, or a tensor-core wait that ran out (bit 2 of the device flag)
-int check_status(wk_mlp *m, cudaStream_t s, const char *what) {
+int check_status(wk_mlp *m, cudaStream_t s, const char *what, bool copied = false) {
     int st = m->status;
     m->status = WK_OK;
     if (st) return st;
     cudaError_t e = cudaGetLastError();
-    if (e == cudaSuccess) e = cudaMemcpyAsync(m->h_err, m->d_err, sizeof(int), cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess && !copied) e = copy_status(m, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return cuda_fail(e, what);
-    if (*m->h_err) {
-        const int f = *m->h_err;
-        *m->h_err = 0;
+    int f;
+    std::memcpy(&f, m->h_loss + 2, sizeof(f));
+    if (f) {
         cudaMemsetAsync(m->d_err, 0, sizeof(int), s);
         if (f & 8) {
             // copies or products may still be in flight and their CTA kept its
@@ -348,25 +318,6 @@ int check_status(wk_mlp *m, cudaStream_t s, const char *what) {
     return WK_OK;
 }
 
-// forward of a training step over M rows already uploaded (feats, pids); Y in z[3] col 0
-void forward(wk_mlp *m, int M, cudaStream_t s) {
-    const int Mp = pad64(M);
-    build_input_kernel<<<nblk((int64_t)Mp * kX), 256, 0, s>>>(m->feats, m->pids, M, Mp, m->params + m->off_emb,
-                                                              m->n_ids, m->x0, m->x0t);
-    const __nv_bfloat16 *in = m->x0;
-    int kin = kX;
-    for (int l = 0; l < 3; ++l) {
-        // Z_l = X W_l^T + b_l, and H_l = GELU(Z_l) from the epilogue
-        gemm<tc::kEpiGeluFwd>(m, in, kin, m->wb[l], kin, m->z[l], kH, Mp, kH, kin, m->params + m->off_b[l], s,
-                              act_args(M, Mp, m->h[l], m->ht[l]));
-        in = m->h[l];
-        kin = kH;
-    }
-    gemm(m, in, kH, m->wb[3], kH, m->z[3], kOutPad, Mp, kOutPad, kH, nullptr, s);
-    // output bias (layer 4 has one real output): added before the loss
-    m->kernels += 1;
-}
-
 // Calls of up to kSmallRows samples go through the pinned block, which the
 // kernel reads and writes in place: one host copy of at most 100 KB instead of
 // two device copies in and one out, each some 10 us whatever it holds.
@@ -376,12 +327,7 @@ constexpr size_t kSmallBytes = kSmallOut + sizeof(float) * kSmallRows;
 
 // predictions for n samples in device-readable memory (wk_mlp_forward.cuh)
 void predict(wk_mlp *m, const float *feats, const int32_t *pids, int64_t n, float *out, cudaStream_t s) {
-    if (m->broken) {
-        if (!m->status)
-            m->status = set_error(WK_EDEVICE, "estimator: an earlier tensor-core GEMM left work in flight; "
-                                              "destroy the estimator");
-        return;
-    }
+    if (refused(m)) return;
     mlpf::Args a;
     a.feats = feats;
     a.pids = pids;
@@ -406,60 +352,106 @@ void predict(wk_mlp *m, const float *feats, const int32_t *pids, int64_t n, floa
     m->kernels++;
 }
 
-// loss + backward + Adam on M rows (targets uploaded)
-void backward_step(wk_mlp *m, int M, float lr, bool update, cudaStream_t s) {
-    const int Mp = pad64(M);
-    float *g = m->grads;
-    cudaMemsetAsync(g, 0, sizeof(float) * (size_t)m->n_params, s);
-    // dY: y includes the output bias
-    loss_kernel<<<1, 1024, 0, s>>>(m->z[3], m->tgt, M, Mp, m->dy, m->dyt, m->loss);
-    // layer 4: dW4 = dY^T . H3 (B = H3^T [256 x Mp]); db4 = sum dY; dZ3 = (dY . W4) * GELU'(Z3)
-    // (B = W4^T [256 x 64]) with db3 from the same epilogue
-    int cur = 0;
-    {
-        float *dw4 = g + m->off_w[3];   // [1 x 256] real, GEMM writes [64 x 256]
-        gemm(m, m->dyt, Mp, m->ht[2], Mp, m->dx /*scratch [64 x 256]*/, kH, kOutPad, kH, Mp, nullptr, s);
-        cudaMemcpyAsync(dw4, m->dx, sizeof(float) * kH, cudaMemcpyDeviceToDevice, s);   // row 0
-        colsum_kernel<<<1, 256, 0, s>>>(m->dyt, Mp, g + m->off_b[3]);
-        gemm<tc::kEpiGeluBwd>(m, m->dy, kOutPad, m->wt[3], kOutPad, nullptr, kH, Mp, kH, kOutPad, nullptr, s,
-                              act_args(M, Mp, m->dz[cur], m->dzt[cur], m->z[2], g + m->off_b[2]));
+// The weight gradients dW_l = dZ_l^T . X_l (the layer's input), K the batch, and
+// the embedding's from dX = dZ_0 . W_0, in one launch: nothing waits for any of
+// them, and each alone is 6 to 16 CTAs.
+void gradient_group(wk_mlp *m, int M, int Mp, cudaStream_t s) {
+    if (refused(m)) return;
+    tc::GroupArgs g;
+    bool ok = true;
+    int at = 0;
+    for (int i = 0; i < 3; ++i) {   // layers 2, 1, 0
+        const int l = 2 - i, kin = kCols[l];
+        ok = ok && tc::make_map(&g.a[i], m->dzt[l], kH, (uint64_t)Mp, (uint64_t)Mp, tc::kTM) &&
+             tc::make_map(&g.b[i], l ? m->ht[l - 1] : m->x0t, (uint64_t)kin, (uint64_t)Mp, (uint64_t)Mp, 32);
+        g.first[i] = at;
+        g.mt[i] = kH / tc::kTM;
+        g.n0[i] = 0;
+        g.C[i] = m->grads + m->off_w[l];
+        g.ldc[i] = g.n_real[i] = kin;
+        g.M[i] = kH;
+        g.K[i] = Mp;
+        at += g.mt[i] * ((kin + 31) / 32);
     }
-    for (int l = 2; l >= 0; --l) {
-        // dZ_l is in dz[cur] / dzt[cur], db_l already summed
-        const __nv_bfloat16 *inT = (l == 0) ? m->x0t : m->ht[l - 1];
-        const int kin = (l == 0) ? kX : kH;
-        // dW_l [256 x kin] = dZ^T [256 x Mp] . (X^T [kin x Mp])^T ; N = kin must be a multiple of 64
-        if (kin % 64 == 0) {
-            gemm(m, m->dzt[cur], Mp, inT, Mp, g + m->off_w[l], kin, kH, kin, Mp, nullptr, s);
-        } else {
-            // layer 0: kin = 80 -> compute into scratch [256 x 128] then copy the first 80 columns
-            gemm(m, m->dzt[cur], Mp, inT, Mp, m->dx, kXPadN, kH, kXPadN, Mp, nullptr, s);
-            cudaMemcpy2DAsync(g + m->off_w[0], sizeof(float) * kX, m->dx, sizeof(float) * kXPadN, sizeof(float) * kX,
-                              kH, cudaMemcpyDeviceToDevice, s);
-        }
-        // dZ_{l-1} = (dZ_l . W_l) * GELU'(Z_{l-1}) (B = W_l^T [256 x 256]), with db_{l-1};
-        // layer 0: dX = dZ_0 . W_0 (B = W_0^T [128 x 256]) for the embedding gradient
-        if (l > 0) {
-            gemm<tc::kEpiGeluBwd>(m, m->dz[cur], kH, m->wt[l], kH, nullptr, kH, Mp, kH, kH, nullptr, s,
-                                  act_args(M, Mp, m->dz[1 - cur], m->dzt[1 - cur], m->z[l - 1], g + m->off_b[l - 1]));
-            cur = 1 - cur;
-        } else {
-            gemm(m, m->dz[cur], kH, m->wt[0], kH, m->dx, kXPadN, Mp, kXPadN, kH, nullptr, s);
-        }
+    // columns 48..79 of dX: a tile of 32 from row 48 of W_0^T
+    ok = ok && tc::make_map(&g.a[3], m->dz[0], (uint64_t)Mp, kH, kH, tc::kTM) &&
+         tc::make_map(&g.b[3], m->wt[0], kXPadN, kH, kH, 32);
+    g.first[3] = at;
+    g.mt[3] = (Mp + tc::kTM - 1) / tc::kTM;
+    g.n0[3] = kIn;
+    g.C[3] = nullptr;
+    g.ldc[3] = 0;
+    g.n_real[3] = 0;
+    g.M[3] = Mp;
+    g.K[3] = kH;
+    at += g.mt[3];
+    g.first[4] = at;
+    g.n = 4;
+    g.demb = m->grads + m->off_emb;
+    g.pids = m->pids;
+    g.n_ids = m->n_ids;
+    g.m_real = M;
+    g.err = m->d_err;
+    if (!ok) {
+        if (!m->status) m->status = set_error(WK_EDEVICE, "estimator: tensor map of the weight gradients (M %d)", M);
+        return;
     }
-    emb_grad_kernel<<<nblk((int64_t)M * kEmb), 256, 0, s>>>(m->dx, kXPadN, m->pids, M, m->n_ids, g + m->off_emb);
-    m->kernels += 3;
-    if (update) {
-        adam_kernel<<<nblk(m->n_params), 256, 0, s>>>(m->params, g, m->m1, m->m2, m->n_params, lr, kB1, kB2, 1e-8f,
-                                                      m->cbias, m->bidx);
-        refresh_bf16(m, s);
-        m->kernels++;
-    }
+    launch_ahead(tc::gemm_group_kernel, dim3((unsigned)at), tc::kThreads, tc::smem_bytes(32, tc::kDeepStages), s, g);
+    m->kernels++;
 }
 
-// add the output bias to column 0 of Y in place (so the loss sees y = H3 . w4 + b4)
-__global__ void add_out_bias_kernel(float *Y, const float *b4, int M) {
-    for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < M; r += gridDim.x * blockDim.x) Y[(size_t)r * kOutPad] += b4[0];
+// The loss and every gradient for M rows already uploaded (feats, pids, tgt).
+void gradient_step(wk_mlp *m, int M, cudaStream_t s) {
+    const int Mp = pad64(M);
+    float *g = m->grads;
+    // w4's gradient, the biases' and the embedding's are added into; they lie together
+    launch_ahead(build_input_kernel, dim3((unsigned)(Mp / 32)), 256, 0, s, (const float *)m->feats,
+                 (const int32_t *)m->pids, M, Mp, (const float *)(m->params + m->off_emb), m->n_ids, m->x0, m->x0t,
+                 g + m->off_w[3], m->n_params - m->off_w[3], m->done);
+    m->kernels++;
+    const __nv_bfloat16 *in = m->x0;
+    int kin = kX;
+    for (int l = 0; l < 3; ++l) {
+        // Z_l = X W_l^T + b_l, and H_l = GELU(Z_l) from the epilogue
+        gemm<tc::kEpiGeluFwd>(m, in, kin, m->wb[l], kin, m->z[l], kH, Mp, kH, kin, m->params + m->off_b[l], s,
+                              act_args(M, Mp, m->h[l], m->ht[l]));
+        in = m->h[l];
+        kin = kH;
+    }
+    // the output layer, the loss, dZ_2 and the gradients of w4, b4, b3
+    if (!refused(m)) {
+        tc::EpiArgs ea = act_args(M, Mp, m->dz[2], m->dzt[2], m->z[2], g + m->off_b[2]);
+        ea.hin = m->h[2];
+        ea.w = m->wb[3];
+        ea.b = m->params + m->off_b[3];
+        ea.tgt = m->tgt;
+        ea.dw = g + m->off_w[3];
+        ea.db = g + m->off_b[3];
+        ea.loss = m->loss;
+        ea.part = m->part;
+        ea.done = m->done;
+        CUtensorMap ta, tb;
+        if (tc::make_map(&ta, m->h[2], (uint64_t)Mp, kH, kH, tc::kTM) && tc::make_map(&tb, m->wb[3], kOutPad, kH, kH, 32)) {
+            launch_ahead(tc::gemm_tc_kernel<32, tc::kEpiHead>, dim3((unsigned)(Mp / 16)), tc::kThreads, tc::smem_bytes(32),
+                         s, ta, tb, (float *)nullptr, 0, Mp, kH, (const float *)nullptr, m->d_err, ea);
+            m->kernels++;
+        } else if (!m->status) {
+            m->status = set_error(WK_EDEVICE, "estimator: tensor map of the output layer (M %d)", M);
+        }
+    }
+    // dZ_{l-1} = (dZ_l . W_l) * GELU'(Z_{l-1}) (B = W_l^T [256 x 256]), with db_{l-1}
+    for (int l = 2; l > 0; --l)
+        gemm<tc::kEpiGeluBwd>(m, m->dz[l], kH, m->wt[l], kH, nullptr, kH, Mp, kH, kH, nullptr, s,
+                              act_args(M, Mp, m->dz[l - 1], m->dzt[l - 1], m->z[l - 1], g + m->off_b[l - 1]));
+    gradient_group(m, M, Mp, s);
+}
+
+// an Adam update from the gradients
+void update(wk_mlp *m, float lr, cudaStream_t s) {
+    adam_kernel<<<nblk(m->n_params), 256, 0, s>>>(m->params, m->grads, m->m1, m->m2, m->n_params, lr, kB1, kB2, 1e-8f,
+                                                  m->cbias, m->bidx);
+    m->kernels++;
+    refresh_bf16(m, s);
 }
 
 int upload(wk_mlp *m, const float *feats, const int32_t *pids, const float *tgt, int M, cudaStream_t s) {
@@ -475,15 +467,15 @@ void free_mlp(wk_mlp *m) {
     cudaFree(m->grads);
     cudaFree(m->m1);
     cudaFree(m->m2);
-    for (int l = 0; l < 4; ++l) { cudaFree(m->wb[l]); cudaFree(m->wt[l]); cudaFree(m->z[l]); }
-    for (int l = 0; l < 3; ++l) { cudaFree(m->h[l]); cudaFree(m->ht[l]); }
-    cudaFree(m->x0); cudaFree(m->x0t); cudaFree(m->dy); cudaFree(m->dyt);
-    for (int i = 0; i < 2; ++i) { cudaFree(m->dz[i]); cudaFree(m->dzt[i]); }
-    cudaFree(m->dx); cudaFree(m->feats); cudaFree(m->tgt); cudaFree(m->loss); cudaFree(m->pids);
-    cudaFree(m->d_err);
+    for (int l = 0; l < 4; ++l) { cudaFree(m->wb[l]); cudaFree(m->wt[l]); }
+    for (int l = 0; l < 3; ++l) {
+        cudaFree(m->h[l]); cudaFree(m->ht[l]); cudaFree(m->z[l]); cudaFree(m->dz[l]); cudaFree(m->dzt[l]);
+    }
+    cudaFree(m->x0); cudaFree(m->x0t);
+    cudaFree(m->feats); cudaFree(m->tgt); cudaFree(m->loss); cudaFree(m->part); cudaFree(m->pids);
     cudaFree(m->bidx);
     cudaFree(m->cbias);
-    if (m->h_err) cudaFreeHost(m->h_err);
+    if (m->h_loss) cudaFreeHost(m->h_loss);
     if (m->h_small) cudaFreeHost(m->h_small);
     for (int i = 0; i < 2; ++i) {
         if (m->copied[i]) cudaEventDestroy(m->copied[i]);
@@ -518,21 +510,18 @@ extern "C" int wk_mlp_create(wk_ctx *ctx, int32_t n_ids, int32_t max_batch, uint
     for (int l = 0; ok && l < 4; ++l) {
         const int tcols = (l == 0) ? kXPadN : kH;
         ok = cudaMalloc(&m->wb[l], 2 * (size_t)kRowsPad[l] * kCols[l]) == cudaSuccess &&
-             cudaMalloc(&m->wt[l], 2 * (size_t)tcols * kRowsPad[l]) == cudaSuccess &&
-             cudaMalloc(&m->z[l], 4 * Mp * (size_t)(l < 3 ? kH : kOutPad)) == cudaSuccess;
+             (l == 3 || cudaMalloc(&m->wt[l], 2 * (size_t)tcols * kRowsPad[l]) == cudaSuccess);
     }
     for (int l = 0; ok && l < 3; ++l)
-        ok = cudaMalloc(&m->h[l], 2 * Mp * kH) == cudaSuccess && cudaMalloc(&m->ht[l], 2 * Mp * kH) == cudaSuccess;
-    // X0^T has kXPadN rows: the layer-0 weight-gradient product pads N = 80 to 128 and reads rows 80..127 (zero)
-    ok = ok && cudaMalloc(&m->x0, 2 * Mp * kX) == cudaSuccess && cudaMalloc(&m->x0t, 2 * Mp * kXPadN) == cudaSuccess &&
-         cudaMalloc(&m->dz[0], 2 * Mp * kH) == cudaSuccess && cudaMalloc(&m->dzt[0], 2 * Mp * kH) == cudaSuccess &&
-         cudaMalloc(&m->dz[1], 2 * Mp * kH) == cudaSuccess && cudaMalloc(&m->dzt[1], 2 * Mp * kH) == cudaSuccess &&
-         cudaMalloc(&m->dy, 2 * Mp * kOutPad) == cudaSuccess && cudaMalloc(&m->dyt, 2 * Mp * kOutPad) == cudaSuccess &&
-         cudaMalloc(&m->dx, 4 * std::max(Mp * (size_t)kXPadN, (size_t)kH * kXPadN)) == cudaSuccess &&
+        ok = cudaMalloc(&m->h[l], 2 * Mp * kH) == cudaSuccess && cudaMalloc(&m->ht[l], 2 * Mp * kH) == cudaSuccess &&
+             cudaMalloc(&m->z[l], 4 * Mp * kH) == cudaSuccess && cudaMalloc(&m->dz[l], 2 * Mp * kH) == cudaSuccess &&
+             cudaMalloc(&m->dzt[l], 2 * Mp * kH) == cudaSuccess;
+    ok = ok && cudaMalloc(&m->x0, 2 * Mp * kX) == cudaSuccess && cudaMalloc(&m->x0t, 2 * Mp * kX) == cudaSuccess &&
+         cudaMalloc(&m->part, sizeof(float2) * Mp / 16) == cudaSuccess &&
          cudaMalloc(&m->feats, 4 * Mp * kIn) == cudaSuccess && cudaMalloc(&m->tgt, 4 * Mp) == cudaSuccess &&
          cudaMalloc(&m->loss, 16) == cudaSuccess && cudaMalloc(&m->pids, 4 * Mp) == cudaSuccess &&
-         cudaMalloc(&m->d_err, sizeof(int)) == cudaSuccess && cudaMalloc(&m->bidx, sizeof(int)) == cudaSuccess &&
-         cudaHostAlloc((void **)&m->h_err, sizeof(int), 0) == cudaSuccess &&
+         cudaMalloc(&m->bidx, sizeof(int)) == cudaSuccess &&
+         cudaHostAlloc((void **)&m->h_loss, 16, 0) == cudaSuccess &&
          cudaHostAlloc((void **)&m->h_small, kSmallBytes, cudaHostAllocMapped) == cudaSuccess &&
          cudaHostGetDevicePointer((void **)&m->h_small_dev, m->h_small, 0) == cudaSuccess &&
          cudaStreamCreateWithFlags(&m->copy, cudaStreamNonBlocking) == cudaSuccess &&
@@ -542,13 +531,17 @@ extern "C" int wk_mlp_create(wk_ctx *ctx, int32_t n_ids, int32_t max_batch, uint
          cudaEventCreateWithFlags(&m->used[1], cudaEventDisableTiming) == cudaSuccess &&
          cudaFuncSetAttribute(mlpf::forward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mlpf::kSmem) ==
              cudaSuccess &&
-         set_gemm_smem_all<tc::kEpiStore>() && set_gemm_smem_all<tc::kEpiGeluFwd>() &&
-         set_gemm_smem_all<tc::kEpiGeluBwd>();
+         set_gemm_smem_all<tc::kEpiGeluFwd>() && set_gemm_smem_all<tc::kEpiGeluBwd>() &&
+         set_gemm_smem<32, tc::kEpiHead>() &&
+         cudaFuncSetAttribute(tc::gemm_group_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              (int)tc::smem_bytes(32, tc::kDeepStages)) == cudaSuccess;
     if (!ok) {
         cudaGetLastError();
         free_mlp(m);
         return set_error(WK_ENOMEM, "wk_mlp_create: allocation failed");
     }
+    m->d_err = reinterpret_cast<int *>(m->loss + 2);
+    m->done = m->d_err + 1;
     // He-style initialisation (uniform with the fan-in bound), zero biases, small embeddings
     std::vector<float> h((size_t)at, 0.f);
     std::mt19937_64 rng(seed);
@@ -563,17 +556,13 @@ extern "C" int wk_mlp_create(wk_ctx *ctx, int32_t n_ids, int32_t max_batch, uint
     e = cudaMemcpyAsync(m->params, h.data(), P, cudaMemcpyHostToDevice, s);
     if (e == cudaSuccess) e = cudaMemsetAsync(m->m1, 0, P, s);
     if (e == cudaSuccess) e = cudaMemsetAsync(m->m2, 0, P, s);
-    for (int l = 0; e == cudaSuccess && l < 4; ++l) {
+    for (int l = 0; e == cudaSuccess && l < 3; ++l) {
         const int tcols = (l == 0) ? kXPadN : kH;
         e = cudaMemsetAsync(m->wt[l], 0, 2 * (size_t)tcols * kRowsPad[l], s);
     }
-    if (e == cudaSuccess) e = cudaMemsetAsync(m->x0t, 0, 2 * Mp * kXPadN, s);
-    if (e == cudaSuccess) e = cudaMemsetAsync(m->dy, 0, 2 * Mp * kOutPad, s);
-    if (e == cudaSuccess) e = cudaMemsetAsync(m->dyt, 0, 2 * Mp * kOutPad, s);
-    if (e == cudaSuccess) e = cudaMemsetAsync(m->d_err, 0, sizeof(int), s);
+    if (e == cudaSuccess) e = cudaMemsetAsync(m->grads, 0, P, s);
     if (e == cudaSuccess) e = cudaMemsetAsync(m->bidx, 0, sizeof(int), s);
     if (e == cudaSuccess) e = cudaMemsetAsync(m->loss, 0, 16, s);
-    if (m->h_err) *m->h_err = 0;
     if (e != cudaSuccess) { int r = cuda_fail(e, "wk_mlp_create init"); free_mlp(m); return r; }
     refresh_bf16(m, s);
     if ((e = cudaStreamSynchronize(s)) != cudaSuccess) { int r = cuda_fail(e, "wk_mlp_create sync"); free_mlp(m); return r; }
@@ -614,15 +603,16 @@ extern "C" int wk_mlp_gradients(wk_mlp *m, const float *feats, const int32_t *pi
     cudaStream_t s = m->ctx->stream;
     int st = upload(m, feats, pids, tgt, M, s);
     if (st) return st;
-    forward(m, M, s);
-    add_out_bias_kernel<<<nblk(M), 256, 0, s>>>(m->z[3], m->params + m->off_b[3], M);
-    backward_step(m, M, 0.f, false, s);
+    gradient_step(m, M, s);
     cudaError_t e = cudaGetLastError();
+    // the status first: the copy to the caller's memory holds the host until it is done
+    if (e == cudaSuccess) e = copy_status(m, s);
     if (e == cudaSuccess && grads_host)
         e = cudaMemcpyAsync(grads_host, m->grads, sizeof(float) * (size_t)m->n_params, cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess && loss_host) e = cudaMemcpyAsync(loss_host, m->loss, 4, cudaMemcpyDeviceToHost, s);
     if (e != cudaSuccess) return cuda_fail(e, "wk_mlp_gradients");
-    return check_status(m, s, "wk_mlp_gradients");
+    if ((st = check_status(m, s, "wk_mlp_gradients", true))) return st;
+    if (loss_host) *loss_host = m->h_loss[0];
+    return WK_OK;
 }
 
 // Mini-batch training: `epochs` passes over n samples in batches of `batch`
@@ -677,11 +667,10 @@ extern "C" int wk_mlp_train(wk_mlp *m, const float *feats, const int32_t *pids, 
         gather_batch_kernel<<<nblk((int64_t)M * kIn), 256, 0, s>>>(d_feats.as<float>(), d_pids.as<int32_t>(),
                                                                    d_tgt.as<float>(), d_order.as<int64_t>(), m->bidx,
                                                                    batch, M, m->feats, m->pids, m->tgt);
-        forward(m, M, s);
-        add_out_bias_kernel<<<nblk(M), 256, 0, s>>>(m->z[3], m->params + m->off_b[3], M);
-        backward_step(m, M, lr, true, s);
+        gradient_step(m, M, s);
+        update(m, lr, s);
         bump_kernel<<<1, 1, 0, s>>>(m->bidx);
-        m->kernels += 4;   // gather, output bias, Adam, bump
+        m->kernels += 2;   // gather, bump
     };
     auto finish = [&](int rc) {
         if (exec) cudaGraphExecDestroy(exec);
@@ -773,6 +762,9 @@ extern "C" int wk_mlp_predict(wk_mlp *m, const float *feats, const int32_t *pids
             predict(m, f, p + b0, rows, m->pred.as<float>() + b0, s);
             if (in != s) e = cudaEventRecord(m->used[b], s);
         }
+        // the status first: the copy to the caller's memory holds the host until it is done
+        if (e == cudaSuccess) e = cudaGetLastError();
+        if (e == cudaSuccess) e = copy_status(m, s);
         if (e == cudaSuccess)
             e = cudaMemcpyAsync(out, m->pred.ptr, sizeof(float) * (size_t)n, cudaMemcpyDeviceToHost, s);
         if (e != cudaSuccess) {
@@ -780,7 +772,7 @@ extern "C" int wk_mlp_predict(wk_mlp *m, const float *feats, const int32_t *pids
             cudaStreamSynchronize(s);
             return cuda_fail(e, "wk_mlp_predict");
         }
-        if ((st = check_status(m, s, "wk_mlp_predict"))) return st;
+        if ((st = check_status(m, s, "wk_mlp_predict", true))) return st;
     }
     m->ctx->launches += m->kernels;
     m->kernels = 0;

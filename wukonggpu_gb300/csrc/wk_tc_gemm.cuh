@@ -15,14 +15,23 @@
 //   - after the last commit, warp w reads TMEM lanes 32w..32w+31 (rows) in
 //     32-column chunks with tcgen05.ld and runs the epilogue the template
 //     names (EpiArgs):
-//       kEpiStore:   C = acc (+ bias), staged in shared memory (the pipeline
-//                    stages are free by then) and written as whole rows of
-//                    float4, so a store instruction covers 4 rows x 128 B;
-//       kEpiGeluFwd: the same C (the pre-activation Z), and H = GELU(Z) in
-//                    bf16, row-major and transposed (zero for rows >= m_real);
+//       kEpiGeluFwd: C = Z = acc + bias (the pre-activation), staged in shared
+//                    memory (the pipeline stages are free by then) and written
+//                    as whole rows of float4, so a store instruction covers 4
+//                    rows x 128 B, and H = GELU(Z) in bf16, row-major and
+//                    transposed (zero for rows >= m_real);
 //       kEpiGeluBwd: dZ = acc * GELU'(Z) in bf16, row-major and transposed
 //                    (zero for rows >= m_real), and the column sums of the
-//                    rounded dZ added into colsum[] -- C is not written.
+//                    rounded dZ added into colsum[] -- C is not written;
+//       kEpiHead:    the end of the forward pass and the start of the backward
+//                    one, 16 rows a CTA (head_rows);
+//       kEpiGroup:   C = acc for columns below n_real, or the tile's 32 columns added to
+//                    the rows' embedding gradients (demb).
+// The products of a training step are small and follow one another, so their
+// kernels are launched ahead of their turn (programmatic dependent launch): a
+// CTA sets up its barriers and TMEM and reads its tensor maps, then waits for
+// the kernel before.  It lets the next one start only once it holds its TMEM,
+// so no CTA waits for columns that one behind it has taken.
 // Every mbarrier wait is bounded.  A wait that runs out sets bit 2 of *err and
 // stops the pipeline: the producer waits (bounded) for the copies it issued
 // and the issuer for the last commit of the products it issued.  If those
@@ -44,14 +53,15 @@ namespace tc {
 
 constexpr int kTM = 128;            // tile rows = MMA M
 constexpr int kSlab = 64;           // K elements per stage (128 B rows)
-constexpr int kStages = 4;
+constexpr int kStages = 4;          // kDeepStages where K is the batch and the tiles are few
+constexpr int kDeepStages = 8;
 constexpr int kThreads = 128;
 constexpr int kEpiPitch = 36;       // floats per staged output row: rows 16 B apart modulo 128 B
 constexpr long kWaitIters = 1l << 22;
 
-enum { kEpiStore = 0, kEpiGeluFwd = 1, kEpiGeluBwd = 2 };
+enum { kEpiGeluFwd, kEpiGeluBwd, kEpiHead, kEpiGroup };
 
-// The epilogue's extra operands (unused by kEpiStore).  Rows below m_store get
+// The epilogue's extra operands.  Rows below m_store get
 // h / ht written (row-major with ld ldh, transposed with ld ldt); rows below
 // m_real carry values, the rest zeros.
 struct EpiArgs {
@@ -62,7 +72,20 @@ struct EpiArgs {
     int ldt = 0;
     const float *z = nullptr;   // kEpiGeluBwd: the layer's pre-activation (ld ldz)
     int ldz = 0;
-    float *colsum = nullptr;    // kEpiGeluBwd: column sums of dZ are added here
+    float *colsum = nullptr;    // kEpiGeluBwd, kEpiHead: column sums of dZ are added here
+    int n_real = 1 << 30;       // kEpiGroup: columns of C
+    // kEpiGroup, demb not null: column c of row r is added to demb[32 pids[r] + c]
+    float *demb = nullptr;
+    const int32_t *pids = nullptr;
+    int n_ids = 0;
+    // kEpiHead: the last hidden layer's output (ld ldh), the output layer's
+    // weights and bias, the targets; the gradients of both, the loss and its
+    // running sum; each CTA's sums and the count of CTAs done (zero between launches)
+    const __nv_bfloat16 *hin = nullptr, *w = nullptr;
+    const float *b = nullptr, *tgt = nullptr;
+    float *dw = nullptr, *db = nullptr, *loss = nullptr;
+    float2 *part = nullptr;
+    int *done = nullptr;
 };
 
 // The estimator's activation, exact GELU: x Phi(x), and its derivative
@@ -118,25 +141,124 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
-// C must be 16 B aligned with ldc a multiple of 4, and bias (if any) 16 B
-// aligned; h (and z) 16 B aligned with ldh (ldz) a multiple of 8 (4).
-template <int BN, int EPI>
-__global__ void __launch_bounds__(kThreads)
-gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-               float *__restrict__ C, int ldc, int M, int K, const float *__restrict__ bias, int *err,
-               const EpiArgs ea) {
+// The step's output layer, loss and first backward layer for the CTA's 16 rows,
+// a warp four of them: y = acc + b, loss mean((y - t)^2), dY = 2 (y - t) / M in
+// bf16 (rows >= m_real: zero), dw += dY^T H, db = sum dY, and of the hidden
+// layer below dZ = dY w GELU'(Z) in bf16, row-major and transposed, with its
+// column sums.  The layer has one output, so these are row-wise: as products
+// padded to tiles of 64 with kernels of their own for bias, loss and sums they
+// were seven launches and 30 us of a step of 1024 rows.  y: the CTA's 16 accumulators.
+// sm: 12 KB, free.
+__device__ __forceinline__ void head_rows(const EpiArgs &ea, const float *y, int row0, unsigned char *sm) {
+    constexpr int kCols = 256, kPitch = 18;   // an odd number of words: the 32 lanes' columns fall in 32 banks
+    __nv_bfloat16 *st = reinterpret_cast<__nv_bfloat16 *>(sm);                    // dZ^T: [256][16]
+    float *s_cs = reinterpret_cast<float *>(sm + kCols * kPitch * 2);             // per warp: column sums of dZ
+    float *s_dw = s_cs + kCols;                                                   // and of dY H
+    __shared__ float2 s_sum[kThreads / 32];
+    __shared__ int s_last;
+    const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+    for (int i = t; i < 2 * kCols; i += kThreads) s_cs[i] = 0.f;
+    __syncthreads();
+    float w[8], cs[8] = {}, dw[8] = {};
+#pragma unroll
+    for (int j = 0; j < 8; ++j) w[j] = __bfloat162float(ea.w[lane + 32 * j]);
+    const float b = *ea.b;
+    float sq = 0.f, sdy = 0.f;
+    for (int i = 0; i < 4; ++i) {
+        const int r = warp * 4 + i, row = row0 + r;
+        float dy = 0.f;
+        if (row < ea.m_real) {   // the same in every lane
+            const float d = (y[r] + b) - ea.tgt[row];
+            sq += d * d;
+            dy = __bfloat162float(__float2bfloat16(2.f * d / (float)ea.m_real));
+            sdy += dy;
+        }
+        const __nv_bfloat16 *hr = ea.hin + (size_t)row * ea.ldh + lane;
+        const float *zr = ea.z + (size_t)row * ea.ldz + lane;
+        __nv_bfloat16 *out = ea.h + (size_t)row * ea.ldh + lane;
+        float z[8], h[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            z[j] = zr[32 * j];
+            h[j] = __bfloat162float(hr[32 * j]);
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const __nv_bfloat16 v = __float2bfloat16(row < ea.m_real ? __fmul_rn(dy, w[j]) * gelu_grad(z[j]) : 0.f);
+            out[32 * j] = v;
+            st[(lane + 32 * j) * kPitch + r] = v;
+            cs[j] += __bfloat162float(v);
+            dw[j] += dy * h[j];
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        atomicAdd(s_cs + lane + 32 * j, cs[j]);
+        atomicAdd(s_dw + lane + 32 * j, dw[j]);
+    }
+    if (lane == 0) s_sum[warp] = make_float2(sq, sdy);
+    __syncthreads();
+    for (int c = t; c < kCols; c += kThreads) {
+        const uint32_t *src = reinterpret_cast<const uint32_t *>(st + c * kPitch);
+        uint4 *dst = reinterpret_cast<uint4 *>(ea.ht + (size_t)c * ea.ldt + row0);
+        dst[0] = make_uint4(src[0], src[1], src[2], src[3]);
+        dst[1] = make_uint4(src[4], src[5], src[6], src[7]);
+        if (s_cs[c] != 0.f) atomicAdd(ea.colsum + c, s_cs[c]);
+        if (s_dw[c] != 0.f) atomicAdd(ea.dw + c, s_dw[c]);
+    }
+    // the sums over all rows: the last CTA adds up every CTA's
+    if (t == 0) {
+        float2 v = s_sum[0];
+        for (int i = 1; i < kThreads / 32; ++i) { v.x += s_sum[i].x; v.y += s_sum[i].y; }
+        ea.part[blockIdx.x] = v;
+        __threadfence();
+        s_last = atomicAdd(ea.done, 1) == (int)gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    sq = sdy = 0.f;
+    for (int i = t; i < (int)gridDim.x; i += kThreads) {
+        const float2 v = __ldcg(ea.part + i);
+        sq += v.x;
+        sdy += v.y;
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+        sq += __shfl_xor_sync(0xffffffffu, sq, o);
+        sdy += __shfl_xor_sync(0xffffffffu, sdy, o);
+    }
+    if (lane == 0) s_sum[warp] = make_float2(sq, sdy);
+    __syncthreads();
+    if (t == 0) {
+        float2 v = s_sum[0];
+        for (int i = 1; i < kThreads / 32; ++i) { v.x += s_sum[i].x; v.y += s_sum[i].y; }
+        const float l = v.x / (float)(ea.m_real > 0 ? ea.m_real : 1);
+        ea.loss[0] = l;
+        ea.loss[1] += l;
+        *ea.db = v.y;
+        *ea.done = 0;
+    }
+}
+
+// One tile: rows m0.. and columns n0.. of C.  C must be 16 B aligned with ldc a
+// multiple of 4, and bias (if any) 16 B aligned; h (and z) 16 B aligned with
+// ldh (ldz) a multiple of 8 (4).
+template <int BN, int EPI, int STAGES>
+__device__ __forceinline__ void gemm_tile(const CUtensorMap *tmA, const CUtensorMap *tmB, int m0, int n0,
+                                          float *__restrict__ C, int ldc, int M, int K,
+                                          const float *__restrict__ bias, int *err, const EpiArgs &ea) {
     static_assert(BN == 32 || BN == 64 || BN == 128 || BN == 256, "tile width: an MMA N and a TMEM allocation");
     constexpr uint32_t kABytes = kTM * 128, kBBytes = BN * 128, kStage = kABytes + kBBytes;
     static_assert(4 * 32 * kEpiPitch * 4 <= kStage, "the output staging fits in stage 0");
     extern __shared__ unsigned char smem_raw[];
     __shared__ uint32_t s_tmem;
-    __shared__ __align__(8) uint64_t s_full[kStages], s_empty[kStages];
+    __shared__ __align__(8) uint64_t s_full[STAGES], s_empty[STAGES];
+    __shared__ float s_y[16];             // kEpiHead
     __shared__ volatile int s_fail;
     __shared__ volatile int s_inflight;   // a drain wait ran out: copies or products may be in flight
     // 128 B swizzle: stage bases 1024 B aligned
     unsigned char *sm = (unsigned char *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
-    const int m0 = blockIdx.x * kTM, n0 = blockIdx.y * BN;
     const int nslab = (K + kSlab - 1) / kSlab;
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
@@ -146,35 +268,39 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     if (t == 0) {
         s_fail = 0;
         s_inflight = 0;
-        for (int i = 0; i < kStages; ++i) {
+        for (int i = 0; i < STAGES; ++i) {
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&s_full[i])));
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&s_empty[i])));
         }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("prefetch.tensormap [%0];" ::"l"(tmA) : "memory");
+        asm volatile("prefetch.tensormap [%0];" ::"l"(tmB) : "memory");
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = s_tmem;
-    // slab j lives in stage j % kStages as that stage's use u = j / kStages; each
+    asm volatile("griddepcontrol.launch_dependents;");
+    asm volatile("griddepcontrol.wait;" ::: "memory");   // nothing of the kernels before is read or written until here
+    // slab j lives in stage j % STAGES as that stage's use u = j / STAGES; each
     // barrier completes once per use, so the wait for use u is parity u % 2
     if (t == 0) {
         int issued = 0;
         for (int j = 0; j < nslab; ++j) {
-            const int s = j % kStages, u = j / kStages;
+            const int s = j % STAGES, u = j / STAGES;
             if (u > 0 && !mbar_wait(smem_u32(&s_empty[s]), (uint32_t)((u - 1) & 1))) {
                 s_fail = 1;
                 break;
             }
             const uint32_t a = smem_u32(sm + s * kStage), b = a + kABytes, fb = smem_u32(&s_full[s]);
             asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(fb), "r"(kStage) : "memory");
-            tma_load_2d(a, &tmA, j * kSlab, m0, fb);
-            tma_load_2d(b, &tmB, j * kSlab, n0, fb);
+            tma_load_2d(a, tmA, j * kSlab, m0, fb);
+            tma_load_2d(b, tmB, j * kSlab, n0, fb);
             issued = j + 1;
         }
         // every copy in flight lands before the CTA can leave (immediate when all were consumed)
-        for (int j = issued > kStages ? issued - kStages : 0; j < issued; ++j)
-            if (!mbar_wait(smem_u32(&s_full[j % kStages]), (uint32_t)((j / kStages) & 1))) {
+        for (int j = issued > STAGES ? issued - STAGES : 0; j < issued; ++j)
+            if (!mbar_wait(smem_u32(&s_full[j % STAGES]), (uint32_t)((j / STAGES) & 1))) {
                 s_fail = 1;
                 s_inflight = 1;
                 break;
@@ -182,8 +308,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     } else if (t == 32) {
         int committed = 0;
         for (int sl = 0; sl < nslab; ++sl) {
-            const int s = sl % kStages;
-            if (!mbar_wait(smem_u32(&s_full[s]), (uint32_t)((sl / kStages) & 1))) {
+            const int s = sl % STAGES;
+            if (!mbar_wait(smem_u32(&s_full[s]), (uint32_t)((sl / STAGES) & 1))) {
                 s_fail = 1;
                 break;
             }
@@ -204,7 +330,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         // the last commit covers every product issued: they complete before TMEM is read or freed
         if (committed > 0) {
             const int c = committed - 1;
-            if (!mbar_wait(smem_u32(&s_empty[c % kStages]), (uint32_t)((c / kStages) & 1))) {
+            if (!mbar_wait(smem_u32(&s_empty[c % STAGES]), (uint32_t)((c / STAGES) & 1))) {
                 s_fail = 1;
                 s_inflight = 1;
             }
@@ -217,12 +343,33 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         float *stg = reinterpret_cast<float *>(sm) + warp * 32 * kEpiPitch;
         const int q = lane & 7;
         const int myrow = m0 + warp * 32 + lane;   // the row of this lane's TMEM lane
-        for (int c0 = 0; c0 < BN; c0 += 32) {
+        if constexpr (EPI == kEpiHead) {
+            const int row0 = blockIdx.x * 16;
+            uint32_t r[32];
+            tmem_ld32(tmem + ((uint32_t)(warp * 32) << 16), r);   // column 0: the layer's one output
+            if (myrow >= row0 && myrow < row0 + 16) s_y[myrow - row0] = __uint_as_float(r[0]);
+            __syncthreads();
+            head_rows(ea, s_y, row0, sm);
+        }
+        for (int c0 = 0; EPI != kEpiHead && c0 < BN; c0 += 32) {
             uint32_t r[32];
             tmem_ld32(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0, r);
             const int cb = n0 + c0;   // the chunk's first column
             float4 *mine = reinterpret_cast<float4 *>(stg + lane * kEpiPitch);
-            if constexpr (EPI != kEpiGeluBwd) {
+            if (EPI == kEpiGroup && ea.demb != nullptr) {
+                // one row's 32 columns at a time, a lane each: rows of one vertex meet in 32 addresses
+#pragma unroll
+                for (int i = 0; i < 8; ++i)
+                    mine[i] = make_float4(__uint_as_float(r[4 * i]), __uint_as_float(r[4 * i + 1]),
+                                          __uint_as_float(r[4 * i + 2]), __uint_as_float(r[4 * i + 3]));
+                int p = myrow < ea.m_real ? ea.pids[myrow] : 0;
+                p = p < 0 ? 0 : (p > ea.n_ids ? ea.n_ids : p);
+                __syncwarp();
+                const int rows = min(32, ea.m_real - (m0 + warp * 32));
+                for (int rr = 0; rr < rows; ++rr)
+                    atomicAdd(ea.demb + (size_t)__shfl_sync(0xffffffffu, p, rr) * 32 + lane, stg[rr * kEpiPitch + lane]);
+                __syncwarp();
+            } else if constexpr (EPI != kEpiGeluBwd) {
 #pragma unroll
                 for (int i = 0; i < 8; ++i)
                     mine[i] = make_float4(__uint_as_float(r[4 * i]), __uint_as_float(r[4 * i + 1]),
@@ -236,7 +383,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                     const int row = m0 + warp * 32 + rr;
                     float4 v = *reinterpret_cast<const float4 *>(stg + rr * kEpiPitch + q * 4);
                     v.x += bv.x; v.y += bv.y; v.z += bv.z; v.w += bv.w;
-                    if (row < M) *reinterpret_cast<float4 *>(C + (size_t)row * ldc + col) = v;
+                    if (row < M && (EPI != kEpiGroup || col < ea.n_real))
+                        *reinterpret_cast<float4 *>(C + (size_t)row * ldc + col) = v;
                 }
                 __syncwarp();
             }
@@ -300,7 +448,47 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     }
 }
 
-inline size_t smem_bytes(int BN) { return kStages * ((size_t)kTM * 128 + (size_t)BN * 128) + 1024; }
+template <int BN, int EPI>
+__global__ void __launch_bounds__(kThreads)
+gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
+               float *__restrict__ C, int ldc, int M, int K, const float *__restrict__ bias, int *err,
+               const EpiArgs ea) {
+    // kEpiHead: a CTA for each 16 rows, all of a tile's CTAs taking its product
+    const int m0 = EPI == kEpiHead ? (int)(blockIdx.x * 16 / kTM) * kTM : (int)blockIdx.x * kTM;
+    gemm_tile<BN, EPI, kStages>(&tmA, &tmB, m0, blockIdx.y * BN, C, ldc, M, K, bias, err, ea);
+}
+
+// Up to kGroup products of one launch, tiles of 128 x 32 numbered product by product
+constexpr int kGroup = 4;
+struct GroupArgs {
+    CUtensorMap a[kGroup], b[kGroup];
+    int first[kGroup + 1];        // first tile of each product; the number of tiles
+    int mt[kGroup], n0[kGroup];   // tiles along M; the first column
+    float *C[kGroup];
+    int ldc[kGroup], M[kGroup], K[kGroup], n_real[kGroup];
+    // the last product's columns go to the embedding gradients
+    float *demb;
+    const int32_t *pids;
+    int n_ids, m_real, n;
+    int *err;
+};
+__global__ void __launch_bounds__(kThreads) gemm_group_kernel(const __grid_constant__ GroupArgs g) {
+    int p = 0;
+    while (p + 1 < g.n && (int)blockIdx.x >= g.first[p + 1]) ++p;
+    const int i = (int)blockIdx.x - g.first[p];
+    EpiArgs ea;
+    ea.n_real = g.n_real[p];
+    ea.m_real = g.m_real;
+    ea.demb = p == g.n - 1 ? g.demb : nullptr;
+    ea.pids = g.pids;
+    ea.n_ids = g.n_ids;
+    gemm_tile<32, kEpiGroup, kDeepStages>(&g.a[p], &g.b[p], i % g.mt[p] * kTM, g.n0[p] + i / g.mt[p] * 32, g.C[p],
+                                          g.ldc[p], g.M[p], g.K[p], nullptr, g.err, ea);
+}
+
+inline size_t smem_bytes(int BN, int stages = kStages) {
+    return stages * ((size_t)kTM * 128 + (size_t)BN * 128) + 1024;
+}
 
 // 2-D tensor map of a row-major bf16 matrix (rows x cols, row pitch ld elements,
 // 16 B aligned): boxes of 64 columns x box_rows rows, 128 B swizzle, zero outside.
