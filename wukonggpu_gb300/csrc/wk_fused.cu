@@ -21,7 +21,7 @@
 // through it in 130 us on 12M rows of 4 columns, a third of it look-ups).
 //
 // Two kernels and a host round trip before, this launch after, us a call:
-// k2u on 12M rows of 4 columns 163 -> 138, k2k on 10M rows of 3 105.7 -> 89,
+// k2u on 12M rows of 4 columns 163 -> 138 (132 since), k2k on 10M rows of 3 105.7 -> 89,
 // k2c on 3M rows of 6 49 -> 42; k2u on 50k rows of 6 about 49 -> 22.  A
 // single pass with a decoupled look-back was slower (177 / 139 / 65): every tile
 // waited for the slowest load among the 300 tiles in flight before it.
@@ -286,7 +286,9 @@ __device__ __forceinline__ unsigned int blocks_before(const Fused &a, int64_t b)
 }
 
 // Write block b of a k2u op: its matched rows with the neighbour appended,
-// packed in shared memory at the output's 16 B phase and stored as vectors.
+// packed in shared memory at the output's 16 B phase; its whole vectors leave
+// by the copy engine, which spares the load-store unit the look-ups need (12M
+// rows of 4 columns 138 -> 132 us a step).
 // The rows are loaded before the wait for the groups: nearly every row of a
 // functional step is kept, and they are in L2.  False when the wait ran out.
 template <int C>
@@ -347,17 +349,22 @@ __device__ __forceinline__ bool write_k2u(const Fused &a, int64_t b, WaitShared 
         }
         at += (unsigned)__popc(m[q]);
     }
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     __syncthreads();
     int32_t *o = a.out + (P * W - (unsigned)lead);
-    for (int i = 4 * t; i < end; i += 4 * kThreads) {
-        if (i >= lead && i + 4 <= end) {
-            __stcs(reinterpret_cast<int4 *>(o + i), *reinterpret_cast<const int4 *>(buf + i));
-        } else {
-#pragma unroll
-            for (int j = 0; j < 4; ++j)
-                if (i + j >= lead && i + j < end) o[i + j] = buf[i + j];
-        }
+    const int i0 = (lead + 3) & ~3, i1 = end & ~3;   // whole vectors: the copy engine's
+    if (t == 0 && i1 > i0) {
+        uint64_t first;
+        asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(first));
+        asm volatile("cp.async.bulk.global.shared::cta.bulk_group.L2::cache_hint [%0], [%1], %2, %3;\n\t"
+                     "cp.async.bulk.commit_group;" ::"l"(o + i0), "r"((uint32_t)__cvta_generic_to_shared(buf + i0)),
+                     "r"((uint32_t)(i1 - i0) * 4u), "l"(first)
+                     : "memory");
     }
+    // the words before and behind them, at most three each
+    if (t < 4 && lead + t < i0 && lead + t < end) o[lead + t] = buf[lead + t];
+    if (t >= 4 && t < 8 && i1 + t - 4 < end && i1 >= i0) o[i1 + t - 4] = buf[i1 + t - 4];
+    if (t == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");   // the buffer goes with the CTA
     return true;
 }
 
