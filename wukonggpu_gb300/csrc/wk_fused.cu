@@ -21,8 +21,8 @@
 // through it in 130 us on 12M rows of 4 columns, a third of it look-ups).
 //
 // Two kernels and a host round trip before, this launch after, us a call:
-// k2u on 12M rows of 4 columns 163 -> 138 (132 since), k2k on 10M rows of 3 105.7 -> 89,
-// k2c on 3M rows of 6 49 -> 42; k2u on 50k rows of 6 about 49 -> 22.  A
+// k2u on 12M rows of 4 columns 163 -> 138 (132 since), k2k on 10M rows of 3 105.7 -> 99,
+// k2c on 3M rows of 6 49 -> 47; k2u on 50k rows of 6 about 49 -> 22.  A
 // single pass with a decoupled look-back was slower (177 / 139 / 65): every tile
 // waited for the slowest load among the 300 tiles in flight before it.
 //
@@ -34,8 +34,9 @@
 // Per-block counts and per-group sums are those of the two-kernel ops: a
 // group's word holds its counted blocks (low 16 bits) and kept rows.  One CTA
 // placed behind the last count waits for every group and writes the op's
-// totals into pinned host memory, so that the host goes on while the last
-// blocks are still written.
+// totals into pinned host memory, so that the host goes on while a k2u op's last
+// blocks are still written.  A filter's host waits for every kept row too: a
+// caller may reuse the input of a k2k or k2c op as soon as it returns.
 #include "wk_kernels.h"
 #include "wk_probe.cuh"
 
@@ -73,6 +74,7 @@ struct Fused {
     unsigned int *blk_nz;         // kept rows per block
     unsigned long long *gs;       // two words per group, zero at launch
     int *err;
+    unsigned long long *written;  // filter: write CTAs done
     unsigned long long *clear;    // the other sums buffer, cleared for the next op
     int64_t nclear;
     int32_t *out;
@@ -368,9 +370,10 @@ __device__ __forceinline__ bool write_k2u(const Fused &a, int64_t b, WaitShared 
     return true;
 }
 
-// Write a filter's octet of blocks, one per warp: the block's kept rows from
-// its mask words, its output words as vectors, each gathered from its row.
-template <int CT>
+// Write a filter's blocks: the block's kept rows from its mask words, its
+// output words as vectors, each gathered from its row.  An octet of blocks a
+// CTA, one per warp; or, PB, one block by the whole CTA (filter_per_block).
+template <int CT, bool PB>
 __device__ __forceinline__ void write_filter(const Fused &a, int64_t b0, unsigned long long P, uint16_t *sel,
                                              unsigned int *s_nz, unsigned int *s_b) {
     const int C = CT > 0 ? CT : a.C;
@@ -381,10 +384,11 @@ __device__ __forceinline__ void write_filter(const Fused &a, int64_t b0, unsigne
     __syncthreads();
 #pragma unroll
     for (int i = 0; i < kThreads / 32; ++i) P += s_b[i];
-    for (int i = 0; i < w; ++i) P += s_nz[i];
-    const unsigned int nb = s_nz[w];
-    if (nb == 0u) return;   // the warp's block keeps nothing (or lies past the table)
-    const int64_t r0 = (b0 + w) * kRowsPerBlock;
+    if constexpr (!PB)
+        for (int i = 0; i < w; ++i) P += s_nz[i];
+    const unsigned int nb = s_nz[PB ? 0 : w];
+    if (nb == 0u) return;   // the block keeps nothing (or lies past the table)
+    const int64_t r0 = (PB ? b0 : b0 + w) * kRowsPerBlock;
     const int64_t wi = (r0 >> 5) + lane, nwords = (a.R + 31) >> 5;
     uint32_t m = wi < nwords ? __ldcg(a.mask + wi) : 0u;   // bits past R are 0
     const unsigned int c = __popc(m);
@@ -395,17 +399,19 @@ __device__ __forceinline__ void write_filter(const Fused &a, int64_t b0, unsigne
         if (lane >= o) pos += v;
     }
     pos -= c;
-    uint16_t *ws = sel + w * kRowsPerBlock;
+    uint16_t *ws = PB ? sel : sel + w * kRowsPerBlock;
+    if (PB && lane / (32 / (kThreads / 32)) != w) m = 0u;   // each warp lists its four words' rows
     while (m) {
         ws[pos++] = (uint16_t)(lane * 32 + __ffs(m) - 1);
         m &= m - 1u;
     }
-    __syncwarp();
+    if constexpr (PB) __syncthreads();
+    else __syncwarp();
     const int32_t *hb = a.hist + r0 * C;
     const uint32_t words = nb * (uint32_t)C;
     const uint32_t lead = (uint32_t)((P * (unsigned long long)C) & 3ull);
     int32_t *gout = a.out + (P * (unsigned long long)C - lead);
-    for (uint32_t u = (uint32_t)lane; 4u * u < lead + words; u += 32u) {
+    for (uint32_t u = (uint32_t)(PB ? t : lane); 4u * u < lead + words; u += PB ? kThreads : 32u) {
         int32_t v[4];
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
@@ -424,12 +430,13 @@ __device__ __forceinline__ void write_filter(const Fused &a, int64_t b0, unsigne
     }
 }
 
-// CT columns (0: any, filters only).  BPC: blocks per count CTA.
-template <int CT, bool FILTER, int BPC>
+// CT columns (0: any, filters only).  BPC: blocks per count CTA.  PB (filters): a
+// block per write CTA, as k2u always.
+template <int CT, bool FILTER, int BPC, bool PB>
 __global__ void __launch_bounds__(kThreads, FILTER ? 6 : (CT <= 4 ? 6 : (CT <= 6 ? 5 : 4)))
 fused_kernel(const __grid_constant__ Fused a, const __grid_constant__ PredView pv) {
-    constexpr int NC = kOct / BPC, NW = FILTER ? 1 : kOct;
-    __shared__ __align__(16) int32_t buf[FILTER ? kOct * kRowsPerBlock / 2 : kRowsPerBlock * (CT + 1) + 4];
+    constexpr int NC = kOct / BPC, NW = PB ? kOct : 1;
+    __shared__ __align__(16) int32_t buf[FILTER ? (PB ? 1 : kOct) * kRowsPerBlock / 2 : kRowsPerBlock * (CT + 1) + 4];
     __shared__ unsigned long long s_part[kThreads / 32];
     __shared__ unsigned int s_n[BPC][kThreads / 32], s_b[kThreads / 32];
     __shared__ WaitShared s_wait;
@@ -449,7 +456,16 @@ fused_kernel(const __grid_constant__ Fused a, const __grid_constant__ PredView p
     if (role.kind == 2) {
         // every group counted: the op's totals for the host
         const int64_t ng = (a.nblk + (1 << kGroupShift) - 1) >> kGroupShift;
-        const bool ok = groups_before(a, ng, kPublishPolls, s_wait, P);
+        bool ok = groups_before(a, ng, kPublishPolls, s_wait, P);
+        if (FILTER && ok) {   // and every write CTA done
+            const unsigned long long want = PB ? (unsigned long long)a.nblk : (unsigned long long)a.steps;
+            bool all = false;
+            for (int poll = 0; poll < kPublishPolls && !all; ++poll) {
+                all = ld_acquire64(a.written) == want;
+                if (!all) __nanosleep(100);
+            }
+            ok = __syncthreads_and(all) != 0;
+        }
         unsigned long long x = 0ull;
         for (int64_t i = threadIdx.x; ok && i < ng; i += kThreads) x += __ldcg(a.gs + 2 * i + 1);
         x = warp_add(x);
@@ -472,7 +488,14 @@ fused_kernel(const __grid_constant__ Fused a, const __grid_constant__ PredView p
     bool ok;
     if constexpr (FILTER) {
         ok = groups_before(a, b >> kGroupShift, kWritePolls, s_wait, P);
-        if (ok) write_filter<CT>(a, b, P, reinterpret_cast<uint16_t *>(buf), s_n[0], s_b);
+        if (ok) {
+            write_filter<CT, PB>(a, b, P, reinterpret_cast<uint16_t *>(buf), s_n[0], s_b);
+            __syncthreads();
+            if (threadIdx.x == 0) {
+                __threadfence();
+                atomicAdd(a.written, 1ull);
+            }
+        }
     } else {
         ok = write_k2u<CT>(a, b, s_wait, buf, s_n[0], s_b);
     }
@@ -481,9 +504,9 @@ fused_kernel(const __grid_constant__ Fused a, const __grid_constant__ PredView p
 
 bool fused_takes(int C, bool filter) { return filter || C + 1 <= kFusedCols; }
 
-template <int CT, bool FILTER, int BPC>
+template <int CT, bool FILTER, int BPC, bool PB>
 static int run_fused(const Fused &a, const PredView &pv, cudaStream_t st) {
-    constexpr int NC = kOct / BPC, NW = FILTER ? 1 : kOct;
+    constexpr int NC = kOct / BPC, NW = PB ? kOct : 1;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
@@ -493,7 +516,7 @@ static int run_fused(const Fused &a, const PredView &pv, cudaStream_t st) {
     cfg.stream = st;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return (int)cudaLaunchKernelEx(&cfg, fused_kernel<CT, FILTER, BPC>, a, pv);
+    return (int)cudaLaunchKernelEx(&cfg, fused_kernel<CT, FILTER, BPC, PB>, a, pv);
 }
 
 int launch_fused(const FusedOp &op, cudaStream_t st) {
@@ -514,6 +537,7 @@ int launch_fused(const FusedOp &op, cudaStream_t st) {
     a.blk_nz = op.blk_nz;
     a.gs = op.group_sums;
     a.err = op.err;
+    a.written = op.written;
     a.clear = op.clear;
     a.nclear = op.nclear;
     a.out = op.out;
@@ -531,7 +555,7 @@ int launch_fused(const FusedOp &op, cudaStream_t st) {
     // enough of them to fill the GPU
     const bool pair = !op.filter && a.nblk >= 16 * (int64_t)op.sms;
 #define WK_FUSED(CC)                                                      \
-    case CC: return pair ? run_fused<CC, false, 2>(a, op.pv, st) : run_fused<CC, false, 1>(a, op.pv, st)
+    case CC: return pair ? run_fused<CC, false, 2, true>(a, op.pv, st) : run_fused<CC, false, 1, true>(a, op.pv, st)
     if (!op.filter) {
         switch (op.C) {
             WK_FUSED(1); WK_FUSED(2); WK_FUSED(3); WK_FUSED(4); WK_FUSED(5);
@@ -540,17 +564,20 @@ int launch_fused(const FusedOp &op, cudaStream_t st) {
         return (int)cudaErrorInvalidValue;   // not reached: fused_takes
     }
 #undef WK_FUSED
+    const bool pb = filter_per_block(a.nblk, op.sms);
+#define WK_FUSED(CC) return pb ? run_fused<CC, true, 1, true>(a, op.pv, st) : run_fused<CC, true, 1, false>(a, op.pv, st)
     switch (op.C) {
-        case 1: return run_fused<1, true, 1>(a, op.pv, st);
-        case 2: return run_fused<2, true, 1>(a, op.pv, st);
-        case 3: return run_fused<3, true, 1>(a, op.pv, st);
-        case 4: return run_fused<4, true, 1>(a, op.pv, st);
-        case 5: return run_fused<5, true, 1>(a, op.pv, st);
-        case 6: return run_fused<6, true, 1>(a, op.pv, st);
-        case 7: return run_fused<7, true, 1>(a, op.pv, st);
-        case 8: return run_fused<8, true, 1>(a, op.pv, st);
-        default: return run_fused<0, true, 1>(a, op.pv, st);
+        case 1: WK_FUSED(1);
+        case 2: WK_FUSED(2);
+        case 3: WK_FUSED(3);
+        case 4: WK_FUSED(4);
+        case 5: WK_FUSED(5);
+        case 6: WK_FUSED(6);
+        case 7: WK_FUSED(7);
+        case 8: WK_FUSED(8);
+        default: WK_FUSED(0);
     }
+#undef WK_FUSED
 }
 
 }  // namespace dev

@@ -14,6 +14,7 @@
 //   k2k/k2c : probe + membership (per-row ballot masks; per-block counts;
 //             per-group sums) -> filtered copy (per input block: output prefix
 //             from the group sums and its group's counts, selected rows copied)
+//             -> publish (the sums to the host)
 //
 // A dense functional direction takes one launch for either (wk_fused.cu).
 //
@@ -787,32 +788,28 @@ k2u_expand_func_kernel(const int32_t *__restrict__ hist, int64_t R, const int32_
 }
 
 // ------------------------------------------------------- k2k / k2c probe
-// lower_bound of `v` in the ascending list e[0..n).  Lists hold distinct ids,
-// so lower_bound is also the position where the reference's linear scan
-// (core/engine.hpp:172-179) stops; *scanned receives the entries that scan
-// touches (position + 1 on a match, n otherwise).
-__device__ __forceinline__ bool list_contains(const int32_t *__restrict__ e, uint32_t n, int32_t v,
-                                              uint32_t *scanned) {
-    uint32_t lo = 0, hi = n;
-    while (lo < hi) {
-        const uint32_t mid = (lo + hi) >> 1;
-        if (__ldg(e + mid) < v) lo = mid + 1;
-        else hi = mid;
-    }
-    const bool f = lo < n && __ldg(e + lo) == v;
-    *scanned = f ? lo + 1 : n;
-    return f;
-}
-
-// totals[0] += adjacency entries a linear scan would touch, totals[1] += rows kept.
 // One CTA per block of input rows (two blocks per CTA, with eight rounds of
-// loads in flight per lane, took 48 registers and ran slower).
+// loads in flight per lane, took 48 registers and ran slower).  Membership is
+// the lower bound of the end value in the row's ascending list.  Lists hold
+// distinct ids, so that is also the position where the reference's linear scan
+// (core/engine.hpp:172-179) stops: group_sums[2 g + 1] += the entries that scan
+// touches (position + 1 on a match, the whole list otherwise), group_sums[2 g]
+// += rows kept.
+//
+// The searches are chains of dependent reads, so a lane's rounds are searched
+// side by side, as their offsets are looked up: one after another, 422k rows of
+// 8 columns in runs of 40 took 51.1 us a step, 48.6 so, and 2.8k rows 43 and 37.6.
+template <bool DENSE>
 __global__ void __launch_bounds__(kThreads, 6)
 filter_probe_kernel(const int32_t *__restrict__ hist, int64_t R, int C, int scol, int ecol,
                     int32_t end_const, uint32_t dir, PredView pv,
                     uint32_t *__restrict__ mask, unsigned int *__restrict__ blk_nz,
                     unsigned long long *__restrict__ group_sums, unsigned long long *__restrict__ clear,
-                    int64_t nclear, unsigned long long *__restrict__ totals, int *err) {
+                    int64_t nclear, int *err) {
+    wait_prior_grid();   // before anything is read or cleared
+    // the copy behind it does not start early: its CTAs would keep to the small
+    // shared memory of this kernel's SMs, few at a time (51 -> 75 us a step on 422k
+    // rows of 8 columns)
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     // the other sums buffer, read by the previous op's write or expansion, is
     // cleared for the next op (a few hundred words at most)
@@ -827,25 +824,71 @@ filter_probe_kernel(const int32_t *__restrict__ hist, int64_t R, int C, int scol
         v[rd] = r < R ? __ldg(hist + r * C + scol) : -1;
         tg[rd] = (r < R && ecol >= 0) ? __ldg(hist + r * C + ecol) : end_const;
     }
-    unsigned int my_nz = 0u;   // kept rows (lane 0)
-    unsigned long long my_scan = 0;
-    const bool dense = (dir ? pv.rp[1] : pv.rp[0]) != nullptr;
-    const unsigned present = dense ? ~0u : may_hold(pv, dir, v);
+    // every round's list: offset and entries (none past the table)
+    uint32_t o[kRounds], d[kRounds];
+    if constexpr (DENSE) {
+        const uint32_t vmin = dir ? pv.vmin[1] : pv.vmin[0], dn = dir ? pv.dn[1] : pv.dn[0];
+        const uint32_t *rp = dir ? pv.rp[1] : pv.rp[0];
+#pragma unroll
+        for (int rd = 0; rd < kRounds; ++rd) {
+            o[rd] = d[rd] = 0u;
+            const uint32_t x = (uint32_t)v[rd] - vmin;   // wraps above dn below vmin
+            if (v[rd] > 0 && x < dn) {
+                o[rd] = __ldg(rp + x);
+                d[rd] = __ldg(rp + x + 1);
+            } else if (v[rd] == 0) {   // index key: the hash table
+                d[rd] = probe_seg(pv.buckets, pv.nmain, pv.nover, seg_key(0u, dir), &o[rd], err);
+                d[rd] += o[rd];
+            }
+        }
+#pragma unroll
+        for (int rd = 0; rd < kRounds; ++rd) d[rd] -= o[rd];
+    } else {
+        const unsigned present = may_hold(pv, dir, v);
+#pragma unroll
+        for (int rd = 0; rd < kRounds; ++rd) {
+            o[rd] = d[rd] = 0u;
+            const bool here = (present >> rd) & 1u;
+            if (__any_sync(FULL, here)) probe_warp(pv, here ? v[rd] : -1, dir, o[rd], d[rd], err);
+        }
+    }
+    // lo[rd]: the first entry not below tg[rd]
+    uint32_t lo[kRounds], hi[kRounds];
+    bool more = false;
 #pragma unroll
     for (int rd = 0; rd < kRounds; ++rd) {
-        const int64_t row0 = wrow0 + rd * 32, r = row0 + lane;
-        if (row0 >= R) break;   // warp-uniform
-        bool found = false;
-        uint32_t o = 0u, d = 0u;
-        const bool here = (present >> rd) & 1u;
-        if (__any_sync(FULL, here)) probe_warp(pv, here ? v[rd] : -1, dir, o, d, err);
-        if (r < R && d > 0u) {
-            uint32_t sc = 0;
-            found = list_contains(pv.edges + o, d, tg[rd], &sc);
-            my_scan += sc;
+        lo[rd] = 0u;
+        hi[rd] = d[rd];
+        more |= d[rd] != 0u;
+    }
+    while (more) {
+        int32_t e[kRounds];
+#pragma unroll
+        for (int rd = 0; rd < kRounds; ++rd)
+            e[rd] = lo[rd] < hi[rd] ? __ldg(pv.edges + o[rd] + ((lo[rd] + hi[rd]) >> 1)) : 0;
+        more = false;
+#pragma unroll
+        for (int rd = 0; rd < kRounds; ++rd) {
+            if (lo[rd] < hi[rd]) {
+                const uint32_t mid = (lo[rd] + hi[rd]) >> 1;
+                if (e[rd] < tg[rd]) lo[rd] = mid + 1;
+                else hi[rd] = mid;
+                more |= lo[rd] < hi[rd];
+            }
         }
+    }
+    int32_t e[kRounds];
+#pragma unroll
+    for (int rd = 0; rd < kRounds; ++rd) e[rd] = lo[rd] < d[rd] ? __ldg(pv.edges + o[rd] + lo[rd]) : 0;
+    unsigned int my_nz = 0u;   // kept rows (lane 0)
+    unsigned long long my_scan = 0ull;
+#pragma unroll
+    for (int rd = 0; rd < kRounds; ++rd) {
+        const bool found = lo[rd] < d[rd] && e[rd] == tg[rd];
+        my_scan += found ? lo[rd] + 1u : d[rd];
         const uint32_t m = __ballot_sync(FULL, found);
-        if (lane == 0) {
+        const int64_t row0 = wrow0 + rd * 32;
+        if (lane == 0 && row0 < R) {
             mask[row0 >> 5] = m;
             my_nz += __popc(m);
         }
@@ -853,17 +896,15 @@ filter_probe_kernel(const int32_t *__restrict__ hist, int64_t R, int C, int scol
     block_sum2(my_scan, my_nz);
     if (threadIdx.x == 0) {
         blk_nz[b] = my_nz;
-        if (my_scan) atomicAdd(totals, my_scan);
-        if (my_nz) {
-            atomicAdd(totals + 1, (unsigned long long)my_nz);
-            atomicAdd(group_sums + 2 * (b >> kGroupShift), (unsigned long long)my_nz);
-        }
+        unsigned long long *gs = group_sums + 2 * (b >> kGroupShift);
+        if (my_nz) atomicAdd(gs, (unsigned long long)my_nz);
+        if (my_scan) atomicAdd(gs + 1, my_scan);
     }
 }
 
 // ----------------------------------------------------------- filter write
 // A write CTA takes kWriteBlocks consecutive blocks of input rows, one per
-// warp, all in one group of 2^kGroupShift blocks.  Their output prefixes need
+// warp (or one block, filter_per_block), all in one group of 2^kGroupShift blocks.  Their output prefixes need
 // no look-back and no wait: the probe kernel added every block's kept-row
 // count into its group's sum, so the prefix of the CTA's first block is the
 // sum of the group sums before its group and of the block counts before it in
@@ -876,19 +917,20 @@ filter_probe_kernel(const int32_t *__restrict__ hist, int64_t R, int C, int scol
 constexpr int kWriteBlocks = kThreads / 32;
 static_assert(((1 << kGroupShift) % kWriteBlocks) == 0, "a write CTA's blocks share a group");
 
-template <int CT>   // the columns, or 0 for any (C_rt)
+template <int CT, bool PB>   // CT: the columns, or 0 for any (C_rt); PB: a block per CTA
 __global__ void __launch_bounds__(kThreads)
 filter_write_kernel(const int32_t *__restrict__ hist, int64_t R, int C_rt, const uint32_t *__restrict__ mask,
                     const unsigned int *__restrict__ blk_nz, const unsigned long long *__restrict__ group_sums,
                     int32_t *__restrict__ out) {
-    __shared__ uint16_t sel[kWriteBlocks][kRowsPerBlock];   // each warp's kept rows, in order
+    __shared__ uint16_t sel[PB ? 1 : kWriteBlocks][kRowsPerBlock];   // each block's kept rows, in order
     __shared__ unsigned long long s_part[kThreads / 32];
     __shared__ unsigned int s_nz[kWriteBlocks];
     const int C = CT > 0 ? CT : C_rt;
     const int t = threadIdx.x, lane = t & 31, w = t >> 5;
     const int64_t nblk = (R + kRowsPerBlock - 1) / kRowsPerBlock;
-    const int64_t b0 = (int64_t)blockIdx.x * kWriteBlocks;
+    const int64_t b0 = (int64_t)blockIdx.x * (PB ? 1 : kWriteBlocks);
     const int64_t g = b0 >> kGroupShift;
+    wait_prior_grid();
 
     // 1. the prefix of block b0, and the CTA's blocks' counts
     unsigned long long x = 0ull;
@@ -901,12 +943,13 @@ filter_write_kernel(const int32_t *__restrict__ hist, int64_t R, int C_rt, const
     unsigned long long P = 0ull;
 #pragma unroll
     for (int i = 0; i < kThreads / 32; ++i) P += s_part[i];
-    for (int i = 0; i < w; ++i) P += s_nz[i];
-    const unsigned int nb = s_nz[w];
-    if (nb == 0u) return;   // the warp's block keeps nothing (or lies past the table)
+    if constexpr (!PB)
+        for (int i = 0; i < w; ++i) P += s_nz[i];
+    const unsigned int nb = s_nz[PB ? 0 : w];
+    if (nb == 0u) return;   // the block keeps nothing (or lies past the table)
 
     // 2. the block's kept rows, in order
-    const int64_t b = b0 + w, r0 = b * kRowsPerBlock;
+    const int64_t b = PB ? b0 : b0 + w, r0 = b * kRowsPerBlock;
     const int64_t wi = (r0 >> 5) + lane, nwords = (R + 31) >> 5;
     uint32_t m = wi < nwords ? mask[wi] : 0u;   // bits past R are 0
     const unsigned int c = __popc(m);
@@ -917,19 +960,21 @@ filter_write_kernel(const int32_t *__restrict__ hist, int64_t R, int C_rt, const
         if (lane >= o) pos += v;
     }
     pos -= c;
-    uint16_t *ws = sel[w];
+    uint16_t *ws = sel[PB ? 0 : w];
+    if (PB && lane / (32 / (kThreads / 32)) != w) m = 0u;   // each warp lists its four words' rows
     while (m) {
         ws[pos++] = (uint16_t)(lane * 32 + __ffs(m) - 1);
         m &= m - 1u;
     }
-    __syncwarp();
+    if constexpr (PB) __syncthreads();
+    else __syncwarp();
 
     // 3. output words [P C, (P + nb) C) as int4 stores aligned to 16 B of out
     const int32_t *hb = hist + r0 * C;
     const uint32_t words = nb * (uint32_t)C;
     const uint32_t lead = (uint32_t)((P * (unsigned long long)C) & 3ull);
     int32_t *gout = out + (P * (unsigned long long)C - lead);
-    for (uint32_t u = (uint32_t)lane; 4u * u < lead + words; u += 32u) {
+    for (uint32_t u = (uint32_t)(PB ? t : lane); 4u * u < lead + words; u += PB ? kThreads : 32u) {
         int32_t v[4];
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
@@ -1099,16 +1144,24 @@ int preload_k2u_kernels() {
 void launch_filter_probe(const int32_t *hist, int64_t R, int C, int scol, int ecol, int32_t end_const,
                          uint32_t dir, PredView pv, uint32_t *mask, unsigned int *blk_nz,
                          unsigned long long *group_sums, unsigned long long *clear, int64_t nclear,
-                         unsigned long long *totals, int *err, cudaStream_t st) {
-    const unsigned int nb = nblocks_rows(R);
-    filter_probe_kernel<<<nb, kThreads, 0, st>>>(hist, R, C, scol, ecol, end_const, dir, pv, mask, blk_nz, group_sums,
-                                                 clear, nclear, totals, err);
+                         int *err, cudaStream_t st) {
+    cudaLaunchAttribute attr[1];
+    const cudaLaunchConfig_t cfg = dependent_launch(attr, nblocks_rows(R), st);
+    auto *k = (dir ? pv.rp[1] : pv.rp[0]) != nullptr ? filter_probe_kernel<true> : filter_probe_kernel<false>;
+    cudaLaunchKernelEx(&cfg, k, hist, R, C, scol, ecol, end_const, dir, pv, mask, blk_nz, group_sums, clear, nclear, err);
 }
 
 void launch_filter_write(const int32_t *hist, int64_t R, int C, const uint32_t *mask, const unsigned int *blk_nz,
-                         const unsigned long long *group_sums, int32_t *out, cudaStream_t st) {
-    const unsigned int g = (nblocks_rows(R) + kWriteBlocks - 1) / kWriteBlocks;
-#define WK_FWRITE(CC) filter_write_kernel<CC><<<g, kThreads, 0, st>>>(hist, R, C, mask, blk_nz, group_sums, out)
+                         const unsigned long long *group_sums, int32_t *out, int sms, cudaStream_t st) {
+    const unsigned int nb = nblocks_rows(R);
+    const bool pb = filter_per_block(nb, sms);
+    cudaLaunchAttribute attr[1];
+    const cudaLaunchConfig_t cfg = dependent_launch(attr, pb ? nb : (nb + kWriteBlocks - 1) / kWriteBlocks, st);
+#define WK_FWRITE(CC)                                                                                             \
+    do {                                                                                                          \
+        if (pb) cudaLaunchKernelEx(&cfg, filter_write_kernel<CC, true>, hist, R, C, mask, blk_nz, group_sums, out); \
+        else cudaLaunchKernelEx(&cfg, filter_write_kernel<CC, false>, hist, R, C, mask, blk_nz, group_sums, out);   \
+    } while (0)
     switch (C) {
         case 1: WK_FWRITE(1); break;
         case 2: WK_FWRITE(2); break;

@@ -93,30 +93,40 @@ void launch_k2u_expand(const int32_t *hist, int C, const int32_t *edges, const E
                        unsigned int n, const uint32_t *head, bool wide, int32_t *out, cudaStream_t st);
 
 // k2k/k2c pass 1: probe + membership of the end value; per-row ballot masks,
-// per-block kept-row counts, each added into its group's sum (group_sums[2 g],
-// 2^kGroupShift blocks a group, zero on entry); totals[0] += adjacency entries
-// a linear scan touches, totals[1] += kept rows.  The nclear words at `clear`
-// (the other sums buffer) are zeroed.
+// per-block kept-row counts; group_sums[2 g] += kept rows and
+// group_sums[2 g + 1] += adjacency entries a linear scan touches, of the
+// 2^kGroupShift blocks of group g (zero on entry).  The nclear words at `clear`
+// (the other sums buffer) are zeroed.  err bit 0: corrupt overflow chain.
 // ecol >= 0: end is column ecol (k2k); ecol < 0: end is the constant `end_const` (k2c).
 void launch_filter_probe(const int32_t *hist, int64_t R, int C, int scol, int ecol, int32_t end_const,
                          uint32_t dir, PredView pv, uint32_t *mask, unsigned int *blk_nz,
                          unsigned long long *group_sums, unsigned long long *clear, int64_t nclear,
-                         unsigned long long *totals, int *err, cudaStream_t st);
+                         int *err, cudaStream_t st);
 
 // k2k/k2c pass 2: copy the kept rows in order (out holds up to R rows of C columns).
 void launch_filter_write(const int32_t *hist, int64_t R, int C, const uint32_t *mask, const unsigned int *blk_nz,
-                         const unsigned long long *group_sums, int32_t *out, cudaStream_t st);
+                         const unsigned long long *group_sums, int32_t *out, int sms, cudaStream_t st);
+
+// Whether a filter of nblk blocks copies its kept rows with a CTA per block;
+// else with a warp per block.  A warp copies a block of 1024 rows in some 70
+// dependent steps, 35 us of them on 11 columns however few blocks there are:
+// 12k rows of 11 columns take 65.9 us with a warp per block and 30.9 with a CTA,
+// 422k rows of 8 51.9 and 36.0.  From about 16 blocks an SM on there are warps
+// enough, and the CTAs' prefixes and barriers cost more (10M rows of 3 columns
+// 99 and 120 us).
+inline bool filter_per_block(int64_t nblk, int sms) { return nblk <= 16 * (int64_t)(sms < 1 ? 1 : sms); }
 
 // k2u, k2k and k2c over a dense functional direction (pv.nb[dir] set) in one
 // launch; k2u for up to kFusedCols output columns (fused_takes).  out holds R
 // rows of C + 1 (k2u) or C columns and is 16 B aligned; nbr (k2u) holds R
 // words, mask (filters) a bit per row, blk_nz a word per block, group_sums two
-// zero words per group.  clear[0 .. nclear) is set to zero.  The op's totals go
+// zero words per group; written (filters) is a zero word.  clear[0 .. nclear) is set to zero.  The op's totals go
 // to pinned host memory: pub[2] = the error word (bit 0: corrupt overflow
 // chain, kErrWait: a wait ran out and the op has to run as two kernels),
 // pub[3] = output rows, pub[4] = k2u: not 0 when a row's start is an index key
 // (the op has to run unspecialised), filter: entries a linear scan touches;
-// then seq into pub[0].  Returns a cudaError_t.
+// then seq into pub[0], once every row is counted (k2u) or every kept row
+// copied (filters: the launch has finished with its input).  Returns a cudaError_t.
 constexpr int kFusedCols = 11;
 constexpr int kErrWait = 16;
 struct FusedOp {
@@ -132,6 +142,7 @@ struct FusedOp {
     unsigned int *blk_nz;
     unsigned long long *group_sums;
     int *err;
+    unsigned long long *written;
     unsigned long long *clear;
     int64_t nclear;
     int32_t *out;

@@ -132,8 +132,7 @@ int wait_published(wk_ctx *ctx, unsigned long long seq) {
     }
 }
 
-int fail_corrupt(wk_ctx *ctx) {
-    cudaMemsetAsync(ctx->dscal.ptr, 0, 8, ctx->stream);
+int fail_corrupt() {
     return set_error(WK_EDEVICE, "probe found an overflow chain longer than the segment's overflow area (corrupt store)");
 }
 
@@ -218,12 +217,6 @@ int take(wk_ctx *ctx, DevBuf &b, size_t bytes) {
     return b.reserve(bytes);
 }
 
-// zero the op totals (dscal[1..3]) before a first pass accumulates into them
-int clear_totals(wk_ctx *ctx) {
-    cudaError_t e = cudaMemsetAsync(ctx->dscal.as<unsigned long long>() + 1, 0, 24, ctx->stream);
-    return e == cudaSuccess ? WK_OK : cuda_fail(e, "clear totals");
-}
-
 bool alloc_failure_pending(wk_ctx *ctx) { return ctx->inject_alloc_fail.load(std::memory_order_relaxed) > 0; }
 
 // A k2u or filter op over a dense functional direction in one launch
@@ -269,6 +262,7 @@ int op_fused(wk_ctx *ctx, wk_history *h, int scol, int ecol, int32_t end_const, 
     op.blk_nz = ctx->blk_nz.as<unsigned int>();
     op.group_sums = gs + 2;
     op.err = reinterpret_cast<int *>(gs);
+    op.written = gs + 1;
     op.clear = gsum_buffer(ctx, par ^ 1);
     op.nclear = 2 + 2 * ctx->gs_used[par ^ 1];
     op.out = ob.as<int32_t>();
@@ -285,7 +279,7 @@ int op_fused(wk_ctx *ctx, wk_history *h, int scol, int ecol, int32_t end_const, 
     const unsigned long long err = ctx->h_gs[2];
     const int64_t R_out = (int64_t)ctx->h_gs[3], extra = (int64_t)ctx->h_gs[4];
     if (err & 1ull)
-        return set_error(WK_EDEVICE, "probe found an overflow chain longer than the segment's overflow area (corrupt store)");
+        return fail_corrupt();
     if ((err & (unsigned long long)dev::kErrWait) || (!filter && extra)) return WK_OK;
     if (!filter && R_out > ctx->row_limit)
         return set_error(WK_EOVERFLOW, "k2u: %lld output rows exceed the context's row limit %lld", (long long)R_out,
@@ -401,7 +395,7 @@ int op_k2u(wk_ctx *ctx, wk_history *h, int scol, uint32_t pid, uint32_t dir) {
         func = false;   // the next count adds into the other, cleared buffer
     }
     if (errf & 1)
-        return set_error(WK_EDEVICE, "probe found an overflow chain longer than the segment's overflow area (corrupt store)");
+        return fail_corrupt();
     if (errf & 2) return set_error(WK_EOVERFLOW, "k2u: 1024 consecutive input rows expand to 2^31 rows or more");
     unsigned long long rows_out = 0ull, slices = 0ull;
     for (int64_t g = 0; g < groups; ++g) {
@@ -474,37 +468,38 @@ int op_filter(wk_ctx *ctx, wk_history *h, int scol, int ecol, int32_t end_const,
     const int64_t nblk = (R + dev::kRowsPerBlock - 1) / dev::kRowsPerBlock;
     const int64_t groups = (nblk + (1 << dev::kGroupShift) - 1) >> dev::kGroupShift;
     if ((st = take(ctx, ctx->mask, (size_t)((R + 31) / 32) * 4)) || (st = take(ctx, ctx->blk_nz, (size_t)nblk * 4)) ||
-        (st = reserve_gsum(ctx, groups)) || (st = take(ctx, ob, (size_t)R * C * 4)) || (st = clear_totals(ctx)))
+        (st = reserve_gsum(ctx, groups)) || (st = take(ctx, ob, (size_t)R * C * 4)))
         return st;
-    unsigned long long *tot = ctx->dscal.as<unsigned long long>() + 1;
-    int *err = ctx->dscal.as<int>();
-    // the block counts' group sums go to one of the two sums buffers k2u uses,
-    // and the probe clears the other
+    // as in a k2u op: the error word and the group sums in one of two buffers,
+    // the other cleared for the next op, and the sums to the host through pinned
+    // memory, here behind the copy of the kept rows: the op has finished with its
+    // input when it returns
     const int par = ctx->gs_par;
-    unsigned long long *gs = gsum_buffer(ctx, par) + 2;
+    unsigned long long *gs = gsum_buffer(ctx, par);
     if ((st = clk.begin())) return st;
     dev::launch_filter_probe(h->data, R, C, scol, ecol, end_const, dir, pv, ctx->mask.as<uint32_t>(),
-                             ctx->blk_nz.as<unsigned int>(), gs, gsum_buffer(ctx, par ^ 1),
-                             2 + 2 * ctx->gs_used[par ^ 1], tot, err, ctx->stream);
+                             ctx->blk_nz.as<unsigned int>(), gs + 2, gsum_buffer(ctx, par ^ 1),
+                             2 + 2 * ctx->gs_used[par ^ 1], reinterpret_cast<int *>(gs), ctx->stream);
     if ((st = launch_check("filter probe"))) return st;
     ctx->gs_par = par ^ 1;
     ctx->gs_used[par ^ 1] = 0;
     ctx->gs_used[par] = groups;
     if ((st = clk.end(true)) || (st = clk.begin())) return st;
-    dev::launch_filter_write(h->data, R, C, ctx->mask.as<uint32_t>(), ctx->blk_nz.as<unsigned int>(), gs,
-                             ob.as<int32_t>(), ctx->stream);
+    dev::launch_filter_write(h->data, R, C, ctx->mask.as<uint32_t>(), ctx->blk_nz.as<unsigned int>(), gs + 2,
+                             ob.as<int32_t>(), ctx->sms, ctx->stream);
     if ((st = launch_check("filter write")) || (st = clk.end(false))) return st;
-    // the error word and totals come to the host through pinned memory, as a
-    // k2u op's group sums do
-    const dev::Publish pub{ctx->dscal.as<unsigned long long>(), ctx->h_gs_dev, 4, ++ctx->pub_seq};
+    const dev::Publish pub{gs, ctx->h_gs_dev, 2 + 2 * groups, ++ctx->pub_seq};
     dev::launch_publish(pub, dev::SlicePlan{}, ctx->stream);
     if ((st = launch_check("filter publish"))) return st;
     ++ctx->launches;
     ++ctx->last.kernels;
     if ((st = wait_published(ctx, pub.seq))) return st;
-    if (ctx->h_gs[2] & 0xffffffffull) return fail_corrupt(ctx);
-    const int64_t E = (int64_t)ctx->h_gs[3];
-    const int64_t nz = (int64_t)ctx->h_gs[4];
+    if (ctx->h_gs[2] & 0xffffffffull) return fail_corrupt();
+    int64_t nz = 0, E = 0;
+    for (int64_t g = 0; g < groups; ++g) {
+        nz += (int64_t)ctx->h_gs[4 + 2 * g];
+        E += (int64_t)ctx->h_gs[5 + 2 * g];
+    }
     clk.finish();
     ctx->last.rows_out = nz;
     ctx->last.alg_bytes = 4 * R * C + 16 * R + 4 * E + 4 * nz * C;
