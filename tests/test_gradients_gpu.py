@@ -33,3 +33,16 @@ def test_gradients_after_a_larger_batch(gpu_small, M):
     for a, b in zip(np.r_[0, ends[:-1]], ends):
         x, y = g_gpu[a:b].astype(np.float64), g_ref[a:b].astype(np.float64)
         assert np.linalg.norm(x - y) <= 0.005 * np.linalg.norm(y) + 1e-6, (a, b)
+
+
+@pytest.mark.parametrize("n", [1023, 1024, 1025, 16383, 16384, 16385])
+def test_predictions_at_the_copy_limits(gpu_small, n):
+    """features through the pinned block up to 1024 samples, ids and outputs up to 16,384: the same bits in pieces"""
+    est = W.Estimator(gpu_small, 26, max_batch=64, seed=5)
+    rng = np.random.default_rng(n)
+    feats = rng.normal(0, 1, size=(n, 48)).astype(np.float32)
+    pids = rng.integers(-1, 28, size=n).astype(np.int32)
+    whole = est.predict(feats, pids)
+    cut = [0, 100, n // 2, n - 7, n]
+    parts = [est.predict(feats[a:b], pids[a:b]) for a, b in zip(cut, cut[1:])]
+    assert np.array_equal(whole, np.concatenate(parts))

@@ -53,31 +53,40 @@ constexpr float kB1 = 0.9f, kB2 = 0.999f;   // Adam moment decay rates
 
 // ------------------------------------------------------------ elementwise
 // X0 [Mp x 80] bf16 = [feats | emb[pid]] for real rows, 0 for padding, and its
-// transpose, 32 rows a CTA; and the words that the step adds into, cleared.
+// transpose, 32 rows a CTA; the ids and targets, which may lie in host memory,
+// brought to the device (pids_to and tgt_to, or in place); and the words that
+// the step adds into, cleared.
 __global__ void __launch_bounds__(256)
-build_input_kernel(const float *__restrict__ feats, const int32_t *__restrict__ pids, int M, int Mp,
+build_input_kernel(const float *__restrict__ feats, const int32_t *pids, const float *tgt,
+                   int32_t *pids_to, float *tgt_to, int M, int Mp,
                    const float *__restrict__ emb, int n_ids, __nv_bfloat16 *__restrict__ X0,
                    __nv_bfloat16 *__restrict__ X0t, float *__restrict__ zero, int64_t nzero, int *done) {
     __shared__ __nv_bfloat16 tile[kX][34];   // 17 words a column: the transposing reads and writes spread over the banks
+    __shared__ int s_pid[32];
     asm volatile("griddepcontrol.launch_dependents;");
     asm volatile("griddepcontrol.wait;" ::: "memory");
     const int r0 = blockIdx.x * 32, t = threadIdx.x;
-    for (int i = t; i < 32 * kX; i += 256) {
-        const int r = i / kX, c = i % kX, row = r0 + r;
-        float v = 0.f;
-        if (row < M) {
-            if (c < kIn) v = feats[(size_t)row * kIn + c];
-            else {
-                int p = pids[row];
-                p = p < 0 ? 0 : (p > n_ids ? n_ids : p);
-                v = emb[(size_t)p * kEmb + (c - kIn)];
-            }
-        }
-        const __nv_bfloat16 bv = __float2bfloat16(v);
-        X0[(size_t)r0 * kX + i] = bv;
-        tile[c][r] = bv;
+    if (t < 32 && r0 + t < M) {
+        const int p = pids[r0 + t];
+        s_pid[t] = p < 0 ? 0 : (p > n_ids ? n_ids : p);
+        pids_to[r0 + t] = p;
+        tgt_to[r0 + t] = tgt[r0 + t];
+    }
+    float fv[32 * kIn / 256];   // the features, in flight with the ids
+#pragma unroll
+    for (int q = 0; q < 32 * kIn / 256; ++q) {
+        const int i = q * 256 + t;
+        fv[q] = r0 + i / kIn < M ? feats[(size_t)r0 * kIn + i] : 0.f;
     }
     __syncthreads();
+#pragma unroll
+    for (int q = 0; q < 32 * kIn / 256; ++q) tile[(q * 256 + t) % kIn][(q * 256 + t) / kIn] = __float2bfloat16(fv[q]);
+    for (int i = t; i < 32 * kEmb; i += 256) {
+        const int r = i / kEmb, c = i % kEmb;
+        tile[kIn + c][r] = __float2bfloat16(r0 + r < M ? emb[(size_t)s_pid[r] * kEmb + c] : 0.f);
+    }
+    __syncthreads();
+    for (int i = t; i < 32 * kX; i += 256) X0[(size_t)r0 * kX + i] = tile[i % kX][i / kX];
     for (int i = t; i < 32 * kX; i += 256) X0t[(size_t)(i / 32) * Mp + r0 + i % 32] = tile[i / 32][i % 32];
     for (int64_t i = (int64_t)blockIdx.x * 256 + t; i < nzero; i += (int64_t)gridDim.x * 256) zero[i] = 0.f;
     if (blockIdx.x == 0 && t == 0) *done = 0;
@@ -318,12 +327,13 @@ int check_status(wk_mlp *m, cudaStream_t s, const char *what, bool copied = fals
     return WK_OK;
 }
 
-// Calls of up to kSmallRows samples go through the pinned block, which the
-// kernel reads and writes in place: one host copy of at most 100 KB instead of
-// two device copies in and one out, each some 10 us whatever it holds.
-constexpr int kSmallRows = 512;
-constexpr size_t kSmallPids = sizeof(float) * kIn * kSmallRows, kSmallOut = kSmallPids + sizeof(int32_t) * kSmallRows;
-constexpr size_t kSmallBytes = kSmallOut + sizeof(float) * kSmallRows;
+// The pinned block of small calls, which the kernels read and write in place: a
+// copy to or from the caller's memory holds the host for some 14 us whatever its
+// size.  The features of up to kSmallRows samples go through it (100 KB in 6 us
+// on the host), ids, targets and predictions of up to kMidRows.
+constexpr int kSmallRows = 1024, kMidRows = 16384;
+constexpr size_t kSmallPids = sizeof(float) * kIn * kSmallRows, kSmallOut = kSmallPids + sizeof(int32_t) * kMidRows;
+constexpr size_t kSmallBytes = kSmallOut + sizeof(float) * kMidRows;
 
 // predictions for n samples in device-readable memory (wk_mlp_forward.cuh)
 void predict(wk_mlp *m, const float *feats, const int32_t *pids, int64_t n, float *out, cudaStream_t s) {
@@ -400,13 +410,13 @@ void gradient_group(wk_mlp *m, int M, int Mp, cudaStream_t s) {
     m->kernels++;
 }
 
-// The loss and every gradient for M rows already uploaded (feats, pids, tgt).
-void gradient_step(wk_mlp *m, int M, cudaStream_t s) {
+// The loss and every gradient for M rows of device-readable feats, pids and tgt
+// (the latter two brought to m->pids and m->tgt).
+void gradient_step(wk_mlp *m, const float *feats, const int32_t *pids, const float *tgt, int M, cudaStream_t s) {
     const int Mp = pad64(M);
     float *g = m->grads;
     // w4's gradient, the biases' and the embedding's are added into; they lie together
-    launch_ahead(build_input_kernel, dim3((unsigned)(Mp / 32)), 256, 0, s, (const float *)m->feats,
-                 (const int32_t *)m->pids, M, Mp, (const float *)(m->params + m->off_emb), m->n_ids, m->x0, m->x0t,
+    launch_ahead(build_input_kernel, dim3((unsigned)(Mp / 32)), 256, 0, s, feats, pids, tgt, m->pids, m->tgt, M, Mp, (const float *)(m->params + m->off_emb), m->n_ids, m->x0, m->x0t,
                  g + m->off_w[3], m->n_params - m->off_w[3], m->done);
     m->kernels++;
     const __nv_bfloat16 *in = m->x0;
@@ -452,13 +462,6 @@ void update(wk_mlp *m, float lr, cudaStream_t s) {
                                                   m->cbias, m->bidx);
     m->kernels++;
     refresh_bf16(m, s);
-}
-
-int upload(wk_mlp *m, const float *feats, const int32_t *pids, const float *tgt, int M, cudaStream_t s) {
-    cudaError_t e = cudaMemcpyAsync(m->feats, feats, sizeof(float) * (size_t)M * kIn, cudaMemcpyHostToDevice, s);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(m->pids, pids, sizeof(int32_t) * (size_t)M, cudaMemcpyHostToDevice, s);
-    if (e == cudaSuccess && tgt) e = cudaMemcpyAsync(m->tgt, tgt, sizeof(float) * (size_t)M, cudaMemcpyHostToDevice, s);
-    return e == cudaSuccess ? WK_OK : cuda_fail(e, "mlp upload");
 }
 
 void free_mlp(wk_mlp *m) {
@@ -601,10 +604,28 @@ extern "C" int wk_mlp_gradients(wk_mlp *m, const float *feats, const int32_t *pi
     if (!m || !feats || !pids || !tgt || M < 1 || M > m->cap_m) return set_error(WK_EINVAL, "wk_mlp_gradients");
     cudaSetDevice(m->ctx->device);
     cudaStream_t s = m->ctx->stream;
-    int st = upload(m, feats, pids, tgt, M, s);
-    if (st) return st;
-    gradient_step(m, M, s);
-    cudaError_t e = cudaGetLastError();
+    int st;
+    cudaError_t e = cudaSuccess;
+    const float *f = m->feats, *t = m->tgt;
+    const int32_t *p = m->pids;
+    if (M <= kSmallRows) {
+        std::memcpy(m->h_small, feats, sizeof(float) * (size_t)M * kIn);
+        f = reinterpret_cast<const float *>(m->h_small_dev);
+    } else {
+        e = cudaMemcpyAsync(m->feats, feats, sizeof(float) * (size_t)M * kIn, cudaMemcpyHostToDevice, s);
+    }
+    if (M <= kMidRows) {
+        std::memcpy(m->h_small + kSmallPids, pids, sizeof(int32_t) * (size_t)M);
+        std::memcpy(m->h_small + kSmallOut, tgt, sizeof(float) * (size_t)M);
+        p = reinterpret_cast<const int32_t *>(m->h_small_dev + kSmallPids);
+        t = reinterpret_cast<const float *>(m->h_small_dev + kSmallOut);
+    } else {
+        if (e == cudaSuccess) e = cudaMemcpyAsync(m->pids, pids, sizeof(int32_t) * (size_t)M, cudaMemcpyHostToDevice, s);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(m->tgt, tgt, sizeof(float) * (size_t)M, cudaMemcpyHostToDevice, s);
+    }
+    if (e != cudaSuccess) return cuda_fail(e, "mlp upload");
+    gradient_step(m, f, p, t, M, s);
+    e = cudaGetLastError();
     // the status first: the copy to the caller's memory holds the host until it is done
     if (e == cudaSuccess) e = copy_status(m, s);
     if (e == cudaSuccess && grads_host)
@@ -667,7 +688,7 @@ extern "C" int wk_mlp_train(wk_mlp *m, const float *feats, const int32_t *pids, 
         gather_batch_kernel<<<nblk((int64_t)M * kIn), 256, 0, s>>>(d_feats.as<float>(), d_pids.as<int32_t>(),
                                                                    d_tgt.as<float>(), d_order.as<int64_t>(), m->bidx,
                                                                    batch, M, m->feats, m->pids, m->tgt);
-        gradient_step(m, M, s);
+        gradient_step(m, m->feats, m->pids, m->tgt, M, s);
         update(m, lr, s);
         bump_kernel<<<1, 1, 0, s>>>(m->bidx);
         m->kernels += 2;   // gather, bump
@@ -725,18 +746,25 @@ extern "C" int wk_mlp_train(wk_mlp *m, const float *feats, const int32_t *pids, 
 }
 
 // Predictions (log(1 + rows)) for n samples: a small call through the pinned
-// block, a larger one in chunks of two tiles per SM, whose copies in run on
+// block, up to kMidRows samples with their features copied, more in chunks of two tiles per SM, whose copies in run on
 // their own stream while the chunk before is computed.
 extern "C" int wk_mlp_predict(wk_mlp *m, const float *feats, const int32_t *pids, int64_t n, float *out) {
     if (!m || (n > 0 && (!feats || !pids || !out)) || n < 0) return set_error(WK_EINVAL, "wk_mlp_predict");
     cudaSetDevice(m->ctx->device);
     cudaStream_t s = m->ctx->stream;
     int st = WK_OK;
-    if (n > 0 && n <= kSmallRows) {
-        std::memcpy(m->h_small, feats, sizeof(float) * (size_t)n * kIn);
+    if (n > 0 && n <= kMidRows) {
+        const float *f = reinterpret_cast<const float *>(m->h_small_dev);
+        if (n <= kSmallRows) {
+            std::memcpy(m->h_small, feats, sizeof(float) * (size_t)n * kIn);
+        } else {
+            if ((st = m->stage[0].reserve(sizeof(float) * (size_t)n * kIn))) return st;
+            const cudaError_t e = cudaMemcpyAsync(m->stage[0].ptr, feats, sizeof(float) * (size_t)n * kIn, cudaMemcpyHostToDevice, s);
+            if (e != cudaSuccess) return cuda_fail(e, "wk_mlp_predict");
+            f = m->stage[0].as<float>();
+        }
         std::memcpy(m->h_small + kSmallPids, pids, sizeof(int32_t) * (size_t)n);
-        predict(m, reinterpret_cast<const float *>(m->h_small_dev),
-                reinterpret_cast<const int32_t *>(m->h_small_dev + kSmallPids), n,
+        predict(m, f, reinterpret_cast<const int32_t *>(m->h_small_dev + kSmallPids), n,
                 reinterpret_cast<float *>(m->h_small_dev + kSmallOut), s);
         if ((st = check_status(m, s, "wk_mlp_predict"))) return st;
         std::memcpy(out, m->h_small + kSmallOut, sizeof(float) * (size_t)n);
