@@ -153,6 +153,32 @@ struct FusedOp {
 bool fused_takes(int C, bool filter);
 int launch_fused(const FusedOp &op, cudaStream_t st);
 
+// A request of up to kLightSteps steps from a list of at most kLightRows rows in
+// one launch of one CTA (wk_light.cu).  The list's table goes to buf[0], step i's
+// to buf[(i + 1) & 1]; each holds kLightRows rows of the widest table.  The host
+// gets pub[2] = the error word (bit 0: corrupt overflow chain), pub[3] = steps
+// done (the next one's output has more than kLightRows rows, or than row_limit),
+// pub[4] = entries a linear scan touches in the last filter done, pub[kLightWords
+// + i] = rows after step i; then seq in pub[0].
+constexpr int kLightRows = 2048, kLightSteps = 8, kLightWords = 6;
+enum { kLightK2U, kLightFilter };
+struct LightStep {
+    PredView pv;
+    int kind, C, scol, ecol;   // C: input columns; filters: ecol < 0 for end_const
+    int32_t end_const;
+    uint32_t dir;
+};
+struct LightOp {
+    int n, deg;
+    const int32_t *src;
+    int32_t *buf[2];
+    long long row_limit;
+    unsigned long long *pub;
+    unsigned long long seq;
+    LightStep s[kLightSteps];
+};
+void launch_light(const LightOp &op, cudaStream_t st);
+
 // Copy an adjacency list (index or constant start) into a one-column table.
 void launch_copy_list(const int32_t *src, int64_t n, int32_t *dst, cudaStream_t st);
 

@@ -614,6 +614,98 @@ static int vtype(int64_t v, int col_num) {   // 0 known, 1 unknown, 2 const
     return (-v > col_num) ? 1 : 0;
 }
 
+// Run a request's first steps as a light query (wk_light.cu) when it starts from
+// a short list: *done receives the patterns done, the start among them, and h the
+// table after them (0: nothing was run).  Not taken: a paged store, which loads
+// segments step by step; timing, which times each step; anything the steps' own
+// checks would refuse, which is left for them to refuse.
+static int execute_light(wk_ctx *ctx, const int64_t *cmd, int32_t n, wk_history *h, int64_t *step_rows, int *done) {
+    *done = 0;
+    DeviceStore &ds = *ctx->store;
+    if (ds.pool || ctx->timing || alloc_failure_pending(ctx) || n < 2 || n > dev::kLightSteps + 1) return WK_OK;
+    const auto pid_ok = [&](int64_t pid, int64_t d) {
+        return pid >= 1 && pid <= ds.hs->num_ids && (d == WK_DIR_IN || d == WK_DIR_OUT);
+    };
+    const int64_t start = cmd[0];
+    const bool index = is_tpid(start);
+    const int64_t lpid = index ? start : cmd[1];
+    if (cmd[3] != -1 || start < 0 || start > 0xffffffffll || !pid_ok(lpid, cmd[2]) || (!index && start < WK_VID_BASE)) return WK_OK;
+    const int32_t *e = nullptr;
+    const uint64_t deg = ds.hs->lookup(index ? 0ull : (uint64_t)start, (uint32_t)lpid, (uint32_t)cmd[2], &e);
+    if (deg == 0 || deg > (uint64_t)dev::kLightRows) return WK_OK;
+    dev::LightOp op;
+    op.n = n - 1;
+    op.deg = (int)deg;
+    int cols = 1;
+    for (int i = 1; i < n; ++i) {
+        const int64_t *c = cmd + 4 * i;
+        if (!pid_ok(c[1], c[2]) || vtype(c[0], cols) != 0) return WK_OK;
+        dev::LightStep &s = op.s[i - 1];
+        s.pv = ds.views[(size_t)c[1]];
+        s.C = cols;
+        s.scol = (int)(-c[0] - 1);
+        s.ecol = -1;
+        s.end_const = 0;
+        s.dir = (uint32_t)c[2];
+        const int te = vtype(c[3], cols);
+        s.kind = te == 1 ? dev::kLightK2U : dev::kLightFilter;
+        if (te == 1) {
+            if (-c[3] - 1 != cols) return WK_OK;
+            ++cols;
+        } else if (te == 0) {
+            s.ecol = (int)(-c[3] - 1);
+        } else {
+            if (c[3] > 0x7fffffffll) return WK_OK;
+            s.end_const = (int32_t)c[3];
+        }
+    }
+    int st;
+    const size_t bytes = (size_t)dev::kLightRows * (size_t)cols * 4;
+    if ((st = take(ctx, ctx->hbuf[0], bytes)) || (st = take(ctx, ctx->hbuf[1], bytes)) ||
+        (st = wk::reserve_published(ctx, dev::kLightWords + dev::kLightSteps)))
+        return st;
+    op.src = ds.views[(size_t)lpid].edges + (e - (ds.hs->edges + ds.hs->segs[lpid].edge_off));
+    op.buf[0] = ctx->hbuf[0].as<int32_t>();
+    op.buf[1] = ctx->hbuf[1].as<int32_t>();
+    op.row_limit = ctx->row_limit;
+    op.pub = ctx->h_gs_dev;
+    op.seq = ++ctx->pub_seq;
+    dev::launch_light(op, ctx->stream);
+    if ((st = launch_check("light query"))) return st;
+    ++ctx->launches;
+    if ((st = wait_published(ctx, op.seq))) return st;
+    if (ctx->h_gs[2] & 1ull) return fail_corrupt();
+    const int k = (int)ctx->h_gs[3];   // steps behind the start
+    h->data = op.buf[k & 1];
+    h->col_num = k == 0 ? 1 : op.s[k - 1].C + (op.s[k - 1].kind == dev::kLightK2U ? 1 : 0);
+    h->step = k + 1;
+    int64_t rows = (int64_t)deg, rows_in = 1;
+    if (step_rows) step_rows[0] = rows;
+    for (int i = 0; i < k; ++i) {
+        rows_in = rows;
+        rows = (int64_t)ctx->h_gs[dev::kLightWords + i];
+        if (step_rows) step_rows[i + 1] = rows;
+    }
+    h->size = rows * h->col_num;
+    ctx->last = wk_op_stats{};
+    ctx->last.rows_in = rows_in;
+    ctx->last.rows_out = rows;
+    ctx->last.kernels = 1;
+    if (k == 0) {
+        ctx->last.kind = index ? KIND_I2U : KIND_C2U;
+        ctx->last.alg_bytes = 16 + 8 * rows;
+    } else {
+        const dev::LightStep &s = op.s[k - 1];
+        ctx->last.cols_in = s.C;
+        ctx->last.kind = s.kind == dev::kLightK2U ? KIND_K2U : (s.ecol >= 0 ? KIND_K2K : KIND_K2C);
+        ctx->last.alg_bytes = 4 * rows_in * s.C + 16 * rows_in +
+                              (s.kind == dev::kLightK2U ? 4 * rows + 4 * rows * (s.C + 1)
+                                                        : 4 * (int64_t)ctx->h_gs[4] + 4 * rows * s.C);
+    }
+    *done = k + 1;
+    return WK_OK;
+}
+
 extern "C" int wk_execute(wk_ctx *ctx, const int64_t *cmd, int32_t n, wk_history *h, int64_t *step_rows) {
     if (!ctx || !cmd || !h || n <= 0) return set_error(WK_EINVAL, "wk_execute: bad arguments");
     if (!ctx->store) return set_error(WK_ENOSTORE, "wk_execute: no store");
@@ -623,8 +715,9 @@ extern "C" int wk_execute(wk_ctx *ctx, const int64_t *cmd, int32_t n, wk_history
     ctx->query_rest.clear();
     ctx->qstats.clear();
     DeviceStore &ds = *ctx->store;
-    int st = WK_OK;
-    for (int i = 0; i < n && st == WK_OK; ++i) {
+    int first = 0;
+    int st = execute_light(ctx, cmd, n, h, step_rows, &first);
+    for (int i = first; i < n && st == WK_OK; ++i) {
         const int64_t start = cmd[i * 4], pid = cmd[i * 4 + 1], d = cmd[i * 4 + 2], end = cmd[i * 4 + 3];
         if (ds.pool) {
             // the segments of steps i.. (an index start's segment is its index id)

@@ -313,11 +313,11 @@ wk_ctx::~wk_ctx() {
     if (stream) cudaStreamSynchronize(stream);
     for (auto &b : hbuf) b.release();
     deg.release(); off.release(); mask.release(); blk_sum.release(); blk_nz.release();
-    dscal.release();
     part_cnt.release();
     part_scan.release();
     if (h_scal) cudaFreeHost(h_scal);
     if (h_gs) cudaFreeHost(h_gs);
+    if (h_stage) cudaFreeHost(h_stage);
     for (auto &e : tev) cudaEventDestroy(e);
     if (use_ready) cudaEventDestroy(use_ready);
     if (tm0) cudaEventDestroy(tm0);
@@ -366,7 +366,8 @@ extern "C" int wk_ctx_create(const wk_config *cfg_in, wk_ctx **out) {
     if ((e = cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking)) != cudaSuccess ||
         (e = cudaStreamCreateWithFlags(&ctx->side, cudaStreamNonBlocking)) != cudaSuccess ||
         (e = cudaEventCreateWithFlags(&ctx->use_ready, cudaEventDisableTiming)) != cudaSuccess ||
-        (e = cudaHostAlloc((void **)&ctx->h_scal, 64, cudaHostAllocDefault)) != cudaSuccess) {
+        (e = cudaHostAlloc((void **)&ctx->h_scal, 64, cudaHostAllocDefault)) != cudaSuccess ||
+        (e = cudaHostAlloc(&ctx->h_stage, wk_ctx::kStageBytes, cudaHostAllocDefault)) != cudaSuccess) {
         int r = cuda_fail(e, "wk_ctx_create");
         delete ctx;
         return r;
@@ -377,8 +378,6 @@ extern "C" int wk_ctx_create(const wk_config *cfg_in, wk_ctx **out) {
         return r;
     }
     if ((st = wk::noalloc_prepare(&ctx->noalloc_scratch)) != WK_OK) { delete ctx; return st; }
-    if ((st = ctx->dscal.reserve(4096)) != WK_OK) { delete ctx; return st; }
-    if ((e = cudaMemset(ctx->dscal.ptr, 0, 4096)) != cudaSuccess) { int r = cuda_fail(e, "wk_ctx_create"); delete ctx; return r; }
     const int64_t hc = cfg.history_capacity > 0 ? cfg.history_capacity : (16ll << 20);
     for (auto &b : ctx->hbuf)
         if ((st = b.reserve((size_t)hc * 4)) != WK_OK) { delete ctx; return st; }
@@ -620,8 +619,13 @@ extern "C" int wk_history_download(wk_ctx *ctx, const wk_history *h, int32_t *ho
     int st = make_current(ctx);
     if (st) return st;
     cudaError_t e;
-    if (h->size > 0 && (e = cudaMemcpyAsync(host, h->data, (size_t)h->size * 4, cudaMemcpyDeviceToHost, ctx->stream)) != cudaSuccess)
+    // a small table by way of pinned memory: a copy to pageable memory holds the
+    // host for some 14 us, this and a copy on the host take 9
+    const size_t bytes = (size_t)h->size * 4;
+    const bool staged = h->size > 0 && bytes <= wk_ctx::kStageBytes;
+    if (h->size > 0 && (e = cudaMemcpyAsync(staged ? ctx->h_stage : host, h->data, bytes, cudaMemcpyDeviceToHost, ctx->stream)) != cudaSuccess)
         return cuda_fail(e, "wk_history_download");
     if ((e = cudaStreamSynchronize(ctx->stream)) != cudaSuccess) return cuda_fail(e, "wk_history_download sync");
+    if (staged) std::memcpy(host, ctx->h_stage, bytes);
     return WK_OK;
 }

@@ -95,8 +95,9 @@ struct wk_ctx {
     unsigned long long *h_gs = nullptr;
     unsigned long long *h_gs_dev = nullptr;   // its device address
     size_t h_gs_bytes = 0;
+    static constexpr size_t kStageBytes = 64 << 10;
+    void *h_stage = nullptr;   // pinned, for downloads of small tables
     unsigned long long pub_seq = 0;  // the last count kernel's sequence number
-    wk::DevBuf dscal;                // [0] error flags, [8..32) totals
     // wk_history_partition: rows per (owner, tile) and their scan's block
     // sums (grown on demand, kept for the next call)
     wk::DevBuf part_cnt, part_scan;
