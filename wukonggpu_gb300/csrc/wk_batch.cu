@@ -150,6 +150,7 @@ struct StepIO {
     unsigned long long *tile_sum;   // per tile
     unsigned long long *q_rows;     // per query output rows (zeroed by the scan)
     int *flags;               // [0] error bits, [1] overflow
+    int32_t *pub;             // last step: pinned words for the flags and the layout behind them, or null
     int64_t cap_ints, cap_rows;
     int Q;
     int64_t warps;            // of the count and write grids
@@ -434,6 +435,13 @@ template <int BT>
 __global__ void __launch_bounds__(BT)
 batch_write_kernel(StepIO io, int rounds, int split) {
     after_prior_kernel();
+    // the flags and the final tables' layout, complete since the scan: on their way
+    // to the host while the rows are written (by a copy behind the batch, 41 queries
+    // took 93 us, 4096 200; this way 84 and 192)
+    if (io.pub != nullptr) {
+        const int n = 2 * (2 * io.Q + 2) + io.Q;
+        for (int i = blockIdx.x * BT + threadIdx.x; i < n; i += gridDim.x * BT) io.pub[i] = __ldcg(io.flags + i);
+    }
     if (io.flags[1]) return;
     write_phase<BT>(io, rounds, split);
 }
@@ -500,9 +508,20 @@ batch_step_kernel(StepIO io, int rounds, int split, unsigned int *bar) {
     write_phase<BT>(io, rounds, split);
 }
 
-// step-0 layout: every query has one virtual row and no columns
+// The step descriptors from pinned host memory (Q of each of `steps` rows of
+// `pitch` 8 B words), and the step-0 layout: every query has one virtual row and
+// no columns.  Reading them here takes as long as a copy ahead of this kernel
+// (786 KB in 4 us), but a kernel behind a copy starts late: a batch of 4096
+// queries took 206 us so, 200 this way.
 __global__ void batch_init_kernel(int Q, int64_t *row_off, int64_t *int_off, int32_t *cols,
-                                  unsigned long long *q_rows, int *flags) {
+                                  unsigned long long *q_rows, int *flags, const uint64_t *__restrict__ h_desc,
+                                  uint64_t *__restrict__ desc, int64_t pitch, int steps) {
+    constexpr int kWords = sizeof(StepDesc) / 8;
+    const int64_t row = (int64_t)Q * kWords, n = row * steps;
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t at = i / row * pitch + i % row;
+        desc[at] = h_desc[at];
+    }
     for (int q = blockIdx.x * blockDim.x + threadIdx.x; q <= Q; q += gridDim.x * blockDim.x) {
         row_off[q] = q;
         if (q < Q) { int_off[q] = 0; cols[q] = 0; q_rows[q] = 0ull; }
@@ -534,11 +553,12 @@ struct wk_batch {
     unsigned long long *d_tile = nullptr, *d_qrows = nullptr;
     int *d_flags = nullptr;                 // d_block
     unsigned int *d_bar = nullptr;          // grid barrier of the one-kernel steps (count, generation)
-    // host (pinned)
-    StepDesc *h_desc = nullptr;
+    // host (pinned), read by the first kernel of a batch
+    StepDesc *h_desc = nullptr, *h_desc_dev = nullptr;
     // the flags (one word) and the final tables' layout -- row_off (Q+1), int_off
     // (Q), cols as int32 (Q) -- on the device, and their pinned copy
     int64_t *d_block = nullptr, *h_block = nullptr;
+    int32_t *h_block_dev = nullptr;         // the copy's device address
     int64_t *h_layout = nullptr;            // h_block + 1
     int *h_flags = nullptr;                 // h_block
     // graph
@@ -605,6 +625,7 @@ StepIO make_io(wk_batch *b, int s, int Q, int64_t warps) {
     io.tile_sum = b->d_tile;
     io.q_rows = b->d_qrows;
     io.flags = b->d_flags;
+    io.pub = nullptr;
     io.cap_ints = b->cap_ints;
     io.cap_rows = b->cap_rows;
     io.Q = Q;
@@ -655,6 +676,7 @@ int enqueue_steps(wk_batch *b, int Q, const BatchTune &t, unsigned grid, cudaStr
         cfg.numAttrs = 1;
         for (int s = 0; s < b->max_steps; ++s) {
             StepIO io = make_io(b, s, Q, (int64_t)grid * (BT / 32));
+            if (s == b->max_steps - 1) io.pub = b->h_block_dev;
             cfg.gridDim = dim3(grid);
             cfg.blockDim = dim3(BT);
             cudaError_t e = cudaLaunchKernelEx(&cfg, batch_count_kernel<BT>, io, t.rounds);
@@ -675,16 +697,16 @@ int64_t batch_kernels(const wk_batch *b, const BatchTune &t) {
     return 1 + (t.fused ? 1 : 3) * (int64_t)b->max_steps;
 }
 
-// the whole batch: descriptor upload, layout init, max_steps x (count, scan,
+// the whole batch: descriptors and layout init, max_steps x (count, scan,
 // write) as three kernels or as one cooperative kernel
 int enqueue(wk_batch *b, int Q, const BatchTune &t, cudaStream_t st) {
-    // the Q descriptors of each step (step s's start at s * max_q)
-    const size_t pitch = sizeof(StepDesc) * (size_t)b->max_q;
-    cudaError_t ce = cudaMemcpy2DAsync(b->d_desc, pitch, b->h_desc, pitch, sizeof(StepDesc) * (size_t)Q,
-                                       (size_t)b->max_steps, cudaMemcpyHostToDevice, st);
-    if (ce != cudaSuccess) return cuda_fail(ce, "batch descriptors");
-    batch_init_kernel<<<(Q + 256) / 256, 256, 0, st>>>(Q, b->d_row_off[0], b->d_int_off[0], b->d_cols[0], b->d_qrows,
-                                                       b->d_flags);
+    static_assert(sizeof(StepDesc) % 8 == 0, "descriptors are copied as 8 B words");
+    const int64_t words = (int64_t)(sizeof(StepDesc) / 8) * Q * b->max_steps;
+    const unsigned gi = (unsigned)std::min<int64_t>((words + 511) / 512, 2 * (int64_t)b->sms);   // two words a thread
+    batch_init_kernel<<<std::max(gi, 1u), 256, 0, st>>>(
+        Q, b->d_row_off[0], b->d_int_off[0], b->d_cols[0], b->d_qrows, b->d_flags,
+        reinterpret_cast<const uint64_t *>(b->h_desc_dev), reinterpret_cast<uint64_t *>(b->d_desc),
+        (int64_t)(sizeof(StepDesc) / 8) * b->max_q, b->max_steps);
     // The step kernels loop over tiles, so any grid gives the same rows.  A
     // small batch gets a grid in proportion to its queries (at least a
     // quarter of the SMs): beside a large query on another stream, a few
@@ -728,8 +750,11 @@ extern "C" int wk_batch_create(wk_ctx *ctx, int32_t max_queries, int32_t max_ste
               cudaMalloc(&b->d_qrows, 8 * (size_t)max_queries) == cudaSuccess &&
               cudaMalloc(&b->d_block, 8 * (size_t)(3 * max_queries + 2)) == cudaSuccess &&
               cudaMalloc(&b->d_bar, 2 * sizeof(unsigned int)) == cudaSuccess &&
-              cudaHostAlloc((void **)&b->h_desc, sizeof(StepDesc) * (size_t)max_queries * max_steps, 0) == cudaSuccess &&
-              cudaHostAlloc((void **)&b->h_block, 8 * (size_t)(3 * max_queries + 2), 0) == cudaSuccess &&
+              cudaHostAlloc((void **)&b->h_desc, sizeof(StepDesc) * (size_t)max_queries * max_steps, cudaHostAllocMapped) ==
+                  cudaSuccess &&
+              cudaHostGetDevicePointer((void **)&b->h_desc_dev, b->h_desc, 0) == cudaSuccess &&
+              cudaHostAlloc((void **)&b->h_block, 8 * (size_t)(3 * max_queries + 2), cudaHostAllocMapped) == cudaSuccess &&
+              cudaHostGetDevicePointer((void **)&b->h_block_dev, b->h_block, 0) == cudaSuccess &&
               create_priority_stream(&b->stream) == cudaSuccess &&
               cudaEventCreateWithFlags(&b->done, cudaEventDisableTiming) == cudaSuccess;
     for (int i = 0; ok && i < 2; ++i)
@@ -882,9 +907,10 @@ extern "C" int wk_batch_launch(wk_batch *b, const int64_t *cmd_chains, const int
     ctx->launches += batch_kernels(b, b->tune);
     b->last_q = nq;
     b->final_buf = b->max_steps & 1;
-    // the flags and the layout of the final tables, then the completion event
-    if ((e = cudaMemcpyAsync(b->h_block, b->d_block, 8 * (2 * (size_t)nq + 2) + 4 * (size_t)nq, cudaMemcpyDeviceToHost,
-                             s)) != cudaSuccess ||
+    // the flags and the layout of the final tables (the last write kernel has sent
+    // them where there is one), then the completion event
+    if ((b->tune.fused && (e = cudaMemcpyAsync(b->h_block, b->d_block, 8 * (2 * (size_t)nq + 2) + 4 * (size_t)nq,
+                                               cudaMemcpyDeviceToHost, s)) != cudaSuccess) ||
         (e = cudaEventRecord(b->done, s)) != cudaSuccess)
         return cuda_fail(e, "batch layout readback");
     return WK_OK;
