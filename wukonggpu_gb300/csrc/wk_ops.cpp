@@ -178,14 +178,34 @@ unsigned long long *gsum_buffer(wk_ctx *ctx, int par) {
 
 // Slice records kept for an op of nblk blocks: enough for a mean fan-out of 128;
 // an op with more slices expands in rounds of that many (33M output rows at
-// least).  They lie behind the entries' offsets and rows in the context's `off`
-// buffer, and are few for a small op: as 64k records in a buffer of their own
-// they cost a new context's first light query 110 us of allocation.
+// least).
 namespace {
 inline int64_t slice_records(int64_t nblk) { return 16 * nblk + 4096; }
-inline size_t off_bytes(int64_t nblk) {
-    return (size_t)nblk * dev::kRowsPerBlock * 6 + (size_t)(slice_records(nblk) + 1) * sizeof(dev::SliceRec);
-}
+
+// The scratch of a k2u op of nblk blocks, in the context's `deg` buffer: per row
+// pos, rel and row (Entries), per block its sum, the slice records, the head.  In
+// one buffer, and with few records for a small op, because a new context's first
+// step pays for each allocation, some 60 us where it takes a new piece of device
+// memory.
+struct K2uScratch {
+    dev::Entries en;
+    unsigned long long *blk_sum;
+    dev::SliceRec *recs;
+    uint32_t *head;
+    static size_t bytes(int64_t nblk) {
+        return (size_t)nblk * dev::kRowsPerBlock * 10 + (size_t)(nblk + (nblk & 1)) * 8 +
+               (size_t)(slice_records(nblk) + 1) * sizeof(dev::SliceRec);
+    }
+    K2uScratch(const DevBuf &b, int64_t nblk) {
+        const size_t whole = (size_t)nblk * dev::kRowsPerBlock;   // entries come by whole blocks
+        unsigned char *p = b.as<unsigned char>();
+        en = dev::Entries{reinterpret_cast<uint32_t *>(p), reinterpret_cast<uint32_t *>(p + whole * 4),
+                          reinterpret_cast<uint16_t *>(p + whole * 8)};
+        blk_sum = reinterpret_cast<unsigned long long *>(p + whole * 10);
+        recs = reinterpret_cast<dev::SliceRec *>(blk_sum + nblk + (nblk & 1));
+        head = reinterpret_cast<uint32_t *>(recs + slice_records(nblk));
+    }
+};
 }
 
 int wk::reserve_published(wk_ctx *ctx, int64_t words) { return reserve_gsum(ctx, (words + 1) / 2); }
@@ -197,8 +217,8 @@ int wk::reserve_op_scratch(wk_ctx *ctx, int64_t rows) {
     if (e != cudaSuccess) return cuda_fail(e, "cudaSetDevice");
     const int64_t nblk = (rows + dev::kRowsPerBlock - 1) / dev::kRowsPerBlock + 1;
     int st;
-    if ((st = ctx->deg.reserve((size_t)nblk * dev::kRowsPerBlock * 4)) || (st = ctx->off.reserve(off_bytes(nblk))) ||
-        (st = ctx->mask.reserve((size_t)((rows + 31) / 32) * 4)) || (st = ctx->blk_sum.reserve((size_t)nblk * 8)) ||
+    if ((st = ctx->deg.reserve(K2uScratch::bytes(nblk))) ||
+        (st = ctx->mask.reserve((size_t)((rows + 31) / 32) * 4)) ||
         (st = ctx->blk_nz.reserve((size_t)nblk * 4)) ||
         (st = reserve_gsum(ctx, (nblk + (1 << dev::kGroupShift) - 1) >> dev::kGroupShift)))
         return st;
@@ -324,17 +344,13 @@ int op_k2u(wk_ctx *ctx, wk_history *h, int scol, uint32_t pid, uint32_t dir) {
     if ((st = op_fused(ctx, h, scol, -1, 0, dir, false, pv, clk, &done)) || done) return st;
     const int64_t nblk = (R + dev::kRowsPerBlock - 1) / dev::kRowsPerBlock;
     const int64_t groups = (nblk + (1 << dev::kGroupShift) - 1) >> dev::kGroupShift;
-    const size_t whole = (size_t)nblk * dev::kRowsPerBlock;   // entries come by whole blocks
-    if ((st = take(ctx, ctx->deg, whole * 4)) || (st = take(ctx, ctx->off, off_bytes(nblk))) ||
-        (st = take(ctx, ctx->blk_sum, (size_t)nblk * 8)) || (st = reserve_gsum(ctx, groups)))
-        return st;
-    unsigned char *off = ctx->off.as<unsigned char>();
-    const dev::Entries en{ctx->deg.as<uint32_t>(), reinterpret_cast<uint32_t *>(off),
-                          reinterpret_cast<uint16_t *>(off + whole * 4)};
-    dev::SliceRec *recs = reinterpret_cast<dev::SliceRec *>(off + whole * 6);
-    uint32_t *head = reinterpret_cast<uint32_t *>(recs + slice_records(nblk));
-    dev::SlicePlan plan{ctx->blk_sum.as<unsigned long long>(), nullptr, nblk, recs, 0ull,
-                        (unsigned long long)slice_records(nblk), nullptr, nullptr, 0ull, 0ull};
+    if ((st = take(ctx, ctx->deg, K2uScratch::bytes(nblk))) || (st = reserve_gsum(ctx, groups))) return st;
+    const K2uScratch sc(ctx->deg, nblk);
+    const dev::Entries &en = sc.en;
+    dev::SliceRec *recs = sc.recs;
+    uint32_t *head = sc.head;
+    dev::SlicePlan plan{sc.blk_sum, nullptr, nblk, recs, 0ull, (unsigned long long)slice_records(nblk), nullptr, nullptr,
+                        0ull, 0ull};
     // a hashed functional direction (at most one neighbour per vertex) expands as a
     // compaction; if a row hits an index list (vertex 0) the op reruns unspecialised
     bool func = pv.func[dir] != 0u && pv.nb[dir] == nullptr && C + 1 <= 8;
@@ -368,7 +384,7 @@ int op_k2u(wk_ctx *ctx, wk_history *h, int scol, uint32_t pid, uint32_t dir) {
         // memory (the publish kernel behind the count, which also writes the
         // expansion's slice records); the host adds up the totals
         const dev::Publish pub{gs, ctx->h_gs_dev, 2 + 2 * groups, ++ctx->pub_seq};
-        dev::launch_k2u_count(h->data, R, C, scol, dir, pv, en, ctx->blk_sum.as<unsigned long long>(), gs + 2,
+        dev::launch_k2u_count(h->data, R, C, scol, dir, pv, en, sc.blk_sum, gs + 2,
                               reinterpret_cast<int *>(gs), func, gsum_buffer(ctx, par ^ 1),
                               2 + 2 * ctx->gs_used[par ^ 1], ctx->sms, ctx->stream);
         if ((st = launch_check("k2u count")) || (st = clk.end(false))) return st;

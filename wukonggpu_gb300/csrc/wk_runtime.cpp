@@ -312,12 +312,11 @@ wk_ctx::~wk_ctx() {
     cudaSetDevice(device);
     if (stream) cudaStreamSynchronize(stream);
     for (auto &b : hbuf) b.release();
-    deg.release(); off.release(); mask.release(); blk_sum.release(); blk_nz.release();
+    deg.release(); mask.release(); blk_nz.release();
     part_cnt.release();
     part_scan.release();
     if (h_scal) cudaFreeHost(h_scal);
     if (h_gs) cudaFreeHost(h_gs);
-    if (h_stage) cudaFreeHost(h_stage);
     for (auto &e : tev) cudaEventDestroy(e);
     if (use_ready) cudaEventDestroy(use_ready);
     if (tm0) cudaEventDestroy(tm0);
@@ -366,12 +365,12 @@ extern "C" int wk_ctx_create(const wk_config *cfg_in, wk_ctx **out) {
     if ((e = cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking)) != cudaSuccess ||
         (e = cudaStreamCreateWithFlags(&ctx->side, cudaStreamNonBlocking)) != cudaSuccess ||
         (e = cudaEventCreateWithFlags(&ctx->use_ready, cudaEventDisableTiming)) != cudaSuccess ||
-        (e = cudaHostAlloc((void **)&ctx->h_scal, 64, cudaHostAllocDefault)) != cudaSuccess ||
-        (e = cudaHostAlloc(&ctx->h_stage, wk_ctx::kStageBytes, cudaHostAllocDefault)) != cudaSuccess) {
+        (e = cudaHostAlloc((void **)&ctx->h_scal, 64 + wk_ctx::kStageBytes, cudaHostAllocDefault)) != cudaSuccess) {
         int r = cuda_fail(e, "wk_ctx_create");
         delete ctx;
         return r;
     }
+    ctx->h_stage = ctx->h_scal + 8;
     if ((e = cudaDeviceGetAttribute(&ctx->sms, cudaDevAttrMultiProcessorCount, ctx->device)) != cudaSuccess) {
         int r = cuda_fail(e, "wk_ctx_create: SM count");
         delete ctx;

@@ -82,7 +82,7 @@ struct wk_ctx {
 
     wk::DevBuf hbuf[2];              // ping-pong history buffers (core/rcache.hpp:87-88)
     // scratch of the two-pass ops
-    wk::DevBuf deg, off, mask, blk_sum, blk_nz;
+    wk::DevBuf deg, mask, blk_nz;
     // k2u: two alternating sums buffers, each a 16 B header (the op's error
     // flags) and 16 B per group of 256 input blocks; a count kernel adds into
     // one and clears the other for the next op
@@ -96,7 +96,7 @@ struct wk_ctx {
     unsigned long long *h_gs_dev = nullptr;   // its device address
     size_t h_gs_bytes = 0;
     static constexpr size_t kStageBytes = 64 << 10;
-    void *h_stage = nullptr;   // pinned, for downloads of small tables
+    void *h_stage = nullptr;   // pinned (behind h_scal), for downloads of small tables
     unsigned long long pub_seq = 0;  // the last count kernel's sequence number
     // wk_history_partition: rows per (owner, tile) and their scan's block
     // sums (grown on demand, kept for the next call)
