@@ -356,22 +356,29 @@ int op_k2u(wk_ctx *ctx, wk_history *h, int scol, uint32_t pid, uint32_t dir) {
     bool func = pv.func[dir] != 0u && pv.nb[dir] == nullptr && C + 1 <= 8;
     // The output buffer an earlier op grew often holds this op's rows too, which
     // the device can tell as well as the host: the expansion then goes in behind
-    // the publish kernel, with a CTA for each slice that the buffer has room for,
-    // and the GPU does not wait while the host adds up the totals and launches it:
-    // back to back, 800k -> 1.66M rows of 11 columns took 47.0 us a step so, 41.4
-    // us this way, 120k -> 12M rows of 4 columns 43.1 and 41.3.  The device runs it only if the op is in order and its rows
-    // and slices fit; else the host sees to it as for an op without a buffer.  No
-    // more than two waves of CTAs, or a mean fan-out of 128, are launched so: a
-    // wave that finds no slice takes half a microsecond.
+    // the publish kernel, and the GPU does not wait while the host adds up the
+    // totals and launches it.  Back to back, 800k -> 1.66M rows of 11 columns took
+    // 47.0 us a step so, 41.4 us this way, 120k -> 12M rows of 4 columns 43.1 and
+    // 41.3.  The device runs it only if the op is in order and its rows and slices
+    // fit; else the host sees to it as for an op without a buffer.  The launch has
+    // a CTA for each slice that the buffer has room for, up to four times what the
+    // direction's mean list gives and at least half a wave: a CTA that finds no
+    // slice is gone in half a microsecond, but a buffer that a large step has grown
+    // has room for thousands (the steps of a query of 61M rows: 761 us with up to
+    // two waves of them, 751 so).
     unsigned int ncta = 0;
     bool ahead_wide = false;
     if (!func && !ctx->timing && !alloc_failure_pending(ctx)) {
         const unsigned long long b = (unsigned long long)nblk, wave = 8ull * (unsigned long long)std::max(ctx->sms, 1);
         plan.max_rows = std::min<unsigned long long>(ob.cap / ((size_t)(C + 1) * 4),
                                                      (unsigned long long)std::max<int64_t>(ctx->row_limit, 0));
+        const PredSeg &sg = ctx->store->hs->segs[pid];
+        const int64_t keys = std::max<int64_t>(dir == WK_DIR_OUT ? sg.subjects : sg.objects, 1);
+        const double expect = (double)R * (double)std::max<int64_t>(sg.triples, 0) / (double)keys / dev::kSliceRows;
         const unsigned long long room = plan.max_rows / dev::kSliceRows;
-        plan.max_slices = std::min(plan.cap, b + std::min(room, std::max(2 * wave, 16 * b)));
-        ahead_wide = b < wave && room >= wave;
+        const unsigned long long likely = std::min(room, (unsigned long long)std::min(expect, 1e9));
+        plan.max_slices = std::min(plan.cap, b + std::min(room, std::max(wave / 2, 4 * likely)));
+        ahead_wide = b < wave && likely >= wave;
         if (plan.max_rows) ncta = (unsigned int)plan.max_slices;
     }
     int errf = 0;
