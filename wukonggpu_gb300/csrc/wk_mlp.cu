@@ -27,7 +27,7 @@
 // embedding's in one.  What bounds a step of 1024 rows is the chain of those
 // launches and a product's latency (5 to 8 us, 64 CTAs).  As 16 kernels and 4
 // copies, each weight gradient in the chain, the step kept the GPU for 155 us,
-// so for 66 us.
+// so for 61 us.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -60,7 +60,7 @@ __global__ void __launch_bounds__(256)
 build_input_kernel(const float *__restrict__ feats, const int32_t *pids, const float *tgt,
                    int32_t *pids_to, float *tgt_to, int M, int Mp,
                    const float *__restrict__ emb, int n_ids, __nv_bfloat16 *__restrict__ X0,
-                   __nv_bfloat16 *__restrict__ X0t, float *__restrict__ zero, int64_t nzero, int *done) {
+                   __nv_bfloat16 *__restrict__ X0t, float *__restrict__ zero, int64_t nzero) {
     __shared__ __nv_bfloat16 tile[kX][34];   // 17 words a column: the transposing reads and writes spread over the banks
     __shared__ int s_pid[32];
     asm volatile("griddepcontrol.launch_dependents;");
@@ -89,7 +89,6 @@ build_input_kernel(const float *__restrict__ feats, const int32_t *pids, const f
     for (int i = t; i < 32 * kX; i += 256) X0[(size_t)r0 * kX + i] = tile[i % kX][i / kX];
     for (int i = t; i < 32 * kX; i += 256) X0t[(size_t)(i / 32) * Mp + r0 + i % 32] = tile[i / 32][i % 32];
     for (int64_t i = (int64_t)blockIdx.x * 256 + t; i < nzero; i += (int64_t)gridDim.x * 256) zero[i] = 0.f;
-    if (blockIdx.x == 0 && t == 0) *done = 0;
 }
 
 // Adam over fp32 master weights; g, m, v, w all of length n.  The bias
@@ -166,7 +165,7 @@ struct wk_mlp {
     // activations (capacity cap_m)
     __nv_bfloat16 *x0 = nullptr, *x0t = nullptr, *h[3] = {}, *ht[3] = {}, *dz[3] = {}, *dzt[3] = {};
     float *z[3] = {}, *feats = nullptr, *tgt = nullptr;
-    float *loss = nullptr;       // the step's, the epoch's sum; then d_err and done, two ints
+    float *loss = nullptr;       // the step's, the epoch's sum; then d_err, an int
     float2 *part = nullptr;      // the output layer's sums per CTA
     int32_t *pids = nullptr;
     int *bidx = nullptr;         // the batch of the epoch a training step takes
@@ -176,7 +175,6 @@ struct wk_mlp {
     int64_t kernels = 0;
     int *d_err = nullptr;        // device flag of the tensor-core GEMM (bit 2: a wait ran out,
                                  // bit 3: work left in flight, TMEM kept)
-    int *done = nullptr;         // the output layer's CTAs done
     float *h_loss = nullptr;     // pinned mirror of loss and what follows it
     int status = 0;              // a host-side GEMM failure since the last check
     int sms = 152;               // multiprocessors of the device (GEMM tile width choice)
@@ -362,9 +360,9 @@ void predict(wk_mlp *m, const float *feats, const int32_t *pids, int64_t n, floa
     m->kernels++;
 }
 
-// The weight gradients dW_l = dZ_l^T . X_l (the layer's input), K the batch, and
-// the embedding's from dX = dZ_0 . W_0, in one launch: nothing waits for any of
-// them, and each alone is 6 to 16 CTAs.
+// The weight gradients dW_l = dZ_l^T . X_l (the layer's input), K the batch, the
+// embedding's from dX = dZ_0 . W_0, and the loss, in one launch: nothing waits for
+// any of them, and each alone is 1 to 16 CTAs.
 void gradient_group(wk_mlp *m, int M, int Mp, cudaStream_t s) {
     if (refused(m)) return;
     tc::GroupArgs g;
@@ -406,7 +404,11 @@ void gradient_group(wk_mlp *m, int M, int Mp, cudaStream_t s) {
         if (!m->status) m->status = set_error(WK_EDEVICE, "estimator: tensor map of the weight gradients (M %d)", M);
         return;
     }
-    launch_ahead(tc::gemm_group_kernel, dim3((unsigned)at), tc::kThreads, tc::smem_bytes(32, tc::kDeepStages), s, g);
+    g.part = m->part;
+    g.nparts = Mp / 16;
+    g.loss = m->loss;
+    g.db = m->grads + m->off_b[3];
+    launch_ahead(tc::gemm_group_kernel, dim3((unsigned)at + 1u), tc::kThreads, tc::smem_bytes(32, tc::kDeepStages), s, g);
     m->kernels++;
 }
 
@@ -417,7 +419,7 @@ void gradient_step(wk_mlp *m, const float *feats, const int32_t *pids, const flo
     float *g = m->grads;
     // w4's gradient, the biases' and the embedding's are added into; they lie together
     launch_ahead(build_input_kernel, dim3((unsigned)(Mp / 32)), 256, 0, s, feats, pids, tgt, m->pids, m->tgt, M, Mp, (const float *)(m->params + m->off_emb), m->n_ids, m->x0, m->x0t,
-                 g + m->off_w[3], m->n_params - m->off_w[3], m->done);
+                 g + m->off_w[3], m->n_params - m->off_w[3]);
     m->kernels++;
     const __nv_bfloat16 *in = m->x0;
     int kin = kX;
@@ -436,10 +438,7 @@ void gradient_step(wk_mlp *m, const float *feats, const int32_t *pids, const flo
         ea.b = m->params + m->off_b[3];
         ea.tgt = m->tgt;
         ea.dw = g + m->off_w[3];
-        ea.db = g + m->off_b[3];
-        ea.loss = m->loss;
         ea.part = m->part;
-        ea.done = m->done;
         CUtensorMap ta, tb;
         if (tc::make_map(&ta, m->h[2], (uint64_t)Mp, kH, kH, tc::kTM) && tc::make_map(&tb, m->wb[3], kOutPad, kH, kH, 32)) {
             launch_ahead(tc::gemm_tc_kernel<32, tc::kEpiHead>, dim3((unsigned)(Mp / 16)), tc::kThreads, tc::smem_bytes(32),
@@ -544,7 +543,6 @@ extern "C" int wk_mlp_create(wk_ctx *ctx, int32_t n_ids, int32_t max_batch, uint
         return set_error(WK_ENOMEM, "wk_mlp_create: allocation failed");
     }
     m->d_err = reinterpret_cast<int *>(m->loss + 2);
-    m->done = m->d_err + 1;
     // He-style initialisation (uniform with the fan-in bound), zero biases, small embeddings
     std::vector<float> h((size_t)at, 0.f);
     std::mt19937_64 rng(seed);

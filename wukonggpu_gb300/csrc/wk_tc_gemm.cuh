@@ -79,13 +79,12 @@ struct EpiArgs {
     const int32_t *pids = nullptr;
     int n_ids = 0;
     // kEpiHead: the last hidden layer's output (ld ldh), the output layer's
-    // weights and bias, the targets; the gradients of both, the loss and its
-    // running sum; each CTA's sums and the count of CTAs done (zero between launches)
+    // weights and bias, the targets; the weights' gradient; each CTA's sums of
+    // (y - t)^2 and dY
     const __nv_bfloat16 *hin = nullptr, *w = nullptr;
     const float *b = nullptr, *tgt = nullptr;
-    float *dw = nullptr, *db = nullptr, *loss = nullptr;
+    float *dw = nullptr;
     float2 *part = nullptr;
-    int *done = nullptr;
 };
 
 // The estimator's activation, exact GELU: x Phi(x), and its derivative
@@ -143,58 +142,61 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
 
 // The step's output layer, loss and first backward layer for the CTA's 16 rows,
 // a warp four of them: y = acc + b, loss mean((y - t)^2), dY = 2 (y - t) / M in
-// bf16 (rows >= m_real: zero), dw += dY^T H, db = sum dY, and of the hidden
+// bf16 (rows >= m_real: zero), dw += dY^T H, and of the hidden
 // layer below dZ = dY w GELU'(Z) in bf16, row-major and transposed, with its
 // column sums.  The layer has one output, so these are row-wise: as products
 // padded to tiles of 64 with kernels of their own for bias, loss and sums they
-// were seven launches and 30 us of a step of 1024 rows.  y: the CTA's 16 accumulators.
-// sm: 12 KB, free.
+// were seven launches and 30 us of a step of 1024 rows; this takes 9.  y: the CTA's 16 accumulators.
+// sm: 18 KB, free.
 __device__ __forceinline__ void head_rows(const EpiArgs &ea, const float *y, int row0, unsigned char *sm) {
     constexpr int kCols = 256, kPitch = 18;   // an odd number of words: the 32 lanes' columns fall in 32 banks
     __nv_bfloat16 *st = reinterpret_cast<__nv_bfloat16 *>(sm);                    // dZ^T: [256][16]
     float *s_cs = reinterpret_cast<float *>(sm + kCols * kPitch * 2);             // per warp: column sums of dZ
-    float *s_dw = s_cs + kCols;                                                   // and of dY H
+    float *s_dw = s_cs + kThreads / 32 * kCols;                                   // and of dY H
     __shared__ float2 s_sum[kThreads / 32];
-    __shared__ int s_last;
     const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
-    for (int i = t; i < 2 * kCols; i += kThreads) s_cs[i] = 0.f;
-    __syncthreads();
-    float w[8], cs[8] = {}, dw[8] = {};
+    // every row's words in flight at once
+    constexpr int kRows = 16 / (kThreads / 32);
+    float w[8], z[kRows][8], cs[8] = {}, dw[8] = {}, tg[kRows];
+    __nv_bfloat16 h[kRows][8];
+#pragma unroll
+    for (int i = 0; i < kRows; ++i) {
+        const int row = row0 + warp * kRows + i;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            z[i][j] = ea.z[(size_t)row * ea.ldz + lane + 32 * j];
+            h[i][j] = ea.hin[(size_t)row * ea.ldh + lane + 32 * j];
+        }
+        tg[i] = row < ea.m_real ? ea.tgt[row] : 0.f;
+    }
 #pragma unroll
     for (int j = 0; j < 8; ++j) w[j] = __bfloat162float(ea.w[lane + 32 * j]);
     const float b = *ea.b;
     float sq = 0.f, sdy = 0.f;
-    for (int i = 0; i < 4; ++i) {
-        const int r = warp * 4 + i, row = row0 + r;
+#pragma unroll
+    for (int i = 0; i < kRows; ++i) {
+        const int r = warp * kRows + i, row = row0 + r;
         float dy = 0.f;
         if (row < ea.m_real) {   // the same in every lane
-            const float d = (y[r] + b) - ea.tgt[row];
+            const float d = (y[r] + b) - tg[i];
             sq += d * d;
             dy = __bfloat162float(__float2bfloat16(2.f * d / (float)ea.m_real));
             sdy += dy;
         }
-        const __nv_bfloat16 *hr = ea.hin + (size_t)row * ea.ldh + lane;
-        const float *zr = ea.z + (size_t)row * ea.ldz + lane;
         __nv_bfloat16 *out = ea.h + (size_t)row * ea.ldh + lane;
-        float z[8], h[8];
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
-            z[j] = zr[32 * j];
-            h[j] = __bfloat162float(hr[32 * j]);
-        }
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const __nv_bfloat16 v = __float2bfloat16(row < ea.m_real ? __fmul_rn(dy, w[j]) * gelu_grad(z[j]) : 0.f);
+            const __nv_bfloat16 v = __float2bfloat16(row < ea.m_real ? __fmul_rn(dy, w[j]) * gelu_grad(z[i][j]) : 0.f);
             out[32 * j] = v;
             st[(lane + 32 * j) * kPitch + r] = v;
             cs[j] += __bfloat162float(v);
-            dw[j] += dy * h[j];
+            dw[j] += dy * __bfloat162float(h[i][j]);
         }
     }
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
-        atomicAdd(s_cs + lane + 32 * j, cs[j]);
-        atomicAdd(s_dw + lane + 32 * j, dw[j]);
+        s_cs[warp * kCols + lane + 32 * j] = cs[j];
+        s_dw[warp * kCols + lane + 32 * j] = dw[j];
     }
     if (lane == 0) s_sum[warp] = make_float2(sq, sdy);
     __syncthreads();
@@ -203,23 +205,26 @@ __device__ __forceinline__ void head_rows(const EpiArgs &ea, const float *y, int
         uint4 *dst = reinterpret_cast<uint4 *>(ea.ht + (size_t)c * ea.ldt + row0);
         dst[0] = make_uint4(src[0], src[1], src[2], src[3]);
         dst[1] = make_uint4(src[4], src[5], src[6], src[7]);
-        if (s_cs[c] != 0.f) atomicAdd(ea.colsum + c, s_cs[c]);
-        if (s_dw[c] != 0.f) atomicAdd(ea.dw + c, s_dw[c]);
+        float a = s_cs[c], d = s_dw[c];
+        for (int i = 1; i < kThreads / 32; ++i) { a += s_cs[i * kCols + c]; d += s_dw[i * kCols + c]; }
+        if (a != 0.f) atomicAdd(ea.colsum + c, a);
+        if (d != 0.f) atomicAdd(ea.dw + c, d);
     }
-    // the sums over all rows: the last CTA adds up every CTA's
-    if (t == 0) {
+    if (t == 0) {   // added up over the CTAs by sum_rows, in a later kernel: nothing waits for it
         float2 v = s_sum[0];
         for (int i = 1; i < kThreads / 32; ++i) { v.x += s_sum[i].x; v.y += s_sum[i].y; }
         ea.part[blockIdx.x] = v;
-        __threadfence();
-        s_last = atomicAdd(ea.done, 1) == (int)gridDim.x - 1;
     }
-    __syncthreads();
-    if (!s_last) return;
-    __threadfence();
-    sq = sdy = 0.f;
-    for (int i = t; i < (int)gridDim.x; i += kThreads) {
-        const float2 v = __ldcg(ea.part + i);
+}
+
+// The loss (the mean over m rows, also added into loss[1]) and the output
+// bias's gradient from the n CTAs' sums.  One CTA.
+__device__ __forceinline__ void sum_rows(const float2 *part, int n, int m, float *loss, float *db) {
+    __shared__ float2 s_sum[kThreads / 32];
+    const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+    float sq = 0.f, sdy = 0.f;
+    for (int i = t; i < n; i += kThreads) {
+        const float2 v = __ldcg(part + i);
         sq += v.x;
         sdy += v.y;
     }
@@ -232,11 +237,10 @@ __device__ __forceinline__ void head_rows(const EpiArgs &ea, const float *y, int
     if (t == 0) {
         float2 v = s_sum[0];
         for (int i = 1; i < kThreads / 32; ++i) { v.x += s_sum[i].x; v.y += s_sum[i].y; }
-        const float l = v.x / (float)(ea.m_real > 0 ? ea.m_real : 1);
-        ea.loss[0] = l;
-        ea.loss[1] += l;
-        *ea.db = v.y;
-        *ea.done = 0;
+        const float l = v.x / (float)(m > 0 ? m : 1);
+        loss[0] = l;
+        loss[1] += l;
+        *db = v.y;
     }
 }
 
@@ -471,8 +475,18 @@ struct GroupArgs {
     const int32_t *pids;
     int n_ids, m_real, n;
     int *err;
+    // sum_rows, by a CTA behind the tiles
+    const float2 *part;
+    int nparts;
+    float *loss, *db;
 };
 __global__ void __launch_bounds__(kThreads) gemm_group_kernel(const __grid_constant__ GroupArgs g) {
+    if ((int)blockIdx.x == g.first[g.n]) {
+        asm volatile("griddepcontrol.launch_dependents;");
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+        sum_rows(g.part, g.nparts, g.m_real, g.loss, g.db);
+        return;
+    }
     int p = 0;
     while (p + 1 < g.n && (int)blockIdx.x >= g.first[p + 1]) ++p;
     const int i = (int)blockIdx.x - g.first[p];
