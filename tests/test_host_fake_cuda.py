@@ -1,0 +1,72 @@
+"""Host code around the kernels, run without a GPU: the library's objects linked
+against a CUDA runtime with two devices whose kernels do nothing
+(fake_cuda/fake_cudart.cpp).  Each test is a program of its own."""
+import os
+import subprocess
+import sys
+from pathlib import Path
+
+import pytest
+
+ROOT = Path(__file__).resolve().parents[1]
+
+PRELUDE = """
+import ctypes as C, sys, threading
+from pathlib import Path
+import numpy as np
+sys.path.insert(0, {root!r})
+import wukonggpu_gb300 as W
+W._LIB_PATH = Path({lib!r})
+lib = W.load_library()
+fake = C.CDLL({lib!r})
+for f in ("fake_wrong_device", "fake_launches", "fake_bytes_on", "fake_pending"):
+    getattr(fake, f).restype = C.c_long
+
+# vertex VID_BASE + i has the one neighbour VID_BASE + 100 + i in predicate 2
+def context(device, **kw):
+    s = (W.VID_BASE + np.arange(64)).astype(np.int32)
+    rc = W.RCache(device=device, **kw)
+    rc.build_store(s, np.full(64, 2, np.int32), s + 100, 2)
+    return rc
+"""
+
+
+@pytest.fixture(scope="session")
+def fake_lib(lib_built, tmp_path_factory):
+    from wukonggpu_gb300 import build as wb
+    out = tmp_path_factory.mktemp("fake") / "libwkgpu_fake.so"
+    objs = [wb.BUILD / (p.name + ".o") for pat in ("*.cpp", "*.cu") for p in sorted(wb.CSRC.glob(pat))]
+    cmd = ["g++", "-O1", "-std=c++17", "-shared", "-fPIC", "-I", str(wb._cuda_home() / "include"), "-o", str(out),
+           str(ROOT / "tests" / "fake_cuda" / "fake_cudart.cpp"), *map(str, objs), "-lpthread", "-Wl,--no-undefined"]
+    subprocess.run(cmd, check=True, capture_output=True, text=True)
+    return out
+
+
+def _run(fake_lib, body):
+    code = PRELUDE.format(root=str(ROOT), lib=str(fake_lib)) + body + "\nprint('ok', flush=True)\nimport os; os._exit(0)\n"
+    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=120,
+                       env={**os.environ, "OPENBLAS_NUM_THREADS": "1"})
+    assert r.returncode == 0 and r.stdout.strip().endswith("ok"), r.stdout + r.stderr
+
+
+def test_light_request_runs_on_its_contexts_device(fake_lib):
+    """Two contexts on two devices in one thread, and a context used from a new
+    thread: every launch and allocation of a short request is its device's."""
+    _run(fake_lib, """
+q = [W.VID_BASE + 1, 2, W.OUT, -1, -1, 2, W.OUT, -2]
+def short(rc):
+    try:
+        rc.execute(q)
+    except W.WkError as e:      # the kernels publish nothing here
+        assert "without publishing" in str(e), e
+a, b = context(0, history_capacity=64), context(1, history_capacity=64)
+on1 = fake.fake_bytes_on(1)
+n = fake.fake_launches()
+short(a)                        # device 1 is current
+assert fake.fake_launches() > n
+assert fake.fake_wrong_device() == 0 and fake.fake_bytes_on(1) == on1
+t = threading.Thread(target=short, args=(b,))    # a new thread: device 0 is current
+on0 = fake.fake_bytes_on(0)
+t.start(); t.join()
+assert fake.fake_wrong_device() == 0 and fake.fake_bytes_on(0) == on0
+""")

@@ -733,6 +733,8 @@ extern "C" int wk_execute(wk_ctx *ctx, const int64_t *cmd, int32_t n, wk_history
     if (!ctx || !cmd || !h || n <= 0) return set_error(WK_EINVAL, "wk_execute: bad arguments");
     if (!ctx->store) return set_error(WK_ENOSTORE, "wk_execute: no store");
     if (ctx->device < 0) return set_error(WK_EDEVICE, "wk_execute: host-only context");
+    // a light query and a prefetch use the device before any step's op makes it current
+    if (const cudaError_t e = cudaSetDevice(ctx->device)) return cuda_fail(e, "cudaSetDevice");
     wk_history_init(h);
     ctx->protect.clear();
     ctx->query_rest.clear();
