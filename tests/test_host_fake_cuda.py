@@ -70,3 +70,33 @@ on0 = fake.fake_bytes_on(0)
 t.start(); t.join()
 assert fake.fake_wrong_device() == 0 and fake.fake_bytes_on(0) == on0
 """)
+
+
+def test_group_sums_after_a_failed_allocation(fake_lib):
+    """An op after one whose group sums could not be allocated allocates them
+    again: the buffer that was given back for the larger one is gone."""
+    _run(fake_lib, """
+rc = context(0)
+h = np.full((300, 1), W.VID_BASE + 1, np.int32)
+def step():
+    req = W.Request([])
+    rc.upload_history(req, h)
+    try:
+        rc.known_to_unknown(req, -1, W.OUT, 2)
+    except W.WkError as e:
+        assert "without publishing" in str(e), e
+    return req
+step()
+fake.fake_fail_mallocs(2)       # the reservation and its retry
+req = W.Request([])
+rc.upload_history(req, h)
+try:
+    rc.partition(req, -1, 2)
+    raise SystemExit("no error")
+except W.WkError as e:
+    assert e.status == W.WK_ENOMEM, e
+fake.fake_fail_mallocs(0)
+before = fake.fake_bytes_on(0)
+step()
+assert fake.fake_bytes_on(0) > before
+""")

@@ -145,6 +145,7 @@ int reserve_gsum(wk_ctx *ctx, int64_t groups) {
     if (groups <= ctx->gs_groups) return WK_OK;
     const int64_t want = std::max(groups, ctx->gs_groups + ctx->gs_groups / 2);
     const size_t buf_bytes = 16 + (size_t)want * 16;
+    ctx->gs_groups = 0;   // until both are there: a failed reservation has given the old ones back
     int st = ctx->gsum.reserve(2 * buf_bytes);
     if (st) return st;
     cudaError_t e = cudaMemsetAsync(ctx->gsum.ptr, 0, ctx->gsum.cap, ctx->stream);
@@ -161,7 +162,6 @@ int reserve_gsum(wk_ctx *ctx, int64_t groups) {
     if (e != cudaSuccess) {
         if (ctx->h_gs) cudaFreeHost(ctx->h_gs);
         ctx->h_gs = ctx->h_gs_dev = nullptr;
-        ctx->gs_groups = 0;
         return cuda_fail(e, "k2u: pinned group sums");
     }
     ctx->h_gs_bytes = 16 + buf_bytes;
