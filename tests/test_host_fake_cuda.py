@@ -100,3 +100,20 @@ before = fake.fake_bytes_on(0)
 step()
 assert fake.fake_bytes_on(0) > before
 """)
+
+
+def test_batch_holds_a_row_for_each_query(fake_lib):
+    """The rows' counts and list offsets of a batch have room for step 0's one
+    row per query however small the capacity is: all that a capacity below the
+    number of queries saves is the two tables."""
+    _run(fake_lib, """
+rc = context(0)
+def size(cap):
+    before = fake.fake_bytes_on(0)
+    b = W.Batch(rc, max_queries=4096, max_steps=2, capacity_ints=cap)
+    n = fake.fake_bytes_on(0) - before
+    b.close()
+    assert fake.fake_bytes_on(0) == before
+    return n
+assert size(4096) - size(1) == 2 * 4 * 4095
+""")

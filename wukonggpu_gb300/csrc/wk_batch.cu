@@ -742,10 +742,12 @@ extern "C" int wk_batch_create(wk_ctx *ctx, int32_t max_queries, int32_t max_ste
     cudaDeviceGetAttribute(&b->sms, cudaDevAttrMultiProcessorCount, ctx->device);
     const size_t npv = ctx->store->views.size();
     const int64_t tiles = max_tiles(b);
+    // a step's input rows: what the step before may leave, or one for each query
+    const size_t rows = (size_t)std::max<int64_t>(b->cap_rows, max_queries);
     bool ok = cudaMalloc(&b->d_pvs, sizeof(PredView) * npv) == cudaSuccess &&
               cudaMalloc(&b->d_desc, sizeof(StepDesc) * (size_t)max_queries * max_steps) == cudaSuccess &&
-              cudaMalloc(&b->d_cnt, 4 * (size_t)b->cap_rows) == cudaSuccess &&
-              cudaMalloc(&b->d_off, 4 * (size_t)b->cap_rows) == cudaSuccess &&
+              cudaMalloc(&b->d_cnt, 4 * rows) == cudaSuccess &&
+              cudaMalloc(&b->d_off, 4 * rows) == cudaSuccess &&
               cudaMalloc(&b->d_tile, 8 * (size_t)tiles) == cudaSuccess &&
               cudaMalloc(&b->d_qrows, 8 * (size_t)max_queries) == cudaSuccess &&
               cudaMalloc(&b->d_block, 8 * (size_t)(3 * max_queries + 2)) == cudaSuccess &&
