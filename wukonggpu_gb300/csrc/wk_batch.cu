@@ -341,7 +341,10 @@ __global__ void __launch_bounds__(kScanThreads)
 batch_scan_kernel(StepIO io, int rounds) {
     __shared__ unsigned long long ws[32];
     after_prior_kernel();
-    if (io.flags[1]) return;   // over capacity: so does the write (also when the other block just found it)
+    // Over capacity: nothing of this step is used.  The other block may be finding
+    // that out just now, so the block's threads, which meet at barriers below, go by
+    // one vote on what they read.
+    if (__syncthreads_or(*(volatile int *)(io.flags + 1))) return;
     if (blockIdx.x == 0) scan_tiles(io, rounds, ws);
     else scan_queries(io, ws);
 }
@@ -491,7 +494,7 @@ __device__ __forceinline__ bool grid_barrier(unsigned int *bar, int *flags) {
     return s_ok != 0;
 }
 
-// One step in one cooperative launch: count, barrier, scan (block 0),
+// One step in one cooperative launch: count, barrier, scan (the first and last block),
 // barrier, write.  Launched with at most as many blocks as fit on the device
 // at once (the cooperative launch refuses more).
 template <int BT>
