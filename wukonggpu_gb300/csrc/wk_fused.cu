@@ -1,9 +1,9 @@
 // k2u, k2k and k2c over a dense functional direction in one launch (sm_103a).
 //
 // A direction that keeps one neighbour per id (PredView::nb) answers a row
-// with one 4 B read and gives at most one output row per input row, so the
-// output is sized by the input, and nothing has to reach the host between
-// counting and writing:
+// with one 4 B read and gives at most one output row per input row, so nothing
+// has to reach the host between counting and writing where the output buffer
+// holds a row for each row in (and the row limit allows as many):
 //
 //   k2u     : the rows that have a neighbour, with it appended
 //   k2k/k2c : the rows whose neighbour is the end value
@@ -81,6 +81,7 @@ struct Fused {
     unsigned long long *pub;      // pinned host words: [0] seq, [2] error bits, [3] rows, [4] second count
     unsigned long long seq;
     int steps, lag;               // octets of blocks, and how many the writing trails by
+    int first;                    // the launch's first CTA in that order
 };
 
 // What CTA `i` does: role 0 counts unit `unit` of octet `oct`, 1 writes it, 2
@@ -442,7 +443,7 @@ fused_kernel(const __grid_constant__ Fused a, const __grid_constant__ PredView p
     __shared__ WaitShared s_wait;
     asm volatile("griddepcontrol.wait;" ::: "memory");   // the previous op's table and sums are complete
     asm volatile("griddepcontrol.launch_dependents;");
-    const Role role = role_of((int)blockIdx.x, a.steps, a.lag, NC, NW);
+    const Role role = role_of(a.first + (int)blockIdx.x, a.steps, a.lag, NC, NW);
     if (role.kind == 0) {
         // the other sums buffer, read by the previous op, is cleared for the next
         for (int64_t w = ((int64_t)role.oct * NC + role.unit) * kThreads + threadIdx.x; w < a.nclear;
@@ -505,13 +506,18 @@ fused_kernel(const __grid_constant__ Fused a, const __grid_constant__ PredView p
 bool fused_takes(int C, bool filter) { return filter || C + 1 <= kFusedCols; }
 
 template <int CT, bool FILTER, int BPC, bool PB>
-static int run_fused(const Fused &a, const PredView &pv, cudaStream_t st) {
+static int run_fused(Fused a, const PredView &pv, int part, cudaStream_t st) {
     constexpr int NC = kOct / BPC, NW = PB ? kOct : 1;
+    // with every octet counted before the first is written, the order is the
+    // counts, the publisher, the writes
+    if (part != kFusedAll) a.lag = a.steps;
+    const int counts = a.steps * NC + 1, all = counts + a.steps * NW;
+    a.first = part == kFusedWrite ? counts : 0;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned int)(a.steps * (NC + NW) + 1));
+    cfg.gridDim = dim3((unsigned int)((part == kFusedCount ? counts : all) - a.first));
     cfg.blockDim = dim3(kThreads);
     cfg.stream = st;
     cfg.attrs = attr;
@@ -555,7 +561,7 @@ int launch_fused(const FusedOp &op, cudaStream_t st) {
     // enough of them to fill the GPU
     const bool pair = !op.filter && a.nblk >= 16 * (int64_t)op.sms;
 #define WK_FUSED(CC)                                                      \
-    case CC: return pair ? run_fused<CC, false, 2, true>(a, op.pv, st) : run_fused<CC, false, 1, true>(a, op.pv, st)
+    case CC: return pair ? run_fused<CC, false, 2, true>(a, op.pv, op.part, st) : run_fused<CC, false, 1, true>(a, op.pv, op.part, st)
     if (!op.filter) {
         switch (op.C) {
             WK_FUSED(1); WK_FUSED(2); WK_FUSED(3); WK_FUSED(4); WK_FUSED(5);
@@ -565,7 +571,7 @@ int launch_fused(const FusedOp &op, cudaStream_t st) {
     }
 #undef WK_FUSED
     const bool pb = filter_per_block(a.nblk, op.sms);
-#define WK_FUSED(CC) return pb ? run_fused<CC, true, 1, true>(a, op.pv, st) : run_fused<CC, true, 1, false>(a, op.pv, st)
+#define WK_FUSED(CC) return pb ? run_fused<CC, true, 1, true>(a, op.pv, kFusedAll, st) : run_fused<CC, true, 1, false>(a, op.pv, kFusedAll, st)
     switch (op.C) {
         case 1: WK_FUSED(1);
         case 2: WK_FUSED(2);

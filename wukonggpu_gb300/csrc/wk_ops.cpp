@@ -239,12 +239,14 @@ int take(wk_ctx *ctx, DevBuf &b, size_t bytes) {
 
 bool alloc_failure_pending(wk_ctx *ctx) { return ctx->inject_alloc_fail.load(std::memory_order_relaxed) > 0; }
 
-// A k2u or filter op over a dense functional direction in one launch
-// (wk_fused.cu): at most one row out per row in, so the output is sized by the
-// input and nothing has to reach the host before it is written.
-// *done is false when the op has to run as two kernels instead: more columns
-// than the launch takes, a start that is an index key (k2u), an output bound
-// that does not fit in device memory, or a device wait that ran out.
+// A k2u or filter op over a dense functional direction (wk_fused.cu), at most
+// one row out per row in: one launch.  A k2u op whose output buffer does not hold
+// that many rows, or whose row limit does not allow them, is counted by one launch
+// and written by another, with the limit checked and the buffer grown to the rows
+// there are in between.
+// *done is false when the op has to run as the general kernels instead: more
+// columns than the launch takes, a start that is an index key (k2u), or a device
+// wait that ran out.
 int op_fused(wk_ctx *ctx, wk_history *h, int scol, int ecol, int32_t end_const, uint32_t dir, bool filter,
              const PredView &pv, OpClock &clk, bool *done) {
     *done = false;
@@ -257,17 +259,15 @@ int op_fused(wk_ctx *ctx, wk_history *h, int scol, int ecol, int32_t end_const, 
     const int64_t groups = (nblk + (1 << dev::kGroupShift) - 1) >> dev::kGroupShift;
     int st;
     if ((st = filter ? take(ctx, ctx->mask, (size_t)((R + 31) / 32) * 4) : take(ctx, ctx->deg, (size_t)R * 4)) ||
-        (st = take(ctx, ctx->blk_nz, (size_t)nblk * 4)) || (st = reserve_gsum(ctx, groups)))
+        (st = take(ctx, ctx->blk_nz, (size_t)nblk * 4)) || (st = reserve_gsum(ctx, groups)) ||
+        (filter && (st = take(ctx, ob, (size_t)R * C * 4))))
         return st;
-    const bool injected = alloc_failure_pending(ctx);
-    if ((st = take(ctx, ob, (size_t)R * width * 4))) {
-        // a k2u op of two kernels asks for its rows only; a filter's asks for as much
-        return injected || st != WK_ENOMEM || filter ? st : WK_OK;
-    }
+    const bool count_first = !filter && (ob.cap < (size_t)R * width * 4 || R > ctx->row_limit);
     if ((st = clk.begin())) return st;
     const int par = ctx->gs_par;
     unsigned long long *gs = gsum_buffer(ctx, par);
     dev::FusedOp op;
+    op.part = count_first ? dev::kFusedCount : dev::kFusedAll;
     op.hist = h->data;
     op.R = R;
     op.C = C;
@@ -289,9 +289,9 @@ int op_fused(wk_ctx *ctx, wk_history *h, int scol, int ecol, int32_t end_const, 
     op.pub = ctx->h_gs_dev;
     op.seq = ++ctx->pub_seq;
     op.sms = ctx->sms;
-    const cudaError_t le = (cudaError_t)dev::launch_fused(op, ctx->stream);
+    cudaError_t le = (cudaError_t)dev::launch_fused(op, ctx->stream);
     if (le != cudaSuccess) return cuda_fail(le, "one-launch op");
-    if ((st = launch_check("one-launch op")) || (st = clk.end(true))) return st;
+    if ((st = launch_check("one-launch op")) || (st = clk.end(!count_first))) return st;
     ctx->gs_par = par ^ 1;
     ctx->gs_used[par ^ 1] = 0;
     ctx->gs_used[par] = groups;
@@ -301,9 +301,19 @@ int op_fused(wk_ctx *ctx, wk_history *h, int scol, int ecol, int32_t end_const, 
     if (err & 1ull)
         return fail_corrupt();
     if ((err & (unsigned long long)dev::kErrWait) || (!filter && extra)) return WK_OK;
-    if (!filter && R_out > ctx->row_limit)
-        return set_error(WK_EOVERFLOW, "k2u: %lld output rows exceed the context's row limit %lld", (long long)R_out,
-                         (long long)ctx->row_limit);
+    if (count_first) {
+        if (R_out > ctx->row_limit)
+            return set_error(WK_EOVERFLOW, "k2u: %lld output rows exceed the context's row limit %lld",
+                             (long long)R_out, (long long)ctx->row_limit);
+        if ((st = take(ctx, ob, (size_t)R_out * width * 4 + 16))) return st;
+        if (R_out > 0) {
+            op.part = dev::kFusedWrite;
+            op.out = ob.as<int32_t>();
+            if ((st = clk.begin())) return st;
+            if ((le = (cudaError_t)dev::launch_fused(op, ctx->stream)) != cudaSuccess) return cuda_fail(le, "functional write");
+            if ((st = launch_check("functional write")) || (st = clk.end(true))) return st;
+        }
+    }
     ctx->last.rows_out = R_out;
     ctx->last.alg_bytes = filter ? 4 * R * C + 16 * R + 4 * extra + 4 * R_out * C
                                  : 4 * R * C + 16 * R + 4 * R_out + 4 * R_out * (C + 1);
