@@ -3,7 +3,8 @@
 // A direction that keeps one neighbour per id (PredView::nb) answers a row
 // with one 4 B read and gives at most one output row per input row, so nothing
 // has to reach the host between counting and writing where the output buffer
-// holds a row for each row in (and the row limit allows as many):
+// holds the rows there are (the device leaves out what it does not hold, and the
+// host, which learns the rows from the same launch, has the blocks written again):
 //
 //   k2u     : the rows that have a neighbour, with it appended
 //   k2k/k2c : the rows whose neighbour is the end value
@@ -78,6 +79,7 @@ struct Fused {
     unsigned long long *clear;    // the other sums buffer, cleared for the next op
     int64_t nclear;
     int32_t *out;
+    unsigned long long max_rows;  // k2u: rows that out has room for
     unsigned long long *pub;      // pinned host words: [0] seq, [2] error bits, [3] rows, [4] second count
     unsigned long long seq;
     int steps, lag;               // octets of blocks, and how many the writing trails by
@@ -292,8 +294,15 @@ __device__ __forceinline__ unsigned int blocks_before(const Fused &a, int64_t b)
 // packed in shared memory at the output's 16 B phase; its whole vectors leave
 // by the copy engine, which spares the load-store unit the look-ups need (12M
 // rows of 4 columns 138 -> 132 us a step).
-// The rows are loaded before the wait for the groups: nearly every row of a
-// functional step is kept, and they are in L2.  False when the wait ran out.
+// A block most of whose rows are kept loads them before the wait for the groups
+// (they are in L2); of another only the kept rows are read, behind it.  Whether
+// most are kept is told by the block's count, which is there already for nearly
+// every block; read too early it is some earlier op's, and costs time only.  With
+// every block's rows loaded ahead and the ballots held in registers, which spilled,
+// 12M rows of 4 columns took 126 / 98 / 82 / 72 us a step with all / half / one in
+// eight / none of the rows kept, 118 / 91 / 80 / 66 so; as two kernels, whose
+// second is not launched for none, 169 / 131 / 102 / 48.
+// False when the wait ran out.
 template <int C>
 __device__ __forceinline__ bool write_k2u(const Fused &a, int64_t b, WaitShared &s_wait, int32_t *buf,
                                           unsigned int *s_w, unsigned int *s_b) {
@@ -303,25 +312,33 @@ __device__ __forceinline__ bool write_k2u(const Fused &a, int64_t b, WaitShared 
     const int n = (int)((a.R - r0) < kRowsPerBlock ? (a.R - r0) : kRowsPerBlock);
     const bool aligned = ((uintptr_t)a.hist & 15u) == 0;
     int32_t x[kPasses], v[kPasses][W];
-    unsigned m[kPasses], kept = 0u;
+    unsigned kept = 0u;
+    const bool most = ld_l2(a.blk_nz + b) >= (unsigned)kRowsPerBlock / 4;
+    if (most) {
 #pragma unroll
-    for (int q = 0; q < kPasses; ++q) {
-        const int r = wid * (32 * kPasses) + q * 32 + lane;
-        if (r < n) copy_row_regs<C>(a.hist + (r0 + r) * C, v[q], aligned);
+        for (int q = 0; q < kPasses; ++q) {
+            const int r = wid * (32 * kPasses) + q * 32 + lane;
+            if (r < n) copy_row_regs<C>(a.hist + (r0 + r) * C, v[q], aligned);
+        }
     }
     unsigned long long P;
     if (!groups_before(a, b >> kGroupShift, kWritePolls, s_wait, P)) return false;
+    const bool any = most || ld_l2(a.blk_nz + b) != 0u;
 #pragma unroll
     for (int q = 0; q < kPasses; ++q) {
         const int r = wid * (32 * kPasses) + q * 32 + lane;
-        x[q] = r < n ? __ldcg(a.nbr + r0 + r) : -1;
+        x[q] = any && r < n ? __ldcg(a.nbr + r0 + r) : -1;
+    }
+    if (!most) {
+#pragma unroll
+        for (int q = 0; q < kPasses; ++q) {
+            const int r = wid * (32 * kPasses) + q * 32 + lane;
+            if (x[q] >= 0) copy_row_regs<C>(a.hist + (r0 + r) * C, v[q], aligned);
+        }
     }
     const unsigned int before = blocks_before(a, b);
 #pragma unroll
-    for (int q = 0; q < kPasses; ++q) {
-        m[q] = __ballot_sync(FULL, x[q] >= 0);
-        kept += (unsigned)__popc(m[q]);
-    }
+    for (int q = 0; q < kPasses; ++q) kept += (unsigned)__popc(__ballot_sync(FULL, x[q] >= 0));
     if (lane == 0) { s_w[wid] = kept; s_b[wid] = before; }
     __syncthreads();
     unsigned at = 0u, T = 0u;
@@ -331,13 +348,15 @@ __device__ __forceinline__ bool write_k2u(const Fused &a, int64_t b, WaitShared 
         T += s_w[w];
         P += s_b[w];
     }
+    if (T == 0u || P + T > a.max_rows) return true;
     const int lead = (int)((P * W) & 3ull), end = lead + (int)T * W;
     const unsigned below = (1u << lane) - 1u;
 #pragma unroll
     for (int q = 0; q < kPasses; ++q) {
+        const unsigned m = __ballot_sync(FULL, x[q] >= 0);
         if (x[q] >= 0) {
             v[q][C] = x[q];
-            int32_t *d = buf + lead + (at + (unsigned)__popc(m[q] & below)) * W;
+            int32_t *d = buf + lead + (at + (unsigned)__popc(m & below)) * W;
             if constexpr (W % 4 == 0) {          // lead is 0
 #pragma unroll
                 for (int c = 0; c < W; c += 4)
@@ -350,7 +369,7 @@ __device__ __forceinline__ bool write_k2u(const Fused &a, int64_t b, WaitShared 
                 for (int c = 0; c < W; ++c) d[c] = v[q][c];
             }
         }
-        at += (unsigned)__popc(m[q]);
+        at += (unsigned)__popc(m);
     }
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     __syncthreads();
@@ -547,6 +566,7 @@ int launch_fused(const FusedOp &op, cudaStream_t st) {
     a.clear = op.clear;
     a.nclear = op.nclear;
     a.out = op.out;
+    a.max_rows = op.max_rows;
     a.pub = op.pub;
     a.seq = op.seq;
     a.steps = (int)((a.nblk + kOct - 1) / kOct);

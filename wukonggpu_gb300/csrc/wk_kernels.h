@@ -117,8 +117,8 @@ void launch_filter_write(const int32_t *hist, int64_t R, int C, const uint32_t *
 inline bool filter_per_block(int64_t nblk, int sms) { return nblk <= 16 * (int64_t)(sms < 1 ? 1 : sms); }
 
 // k2u, k2k and k2c over a dense functional direction (pv.nb[dir] set) in one
-// launch; k2u for up to kFusedCols output columns (fused_takes).  out holds R
-// rows of C + 1 (k2u, kFusedAll) or C columns and is 16 B aligned; nbr (k2u) holds R
+// launch; k2u for up to kFusedCols output columns (fused_takes).  out holds
+// max_rows rows of C + 1 (k2u) or R rows of C columns and is 16 B aligned; nbr (k2u) holds R
 // words, mask (filters) a bit per row, blk_nz a word per block, group_sums two
 // zero words per group; written (filters) is a zero word.  clear[0 .. nclear) is set to zero.  The op's totals go
 // to pinned host memory: pub[2] = the error word (bit 0: corrupt overflow
@@ -126,10 +126,11 @@ inline bool filter_per_block(int64_t nblk, int sms) { return nblk <= 16 * (int64
 // pub[3] = output rows, pub[4] = k2u: not 0 when a row's start is an index key
 // (the op has to run unspecialised), filter: entries a linear scan touches;
 // then seq into pub[0], once every row is counted (k2u) or every kept row
-// copied (filters: the launch has finished with its input).  A k2u op whose output
-// is not there before its rows are counted runs as two launches: kFusedCount
-// counts and publishes and leaves out alone; kFusedWrite, behind it with the same
-// scratch, writes out, which holds the pub[3] rows counted.  Returns a cudaError_t.
+// copied (filters: the launch has finished with its input).  k2u: out holds
+// max_rows rows, and blocks whose rows end past them are not written; kFusedWrite,
+// a launch behind one of the others with the same scratch, writes out (all
+// pub[3] rows of it) and nothing else.  kFusedCount counts and publishes and leaves
+// out alone.  Returns a cudaError_t.
 constexpr int kFusedCols = 11;
 constexpr int kErrWait = 16;
 enum { kFusedAll, kFusedCount, kFusedWrite };
@@ -151,6 +152,7 @@ struct FusedOp {
     unsigned long long *clear;
     int64_t nclear;
     int32_t *out;
+    unsigned long long max_rows;
     unsigned long long *pub;
     unsigned long long seq;
     int sms;

@@ -240,10 +240,11 @@ int take(wk_ctx *ctx, DevBuf &b, size_t bytes) {
 bool alloc_failure_pending(wk_ctx *ctx) { return ctx->inject_alloc_fail.load(std::memory_order_relaxed) > 0; }
 
 // A k2u or filter op over a dense functional direction (wk_fused.cu), at most
-// one row out per row in: one launch.  A k2u op whose output buffer does not hold
-// that many rows, or whose row limit does not allow them, is counted by one launch
-// and written by another, with the limit checked and the buffer grown to the rows
-// there are in between.
+// one row out per row in: one launch.  A k2u op writes as it counts, as long as the
+// output buffer has room; when the buffer turns out too small it is grown to the
+// rows there are and the rows are written by a second launch.  An op whose row
+// limit is below its input's rows is counted, held to the limit and only then
+// written.
 // *done is false when the op has to run as the general kernels instead: more
 // columns than the launch takes, a start that is an index key (k2u), or a device
 // wait that ran out.
@@ -262,7 +263,8 @@ int op_fused(wk_ctx *ctx, wk_history *h, int scol, int ecol, int32_t end_const, 
         (st = take(ctx, ctx->blk_nz, (size_t)nblk * 4)) || (st = reserve_gsum(ctx, groups)) ||
         (filter && (st = take(ctx, ob, (size_t)R * C * 4))))
         return st;
-    const bool count_first = !filter && (ob.cap < (size_t)R * width * 4 || R > ctx->row_limit);
+    const bool count_first = !filter && R > ctx->row_limit;
+    const int64_t room = (int64_t)(ob.cap / ((size_t)width * 4));
     if ((st = clk.begin())) return st;
     const int par = ctx->gs_par;
     unsigned long long *gs = gsum_buffer(ctx, par);
@@ -286,6 +288,7 @@ int op_fused(wk_ctx *ctx, wk_history *h, int scol, int ecol, int32_t end_const, 
     op.clear = gsum_buffer(ctx, par ^ 1);
     op.nclear = 2 + 2 * ctx->gs_used[par ^ 1];
     op.out = ob.as<int32_t>();
+    op.max_rows = (unsigned long long)room;
     op.pub = ctx->h_gs_dev;
     op.seq = ++ctx->pub_seq;
     op.sms = ctx->sms;
@@ -301,18 +304,18 @@ int op_fused(wk_ctx *ctx, wk_history *h, int scol, int ecol, int32_t end_const, 
     if (err & 1ull)
         return fail_corrupt();
     if ((err & (unsigned long long)dev::kErrWait) || (!filter && extra)) return WK_OK;
-    if (count_first) {
-        if (R_out > ctx->row_limit)
-            return set_error(WK_EOVERFLOW, "k2u: %lld output rows exceed the context's row limit %lld",
-                             (long long)R_out, (long long)ctx->row_limit);
-        if ((st = take(ctx, ob, (size_t)R_out * width * 4 + 16))) return st;
-        if (R_out > 0) {
-            op.part = dev::kFusedWrite;
-            op.out = ob.as<int32_t>();
-            if ((st = clk.begin())) return st;
-            if ((le = (cudaError_t)dev::launch_fused(op, ctx->stream)) != cudaSuccess) return cuda_fail(le, "functional write");
-            if ((st = launch_check("functional write")) || (st = clk.end(true))) return st;
-        }
+    if (!filter && R_out > ctx->row_limit)   // nothing was written
+        return set_error(WK_EOVERFLOW, "k2u: %lld output rows exceed the context's row limit %lld", (long long)R_out,
+                         (long long)ctx->row_limit);
+    if (!ob.ptr && (st = take(ctx, ob, 16))) return st;
+    if (!filter && (R_out > room || (count_first && R_out > 0))) {
+        if ((st = take(ctx, ob, (size_t)R_out * width * 4))) return st;
+        op.part = dev::kFusedWrite;
+        op.out = ob.as<int32_t>();
+        op.max_rows = (unsigned long long)R_out;
+        if ((st = clk.begin())) return st;
+        if ((le = (cudaError_t)dev::launch_fused(op, ctx->stream)) != cudaSuccess) return cuda_fail(le, "functional write");
+        if ((st = launch_check("functional write")) || (st = clk.end(true))) return st;
     }
     ctx->last.rows_out = R_out;
     ctx->last.alg_bytes = filter ? 4 * R * C + 16 * R + 4 * extra + 4 * R_out * C

@@ -27,6 +27,14 @@ __device__ __forceinline__ void ld_bucket_half(const uint32_t *p, uint32_t (&v)[
         : "l"(p));
 }
 
+// A word that other CTAs of the same launch write: from L2, at this point of the
+// program (a plain load may come from L1, or be taken from an earlier one).
+__device__ __forceinline__ uint32_t ld_l2(const uint32_t *p) {
+    uint32_t v;
+    asm volatile("ld.global.cg.u32 %0, [%1];" : "=r"(v) : "l"(p));
+    return v;
+}
+
 // Ask L2 for rows [r0, r1) of a table of R rows of C columns, those that lie in
 // the table: one instruction of the calling thread, no registers and no wait.  A
 // first pass reads one column of the rows, every sector of them up to 8 columns,
