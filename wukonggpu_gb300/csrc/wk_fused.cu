@@ -453,7 +453,7 @@ __device__ __forceinline__ void write_filter(const Fused &a, int64_t b0, unsigne
 // CT columns (0: any, filters only).  BPC: blocks per count CTA.  PB (filters): a
 // block per write CTA, as k2u always.
 template <int CT, bool FILTER, int BPC, bool PB>
-__global__ void __launch_bounds__(kThreads, FILTER ? 6 : (CT <= 4 ? 6 : (CT <= 6 ? 5 : 4)))
+__global__ void __launch_bounds__(kThreads, FILTER ? (BPC == 2 ? 5 : 6) : (CT <= 4 ? 6 : (CT <= 6 ? 5 : 4)))
 fused_kernel(const __grid_constant__ Fused a, const __grid_constant__ PredView pv) {
     constexpr int NC = kOct / BPC, NW = PB ? kOct : 1;
     __shared__ __align__(16) int32_t buf[FILTER ? (PB ? 1 : kOct) * kRowsPerBlock / 2 : kRowsPerBlock * (CT + 1) + 4];
@@ -578,8 +578,11 @@ int launch_fused(const FusedOp &op, cudaStream_t st) {
     const int lag = op.sms * 3 / 4 + (1 << kGroupShift) / kOct;
     a.lag = a.steps < lag ? a.steps : lag;
     // two blocks per count CTA (eight look-ups in flight a lane) once there are
-    // enough of them to fill the GPU
-    const bool pair = !op.filter && a.nblk >= 16 * (int64_t)op.sms;
+    // enough of them to fill the GPU.  A filter of 12M rows of 4 columns takes 92 us
+    // with one block a CTA and 84.5 with two when nothing is kept (two kernels: 79),
+    // 100 and 95 (103) at one row in eight, 156 and 156 (169) when all are; of 4M rows
+    // of 8 columns 50, 58.5, 114 and 48, 55, 109
+    const bool pair = a.nblk >= 16 * (int64_t)op.sms;
 #define WK_FUSED(CC)                                                      \
     case CC: return pair ? run_fused<CC, false, 2, true>(a, op.pv, op.part, st) : run_fused<CC, false, 1, true>(a, op.pv, op.part, st)
     if (!op.filter) {
@@ -590,8 +593,10 @@ int launch_fused(const FusedOp &op, cudaStream_t st) {
         return (int)cudaErrorInvalidValue;   // not reached: fused_takes
     }
 #undef WK_FUSED
+    // a filter that is not written block by block has blocks enough for pairs
     const bool pb = filter_per_block(a.nblk, op.sms);
-#define WK_FUSED(CC) return pb ? run_fused<CC, true, 1, true>(a, op.pv, kFusedAll, st) : run_fused<CC, true, 1, false>(a, op.pv, kFusedAll, st)
+#define WK_FUSED(CC) \
+    return pb ? run_fused<CC, true, 1, true>(a, op.pv, kFusedAll, st) : run_fused<CC, true, 2, false>(a, op.pv, kFusedAll, st)
     switch (op.C) {
         case 1: WK_FUSED(1);
         case 2: WK_FUSED(2);
