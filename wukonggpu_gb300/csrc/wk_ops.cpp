@@ -247,7 +247,7 @@ bool alloc_failure_pending(wk_ctx *ctx) { return ctx->inject_alloc_fail.load(std
 // written; so is one whose buffer has room for less than half of the rows that the
 // direction's share of ids with a neighbour lets expect, as it will have to be
 // grown (the first step of a new context on 12M rows that all match, from room for
-// 3.4M: @F0@ us when it writes first, @F1@ so; a step one in fifty of whose rows
+// 3.4M: 494 us when it writes first, 442 so; a step one in fifty of whose rows
 // match, all of which the share lets expect: 98 us each time instead of 76).
 // *done is false when the op has to run as the general kernels instead: more
 // columns than the launch takes, a start that is an index key (k2u), or a device
