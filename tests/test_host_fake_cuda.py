@@ -117,3 +117,13 @@ def size(cap):
     return n
 assert size(4096) - size(1) == 2 * 4 * 4095
 """)
+
+
+def test_new_context_holds_a_small_piece(fake_lib):
+    """Beside its two tables, a context allocates something small when it is made,
+    so that its first step finds the piece of device memory that small
+    allocations come from."""
+    _run(fake_lib, """
+rc = W.RCache(device=0, history_capacity=1 << 20)
+assert 0 < fake.fake_bytes_on(0) - 2 * (4 << 20) <= 1 << 16
+""")
