@@ -461,6 +461,10 @@ int wk_sync(wk_ctx *ctx);
  * (history and op scratch) fail with WK_ENOMEM as a failed cudaMalloc would.
  * For testing the callers' error paths; no device state is touched. */
 int wk_ctx_inject_alloc_failure(wk_ctx *ctx, int32_t n);
+/* For testing what follows when a device wait runs out: the waits inside the
+ * context's one-launch ops (dense functional directions) give up after n polls
+ * (-1: their own bound, about a second), and the op runs as separate kernels. */
+int wk_ctx_set_wait_polls(wk_ctx *ctx, int32_t n);
 /* ------------------------------------------------------- the planner
  * Statistics-based plan of a BGP: Planner::generate_plan
  * (core/planner.hpp:927-1028) over the statistics of

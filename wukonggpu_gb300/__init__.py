@@ -172,6 +172,7 @@ _SIGS = {
     "wk_server_cancel": (C.c_int, [_P, C.c_int64]),
     "wk_server_inject_alloc_failure": (C.c_int, [_P, C.c_int32, C.c_int32]),
     "wk_ctx_inject_alloc_failure": (C.c_int, [_P, C.c_int32]),
+    "wk_ctx_set_wait_polls": (C.c_int, [_P, C.c_int32]),
     "wk_mlp_create": (C.c_int, [_P, C.c_int32, C.c_int32, C.c_uint64, C.POINTER(_P)]),
     "wk_mlp_destroy": (C.c_int, [_P]),
     "wk_mlp_num_params": (C.c_int64, [_P]),
@@ -523,6 +524,10 @@ class RCache:
     def inject_alloc_failure(self, n: int):
         """The next n device-buffer reservations fail with WK_ENOMEM (host-side injection)."""
         _check(load_library().wk_ctx_inject_alloc_failure(self._h, n))
+
+    def set_wait_polls(self, n: int):
+        """The device waits of one-launch ops give up after n polls (-1: their own bound)."""
+        _check(load_library().wk_ctx_set_wait_polls(self._h, n))
 
     def set_row_limit(self, max_rows: int):
         """Cap on k2u output rows (0 = none); larger steps fail with WK_EOVERFLOW."""

@@ -30,7 +30,7 @@
 // A write CTA checks that the groups of 256 blocks up to its own have been
 // counted, and waits if not.  It depends only on CTAs before it in the grid,
 // which the device starts in order, so the wait ends; it is bounded all the
-// same, and an op whose wait ran out runs again as two kernels.
+// same, and an op whose wait ran out runs again as the general kernels.
 //
 // Per-block counts and per-group sums are those of the two-kernel ops: a
 // group's word holds its counted blocks (low 16 bits) and kept rows.  One CTA
@@ -46,9 +46,7 @@ namespace dev {
 
 #define FULL 0xffffffffu
 
-constexpr int kOct = 8;              // blocks per step of the CTA order
-constexpr int kPublishPolls = 1 << 20;
-constexpr int kWritePolls = 1 << 22;   // above the publisher's: it reports first
+constexpr int kOct = 8;   // blocks per step of the CTA order
 
 __device__ __forceinline__ unsigned long long ld_acquire64(const unsigned long long *p) {
     unsigned long long v;
@@ -84,6 +82,7 @@ struct Fused {
     unsigned long long seq;
     int steps, lag;               // octets of blocks, and how many the writing trails by
     int first;                    // the launch's first CTA in that order
+    int pub_polls, write_polls;   // the waits' bounds (FusedOp)
 };
 
 // What CTA `i` does: role 0 counts unit `unit` of octet `oct`, 1 writes it, 2
@@ -119,7 +118,12 @@ __device__ __forceinline__ Role role_of(int i, int steps, int lag, int nc, int n
 
 // Wait until groups 0 .. g are counted; the sum of the kept rows of groups
 // before g, the same in every thread (and of all of them when g is past the
-// last group).  False when the wait ran out.
+// last group).  False when the wait ran out, which the error word says by then.
+//
+// A write CTA's wait may run out at the moment the groups are complete.  So the CTA
+// sets the error first and then looks once more: if the groups are not there now,
+// either, the publisher, which reads the word after it has seen them all, finds
+// the error in it and does not report an op whose block is missing.
 struct WaitShared {
     unsigned long long sum[2][kThreads / 32];
     int there[2][kThreads / 32];
@@ -154,8 +158,14 @@ __device__ __forceinline__ bool groups_before(const Fused &a, int64_t g, int pol
             sum += sh.sum[poll & 1][w];
         }
         if (all) return true;
-        if (poll >= polls) return false;
-        __nanosleep(100);
+        if (poll > polls) return false;
+        if (poll == polls) {
+            if (t == 0) atomicOr(a.err, kErrWait);
+            __threadfence();
+            __syncthreads();
+        } else {
+            __nanosleep(100);
+        }
     }
 }
 
@@ -302,9 +312,9 @@ __device__ __forceinline__ unsigned int blocks_before(const Fused &a, int64_t b)
 // 12M rows of 4 columns took 126 / 98 / 82 / 72 us a step with all / half / one in
 // eight / none of the rows kept, 118 / 91 / 80 / 66 so; as two kernels, whose
 // second is not launched for none, 169 / 131 / 102 / 48.
-// False when the wait ran out.
+// Nothing is written when the wait ran out.
 template <int C>
-__device__ __forceinline__ bool write_k2u(const Fused &a, int64_t b, WaitShared &s_wait, int32_t *buf,
+__device__ __forceinline__ void write_k2u(const Fused &a, int64_t b, WaitShared &s_wait, int32_t *buf,
                                           unsigned int *s_w, unsigned int *s_b) {
     constexpr int W = C + 1, kPasses = kRowsPerBlock / kThreads;
     const int t = threadIdx.x, lane = t & 31, wid = t >> 5;
@@ -322,7 +332,7 @@ __device__ __forceinline__ bool write_k2u(const Fused &a, int64_t b, WaitShared 
         }
     }
     unsigned long long P;
-    if (!groups_before(a, b >> kGroupShift, kWritePolls, s_wait, P)) return false;
+    if (!groups_before(a, b >> kGroupShift, a.write_polls, s_wait, P)) return;
     const bool any = most || ld_l2(a.blk_nz + b) != 0u;
 #pragma unroll
     for (int q = 0; q < kPasses; ++q) {
@@ -348,7 +358,7 @@ __device__ __forceinline__ bool write_k2u(const Fused &a, int64_t b, WaitShared 
         T += s_w[w];
         P += s_b[w];
     }
-    if (T == 0u || P + T > a.max_rows) return true;
+    if (T == 0u || P + T > a.max_rows) return;
     const int lead = (int)((P * W) & 3ull), end = lead + (int)T * W;
     const unsigned below = (1u << lane) - 1u;
 #pragma unroll
@@ -387,7 +397,6 @@ __device__ __forceinline__ bool write_k2u(const Fused &a, int64_t b, WaitShared 
     if (t < 4 && lead + t < i0 && lead + t < end) o[lead + t] = buf[lead + t];
     if (t >= 4 && t < 8 && i1 + t - 4 < end && i1 >= i0) o[i1 + t - 4] = buf[i1 + t - 4];
     if (t == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");   // the buffer goes with the CTA
-    return true;
 }
 
 // Write a filter's blocks: the block's kept rows from its mask words, its
@@ -476,11 +485,11 @@ fused_kernel(const __grid_constant__ Fused a, const __grid_constant__ PredView p
     if (role.kind == 2) {
         // every group counted: the op's totals for the host
         const int64_t ng = (a.nblk + (1 << kGroupShift) - 1) >> kGroupShift;
-        bool ok = groups_before(a, ng, kPublishPolls, s_wait, P);
+        bool ok = groups_before(a, ng, a.pub_polls, s_wait, P);
         if (FILTER && ok) {   // and every write CTA done
             const unsigned long long want = PB ? (unsigned long long)a.nblk : (unsigned long long)a.steps;
             bool all = false;
-            for (int poll = 0; poll < kPublishPolls && !all; ++poll) {
+            for (int poll = 0; poll < a.pub_polls && !all; ++poll) {
                 all = ld_acquire64(a.written) == want;
                 if (!all) __nanosleep(100);
             }
@@ -495,6 +504,7 @@ fused_kernel(const __grid_constant__ Fused a, const __grid_constant__ PredView p
             x = 0ull;
 #pragma unroll
             for (int w = 0; w < kThreads / 32; ++w) x += s_part[w];
+            __threadfence();   // the groups were read before the error word (groups_before)
             a.pub[2] = (unsigned long long)(unsigned int)atomicOr(a.err, 0) | (ok ? 0ull : (unsigned long long)kErrWait);
             a.pub[3] = P;
             a.pub[4] = x;
@@ -505,10 +515,8 @@ fused_kernel(const __grid_constant__ Fused a, const __grid_constant__ PredView p
     }
     const int64_t b = (int64_t)role.oct * kOct + role.unit;
     if (b >= a.nblk) return;   // the same in every thread
-    bool ok;
     if constexpr (FILTER) {
-        ok = groups_before(a, b >> kGroupShift, kWritePolls, s_wait, P);
-        if (ok) {
+        if (groups_before(a, b >> kGroupShift, a.write_polls, s_wait, P)) {
             write_filter<CT, PB>(a, b, P, reinterpret_cast<uint16_t *>(buf), s_n[0], s_b);
             __syncthreads();
             if (threadIdx.x == 0) {
@@ -517,9 +525,8 @@ fused_kernel(const __grid_constant__ Fused a, const __grid_constant__ PredView p
             }
         }
     } else {
-        ok = write_k2u<CT>(a, b, s_wait, buf, s_n[0], s_b);
+        write_k2u<CT>(a, b, s_wait, buf, s_n[0], s_b);
     }
-    if (!ok && threadIdx.x == 0) atomicOr(a.err, kErrWait);
 }
 
 bool fused_takes(int C, bool filter) { return filter || C + 1 <= kFusedCols; }
@@ -569,6 +576,8 @@ int launch_fused(const FusedOp &op, cudaStream_t st) {
     a.max_rows = op.max_rows;
     a.pub = op.pub;
     a.seq = op.seq;
+    a.pub_polls = op.pub_polls;
+    a.write_polls = op.write_polls;
     a.steps = (int)((a.nblk + kOct - 1) / kOct);
     // The writing trails by what the CTAs in flight reach over (6 to 8 a SM, 9 to
     // 16 an octet) and a group's 256 blocks, no more: the rows should still be in

@@ -135,6 +135,9 @@ constexpr int kFusedCols = 11;
 constexpr int kErrWait = 16;
 enum { kFusedAll, kFusedCount, kFusedWrite };
 struct FusedOp {
+    // polls of 100 ns and more after which the publisher and a write CTA give up;
+    // the publisher first: it reports the op
+    int pub_polls = 1 << 20, write_polls = 1 << 22;
     int part = kFusedAll;
     const int32_t *hist;
     int64_t R;

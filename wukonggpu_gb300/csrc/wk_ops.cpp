@@ -275,6 +275,7 @@ int op_fused(wk_ctx *ctx, wk_history *h, int scol, int ecol, int32_t end_const, 
     const int par = ctx->gs_par;
     unsigned long long *gs = gsum_buffer(ctx, par);
     dev::FusedOp op;
+    if (const int polls = ctx->wait_polls.load(std::memory_order_relaxed); polls >= 0) op.pub_polls = op.write_polls = polls;
     op.part = count_first ? dev::kFusedCount : dev::kFusedAll;
     op.hist = h->data;
     op.R = R;
@@ -815,6 +816,12 @@ extern "C" int wk_execute(wk_ctx *ctx, const int64_t *cmd, int32_t n, wk_history
 extern "C" int wk_ctx_inject_alloc_failure(wk_ctx *ctx, int32_t n) {
     if (!ctx || n < 0) return set_error(WK_EINVAL, "wk_ctx_inject_alloc_failure: bad arguments");
     ctx->inject_alloc_fail.store(n);
+    return WK_OK;
+}
+
+extern "C" int wk_ctx_set_wait_polls(wk_ctx *ctx, int32_t n) {
+    if (!ctx || n < -1) return set_error(WK_EINVAL, "wk_ctx_set_wait_polls: bad arguments");
+    ctx->wait_polls.store(n);
     return WK_OK;
 }
 

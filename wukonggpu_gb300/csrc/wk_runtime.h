@@ -121,6 +121,9 @@ struct wk_ctx {
 
     // injected allocation failures still to come (wk_ctx_inject_alloc_failure)
     std::atomic<int> inject_alloc_fail{0};
+    // the one-launch ops' device waits give up after this many polls (< 0: their own
+    // bounds; wk_ctx_set_wait_polls)
+    std::atomic<int> wait_polls{-1};
 
     // the no-allocation entry point's scratch array on this device, resolved
     // when the context is made (wk_noalloc.cu)
