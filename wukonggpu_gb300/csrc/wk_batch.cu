@@ -73,11 +73,11 @@ constexpr int kMaxQ = 4096;                 // queries per batch
 
 // largest q with off[q] <= g (off: the step's input row offsets, Q + 1 of
 // them, read through L1)
-__device__ __forceinline__ int find_query(const int64_t *__restrict__ off, int Q, int64_t g) {
+__device__ __forceinline__ int find_query(const int64_t *off, int Q, int64_t g) {
     int lo = 0, hi = Q - 1;
     while (lo < hi) {
         const int mid = (lo + hi + 1) >> 1;
-        if (__ldg(off + mid) <= g) lo = mid;
+        if (ld_prior(off + mid) <= g) lo = mid;
         else hi = mid - 1;
     }
     return lo;
@@ -86,11 +86,11 @@ __device__ __forceinline__ int find_query(const int64_t *__restrict__ off, int Q
 // As find_query for one row by a whole warp: each round asks 32 pivots with
 // one load, so 4096 queries take three dependent loads instead of twelve (the
 // step kernels are chains of such loads, each starting with a cold L1).
-__device__ __forceinline__ int find_query_warp(const int64_t *__restrict__ off, int Q, int64_t g, int lane) {
+__device__ __forceinline__ int find_query_warp(const int64_t *off, int Q, int64_t g, int lane) {
     int lo = 0, n = Q;
     while (n > 1) {
         const int step = (n + 31) >> 5, i = lane * step;
-        const unsigned m = __ballot_sync(FULL, i < n && __ldg(off + lo + i) <= g);
+        const unsigned m = __ballot_sync(FULL, i < n && ld_prior(off + lo + i) <= g);
         const int k = 31 - __clz((int)m);   // off is ascending: the pivots at or below g come first
         lo += k * step;
         n = n - k * step < step ? n - k * step : step;
@@ -101,8 +101,8 @@ __device__ __forceinline__ int find_query_warp(const int64_t *__restrict__ off, 
 // The queries of 32 consecutive rows g0 + lane, whose first belongs to q0: the
 // boundaries of the next 32 queries, one per lane, searched by shuffles; rows
 // past them (behind that many empty queries) search on their own.
-__device__ __forceinline__ int find_queries(const int64_t *__restrict__ off, int Q, int64_t g0, int q0, int lane) {
-    const int64_t rel = q0 + 1 + lane < Q ? __ldg(off + q0 + 1 + lane) - g0 : 64;
+__device__ __forceinline__ int find_queries(const int64_t *off, int Q, int64_t g0, int q0, int lane) {
+    const int64_t rel = q0 + 1 + lane < Q ? ld_prior(off + q0 + 1 + lane) - g0 : 64;
     const int p = rel < 64 ? (int)rel : 64;   // > 0: q0 is the last query that begins at or before g0
     int k = 0;                                // boundaries at or before row g0 + lane
 #pragma unroll
@@ -175,7 +175,7 @@ __device__ __forceinline__ unsigned long long warp_scan(unsigned long long v, in
 template <int BT>
 __device__ __forceinline__ void count_phase(const StepIO &io, int rounds) {
     const int lane = threadIdx.x & 31;
-    const int64_t total = io.in_row_off[io.Q];
+    const int64_t total = ld_prior(io.in_row_off + io.Q);
     const int rho = rows_per_tile(total, io.warps, rounds);
     const int64_t ntiles = (total + rho - 1) / rho;
     for (int64_t tile = first_tile(); tile < ntiles; tile += (int64_t)gridDim.x * (BT / 32)) {
@@ -197,10 +197,10 @@ __device__ __forceinline__ void count_phase(const StepIO &io, int rounds) {
                 if (d.kind == BK_C2U) {
                     vid = d.cst;
                 } else {
-                    const int64_t r = g - __ldg(io.in_row_off + q);
+                    const int64_t r = g - ld_prior(io.in_row_off + q);
                     const int32_t *row = io.hist + io.in_int_off[q] + r * io.in_cols[q];
-                    vid = __ldg(row + d.scol);
-                    target = d.kind == BK_K2K ? __ldg(row + d.ecol) : d.cst;
+                    vid = ld_prior(row + d.scol);
+                    target = d.kind == BK_K2K ? ld_prior(row + d.ecol) : d.cst;
                 }
             }
             uint32_t o = 0u, deg = 0u;
@@ -272,7 +272,7 @@ __device__ __forceinline__ unsigned long long block_scan(unsigned long long v, u
 constexpr int kScanPer = 4;   // loads in flight
 __device__ __forceinline__ void scan_tiles(const StepIO &io, int rounds, unsigned long long *ws) {
     const int nt = blockDim.x, t = threadIdx.x;
-    const int64_t total = io.in_row_off[io.Q];
+    const int64_t total = ld_prior(io.in_row_off + io.Q);
     const int rho = rows_per_tile(total, io.warps, rounds);
     const int64_t n = (total + rho - 1) / rho;
     unsigned long long carry = 0ull;
@@ -281,7 +281,7 @@ __device__ __forceinline__ void scan_tiles(const StepIO &io, int rounds, unsigne
 #pragma unroll
         for (int k = 0; k < kScanPer; ++k) {
             const int64_t i = i0 + 2 * ((int64_t)k * nt + t);   // the buffer holds an even number of tiles
-            p[k] = i < n ? __ldcg(reinterpret_cast<const ulonglong2 *>(io.tile_sum + i)) : make_ulonglong2(0ull, 0ull);
+            p[k] = i < n ? ld_l2(reinterpret_cast<const ulonglong2 *>(io.tile_sum + i)) : make_ulonglong2(0ull, 0ull);
             if (i + 1 >= n) p[k].y = 0ull;
         }
 #pragma unroll
@@ -310,7 +310,7 @@ __device__ __forceinline__ void scan_queries(const StepIO &io, unsigned long lon
             w[k] = 0;
             if (q < Q) {
                 const int kind = io.desc[q].kind, cols = io.in_cols[q];
-                r[k] = __ldcg(io.q_rows + q);
+                r[k] = ld_l2(io.q_rows + q);
                 w[k] = kind == BK_K2U ? cols + 1 : (kind == BK_C2U ? 1 : cols);
             }
         }
@@ -383,18 +383,18 @@ __device__ __forceinline__ void write_row_warp(int kind, const int32_t *row, con
 template <int BT>
 __device__ __forceinline__ void write_phase(const StepIO &io, int rounds, int split) {
     const int lane = threadIdx.x & 31;
-    const int64_t total = io.in_row_off[io.Q];
+    const int64_t total = ld_prior(io.in_row_off + io.Q);
     const int rho = rows_per_tile(total, io.warps, rounds);
     const int64_t ntiles = (total + rho - 1) / rho;
     const int64_t most = rho < 32 ? ((int64_t)split * rho + 31) / 32 : split;
     for (int64_t tile = first_tile(); tile < ntiles; tile += (int64_t)gridDim.x * (BT / 32)) {
-        unsigned long long base = __ldcg(io.tile_sum + tile);
+        unsigned long long base = ld_l2(io.tile_sum + tile);
         int q0 = find_query_warp(io.in_row_off, io.Q, tile * rho, lane);
         for (int r0 = 0; r0 < rho && tile * rho + r0 < total; r0 += 32) {
             const int64_t g = tile * rho + r0 + lane;
             const int q = find_queries(io.in_row_off, io.Q, g - lane, q0, lane);
             q0 = __shfl_sync(FULL, q, 31);
-            const uint32_t c = r0 + lane < rho && g < total ? __ldcg(io.cnt + g) : 0u;
+            const uint32_t c = r0 + lane < rho && g < total ? ld_l2(io.cnt + g) : 0u;
             const unsigned long long inc = warp_scan(c, lane);
             const unsigned long long pos = base + inc - c;
             base += __shfl_sync(FULL, inc, 31);
@@ -406,9 +406,9 @@ __device__ __forceinline__ void write_phase(const StepIO &io, int rounds, int sp
                 kind = d.kind;
                 cin = io.in_cols[q];
                 w = (kind == BK_K2U) ? cin + 1 : (kind == BK_C2U ? 1 : cin);
-                row = io.hist + io.in_int_off[q] + (g - __ldg(io.in_row_off + q)) * cin;
-                dst = io.out + __ldcg(io.out_int_off + q) + ((int64_t)pos - __ldcg(io.out_row_off + q)) * w;
-                if (kind == BK_K2U || kind == BK_C2U) e = io.pvs[d.pid].edges + __ldcg(io.off + g);
+                row = io.hist + io.in_int_off[q] + (g - ld_prior(io.in_row_off + q)) * cin;
+                dst = io.out + ld_l2(io.out_int_off + q) + ((int64_t)pos - ld_l2(io.out_row_off + q)) * w;
+                if (kind == BK_K2U || kind == BK_C2U) e = io.pvs[d.pid].edges + ld_l2(io.off + g);
             }
             const bool big = c != 0u && (int64_t)c * w > most;
             if (c != 0u && !big) {
@@ -443,7 +443,7 @@ batch_write_kernel(StepIO io, int rounds, int split) {
     // took 93 us, 4096 200; this way 84 and 192)
     if (io.pub != nullptr) {
         const int n = 2 * (2 * io.Q + 2) + io.Q;
-        for (int i = blockIdx.x * BT + threadIdx.x; i < n; i += gridDim.x * BT) io.pub[i] = __ldcg(io.flags + i);
+        for (int i = blockIdx.x * BT + threadIdx.x; i < n; i += gridDim.x * BT) io.pub[i] = ld_l2(io.flags + i);
     }
     if (io.flags[1]) return;
     write_phase<BT>(io, rounds, split);

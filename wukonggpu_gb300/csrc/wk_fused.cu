@@ -202,8 +202,8 @@ __device__ __forceinline__ void count_blocks(const Fused &a, const PredView &pv,
 #pragma unroll
     for (int rd = 0; rd < NR; ++rd) {
         const int64_t r = row_at(rd);
-        v[rd] = r < a.R ? __ldg(a.hist + r * C + a.scol) : -1;
-        if constexpr (FILTER) tg[rd] = r < a.R && a.ecol >= 0 ? __ldg(a.hist + r * C + a.ecol) : a.end_const;
+        v[rd] = r < a.R ? ld_prior(a.hist + r * C + a.scol) : -1;
+        if constexpr (FILTER) tg[rd] = r < a.R && a.ecol >= 0 ? ld_prior(a.hist + r * C + a.ecol) : a.end_const;
     }
     unsigned zeros = 0u;   // rounds in which this lane's row starts at an index key
     int32_t g[NR];
@@ -273,22 +273,22 @@ __device__ __forceinline__ void count_blocks(const Fused &a, const PredView &pv,
 
 // One row of C words, in the widest loads that C (and the table's alignment) allows.
 template <int C>
-__device__ __forceinline__ void copy_row_regs(const int32_t *__restrict__ src, int32_t *v, bool aligned) {
+__device__ __forceinline__ void copy_row_regs(const int32_t *src, int32_t *v, bool aligned) {
     if (C % 4 == 0 && aligned) {
 #pragma unroll
         for (int c = 0; c + 3 < C; c += 4) {
-            const int4 x = __ldg(reinterpret_cast<const int4 *>(src + c));
+            const int4 x = ld_prior(reinterpret_cast<const int4 *>(src + c));
             v[c] = x.x; v[c + 1] = x.y; v[c + 2] = x.z; v[c + 3] = x.w;
         }
     } else if (C % 2 == 0 && aligned) {
 #pragma unroll
         for (int c = 0; c + 1 < C; c += 2) {
-            const int2 x = __ldg(reinterpret_cast<const int2 *>(src + c));
+            const int2 x = ld_prior(reinterpret_cast<const int2 *>(src + c));
             v[c] = x.x; v[c + 1] = x.y;
         }
     } else {
 #pragma unroll
-        for (int c = 0; c < C; ++c) v[c] = __ldg(src + c);
+        for (int c = 0; c < C; ++c) v[c] = ld_prior(src + c);
     }
 }
 
@@ -297,7 +297,7 @@ __device__ __forceinline__ void copy_row_regs(const int32_t *__restrict__ src, i
 __device__ __forceinline__ unsigned int blocks_before(const Fused &a, int64_t b) {
     static_assert(kThreads == (1 << kGroupShift), "one thread per block of a group");
     const int64_t i = ((b >> kGroupShift) << kGroupShift) + threadIdx.x;
-    return __reduce_add_sync(FULL, i < b ? __ldcg(a.blk_nz + i) : 0u);
+    return __reduce_add_sync(FULL, i < b ? ld_l2(a.blk_nz + i) : 0u);
 }
 
 // Write block b of a k2u op: its matched rows with the neighbour appended,
@@ -337,7 +337,7 @@ __device__ __forceinline__ void write_k2u(const Fused &a, int64_t b, WaitShared 
 #pragma unroll
     for (int q = 0; q < kPasses; ++q) {
         const int r = wid * (32 * kPasses) + q * 32 + lane;
-        x[q] = any && r < n ? __ldcg(a.nbr + r0 + r) : -1;
+        x[q] = any && r < n ? ld_l2(a.nbr + r0 + r) : -1;
     }
     if (!most) {
 #pragma unroll
@@ -409,7 +409,7 @@ __device__ __forceinline__ void write_filter(const Fused &a, int64_t b0, unsigne
     const int t = threadIdx.x, lane = t & 31, w = t >> 5;
     const unsigned int before = blocks_before(a, b0);
     if (lane == 0) s_b[w] = before;
-    if (t < kOct) s_nz[t] = b0 + t < a.nblk ? __ldcg(a.blk_nz + b0 + t) : 0u;
+    if (t < kOct) s_nz[t] = b0 + t < a.nblk ? ld_l2(a.blk_nz + b0 + t) : 0u;
     __syncthreads();
 #pragma unroll
     for (int i = 0; i < kThreads / 32; ++i) P += s_b[i];
@@ -419,7 +419,7 @@ __device__ __forceinline__ void write_filter(const Fused &a, int64_t b0, unsigne
     if (nb == 0u) return;   // the block keeps nothing (or lies past the table)
     const int64_t r0 = (PB ? b0 : b0 + w) * kRowsPerBlock;
     const int64_t wi = (r0 >> 5) + lane, nwords = (a.R + 31) >> 5;
-    uint32_t m = wi < nwords ? __ldcg(a.mask + wi) : 0u;   // bits past R are 0
+    uint32_t m = wi < nwords ? ld_l2(a.mask + wi) : 0u;   // bits past R are 0
     const unsigned int c = __popc(m);
     unsigned int pos = c;
 #pragma unroll
@@ -445,7 +445,7 @@ __device__ __forceinline__ void write_filter(const Fused &a, int64_t b0, unsigne
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             const uint32_t kk = 4u * u + (uint32_t)j - lead;   // wraps above `words` before the lead
-            v[j] = kk < words ? __ldg(hb + (int)ws[kk / (uint32_t)C] * C + (int)(kk % (uint32_t)C)) : 0;
+            v[j] = kk < words ? ld_prior(hb + (int)ws[kk / (uint32_t)C] * C + (int)(kk % (uint32_t)C)) : 0;
         }
         if (4u * u >= lead && 4u * u + 4u <= lead + words) {
             reinterpret_cast<int4 *>(gout)[u] = make_int4(v[0], v[1], v[2], v[3]);
@@ -496,7 +496,7 @@ fused_kernel(const __grid_constant__ Fused a, const __grid_constant__ PredView p
             ok = __syncthreads_and(all) != 0;
         }
         unsigned long long x = 0ull;
-        for (int64_t i = threadIdx.x; ok && i < ng; i += kThreads) x += __ldcg(a.gs + 2 * i + 1);
+        for (int64_t i = threadIdx.x; ok && i < ng; i += kThreads) x += ld_l2(a.gs + 2 * i + 1);
         x = warp_add(x);
         if ((threadIdx.x & 31) == 0) s_part[threadIdx.x >> 5] = x;
         __syncthreads();

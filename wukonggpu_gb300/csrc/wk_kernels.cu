@@ -163,7 +163,7 @@ k2u_count_kernel(const int32_t *__restrict__ hist, int64_t R, int C, int scol, u
 #pragma unroll
     for (int rd = 0; rd < NR; ++rd) {
         const int64_t r = row_at(rd);
-        v[rd] = r < R ? __ldg(hist + r * C + scol) : -1;
+        v[rd] = r < R ? ld_prior(hist + r * C + scol) : -1;
     }
     unsigned long long my_sum[BPC];
     unsigned int nent[BPC], run[BPC];   // the warp's entries and output rows so far
@@ -316,14 +316,14 @@ __device__ __forceinline__ void plan_group(const SlicePlan &a, int64_t g) {
     // output rows and slices of the groups before
     unsigned long long op = 0ull, sp = 0ull;
     for (int64_t i = t; i < g; i += kThreads) {
-        op += __ldcg(a.group_sums + 2 * i);
-        sp += __ldcg(a.group_sums + 2 * i + 1);
+        op += ld_prior(a.group_sums + 2 * i);
+        sp += ld_prior(a.group_sums + 2 * i + 1);
     }
     op = warp_sum(op);
     sp = warp_sum(sp);
     if (lane == 0) { s_before[0][wid] = op; s_before[1][wid] = sp; }
     const int64_t bi = (g << kGroupShift) + t;
-    const unsigned long long word = bi < a.nblk ? a.blk_sum[bi] : 0ull;
+    const unsigned long long word = bi < a.nblk ? ld_prior(a.blk_sum + bi) : 0ull;
     unsigned long long x = word & kSumMask, y = slices_of(word & kSumMask);
     const unsigned long long x0 = x, y0 = y;
     cta_scan2(x, y, sw);
@@ -338,7 +338,7 @@ __device__ __forceinline__ void plan_group(const SlicePlan &a, int64_t g) {
     if (t == 0 && a.head != nullptr && (g + 1) << kGroupShift >= a.nblk) {   // the last group
         const unsigned long long rows = op + s_x[kThreads - 1] + (s_word[kThreads - 1] & kSumMask);
         const unsigned long long n = sp + s_y[kThreads];
-        *a.head = *a.err == 0 && n <= a.max_slices && rows <= a.max_rows ? (uint32_t)n : 0u;
+        *a.head = ld_prior(a.err) == 0 && n <= a.max_slices && rows <= a.max_rows ? (uint32_t)n : 0u;
     }
     const unsigned long long last = a.first + a.cap;   // the group's slices of the window
     const uint32_t i0 = a.first > sp ? (uint32_t)min(a.first - sp, (unsigned long long)s_y[kThreads]) : 0u;
@@ -378,7 +378,7 @@ __global__ void __launch_bounds__(kThreads) publish_kernel(const Publish pub, co
         return;
     }
     if (pub.dst == nullptr) return;
-    for (long long w = threadIdx.x; w < pub.n; w += blockDim.x) pub.dst[2 + w] = __ldcg(pub.src + w);
+    for (long long w = threadIdx.x; w < pub.n; w += blockDim.x) pub.dst[2 + w] = ld_prior(pub.src + w);
     __threadfence_system();
     __syncthreads();
     if (threadIdx.x == 0) *(volatile unsigned long long *)pub.dst = pub.seq;
@@ -448,13 +448,6 @@ __device__ __forceinline__ void bulk_store(int32_t *dst, const int32_t *src, uin
                  : "memory");
 }
 __device__ __forceinline__ void bulk_read_done() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
-
-// 16 B that the grid before has written: after wait_prior_grid, in program order
-__device__ __forceinline__ uint4 load16(const void *p) {
-    uint4 v;
-    asm volatile("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
-    return v;
-}
 
 // 16 B from global to shared memory without registers
 __device__ __forceinline__ void copy16(void *dst, const void *src) {
@@ -668,10 +661,11 @@ k2u_expand_kernel(const int32_t *__restrict__ hist, int C_rt, const int32_t *__r
     wait_prior_grid();   // the records are complete
     if constexpr (NT == kThreads) allow_dependent_grid();   // see above
 
-    if (head != nullptr && blockIdx.x >= *head) return;
+    if (head != nullptr && blockIdx.x >= ld_prior(head)) return;
 
     // 1. the slice
-    const uint4 ra = load16(slices + blockIdx.x), rb = load16(reinterpret_cast<const uint4 *>(slices + blockIdx.x) + 1);
+    const uint4 *rec = reinterpret_cast<const uint4 *>(slices + blockIdx.x);
+    const uint4 ra = ld_prior(rec), rb = ld_prior(rec + 1);
     const unsigned long long P = (unsigned long long)ra.y << 32 | ra.x;   // SliceRec: P, block, T | slice, n
     const uint32_t T = ra.w, slice = rb.x;
     const int n = (int)rb.y;
@@ -828,8 +822,8 @@ filter_probe_kernel(const int32_t *__restrict__ hist, int64_t R, int C, int scol
 #pragma unroll
     for (int rd = 0; rd < kRounds; ++rd) {
         const int64_t r = wrow0 + rd * 32 + lane;
-        v[rd] = r < R ? __ldg(hist + r * C + scol) : -1;
-        tg[rd] = (r < R && ecol >= 0) ? __ldg(hist + r * C + ecol) : end_const;
+        v[rd] = r < R ? ld_prior(hist + r * C + scol) : -1;
+        tg[rd] = (r < R && ecol >= 0) ? ld_prior(hist + r * C + ecol) : end_const;
     }
     // every round's list: offset and entries (none past the table)
     uint32_t o[kRounds], d[kRounds];
@@ -941,9 +935,9 @@ filter_write_kernel(const int32_t *__restrict__ hist, int64_t R, int C_rt, const
 
     // 1. the prefix of block b0, and the CTA's blocks' counts
     unsigned long long x = 0ull;
-    for (int64_t i = t; i < g; i += kThreads) x += group_sums[2 * i];
-    for (int64_t i = (g << kGroupShift) + t; i < b0; i += kThreads) x += blk_nz[i];
-    if (t < kWriteBlocks) s_nz[t] = b0 + t < nblk ? blk_nz[b0 + t] : 0u;
+    for (int64_t i = t; i < g; i += kThreads) x += ld_prior(group_sums + 2 * i);
+    for (int64_t i = (g << kGroupShift) + t; i < b0; i += kThreads) x += ld_prior(blk_nz + i);
+    if (t < kWriteBlocks) s_nz[t] = b0 + t < nblk ? ld_prior(blk_nz + b0 + t) : 0u;
     x = warp_sum(x);
     if (lane == 0) s_part[w] = x;
     __syncthreads();
@@ -958,7 +952,7 @@ filter_write_kernel(const int32_t *__restrict__ hist, int64_t R, int C_rt, const
     // 2. the block's kept rows, in order
     const int64_t b = PB ? b0 : b0 + w, r0 = b * kRowsPerBlock;
     const int64_t wi = (r0 >> 5) + lane, nwords = (R + 31) >> 5;
-    uint32_t m = wi < nwords ? mask[wi] : 0u;   // bits past R are 0
+    uint32_t m = wi < nwords ? ld_prior(mask + wi) : 0u;   // bits past R are 0
     const unsigned int c = __popc(m);
     unsigned int pos = c;
 #pragma unroll

@@ -57,7 +57,7 @@ constexpr float kB1 = 0.9f, kB2 = 0.999f;   // Adam moment decay rates
 // brought to the device (pids_to and tgt_to, or in place); and the words that
 // the step adds into, cleared.
 __global__ void __launch_bounds__(256)
-build_input_kernel(const float *__restrict__ feats, const int32_t *pids, const float *tgt,
+build_input_kernel(const float *feats, const int32_t *pids, const float *tgt,
                    int32_t *pids_to, float *tgt_to, int M, int Mp,
                    const float *__restrict__ emb, int n_ids, __nv_bfloat16 *__restrict__ X0,
                    __nv_bfloat16 *__restrict__ X0t, float *__restrict__ zero, int64_t nzero) {

@@ -33,6 +33,7 @@
 // bounds came back through pageable memory.  6M rows of 3 columns over 8 owners
 // took 147 us so, 82 now; the moves are left bound by their issue slots.
 #include "wk_runtime.h"
+#include "wk_loads.cuh"
 
 #include <algorithm>
 
@@ -213,7 +214,7 @@ __global__ void part_bounds_kernel(const uint32_t *__restrict__ start, int64_t n
 // copies its row.  BITS: of the largest owner, or more.
 template <typename V, int PER, int BITS, bool STAGED>
 __global__ void __launch_bounds__(kThreads, 6)
-part_move_kernel(const Split a, const uint32_t *__restrict__ start, int32_t *__restrict__ out) {
+part_move_kernel(const Split a, const uint32_t *start, int32_t *__restrict__ out) {
     __shared__ uint32_t wc[kWarps][kMaxParts];   // per warp: its rows per owner, then its next place per owner
     __shared__ uint32_t s_at[kMaxParts];         // STAGED: an owner's start in `out` minus its place in the tile
     __shared__ uint32_t s_w[kWarps];
@@ -269,7 +270,7 @@ part_move_kernel(const Split a, const uint32_t *__restrict__ start, int32_t *__r
     uint32_t total = 0u, first = 0u;
     const uint32_t p = threadIdx.x;   // kThreads == kMaxParts
     if (p < nparts) {
-        first = start[(int64_t)p * a.ntiles + t];
+        first = dev::ld_prior(start + (int64_t)p * a.ntiles + t);
 #pragma unroll
         for (int x = 0; x < kWarps; ++x) total += wc[x][p];
     }

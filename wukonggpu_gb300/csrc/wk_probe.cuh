@@ -10,6 +10,7 @@
 #pragma once
 
 #include "wk_internal.h"
+#include "wk_loads.cuh"
 
 namespace wk {
 namespace dev {
@@ -25,14 +26,6 @@ __device__ __forceinline__ void ld_bucket_half(const uint32_t *p, uint32_t (&v)[
     asm("ld.global.nc.L1::no_allocate.v8.u32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
         : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
         : "l"(p));
-}
-
-// A word that other CTAs of the same launch write: from L2, at this point of the
-// program (a plain load may come from L1, or be taken from an earlier one).
-__device__ __forceinline__ uint32_t ld_l2(const uint32_t *p) {
-    uint32_t v;
-    asm volatile("ld.global.cg.u32 %0, [%1];" : "=r"(v) : "l"(p));
-    return v;
 }
 
 // Ask L2 for rows [r0, r1) of a table of R rows of C columns, those that lie in

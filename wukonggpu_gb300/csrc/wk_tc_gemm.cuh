@@ -48,6 +48,8 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include "wk_loads.cuh"
+
 namespace wk {
 namespace tc {
 
@@ -224,7 +226,7 @@ __device__ __forceinline__ void sum_rows(const float2 *part, int n, int m, float
     const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
     float sq = 0.f, sdy = 0.f;
     for (int i = t; i < n; i += kThreads) {
-        const float2 v = __ldcg(part + i);
+        const float2 v = dev::ld_prior(part + i);
         sq += v.x;
         sdy += v.y;
     }
