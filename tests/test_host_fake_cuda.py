@@ -127,3 +127,17 @@ def test_new_context_holds_a_small_piece(fake_lib):
 rc = W.RCache(device=0, history_capacity=1 << 20)
 assert 0 < fake.fake_bytes_on(0) - 2 * (4 << 20) <= 1 << 16
 """)
+
+
+@pytest.mark.parametrize("cols", [1 << 23, 1 << 24])
+def test_partition_of_very_wide_rows(fake_lib, cols):
+    """Widths whose words per tile pass 32 bits are copied row by row, as every
+    width above a tile's is."""
+    _run(fake_lib, f"""
+rc = context(0)
+req = W.Request([])
+rc.upload_history(req, np.zeros((1, {cols}), np.int32))
+n = fake.fake_launches()
+rc.partition(req, -1, 2)        # the kernels do nothing: only the launches count
+assert fake.fake_launches() - n == 3
+""")

@@ -224,7 +224,7 @@ part_move_kernel(const Split a, const uint32_t *start, int32_t *__restrict__ out
     const int rows = kThreads * a.rounds;
     const int64_t t = blockIdx.x, r0 = t * rows;
     const int n = (int)((a.R - r0) < rows ? (a.R - r0) : rows);
-    const int per = PER > 0 ? PER : a.C * 4 / (int)sizeof(V);   // vectors a row
+    const int per = PER > 0 ? PER : a.C / (int)(sizeof(V) / 4);   // vectors a row
     V *tile = reinterpret_cast<V *>(smem);
     uint32_t *s_out = reinterpret_cast<uint32_t *>(tile + (STAGED ? rows * per : 0));
     uint16_t *s_src = reinterpret_cast<uint16_t *>(s_out + (STAGED ? rows : 0));
@@ -251,7 +251,7 @@ part_move_kernel(const Split a, const uint32_t *start, int32_t *__restrict__ out
 #pragma unroll
     for (int c = 0; c < kMaxRounds; ++c) {
         const int r = tile_row(w, c, lane, a.rounds);
-        own[c] = c < a.rounds && r < n ? (uint32_t)key[r * a.C + a.col] : 0u;
+        own[c] = c < a.rounds && r < n ? (uint32_t)key[(STAGED ? r * a.C : (int64_t)r * a.C) + a.col] : 0u;
     }
 #pragma unroll
     for (int c = 0; c < kMaxRounds; ++c) {
@@ -388,7 +388,7 @@ extern "C" int wk_history_partition(wk_ctx *ctx, const wk_history *in, int64_t s
         a.by.m = nparts == 1 ? 0xffffffffu : (uint32_t)((1ull << 32) / (unsigned)nparts);
         // a tile of up to 2048 rows: as many as fit 24 KB; rows of more than
         // kTileWords / kThreads columns are copied lane by lane
-        const bool staged = C * kThreads <= kTileWords;
+        const bool staged = C <= kTileWords / kThreads;
         a.rounds = staged ? std::min(kMaxRounds, kTileWords / (C * kThreads)) : kMaxRounds;
         const int rows = kThreads * a.rounds;
         a.ntiles = (R + rows - 1) / rows;
