@@ -141,3 +141,25 @@ n = fake.fake_launches()
 rc.partition(req, -1, 2)        # the kernels do nothing: only the launches count
 assert fake.fake_launches() - n == 3
 """)
+
+
+def test_estimator_errors_leave_nothing_in_flight(fake_lib):
+    """A call that fails on the host once copies are queued returns when they are
+    done: the caller's arrays are the caller's again."""
+    _run(fake_lib, """
+est = W.Estimator(context(0), 4, max_batch=4096, seed=1)
+def samples(n):
+    return np.zeros((n, 48), np.float32), np.ones(n, np.int32), np.zeros(n, np.float32)
+fake.fake_no_driver_entry(1)    # no tensor map can be made
+calls = [lambda n=n: est.predict(*samples(n)[:2]) for n in (16, 2000, 20_000, 100_000)]
+calls += [lambda n=n: est.gradients(*samples(n)) for n in (16, 2000)]
+for call in calls:
+    try:
+        call()
+        raise SystemExit("no error")
+    except W.WkError as e:
+        assert e.status == W.WK_EDEVICE, e
+    assert fake.fake_pending() == 0
+fake.fake_no_driver_entry(0)
+calls[0]()                      # and the next call is its own
+""")

@@ -299,16 +299,25 @@ cudaError_t copy_status(wk_mlp *m, cudaStream_t s) {
     return cudaMemcpyAsync(m->h_loss, m->loss, 16, cudaMemcpyDeviceToHost, s);
 }
 
+// An error return once copies or kernels of the call are queued: nothing of them
+// still reads or writes the caller's arrays or the pinned block when it returns.
+int settled(wk_mlp *m, cudaStream_t s, int st) {
+    cudaStreamSynchronize(m->copy);
+    cudaStreamSynchronize(s);
+    m->status = WK_OK;   // reported with this call
+    return st;
+}
+
 // the status of the work queued since the last check: a host-side failure, a
 // launch error, or a tensor-core wait that ran out (bit 2 of the device flag)
 int check_status(wk_mlp *m, cudaStream_t s, const char *what, bool copied = false) {
     int st = m->status;
     m->status = WK_OK;
-    if (st) return st;
+    if (st) return settled(m, s, st);
     cudaError_t e = cudaGetLastError();
     if (e == cudaSuccess && !copied) e = copy_status(m, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    if (e != cudaSuccess) return cuda_fail(e, what);
+    if (e != cudaSuccess) return settled(m, s, cuda_fail(e, what));
     int f;
     std::memcpy(&f, m->h_loss + 2, sizeof(f));
     if (f) {
@@ -621,14 +630,14 @@ extern "C" int wk_mlp_gradients(wk_mlp *m, const float *feats, const int32_t *pi
         if (e == cudaSuccess) e = cudaMemcpyAsync(m->pids, pids, sizeof(int32_t) * (size_t)M, cudaMemcpyHostToDevice, s);
         if (e == cudaSuccess) e = cudaMemcpyAsync(m->tgt, tgt, sizeof(float) * (size_t)M, cudaMemcpyHostToDevice, s);
     }
-    if (e != cudaSuccess) return cuda_fail(e, "mlp upload");
+    if (e != cudaSuccess) return settled(m, s, cuda_fail(e, "mlp upload"));
     gradient_step(m, f, p, t, M, s);
     e = cudaGetLastError();
     // the status first: the copy to the caller's memory holds the host until it is done
     if (e == cudaSuccess) e = copy_status(m, s);
     if (e == cudaSuccess && grads_host)
         e = cudaMemcpyAsync(grads_host, m->grads, sizeof(float) * (size_t)m->n_params, cudaMemcpyDeviceToHost, s);
-    if (e != cudaSuccess) return cuda_fail(e, "wk_mlp_gradients");
+    if (e != cudaSuccess) return settled(m, s, cuda_fail(e, "wk_mlp_gradients"));
     if ((st = check_status(m, s, "wk_mlp_gradients", true))) return st;
     if (loss_host) *loss_host = m->h_loss[0];
     return WK_OK;
@@ -642,7 +651,7 @@ extern "C" int wk_mlp_gradients(wk_mlp *m, const float *feats, const int32_t *pi
 // its batch there by the epoch's order.  A step of a full batch is the same
 // launch sequence every time (its batch index and Adam bias corrections are
 // read from device memory), so the second full batch is captured as a CUDA
-// graph and every later one replays it: one launch instead of about forty.
+// graph and every later one replays it: one launch instead of fifteen.
 // A shorter last batch runs as plain launches.  The host reads the device
 // once per epoch (the loss sum and the GEMM status).
 extern "C" int wk_mlp_train(wk_mlp *m, const float *feats, const int32_t *pids, const float *tgt, int64_t n,
@@ -793,11 +802,7 @@ extern "C" int wk_mlp_predict(wk_mlp *m, const float *feats, const int32_t *pids
         if (e == cudaSuccess) e = copy_status(m, s);
         if (e == cudaSuccess)
             e = cudaMemcpyAsync(out, m->pred.ptr, sizeof(float) * (size_t)n, cudaMemcpyDeviceToHost, s);
-        if (e != cudaSuccess) {
-            cudaStreamSynchronize(m->copy);   // nothing still reads the caller's arrays
-            cudaStreamSynchronize(s);
-            return cuda_fail(e, "wk_mlp_predict");
-        }
+        if (e != cudaSuccess) return settled(m, s, cuda_fail(e, "wk_mlp_predict"));
         if ((st = check_status(m, s, "wk_mlp_predict", true))) return st;
     }
     m->ctx->launches += m->kernels;
