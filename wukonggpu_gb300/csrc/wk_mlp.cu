@@ -163,7 +163,8 @@ struct wk_mlp {
     // bf16 weights (row-major, padded) and transposes
     __nv_bfloat16 *wb[4] = {}, *wt[4] = {};
     // activations (capacity cap_m)
-    __nv_bfloat16 *x0 = nullptr, *x0t = nullptr, *h[3] = {}, *ht[3] = {}, *dz[3] = {}, *dzt[3] = {};
+    __nv_bfloat16 *x0 = nullptr, *x0t = nullptr, *h[3] = {}, *ht[3] = {}, *dz[3] = {}, *dzt[3] = {},
+                  *dy = nullptr;
     float *z[3] = {}, *feats = nullptr, *tgt = nullptr;
     float *loss = nullptr;       // the step's, the epoch's sum; then d_err, an int
     float2 *part = nullptr;      // the output layer's sums per CTA
@@ -369,8 +370,8 @@ void predict(wk_mlp *m, const float *feats, const int32_t *pids, int64_t n, floa
     m->kernels++;
 }
 
-// The weight gradients dW_l = dZ_l^T . X_l (the layer's input), K the batch, the
-// embedding's from dX = dZ_0 . W_0, and the loss, in one launch: nothing waits for
+// The weight gradients dW_l = dZ_l^T . X_l (the layer's input), K the batch (of the
+// output layer one row, dY^T . H_2), the embedding's from dX = dZ_0 . W_0, and the loss, in one launch: nothing waits for
 // any of them, and each alone is 1 to 16 CTAs.
 void gradient_group(wk_mlp *m, int M, int Mp, cudaStream_t s) {
     if (refused(m)) return;
@@ -390,20 +391,30 @@ void gradient_group(wk_mlp *m, int M, int Mp, cudaStream_t s) {
         g.K[i] = Mp;
         at += g.mt[i] * ((kin + 31) / 32);
     }
-    // columns 48..79 of dX: a tile of 32 from row 48 of W_0^T
-    ok = ok && tc::make_map(&g.a[3], m->dz[0], (uint64_t)Mp, kH, kH, tc::kTM) &&
-         tc::make_map(&g.b[3], m->wt[0], kXPadN, kH, kH, 32);
+    ok = ok && tc::make_map(&g.a[3], m->dy, 1, (uint64_t)Mp, (uint64_t)Mp, tc::kTM) &&
+         tc::make_map(&g.b[3], m->ht[2], kH, (uint64_t)Mp, (uint64_t)Mp, 32);
     g.first[3] = at;
-    g.mt[3] = (Mp + tc::kTM - 1) / tc::kTM;
-    g.n0[3] = kIn;
-    g.C[3] = nullptr;
-    g.ldc[3] = 0;
-    g.n_real[3] = 0;
-    g.M[3] = Mp;
-    g.K[3] = kH;
-    at += g.mt[3];
+    g.mt[3] = 1;
+    g.n0[3] = 0;
+    g.C[3] = m->grads + m->off_w[3];
+    g.ldc[3] = g.n_real[3] = kH;
+    g.M[3] = 1;
+    g.K[3] = Mp;
+    at += kH / 32;
+    // columns 48..79 of dX: a tile of 32 from row 48 of W_0^T
+    ok = ok && tc::make_map(&g.a[4], m->dz[0], (uint64_t)Mp, kH, kH, tc::kTM) &&
+         tc::make_map(&g.b[4], m->wt[0], kXPadN, kH, kH, 32);
     g.first[4] = at;
-    g.n = 4;
+    g.mt[4] = (Mp + tc::kTM - 1) / tc::kTM;
+    g.n0[4] = kIn;
+    g.C[4] = nullptr;
+    g.ldc[4] = 0;
+    g.n_real[4] = 0;
+    g.M[4] = Mp;
+    g.K[4] = kH;
+    at += g.mt[4];
+    g.first[5] = at;
+    g.n = 5;
     g.demb = m->grads + m->off_emb;
     g.pids = m->pids;
     g.n_ids = m->n_ids;
@@ -426,9 +437,9 @@ void gradient_group(wk_mlp *m, int M, int Mp, cudaStream_t s) {
 void gradient_step(wk_mlp *m, const float *feats, const int32_t *pids, const float *tgt, int M, cudaStream_t s) {
     const int Mp = pad64(M);
     float *g = m->grads;
-    // w4's gradient, the biases' and the embedding's are added into; they lie together
+    // the biases' gradients and the embedding's are added into; they lie together
     launch_ahead(build_input_kernel, dim3((unsigned)(Mp / 32)), 256, 0, s, feats, pids, tgt, m->pids, m->tgt, M, Mp, (const float *)(m->params + m->off_emb), m->n_ids, m->x0, m->x0t,
-                 g + m->off_w[3], m->n_params - m->off_w[3]);
+                 g + m->off_b[0], m->n_params - m->off_b[0]);
     m->kernels++;
     const __nv_bfloat16 *in = m->x0;
     int kin = kX;
@@ -439,14 +450,13 @@ void gradient_step(wk_mlp *m, const float *feats, const int32_t *pids, const flo
         in = m->h[l];
         kin = kH;
     }
-    // the output layer, the loss, dZ_2 and the gradients of w4, b4, b3
+    // the output layer, the loss, dY, dZ_2 and the gradients of b4, b3
     if (!refused(m)) {
         tc::EpiArgs ea = act_args(M, Mp, m->dz[2], m->dzt[2], m->z[2], g + m->off_b[2]);
-        ea.hin = m->h[2];
         ea.w = m->wb[3];
         ea.b = m->params + m->off_b[3];
         ea.tgt = m->tgt;
-        ea.dw = g + m->off_w[3];
+        ea.dy = m->dy;
         ea.part = m->part;
         CUtensorMap ta, tb;
         if (tc::make_map(&ta, m->h[2], (uint64_t)Mp, kH, kH, tc::kTM) && tc::make_map(&tb, m->wb[3], kOutPad, kH, kH, 32)) {
@@ -482,7 +492,7 @@ void free_mlp(wk_mlp *m) {
     for (int l = 0; l < 3; ++l) {
         cudaFree(m->h[l]); cudaFree(m->ht[l]); cudaFree(m->z[l]); cudaFree(m->dz[l]); cudaFree(m->dzt[l]);
     }
-    cudaFree(m->x0); cudaFree(m->x0t);
+    cudaFree(m->x0); cudaFree(m->x0t); cudaFree(m->dy);
     cudaFree(m->feats); cudaFree(m->tgt); cudaFree(m->loss); cudaFree(m->part); cudaFree(m->pids);
     cudaFree(m->bidx);
     cudaFree(m->cbias);
@@ -528,6 +538,7 @@ extern "C" int wk_mlp_create(wk_ctx *ctx, int32_t n_ids, int32_t max_batch, uint
              cudaMalloc(&m->z[l], 4 * Mp * kH) == cudaSuccess && cudaMalloc(&m->dz[l], 2 * Mp * kH) == cudaSuccess &&
              cudaMalloc(&m->dzt[l], 2 * Mp * kH) == cudaSuccess;
     ok = ok && cudaMalloc(&m->x0, 2 * Mp * kX) == cudaSuccess && cudaMalloc(&m->x0t, 2 * Mp * kX) == cudaSuccess &&
+         cudaMalloc(&m->dy, 2 * Mp) == cudaSuccess &&
          cudaMalloc(&m->part, sizeof(float2) * Mp / 16) == cudaSuccess &&
          cudaMalloc(&m->feats, 4 * Mp * kIn) == cudaSuccess && cudaMalloc(&m->tgt, 4 * Mp) == cudaSuccess &&
          cudaMalloc(&m->loss, 16) == cudaSuccess && cudaMalloc(&m->pids, 4 * Mp) == cudaSuccess &&

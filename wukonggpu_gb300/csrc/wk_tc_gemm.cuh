@@ -80,12 +80,11 @@ struct EpiArgs {
     float *demb = nullptr;
     const int32_t *pids = nullptr;
     int n_ids = 0;
-    // kEpiHead: the last hidden layer's output (ld ldh), the output layer's
-    // weights and bias, the targets; the weights' gradient; each CTA's sums of
-    // (y - t)^2 and dY
-    const __nv_bfloat16 *hin = nullptr, *w = nullptr;
+    // kEpiHead: the output layer's weights and bias, the targets; dY in bf16; each
+    // CTA's sums of (y - t)^2 and dY
+    const __nv_bfloat16 *w = nullptr;
     const float *b = nullptr, *tgt = nullptr;
-    float *dw = nullptr;
+    __nv_bfloat16 *dy = nullptr;
     float2 *part = nullptr;
 };
 
@@ -144,31 +143,27 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
 
 // The step's output layer, loss and first backward layer for the CTA's 16 rows,
 // a warp four of them: y = acc + b, loss mean((y - t)^2), dY = 2 (y - t) / M in
-// bf16 (rows >= m_real: zero), dw += dY^T H, and of the hidden
-// layer below dZ = dY w GELU'(Z) in bf16, row-major and transposed, with its
-// column sums.  The layer has one output, so these are row-wise: as products
-// padded to tiles of 64 with kernels of their own for bias, loss and sums they
-// were seven launches and 30 us of a step of 1024 rows; this takes 9.  y: the CTA's 16 accumulators.
-// sm: 18 KB, free.
+// bf16 (rows >= m_real: zero), and of the hidden layer below dZ = dY w GELU'(Z) in
+// bf16, row-major and transposed, with its column sums.  The layer has one output,
+// so these are row-wise: as products padded to tiles of 64 with kernels of their
+// own for bias, loss and sums they were seven launches and 30 us of a step of 1024
+// rows; this takes 9 at most.  (The weights' gradient dY^T H is a product of
+// gemm_group_kernel: added up here by atomics it took whichever order the CTAs
+// came in.)  y: the CTA's 16 accumulators.  sm: 14 KB, free.
 __device__ __forceinline__ void head_rows(const EpiArgs &ea, const float *y, int row0, unsigned char *sm) {
     constexpr int kCols = 256, kPitch = 18;   // an odd number of words: the 32 lanes' columns fall in 32 banks
     __nv_bfloat16 *st = reinterpret_cast<__nv_bfloat16 *>(sm);                    // dZ^T: [256][16]
     float *s_cs = reinterpret_cast<float *>(sm + kCols * kPitch * 2);             // per warp: column sums of dZ
-    float *s_dw = s_cs + kThreads / 32 * kCols;                                   // and of dY H
     __shared__ float2 s_sum[kThreads / 32];
     const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
     // every row's words in flight at once
     constexpr int kRows = 16 / (kThreads / 32);
-    float w[8], z[kRows][8], cs[8] = {}, dw[8] = {}, tg[kRows];
-    __nv_bfloat16 h[kRows][8];
+    float w[8], z[kRows][8], cs[8] = {}, tg[kRows];
 #pragma unroll
     for (int i = 0; i < kRows; ++i) {
         const int row = row0 + warp * kRows + i;
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            z[i][j] = ea.z[(size_t)row * ea.ldz + lane + 32 * j];
-            h[i][j] = ea.hin[(size_t)row * ea.ldh + lane + 32 * j];
-        }
+        for (int j = 0; j < 8; ++j) z[i][j] = ea.z[(size_t)row * ea.ldz + lane + 32 * j];
         tg[i] = row < ea.m_real ? ea.tgt[row] : 0.f;
     }
 #pragma unroll
@@ -185,6 +180,7 @@ __device__ __forceinline__ void head_rows(const EpiArgs &ea, const float *y, int
             dy = __bfloat162float(__float2bfloat16(2.f * d / (float)ea.m_real));
             sdy += dy;
         }
+        if (lane == 0) ea.dy[row] = __float2bfloat16(dy);   // its own bf16 value
         __nv_bfloat16 *out = ea.h + (size_t)row * ea.ldh + lane;
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
@@ -192,14 +188,10 @@ __device__ __forceinline__ void head_rows(const EpiArgs &ea, const float *y, int
             out[32 * j] = v;
             st[(lane + 32 * j) * kPitch + r] = v;
             cs[j] += __bfloat162float(v);
-            dw[j] += dy * __bfloat162float(h[i][j]);
         }
     }
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-        s_cs[warp * kCols + lane + 32 * j] = cs[j];
-        s_dw[warp * kCols + lane + 32 * j] = dw[j];
-    }
+    for (int j = 0; j < 8; ++j) s_cs[warp * kCols + lane + 32 * j] = cs[j];
     if (lane == 0) s_sum[warp] = make_float2(sq, sdy);
     __syncthreads();
     for (int c = t; c < kCols; c += kThreads) {
@@ -207,10 +199,9 @@ __device__ __forceinline__ void head_rows(const EpiArgs &ea, const float *y, int
         uint4 *dst = reinterpret_cast<uint4 *>(ea.ht + (size_t)c * ea.ldt + row0);
         dst[0] = make_uint4(src[0], src[1], src[2], src[3]);
         dst[1] = make_uint4(src[4], src[5], src[6], src[7]);
-        float a = s_cs[c], d = s_dw[c];
-        for (int i = 1; i < kThreads / 32; ++i) { a += s_cs[i * kCols + c]; d += s_dw[i * kCols + c]; }
+        float a = s_cs[c];
+        for (int i = 1; i < kThreads / 32; ++i) a += s_cs[i * kCols + c];
         if (a != 0.f) atomicAdd(ea.colsum + c, a);
-        if (d != 0.f) atomicAdd(ea.dw + c, d);
     }
     if (t == 0) {   // added up over the CTAs by sum_rows, in a later kernel: nothing waits for it
         float2 v = s_sum[0];
@@ -465,7 +456,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
 }
 
 // Up to kGroup products of one launch, tiles of 128 x 32 numbered product by product
-constexpr int kGroup = 4;
+constexpr int kGroup = 5;
 struct GroupArgs {
     CUtensorMap a[kGroup], b[kGroup];
     int first[kGroup + 1];        // first tile of each product; the number of tiles
