@@ -81,6 +81,7 @@ def parse():
     ap.add_argument("--serving-mix", default="",
                     help="mix file of the serving section (reference mix_config format); default: the packaged "
                          "wukonggpu_gb300/mixes/serving/mix_config")
+    ap.add_argument("--detail", default="", help="also write the line with every section in full to this file")
     ap.add_argument("--clocks-csv", default="",
                     help="where nvidia-smi clock samples are written (default: a temporary file)")
     return ap.parse_args()
@@ -189,6 +190,35 @@ def peaks():
         d = json.loads(p.read_text())
         return float(d["hbm_gbs"]), "measured"
     return 6800.0, "fallback"
+
+
+SWEEP = ("qps", "p50_ms", "p99_ms", "light_p99_ms", "heavy_p99_ms", "failed")
+
+
+def brief(line):
+    """The line as it is printed, short enough for a reader that keeps the end of the
+    output: the sections' numbers to six digits, the serving sweep's rows as lists
+    (SWEEP by arm) and without the latency CDFs (--detail has all of it)."""
+    def digits(x):
+        if isinstance(x, float):
+            return float(f"{x:.6g}") if np.isfinite(x) else x
+        if isinstance(x, dict):
+            return {k: digits(v) for k, v in x.items() if not (k.endswith("cdf_ms") or k == "cdf_rates")}
+        return [digits(v) for v in x] if isinstance(x, (list, tuple)) else x
+
+    out = {k: digits(v) if k in ("paged", "partition", "batched", "estimator", "serving", "parity", "setup") else v
+           for k, v in line.items()}
+    if "serving" in out:
+        def row(t):
+            return [t[k] for k in SWEEP] if t else None
+        out["serving"] = {**out["serving"], "sweep_columns": list(SWEEP),
+                          "sweep": [[r["rate_qps"], row(r["query_at_a_time_stats"]), row(r["batched_learned"])]
+                                    for r in out["serving"]["sweep"]]}
+        for arm in ("baseline_per_type", "batched_per_type"):
+            t = out["serving"]["headline"].get(arm)
+            if t:
+                out["serving"]["headline"][arm] = {k: [v["completed"], v["p50_ms"], v["p99_ms"]] for k, v in t.items()}
+    return out
 
 
 def profile_traffic_ratio():
@@ -692,7 +722,9 @@ def run_gb300(args, dist):
             "clocks": clocks,
             **sections,
         }
-        print(json.dumps(line), flush=True)
+        if args.detail:
+            Path(args.detail).write_text(json.dumps(line))
+        print(json.dumps(brief(line)), flush=True)
     rc.close()
 
 
