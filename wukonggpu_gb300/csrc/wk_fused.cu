@@ -602,7 +602,12 @@ int launch_fused(const FusedOp &op, cudaStream_t st) {
         return (int)cudaErrorInvalidValue;   // not reached: fused_takes
     }
 #undef WK_FUSED
-    // a filter that is not written block by block has blocks enough for pairs
+    // A filter that is not written block by block has blocks enough for pairs.  Of
+    // more than 8 columns every size is written by CTAs: a warp on its own divides by a
+    // width it does not know and takes 155 / 168 us to write 2.6M / 4M rows of 12
+    // columns, nine in ten kept, where the CTAs take 93 / 128 (9 columns: 125 / 136
+    // and 80 / 109; 8 columns: 84 / 100 and 69 / 94, but 53 and 60 where one in
+    // fourteen of the 4M is kept)
     const bool pb = filter_per_block(a.nblk, op.sms);
 #define WK_FUSED(CC) \
     return pb ? run_fused<CC, true, 1, true>(a, op.pv, kFusedAll, st) : run_fused<CC, true, 2, false>(a, op.pv, kFusedAll, st)
@@ -615,7 +620,7 @@ int launch_fused(const FusedOp &op, cudaStream_t st) {
         case 6: WK_FUSED(6);
         case 7: WK_FUSED(7);
         case 8: WK_FUSED(8);
-        default: WK_FUSED(0);
+        default: return run_fused<0, true, 1, true>(a, op.pv, kFusedAll, st);
     }
 #undef WK_FUSED
 }

@@ -112,8 +112,10 @@ void launch_filter_write(const int32_t *hist, int64_t R, int C, const uint32_t *
 // dependent steps, 35 us of them on 11 columns however few blocks there are:
 // 12k rows of 11 columns take 65.9 us with a warp per block and 30.9 with a CTA,
 // 422k rows of 8 51.9 and 36.0.  From about 16 blocks an SM on there are warps
-// enough, and the CTAs' prefixes and barriers cost more (10M rows of 3 columns
-// 99 and 120 us).
+// enough, and the CTAs' prefixes and barriers cost more.  Around the line, over a
+// functional direction, 0.4 kept: 2.0M rows of 3 columns 35.2 and 35.6, 2.4M 35.9 and
+// 39.1, 3M 41.7 and 44.1; of 8 columns 2.0M 51.2 and 43.0, 3M 64.2 and 61.0, 4M 76.1
+// and 74.2.
 inline bool filter_per_block(int64_t nblk, int sms) { return nblk <= 16 * (int64_t)(sms < 1 ? 1 : sms); }
 
 // k2u, k2k and k2c over a dense functional direction (pv.nb[dir] set) in one
