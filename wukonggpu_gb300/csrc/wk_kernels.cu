@@ -796,9 +796,11 @@ k2u_expand_func_kernel(const int32_t *__restrict__ hist, int64_t R, const int32_
 // touches (position + 1 on a match, the whole list otherwise), group_sums[2 g]
 // += rows kept.
 //
-// The searches are chains of dependent reads, so a lane's rounds are searched
-// side by side, as their offsets are looked up: one after another, 422k rows of
-// 8 columns in runs of 40 took 51.1 us a step, 48.6 so, and 2.8k rows 43 and 37.6.
+// The searches are chains of dependent reads, so a lane's rounds are searched two
+// at a time.  One after another they take longer (422k rows of 8 columns in runs of
+// 40, half kept, 51.7 us a step, 35.3 so; 2.8k rows 46.8 and 31.8), four at a time a
+// short search pays for the longest of four (9M rows of 3 columns, half kept, 275
+// us, 257 so and 266 one after another; nearly all kept 460, 441 and 427).
 template <bool DENSE>
 __global__ void __launch_bounds__(kThreads, 6)
 filter_probe_kernel(const int32_t *__restrict__ hist, int64_t R, int C, int scol, int ecol,
@@ -853,28 +855,28 @@ filter_probe_kernel(const int32_t *__restrict__ hist, int64_t R, int C, int scol
             if (__any_sync(FULL, here)) probe_warp(pv, here ? v[rd] : -1, dir, o[rd], d[rd], err);
         }
     }
-    // lo[rd]: the first entry not below tg[rd]
+    // lo[rd]: the first entry not below tg[rd], two rounds' searches at a time
+    static_assert(kRounds % 2 == 0, "rounds come in pairs");
     uint32_t lo[kRounds], hi[kRounds];
-    bool more = false;
 #pragma unroll
     for (int rd = 0; rd < kRounds; ++rd) {
         lo[rd] = 0u;
         hi[rd] = d[rd];
-        more |= d[rd] != 0u;
     }
-    while (more) {
-        int32_t e[kRounds];
 #pragma unroll
-        for (int rd = 0; rd < kRounds; ++rd)
-            e[rd] = lo[rd] < hi[rd] ? __ldg(pv.edges + o[rd] + ((lo[rd] + hi[rd]) >> 1)) : 0;
-        more = false;
+    for (int q = 0; q < kRounds; q += 2) {
+        while (lo[q] < hi[q] || lo[q + 1] < hi[q + 1]) {
+            int32_t x[2];
 #pragma unroll
-        for (int rd = 0; rd < kRounds; ++rd) {
-            if (lo[rd] < hi[rd]) {
-                const uint32_t mid = (lo[rd] + hi[rd]) >> 1;
-                if (e[rd] < tg[rd]) lo[rd] = mid + 1;
-                else hi[rd] = mid;
-                more |= lo[rd] < hi[rd];
+            for (int k = q; k < q + 2; ++k)
+                x[k - q] = lo[k] < hi[k] ? __ldg(pv.edges + o[k] + ((lo[k] + hi[k]) >> 1)) : 0;
+#pragma unroll
+            for (int k = q; k < q + 2; ++k) {
+                if (lo[k] < hi[k]) {
+                    const uint32_t mid = (lo[k] + hi[k]) >> 1;
+                    if (x[k - q] < tg[k]) lo[k] = mid + 1;
+                    else hi[k] = mid;
+                }
             }
         }
     }
