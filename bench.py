@@ -420,13 +420,14 @@ def run_one_query(args):
     """Query `args.one_query` of the mix, once, op by op with per-kernel timing.
     Kernel launches: the start op's copy, then three per k2u op (count,
     publish, expand) and three per filter op (probe, write, publish), or one
-    for either over a dense functional direction, in pattern order."""
+    for either over a dense functional direction, in pattern order (the tables
+    have room for every step's rows, so that none grows one)."""
     import wukonggpu_gb300 as W
     from wukonggpu_gb300 import build as wb
     from wukonggpu_gb300 import workloads
     wb.build()
     g = W.Graph(W.spec_single_query(scale=args.scale))
-    rc = W.RCache(device=0)
+    rc = W.RCache(device=0, history_capacity=int(args.scale * (1 << 29)))
     rc.build_store_graph(g)
     group = workloads.scale_queries() if args.one_query_group == "mix" else workloads.scale_filter_queries()
     name, q = group[args.one_query]

@@ -22,8 +22,8 @@
 // through it in 130 us on 12M rows of 4 columns, a third of it look-ups).
 //
 // Two kernels and a host round trip before, this launch after, us a call:
-// k2u on 12M rows of 4 columns 163 -> 138 (132 since), k2k on 10M rows of 3 105.7 -> 99,
-// k2c on 3M rows of 6 49 -> 47; k2u on 50k rows of 6 about 49 -> 22.  A
+// k2u on 12M rows of 4 columns 163 -> 131, k2k on 10M rows of 3 105 -> 95, k2c on 3M
+// rows of 6 50 -> 48; k2u on 50k rows of 6 about 49 -> 22.  A
 // single pass with a decoupled look-back was slower (177 / 139 / 65): every tile
 // waited for the slowest load among the 300 tiles in flight before it.
 //
@@ -302,8 +302,8 @@ __device__ __forceinline__ unsigned int blocks_before(const Fused &a, int64_t b)
 
 // Write block b of a k2u op: its matched rows with the neighbour appended,
 // packed in shared memory at the output's 16 B phase; its whole vectors leave
-// by the copy engine, which spares the load-store unit the look-ups need (12M
-// rows of 4 columns 138 -> 132 us a step).
+// by the copy engine, which spares the load-store unit the look-ups need (some 3
+// of 138 us a step on 12M rows of 4 columns).
 // A block most of whose rows are kept loads them before the wait for the groups
 // (they are in L2); of another only the kept rows are read, behind it.  Whether
 // most are kept is told by the block's count, which is there already for nearly
@@ -583,7 +583,8 @@ int launch_fused(const FusedOp &op, cudaStream_t st) {
     // 16 an octet) and a group's 256 blocks, no more: the rows should still be in
     // L2 when they are read again.  222 octets instead of 146 made a k2u op on
     // 12M rows of 4 columns read 392 instead of 278 MB from DRAM (192 MB is the
-    // table) and took it from 144 to 153 us.
+    // table) and took it from 144 to 153 us; 184 octets (an SM's share of 1 instead
+    // of 3/4) take 120.4 where these take 118.7.
     const int lag = op.sms * 3 / 4 + (1 << kGroupShift) / kOct;
     a.lag = a.steps < lag ? a.steps : lag;
     // two blocks per count CTA (eight look-ups in flight a lane) once there are

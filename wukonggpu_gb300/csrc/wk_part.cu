@@ -31,7 +31,7 @@
 // copying its own row to its place, a warp's store touched a sector per row;
 // owners were found by a division, lanes of one owner by match_any, and the
 // bounds came back through pageable memory.  6M rows of 3 columns over 8 owners
-// took 147 us so, 82 now; the moves are left bound by their issue slots.
+// took 148 us so, 85 now; the moves are left bound by their issue slots.
 #include "wk_runtime.h"
 #include "wk_loads.cuh"
 

@@ -147,7 +147,7 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
 // bf16, row-major and transposed, with its column sums.  The layer has one output,
 // so these are row-wise: as products padded to tiles of 64 with kernels of their
 // own for bias, loss and sums they were seven launches and 30 us of a step of 1024
-// rows; this takes 9 at most.  (The weights' gradient dY^T H is a product of
+// rows; this takes 9, with cold caches 11.5.  (The weights' gradient dY^T H is a product of
 // gemm_group_kernel: added up here by atomics it took whichever order the CTAs
 // came in.)  y: the CTA's 16 accumulators.  sm: 14 KB, free.
 __device__ __forceinline__ void head_rows(const EpiArgs &ea, const float *y, int row0, unsigned char *sm) {
