@@ -304,14 +304,16 @@ __device__ __forceinline__ unsigned int blocks_before(const Fused &a, int64_t b)
 // packed in shared memory at the output's 16 B phase; its whole vectors leave
 // by the copy engine, which spares the load-store unit the look-ups need (some 3
 // of 138 us a step on 12M rows of 4 columns).
-// A block most of whose rows are kept loads them before the wait for the groups
-// (they are in L2); of another only the kept rows are read, behind it.  Whether
-// most are kept is told by the block's count, which is there already for nearly
-// every block; read too early it is some earlier op's, and costs time only.  With
-// every block's rows loaded ahead and the ballots held in registers, which spilled,
-// 12M rows of 4 columns took 126 / 98 / 82 / 72 us a step with all / half / one in
-// eight / none of the rows kept, 118 / 91 / 80 / 66 so; as two kernels, whose
-// second is not launched for none, 169 / 131 / 102 / 48.
+// The rows are loaded before the wait for the groups (they are in L2), unless the
+// block's count says that few of them are kept: then only those are read, behind it.
+// The count is there already for nearly every block where the writing trails the
+// counting; read too early it is some earlier op's, and costs time only.  12M rows of
+// 4 columns take 119 / 92 / 80 / 67 us a step with all / half / one in eight / none of the rows
+// kept; with every block's rows loaded ahead 125 / 97 / 81 / 67; as two kernels,
+// whose second is not launched for none, 169 / 131 / 102 / 48.  Rows of one or two
+// columns, and tables short enough to be counted before the first block is written,
+// are loaded ahead always (4M rows of one column 41.1 us, 44 by the count; 600k 18
+// and 23).  The ballots are taken twice: held in registers they made the kernel spill.
 // Nothing is written when the wait ran out.
 template <int C>
 __device__ __forceinline__ void write_k2u(const Fused &a, int64_t b, WaitShared &s_wait, int32_t *buf,
@@ -323,7 +325,7 @@ __device__ __forceinline__ void write_k2u(const Fused &a, int64_t b, WaitShared 
     const bool aligned = ((uintptr_t)a.hist & 15u) == 0;
     int32_t x[kPasses], v[kPasses][W];
     unsigned kept = 0u;
-    const bool most = ld_l2(a.blk_nz + b) >= (unsigned)kRowsPerBlock / 4;
+    const bool most = C <= 2 || a.lag >= a.steps || ld_l2(a.blk_nz + b) >= (unsigned)kRowsPerBlock / 4;
     if (most) {
 #pragma unroll
         for (int q = 0; q < kPasses; ++q) {
@@ -495,6 +497,9 @@ fused_kernel(const __grid_constant__ Fused a, const __grid_constant__ PredView p
             }
             ok = __syncthreads_and(all) != 0;
         }
+        // the groups were read before the error word will be (groups_before): a fence of a
+        // thread whose warp has no sums to load, beside the others' loads
+        if (threadIdx.x == kThreads - 1) __threadfence();
         unsigned long long x = 0ull;
         for (int64_t i = threadIdx.x; ok && i < ng; i += kThreads) x += ld_l2(a.gs + 2 * i + 1);
         x = warp_add(x);
@@ -504,7 +509,6 @@ fused_kernel(const __grid_constant__ Fused a, const __grid_constant__ PredView p
             x = 0ull;
 #pragma unroll
             for (int w = 0; w < kThreads / 32; ++w) x += s_part[w];
-            __threadfence();   // the groups were read before the error word (groups_before)
             a.pub[2] = (unsigned long long)(unsigned int)atomicOr(a.err, 0) | (ok ? 0ull : (unsigned long long)kErrWait);
             a.pub[3] = P;
             a.pub[4] = x;

@@ -244,11 +244,12 @@ bool alloc_failure_pending(wk_ctx *ctx) { return ctx->inject_alloc_fail.load(std
 // output buffer has room; when the buffer turns out too small it is grown to the
 // rows there are and the rows are written by a second launch.  An op whose row
 // limit is below its input's rows is counted, held to the limit and only then
-// written; so is one whose buffer has room for less than half of the rows that the
-// direction's share of ids with a neighbour lets expect, as it will have to be
-// grown (the first step of a new context on 12M rows that all match, from room for
-// 3.4M: 494 us when it writes first, 442 so; a step one in fifty of whose rows
-// match, all of which the share lets expect: 98 us each time instead of 76).
+// written; so is one whose buffer has room for less than half of the rows to expect,
+// as it will have to be grown: those of the direction's share of ids with a
+// neighbour, or of the context's last such step if that kept fewer.  The first step of
+// a new context on 12M rows that all match, from room for 3.4M, takes 494 us when it
+// writes first, 442 so; a step one in ten of whose 8M rows match, with room for 3.4M,
+// 77 us when it is counted first, 59 so.
 // *done is false when the op has to run as the general kernels instead: more
 // columns than the launch takes, a start that is an index key (k2u), or a device
 // wait that ran out.
@@ -270,7 +271,7 @@ int op_fused(wk_ctx *ctx, wk_history *h, int scol, int ecol, int32_t end_const, 
     const int64_t room = (int64_t)(ob.cap / ((size_t)width * 4));
     const PredSeg &sg = ctx->store->hs->segs[pid];
     const double share = (double)(dir == WK_DIR_OUT ? sg.subjects : sg.objects) / (double)std::max(sg.dn[dir], 1u);
-    const bool count_first = !filter && (R > ctx->row_limit || (double)room < 0.5 * share * (double)R);
+    const bool count_first = !filter && (R > ctx->row_limit || (double)room < 0.5 * std::min(share, ctx->func_share) * (double)R);
     if ((st = clk.begin())) return st;
     const int par = ctx->gs_par;
     unsigned long long *gs = gsum_buffer(ctx, par);
@@ -314,6 +315,7 @@ int op_fused(wk_ctx *ctx, wk_history *h, int scol, int ecol, int32_t end_const, 
     if (!filter && R_out > ctx->row_limit)   // nothing was written
         return set_error(WK_EOVERFLOW, "k2u: %lld output rows exceed the context's row limit %lld", (long long)R_out,
                          (long long)ctx->row_limit);
+    if (!filter) ctx->func_share = (double)R_out / (double)R;
     if (!ob.ptr && (st = take(ctx, ob, 16))) return st;
     if (!filter && (R_out > room || (count_first && R_out > 0))) {
         if ((st = take(ctx, ob, (size_t)R_out * width * 4))) return st;

@@ -112,6 +112,7 @@ struct wk_ctx {
     std::vector<wk_op_stats> qstats;   // every op of the last wk_execute, while timing
     int64_t launches = 0;
     int64_t row_limit = INT64_MAX;   // wk_set_row_limit
+    double func_share = 1.0;         // of its input's rows, what the last functional k2u step kept
     cudaEvent_t tm0 = nullptr, tm1 = nullptr;   // wk_timer_begin / wk_timer_end
 
     // query-level state (segment cache protection / prefetch): segments that
