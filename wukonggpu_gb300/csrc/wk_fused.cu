@@ -442,12 +442,39 @@ __device__ __forceinline__ void write_filter(const Fused &a, int64_t b0, unsigne
     const uint32_t words = nb * (uint32_t)C;
     const uint32_t lead = (uint32_t)((P * (unsigned long long)C) & 3ull);
     int32_t *gout = a.out + (P * (unsigned long long)C - lead);
-    for (uint32_t u = (uint32_t)(PB ? t : lane); 4u * u < lead + words; u += PB ? kThreads : 32u) {
+    // The kept row and column of the vector's first word.  CT 0: moved on by steps (a
+    // row of -1 before the lead), not found by a division, which took a warp most of its
+    // time: 2.6M / 4M rows of 12 columns, nine in ten kept, 173 / 188 us a step with it,
+    // 118 / 138 so (the block by a CTA 90 / 123, but 67 where nothing of the 4M is kept
+    // and this takes 56)
+    constexpr int kStep = 4 * (PB ? kThreads : 32);
+    int q = 0, c0 = 0, dq = 0, dc = 0;
+    if constexpr (CT == 0) {
+        const int k = 4 * (PB ? t : lane) - (int)lead;
+        q = k < 0 ? -1 : k / C;
+        c0 = k - q * C;
+        dq = kStep / C;
+        dc = kStep % C;
+    }
+    for (uint32_t u = (uint32_t)(PB ? t : lane); 4u * u < lead + words; u += kStep / 4) {
         int32_t v[4];
+        int row = q, col = c0;
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             const uint32_t kk = 4u * u + (uint32_t)j - lead;   // wraps above `words` before the lead
-            v[j] = kk < words ? ld_prior(hb + (int)ws[kk / (uint32_t)C] * C + (int)(kk % (uint32_t)C)) : 0;
+            if constexpr (CT > 0) {
+                row = (int)(kk / (uint32_t)C);
+                col = (int)(kk % (uint32_t)C);
+            }
+            v[j] = kk < words ? ld_prior(hb + (int)ws[row] * C + col) : 0;
+            if constexpr (CT == 0) {
+                if (++col == C) { col = 0; ++row; }
+            }
+        }
+        if constexpr (CT == 0) {
+            q += dq;
+            c0 += dc;
+            if (c0 >= C) { c0 -= C; ++q; }
         }
         if (4u * u >= lead && 4u * u + 4u <= lead + words) {
             reinterpret_cast<int4 *>(gout)[u] = make_int4(v[0], v[1], v[2], v[3]);
@@ -607,12 +634,7 @@ int launch_fused(const FusedOp &op, cudaStream_t st) {
         return (int)cudaErrorInvalidValue;   // not reached: fused_takes
     }
 #undef WK_FUSED
-    // A filter that is not written block by block has blocks enough for pairs.  Of
-    // more than 8 columns every size is written by CTAs: a warp on its own divides by a
-    // width it does not know and takes 155 / 168 us to write 2.6M / 4M rows of 12
-    // columns, nine in ten kept, where the CTAs take 93 / 128 (9 columns: 125 / 136
-    // and 80 / 109; 8 columns: 84 / 100 and 69 / 94, but 53 and 60 where one in
-    // fourteen of the 4M is kept)
+    // a filter that is not written block by block has blocks enough for pairs
     const bool pb = filter_per_block(a.nblk, op.sms);
 #define WK_FUSED(CC) \
     return pb ? run_fused<CC, true, 1, true>(a, op.pv, kFusedAll, st) : run_fused<CC, true, 2, false>(a, op.pv, kFusedAll, st)
@@ -625,7 +647,7 @@ int launch_fused(const FusedOp &op, cudaStream_t st) {
         case 6: WK_FUSED(6);
         case 7: WK_FUSED(7);
         case 8: WK_FUSED(8);
-        default: return run_fused<0, true, 1, true>(a, op.pv, kFusedAll, st);
+        default: WK_FUSED(0);
     }
 #undef WK_FUSED
 }
